@@ -195,7 +195,7 @@ __device__ __forceinline__ float4 adj_vel(float4 xo, float rd, float2 s01, float
 }
 
 template <int R, bool VARDEN, bool ADJ>
-__global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __grid_constant__ Acou3DArgs a) {
+__global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __grid_constant__ Acou3DArgs a, int seg) {
     using K = K3<R>;
     extern __shared__ __align__(128) float smem[];
     const int tid = threadIdx.x;
@@ -263,13 +263,15 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    // iteration s: new Vx on plane s+R-1 (own points), then, for s >= R, new Vy / Vz on plane s
-    // (column + halo) and new P on plane s.  Planes below R and from nx-R on are the frozen rim.
+    // The CTA's planes [xs, s_end).  iteration s: new Vx on plane s+R-1 (own points), then, for
+    // s >= xs, new Vy / Vz on plane s (column + halo) and new P on plane s.  The iterations before
+    // xs only fill the Vx ring (each thread its own slots: no staged box, no barrier) with planes
+    // the CTA before this one stores.  Planes below R and from nx-R on are the frozen rim.
     // The boxes of plane s+2 are requested once every thread is done with those of plane s.
-    const int s_begin = 1, s_end = nx - R;
+    const int xs = R + (int)blockIdx.z * seg, s_begin = max(1, xs - 2 * R + 1), s_end = min(xs + seg, nx - R);
     if (tid == 0) {
-        issue(s_begin);
-        if (s_begin + 1 < s_end) issue(s_begin + 1);
+        issue(xs);
+        if (xs + 1 < s_end) issue(xs + 1);
     }
     float4 Pq[K::NQ];
 #pragma unroll
@@ -284,15 +286,18 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
 
     for (int s = s_begin; s < s_end; s++) {
         const int stg = s & 1;
-        const bool got = bounded_wait(bars + stg, (phase >> stg) & 1u);
-        phase ^= 1u << stg;
+        bool got = true;
+        if (s >= xs) {
+            got = bounded_wait(bars + stg, (phase >> stg) & 1u);
+            phase ^= 1u << stg;
+        }
         const float* st = smem + stg * K::STAGE;
         float* nby = smem + K::OFF_NB + stg * K::NBUF;  // new Vy region of this plane
         float* nbz = nby + K::NB_NZ;                     // new Vz region of this plane
         // adjoint: D_k and the imaging sum of the own points of plane s, requested before the
         // velocity phases so that their latency is covered
         float4 adk = make_float4(0.f, 0.f, 0.f, 0.f), agk = adk;
-        if (ADJ && s >= R && own_ok) {
+        if (ADJ && s >= xs && own_ok) {
             const long long pofs = shot_off + (long long)s * L.xstride + own_off;
             adk = __ldg(reinterpret_cast<const float4*>(a.adj_div + pofs));
             agk = *reinterpret_cast<const float4*>(a.adj_g + pofs);
@@ -313,7 +318,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
             return make_float4(k.x * kx, k.y * kx, k.z * kx, k.w * kx);
         };
 
-        if (s >= R) {
+        if (s >= xs) {
             const long long plane_off = shot_off + (long long)s * L.xstride;
             // ---- new Vy on the Vy region: rows y0-R .. y0+TY+R-1, two rows x float4 per task ----
             if (tid < K::NVY2) {
@@ -441,11 +446,11 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
                 vout = vn;
             }
             Vxo = ld_own(vx_in, s + R);
-            if (own_ok) st4s(a.vx_out + shot_off + (long long)xv * L.xstride + own_off, vout);
+            if (own_ok && xv >= xs && xv < s_end) st4s(a.vx_out + shot_off + (long long)xv * L.xstride + own_off, vout);
             sVq[((unsigned)xv % K::NQ) * kThreads] = vn;
         }
         // every thread is done with this stage and with the new-velocity buffer of plane s-1
-        if (__syncthreads_or(!got)) {
+        if (s >= xs && __syncthreads_or(!got)) {
             if (tid == 0) {
                 atomicExch(a.err_flag, 1);
                 // let the copies still in flight land before the CTA's shared memory is released
@@ -454,8 +459,8 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
             }
             return;
         }
-        if (tid == 0 && s + 2 < s_end) issue(s + 2);
-        if (s >= R) {
+        if (tid == 0 && s >= xs && s + 2 < s_end) issue(s + 2);
+        if (s >= xs) {
             // ---- new P on plane s (own points) ----
             float wz[4 * K::NFD];
 #pragma unroll
@@ -603,14 +608,37 @@ __global__ void reduce3d_kernel(const double* __restrict__ acc, int nslab, Layou
     }
 }
 
+// Planes of x that one CTA marches over.  A whole column per CTA leaves SMs idle when a launch has
+// fewer columns than the chip has CTA slots (two per SM), or a last wave that is nearly empty; each
+// further segment repeats 2R - 1 planes of Vx (about 0.4 of a full plane's time each).  The choice
+// minimises the modelled time: whole waves of two CTAs per SM, a plane of two resident CTAs costing
+// 1.22 times that of one alone (measured: 2.2 us alone on 176 x 160 x 140 with 50 CTAs, 2.7 us
+// shared on 352 x 336 x 320 with 220).
+int segment_planes(const Layout3D& L, int active, int R) {
+    const int planes = L.nx - 2 * R, sms = num_sms();
+    const long long cols = (long long)L.nty * L.ntz * active;
+    int best = planes;
+    double bt = 1e300;
+    for (int n = 1; n <= planes && planes / n >= 4; n++) {
+        const int len = (planes + n - 1) / n;
+        const long long ctas = cols * ((planes + len - 1) / len);
+        const long long full = ctas / (2 * sms), rest = ctas % (2 * sms);
+        const double waves = 1.22 * full + (rest == 0 ? 0.0 : rest <= sms ? 1.0 : 1.22);
+        const double t = waves * (len + (n > 1 ? 0.4 * (2 * R - 1) : 0.0));
+        if (t < bt) bt = t, best = len;
+    }
+    return best;
+}
+
 template <int R, bool VARDEN, bool ADJ>
 cudaError_t launch_t(const Acou3DArgs& a, int active, cudaStream_t st) {
     const size_t smem = sizeof(float) * K3<R>::SMEM_FLOATS;
     auto k = acoustic3d_step_kernel<R, VARDEN, ADJ>;
     static bool attr[kMaxDevices] = {};
     if (cudaError_t e = smem_attr_once((const void*)k, (int)smem, attr)) return e;
-    const dim3 grid(a.L.nty * a.L.ntz, active);
-    k<<<grid, kThreads, smem, st>>>(a);
+    const int seg = segment_planes(a.L, active, R), nseg = (a.L.nx - 2 * R + seg - 1) / seg;
+    const dim3 grid(a.L.nty * a.L.ntz, active, nseg);
+    k<<<grid, kThreads, smem, st>>>(a, seg);
     return cudaGetLastError();
 }
 

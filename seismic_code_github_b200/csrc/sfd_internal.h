@@ -27,6 +27,14 @@ inline cudaError_t smem_attr_once(const void* fn, int bytes, bool* done) {
     if (e == cudaSuccess && tracked) done[dev] = true;
     return e;
 }
+// SM count of the current device (148 if the query fails: the answer only sizes grids).
+inline int num_sms() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+        return 148;
+    return n;
+}
 // Both 2-D acoustic step kernels work on the same 64 x 64 tiles, so they share the field
 // layout and the per-tile receiver tables.
 constexpr int kTileX = 64;
