@@ -79,6 +79,7 @@ struct sfd_ctx {
     int* d_err = nullptr;      // bounded-wait timeout flag written by the step kernels
     CUtensorMap tmaps[6];      // TMA descriptors: P0 P1 VX0 VX1 VZ0 VZ1
     CUtensorMap mtmaps[6];     // the same buffers with the x-marching kernel's boxes
+    CUtensorMap itmaps[5];     // isotropic elastic sums vx vz strxx strzz strxz (elastic2d.cu box)
     CUtensorMap qtmaps[2];     // default viscoacoustic step: sigma S0 S1 (viscoac2d_fast.cu box)
 
     // 3-D scheme: dense [x][y][pitch] slabs, 8 fields (P, Vx, Vy, Vz, two buffers each)
@@ -524,11 +525,13 @@ EArgs make_eargs(const sfd_ctx* c, int step) {
     return a;
 }
 
-// Arguments of the isotropic elastic step (ten in-place split fields per shot).
+// Arguments of the isotropic elastic step (ten in-place split fields and five sums per shot).
 IArgs make_iargs(const sfd_ctx* c, int step) {
     IArgs a{};
     const long long fs = (long long)c->nshot * c->L.shot_stride;
     for (int i = 0; i < I_NFIELDS; i++) a.f[i] = c->d_state + i * fs;
+    for (int k = 0; k < 5; k++) a.tm[k] = c->itmaps[k];
+    a.err_flag = c->d_err;
     a.L = c->L;
     a.nz = c->g.nz;
     a.npx = a.npz = c->g.pml;
@@ -543,6 +546,7 @@ IArgs make_iargs(const sfd_ctx* c, int step) {
     const float af[5] = {19845.0f / 16384.0f, -735.0f / 8192.0f, 567.0f / 40960.0f, -405.0f / 229376.0f,
                          35.0f / 294912.0f};  // YMOD:23-27
     std::memcpy(a.a, af, sizeof(af));
+    a.one = 1.0f;
     // YMOD:7-20: the lower orders caluz uses next to the free surface
     const float cr[4][4] = {{1.0f, 0.0f, 0.0f, 0.0f},
                             {9.0f / 8.0f, -1.0f / 24.0f, 0.0f, 0.0f},
@@ -2387,6 +2391,12 @@ int sfd_set_shots(sfd_ctx* ctx, int nshot, const sfd_shot* shots) {
         viscoac2d_sponge_tables(ctx->g.pml, ctx->g.pml, ctx->g.dx, ctx->g.dz, ctx->spg_stride, tab.data());
         dfree(ctx->d_spg);
         if ((rc = up(&ctx->d_spg, tab))) return rc;
+        for (int f = 0; iso && f < 5; f++) {
+            int box[2];
+            elastic2d_box(box);
+            float* base = ctx->d_state + (I_VX + f) * (long long)nshot * L.shot_stride;
+            if ((rc = encode_field_map(ctx, &ctx->itmaps[f], base, L, nshot, box))) return rc;
+        }
         if (q_fast(ctx)) {
             int bs[2];
             viscoac2d_fast_boxes(bs);

@@ -2,12 +2,14 @@
 // forward/yang_version_2016_2_2 for a flat surface -- 'abc' (YPRI:234-386, cosine sponge on all
 // four sides) and 'fsbc' (YPRI:57-230, free surface at row zs, no top sponge).  Every field is kept in the reference's split form (x and z parts), ten per cell:
 //   vxx vxz vzx vzz | strxxx strxxz | strzzx strzzz | strxzx strxzz
-// and one step is two kernels (YPUB = Iso_multishot_fd_subroutine_fsbc_zy_m2_pub.f90):
-//   velocity: strxx, strxz, strzz = sums of their parts (YPUB:1410-1426) on the tile plus halo;
+// with the five sums vx, vz, strxx, strzz, strxz (YPUB:1410-1426) beside them, written by the
+// kernel that completes them, and one step is two kernels
+// (YPUB = Iso_multishot_fd_subroutine_fsbc_zy_m2_pub.f90):
+//   velocity: strxx, strxz, strzz staged on the tile plus halo;
 //             vxx += (dt/dx) busg2e Dx0 strxx, vxz += (dt/dz) busg2e Dz0 strxz,
 //             vzx += (dt/dx) busg1e Dx1 strxz, vzz += (dt/dz) busg1e Dz1 strzz
 //             (caluxabs / caluzabs, YPUB:1095-1157, 1347-1407), each part times its sponge
-//   stress:   vx = vxx + vxz, vz = vzx + vzz on the tile plus halo;
+//   stress:   vx, vz staged on the tile plus halo;
 //             strxxx += (dt/dx) lambmusg Dx1 vx, strxxz += (dt/dz) lambsg Dz0 vz,
 //             strzzx += (dt/dx) lambsg Dx1 vx,   strzzz += (dt/dz) lambmusg Dz0 vz,
 //             strxzx += (dt/dx) musge Dx0 vz,    strxzz += (dt/dz) musge Dz1 vx,
@@ -30,6 +32,17 @@
 // update reads it one step later; running the surface kernel after the stress kernel gives the
 // same order.
 //
+// Bound: memory.  A step must read and write ten split fields and read five model arrays (100 B a
+// cell); the two kernels move 140 B (the sums are written once and read once, the halos hit L2).
+// The sums are slabs of their own so that one TMA box per field stages a tile with its halo (no
+// registers, no address arithmetic in the threads) while the threads' own split parts are loaded,
+// and so that the halos re-read one array per field instead of two.  Tiles are 64 rows of z by 8
+// columns, one vector of four cells per thread, five CTAs of 128 threads per SM: the 2.25-fold halo
+// hits L2, and many small CTAs cover one another's loads and the slow vectors at the surface.
+// Free-surface step of 8 shots of 1280 x 483 (4.95 M cells): 277 us before, 122 us now (40.6 Gpts/s,
+// DRAM at 4.2 TB/s).  Tiles of 16 and 32 columns 133 and 160 us; 64 columns and four vectors per
+// thread, which loads and waits four times in turn, 250 us.
+//
 // Model preparation (host, per shot window): substagger (YPUB:323-547); then, in abc mode, on the
 // device the PML smoothing of modipapml (YPUB:549-634), which overwrites each top-sponge cell with the
 // Gaussian-weighted sum of its window while later cells read the already smoothed ones: a
@@ -45,30 +58,51 @@
 namespace sfd {
 namespace {
 
-constexpr int kThreads = 256;
 constexpr int TX = kTileX, TZ = kTileZ;
 constexpr int H = 5;                  // staggered reach: Dx0 reads i-5..i+4, Dx1 i-4..i+5
 constexpr int HZ = 8;                 // z halo rounded for float4 staging
-constexpr int SROWS = TX + 2 * H;     // 74
 constexpr int SW = TZ + 2 * HZ;       // 80
-constexpr int SMEM = SROWS * SW;      // floats per staged field
+constexpr int TC = kIsoCols;          // columns of a CTA's tile
+constexpr int kSmem = (TC + 2 * H) * SW;  // floats per staged field
+constexpr int kThreads = TC * TZ / 4;     // one float4 of cells per thread
 
 __device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float fa(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fs(float a, float b) { return __fsub_rn(a, b); }
+
+// Two cells per instruction with the same roundings as the scalar operations: a difference as
+// fma(b, -1, a) and a sum as fma(a, one, b) are rounded once.  `one` is 1.0 from the kernel's
+// arguments: the compiler, which contracts a paired multiply and a paired add into one paired FMA,
+// cannot see that the factor does nothing.
+__device__ __forceinline__ float2 bc(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b, float one) { return __ffma2_rn(a, bc(one), b); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, bc(-1.0f), a); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
+__device__ __forceinline__ float4 cat4(float2 a, float2 b) { return make_float4(a.x, a.y, b.x, b.y); }
+__device__ __forceinline__ float4 add4(const float4& p, const float4& q, float one) {
+    return cat4(add2(lo2(p), lo2(q), one), add2(hi2(p), hi2(q), one));
+}
+// u + (c k) d, each operation rounded
+__device__ __forceinline__ float4 upd4(const float4& u, float c, const float4& k, const float4& d, float one) {
+    return cat4(add2(mul2(mul2(bc(c), lo2(k)), lo2(d)), lo2(u), one),
+                add2(mul2(mul2(bc(c), hi2(k)), hi2(d)), hi2(u), one));
+}
 
 struct TileRef {
     int shot, tile, x0, z0;
     ShotDev sd;
 };
 
+// CTA b covers TC columns; t.tile is the 64 x 64 tile (of the receiver lists) that holds them
 __device__ __forceinline__ bool tile_of(const IArgs& a, TileRef& t) {
     t.shot = a.slot_to_shot[blockIdx.y];
     t.sd = a.shots[t.shot];
-    t.tile = blockIdx.x;
-    const int tx_i = t.tile / a.L.ntz, tz_i = t.tile - tx_i * a.L.ntz;
-    t.x0 = tx_i * TX;
+    const int tx_i = blockIdx.x / a.L.ntz, tz_i = blockIdx.x - tx_i * a.L.ntz;
+    t.x0 = tx_i * TC;
     t.z0 = tz_i * TZ;
+    t.tile = t.x0 / TX * a.L.ntz + tz_i;
     return t.x0 < t.sd.nx;
 }
 
@@ -76,17 +110,65 @@ __device__ __forceinline__ long long cell(const IArgs& a, int shot, int x, int z
     return (long long)shot * a.L.shot_stride + (long long)(x + a.L.gx) * a.L.pitch + a.L.gz + z;
 }
 
-// stage f0 + f1 (YPUB:1410-1426) on the tile plus halo
-__device__ __forceinline__ void stage(float* s, const IArgs& a, const TileRef& t, const float* f0, const float* f1) {
-    constexpr int W4 = SW / 4;
-#pragma unroll 3  // several rows' loads in flight before their shared-memory stores
-    for (int i = threadIdx.x; i < SROWS * W4; i += kThreads) {
-        const int r = i / W4, c = i - r * W4;
-        const long long off = cell(a, t.shot, t.x0 - H + r, t.z0 - HZ + 4 * c);
-        const float4 u = __ldg(reinterpret_cast<const float4*>(f0 + off));
-        const float4 v = __ldg(reinterpret_cast<const float4*>(f1 + off));
-        *reinterpret_cast<float4*>(s + r * SW + 4 * c) = make_float4(fa(u.x, v.x), fa(u.y, v.y), fa(u.z, v.z), fa(u.w, v.w));
+__device__ __forceinline__ unsigned sptr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+// One thread requests the tile plus halo of NF sum fields, one TMA box each (z coordinate a multiple
+// of 64, x coordinate at least 3: see Layout2D's margins), all completing on one mbarrier.
+template <int NF>
+__device__ __forceinline__ void stage(float* s, uint64_t* bar, const IArgs& a, const TileRef& t, const int* field) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sptr(bar)),
+                 "r"(4u * NF * kSmem)
+                 : "memory");
+#pragma unroll
+    for (int f = 0; f < NF; f++)
+        asm volatile(
+            "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
+            "[%5];" ::"r"(sptr(s + f * kSmem)),
+            "l"(reinterpret_cast<uint64_t>(&a.tm[field[f] - I_VX])), "r"(a.L.gz + t.z0 - HZ), "r"(a.L.gx + t.x0 - H),
+            "r"(t.shot), "r"(sptr(bar))
+            : "memory");
+}
+__device__ __forceinline__ void bar_init(uint64_t* bar) {
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sptr(bar)) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    __syncthreads();
+}
+__device__ __forceinline__ bool bar_try(uint64_t* bar) {
+    unsigned ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(sptr(bar))
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool bar_wait_1s(uint64_t* bar) {
+    bool done = bar_try(bar);
+    if (!done) {
+        uint64_t t0, t1;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+        do {
+            done = bar_try(bar);
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+        } while (!done && t1 - t0 < 1000000000ull);
+    }
+    return done;
+}
+// every thread waits for the boxes; after a second without them it reports the timeout, gives the
+// copies another second to land before the CTA's shared memory is released, and gives up
+__device__ __forceinline__ bool staged(uint64_t* bar, const IArgs& a) {
+    if (bar_wait_1s(bar)) return true;
+    atomicExch(a.err_flag, 1);
+    bar_wait_1s(bar);
+    return false;
+}
+// programmatic dependent launch: let the next kernel's CTAs start their index work, then wait for
+// the previous kernel before the first read of its fields
+__device__ __forceinline__ void dependency() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // one split-sponge factor in YPUB:851-897's order (near-side table, then far-side table)
@@ -96,11 +178,10 @@ __device__ __forceinline__ float xs(float u, int x, int n, int np, const float* 
     return u;
 }
 
-// Work items: thread t takes the z-vector zv = t % 16 (cells z0 + 4 zv .. + 3) of the rows
-// t / 16 + 16 j, j = 0..3; a warp covers two whole tile rows, so every field access is one
-// coalesced 16-byte load or store per lane.  The stencils read float4 windows from shared
-// memory: an x derivative of four cells is ten 16-byte loads, a z derivative four.
-constexpr int kItems = TX * TZ / 4 / kThreads;  // 4
+// Thread t takes the z-vector t % 16 (cells z0 + 4 (t % 16) .. + 3) of row t / 16 of the tile; a warp
+// covers two whole tile rows, so every field access is one coalesced 16-byte load or store per lane.
+// The stencils read float4 windows from shared memory: an x derivative of four cells is ten 16-byte
+// loads, a z derivative five.
 
 __device__ __forceinline__ float4 lds4(const float* s, int r, int c) { return *reinterpret_cast<const float4*>(s + r * SW + c); }
 __device__ __forceinline__ float cmp(const float4& v, int q) { return q == 0 ? v.x : (q == 1 ? v.y : (q == 2 ? v.z : v.w)); }
@@ -108,18 +189,18 @@ __device__ __forceinline__ float& cmpr(float4& v, int q) { return q == 0 ? v.x :
 
 // x derivative (YPUB:1095-1157) of the four cells (row r, columns c..c+3) of a staged field
 template <int FLAG>
-__device__ __forceinline__ float4 dx4(const float* s, int r, int c, const float* a) {
-    float4 acc;
+__device__ __forceinline__ float4 dx4(const float* s, int r, int c, const float* a, float one) {
+    float2 l, h;
 #pragma unroll
     for (int m = 0; m < 5; m++) {
         const float4 p = lds4(s, FLAG == 0 ? r + m : r + 1 + m, c);
         const float4 q = lds4(s, FLAG == 0 ? r - 1 - m : r - m, c);
-        const float4 t = make_float4(fs(p.x, q.x), fs(p.y, q.y), fs(p.z, q.z), fs(p.w, q.w));
-        if (m == 0) acc = make_float4(fm(a[0], t.x), fm(a[0], t.y), fm(a[0], t.z), fm(a[0], t.w));
-        else acc = make_float4(fa(acc.x, fm(a[m], t.x)), fa(acc.y, fm(a[m], t.y)), fa(acc.z, fm(a[m], t.z)),
-                               fa(acc.w, fm(a[m], t.w)));
+        const float2 am = bc(a[m]);
+        const float2 tl = mul2(am, sub2(lo2(p), lo2(q))), th = mul2(am, sub2(hi2(p), hi2(q)));
+        l = m == 0 ? tl : add2(tl, l, one);
+        h = m == 0 ? th : add2(th, h, one);
     }
-    return acc;
+    return cat4(l, h);
 }
 
 // z derivative (YPUB:1347-1407) of the same four cells: the window z-8 .. z+11 (c = column of z).
@@ -140,12 +221,18 @@ __device__ __forceinline__ float4 dz4(const float* s, int r, int c, const IArgs&
         const int M = !FS ? 5 : FLAG == 0 ? (d >= 5 ? 5 : (d < 1 ? 1 : d)) : (d >= 4 ? 5 : (d < 0 ? 1 : d + 1));
         float sum = 0.0f;
 #pragma unroll
-        for (int m = 0; m < 5; m++) {
-            if (m >= M) break;
-            const float cm = M == 5 ? a.a[m] : a.cr[M - 1 > 0 ? (M == 4 ? 3 : M == 3 ? 2 : 1) : 0][m & 3];
+        for (int m = 0; m < 5; m++) {  // selects, not branches: neighbouring threads differ in M
+            float cm = a.a[m];
+            if (FS && m < 4) {
+                cm = M == 4 ? a.cr[3][m] : cm;
+                cm = m < 3 && M == 3 ? a.cr[2][m] : cm;
+                cm = m < 2 && M == 2 ? a.cr[1][m] : cm;
+                cm = m < 1 && M == 1 ? a.cr[0][m] : cm;
+            }
             const int z = 8 + q;  // index of cell q in w
             const float t = FLAG == 0 ? fs(w[z + m], w[z - 1 - m]) : fs(w[z + 1 + m], w[z - m]);
-            sum = (m == 0) ? fm(cm, t) : fa(sum, fm(cm, t));
+            const float next = (m == 0) ? fm(cm, t) : fa(sum, fm(cm, t));
+            sum = !FS || m < M ? next : sum;
         }
         cmpr(acc, q) = sum;
     }
@@ -161,160 +248,246 @@ __device__ __forceinline__ float zsp(float u, int z, int t0, const IArgs& a, con
     return u;
 }
 
-// four cells of a field: one 16-byte access when all four lie inside the grid, else per cell
-__device__ __forceinline__ float4 ld4(const float* f, long long c, int nv) {
-    if (nv == 4) return *reinterpret_cast<const float4*>(f + c);
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int q = 0; q < nv; q++) cmpr(v, q) = f[c + q];
-    return v;
-}
-__device__ __forceinline__ void st4(float* f, long long c, int nv, const float4& v) {
-    if (nv == 4) {
-        *reinterpret_cast<float4*>(f + c) = v;
-        return;
-    }
-    for (int q = 0; q < nv; q++) f[c + q] = cmp(v, q);
+// Four cells of a field.  The rows past nz of the last vector exist in the slab and hold zero, which
+// the stencils rely on: Vec::keep clears them before a store.
+__device__ __forceinline__ float4 ld4(const float* f, long long c) { return *reinterpret_cast<const float4*>(f + c); }
+__device__ __forceinline__ void st4(float* f, long long c, const float4& v) { *reinterpret_cast<float4*>(f + c) = v; }
+
+__device__ __forceinline__ void mul4(float4& v, float f) {
+    v = cat4(mul2(lo2(v), bc(f)), mul2(hi2(v), bc(f)));
 }
 
+// One z-vector of a row: where it lies and which sponges, surface rows and orders it meets.  A plain
+// vector (all but those at the surface and across the bottom edge) updates its four cells alike: the
+// x sponge is one factor per row, the z sponge is applied only by the threads inside it.  Deciding
+// this per cell took 237 (velocity) and 382 (stress) instructions a cell, which bound the kernels.
 template <bool FS>
-__global__ void __launch_bounds__(kThreads, 3) iso_velocity_kernel(const __grid_constant__ IArgs a) {
-    extern __shared__ __align__(16) float smem[];
-    float* sSxx = smem;
-    float* sSxz = smem + SMEM;
-    float* sSzz = smem + 2 * SMEM;
+struct Vec {
+    int gx, gz, top;
+    long long c, mi;
+    bool plain, pad, air;
+    __device__ __forceinline__ Vec(const IArgs& a, const TileRef& t, int r, int z) {
+        gx = t.x0 + r;
+        gz = t.z0 + z;
+        c = cell(a, t.shot, gx, gz);
+        const int mc = min(t.sd.x0 + gx, a.nx_model - 1);
+        mi = (long long)mc * a.mpitch + gz;
+        // first updated row: zs = itopo - 1 (fsbc) or t0 = itopo - npz - 1 (abc)
+        top = __ldg(a.itopo + mc) - (FS ? 1 : a.npz + 1);
+        const bool zpad = (!FS && gz <= top + a.npz) || gz + 3 >= a.nz - a.npz - 1;
+        plain = gz + 3 < a.nz && gz - top >= (FS ? 5 : 0);
+        pad = zpad || gx <= a.npx || gx >= t.sd.nx - a.npx - 1;
+        // above the row over the surface (which the surface kernel rewrites) nothing changes
+        air = gz + 3 < top - 1 && !zpad;
+    }
+    // both sponge tables of the x part, near side then far side (YPUB:851-897)
+    __device__ __forceinline__ void xsp(float4& v, const IArgs& a, int nx, const float* tn) const {
+        if (gx <= a.npx) mul4(v, tn[gx]);
+        if (gx >= nx - a.npx - 1) mul4(v, tn[a.spg_stride + nx - 1 - gx]);
+    }
+    __device__ __forceinline__ void zsp4(float4& v, const IArgs& a, const float* tn) const {
+#pragma unroll
+        for (int q = 0; q < 4; q++) cmpr(v, q) = zsp<FS>(cmp(v, q), gz + q, top, a, tn, tn + a.spg_stride);
+    }
+    __device__ __forceinline__ void keep(float4& v, int nz) const {
+#pragma unroll
+        for (int q = 1; q < 4; q++)
+            if (gz + q >= nz) cmpr(v, q) = 0.0f;
+    }
+};
+
+template <bool FS>
+__global__ void __launch_bounds__(kThreads, 5) iso_velocity_kernel(const __grid_constant__ IArgs a) {
+    extern __shared__ __align__(128) float smem[];
+    const float* sSxx = smem;
+    const float* sSxz = smem + kSmem;
+    const float* sSzz = smem + 2 * kSmem;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + 3 * kSmem);
     TileRef t;
-    if (!tile_of(a, t)) return;
-    stage(sSxx, a, t, a.f[I_SXXX], a.f[I_SXXZ]);
-    stage(sSxz, a, t, a.f[I_SXZX], a.f[I_SXZZ]);
-    stage(sSzz, a, t, a.f[I_SZZX], a.f[I_SZZZ]);
-    __syncthreads();
+    const bool on = tile_of(a, t);
+    bar_init(bar);
+    dependency();
+    if (!on) return;
+    if (threadIdx.x == 0) {
+        const int f[3] = {I_SXX, I_SXZ, I_SZZ};
+        stage<3>(smem, bar, a, t, f);
+    }
     const int nx = t.sd.nx, nz = a.nz;
     const float* tb = a.spg;
     const int st = a.spg_stride;
-    const int zv = threadIdx.x & 15, z = 4 * zv, gz = t.z0 + z;
-    const int nv = min(4, nz - gz);  // cells of the vector inside the grid
-    if (nv <= 0) return;             // no barrier follows
-#pragma unroll 1
-    for (int j = 0; j < kItems; j++) {
-        const int r = (threadIdx.x >> 4) + 16 * j, gx = t.x0 + r;
-        if (gx >= nx) break;
-        const long long c = cell(a, t.shot, gx, gz);
-        const int mc = min(t.sd.x0 + gx, a.nx_model - 1);
-        const long long mi = (long long)mc * a.mpitch + gz;
-        // first updated row: zs = itopo - 1 (fsbc) or t0 = itopo - npz - 1 (abc)
-        const int top = __ldg(a.itopo + mc) - (FS ? 1 : a.npz + 1);
-        const int d0 = FS ? gz - top : (1 << 20);
-        float4 vxx = ld4(a.f[I_VXX], c, nv), vxz = ld4(a.f[I_VXZ], c, nv);
-        float4 vzx = ld4(a.f[I_VZX], c, nv), vzz = ld4(a.f[I_VZZ], c, nv);
-        const float4 b2 = __ldg(reinterpret_cast<const float4*>(a.b2e + mi));
-        const float4 b1 = __ldg(reinterpret_cast<const float4*>(a.b1e + mi));
-        const float4 d_xx = dx4<0>(sSxx, r + H, z + HZ, a.a);      // Dx0 strxx
-        const float4 d_xz = dz4<0, FS>(sSxz, r + H, z + HZ, a, d0);    // Dz0 strxz
-        const float4 d_zx = dx4<1>(sSxz, r + H, z + HZ, a.a);      // Dx1 strxz
-        const float4 d_zz = dz4<1, FS>(sSzz, r + H, z + HZ, a, d0);    // Dz1 strzz
+    const int z = 4 * (threadIdx.x & 15);
+    const int r = threadIdx.x >> 4;
+    const Vec<FS> e(a, t, r, z);
+    if (t.x0 + r >= nx || e.gz >= nz || e.air) {
+        staged(bar, a);  // leave with the CTA's copies landed
+        return;
+    }
+    float4 vxx = ld4(a.f[I_VXX], e.c), vxz = ld4(a.f[I_VXZ], e.c);
+    float4 vzx = ld4(a.f[I_VZX], e.c), vzz = ld4(a.f[I_VZZ], e.c);
+    const float4 b2 = __ldg(reinterpret_cast<const float4*>(a.b2e + e.mi));
+    const float4 b1 = __ldg(reinterpret_cast<const float4*>(a.b1e + e.mi));
+    if (!staged(bar, a)) return;
+    const float4 d_xx = dx4<0>(sSxx, r + H, z + HZ, a.a, a.one);  // Dx0 strxx
+    const float4 d_zx = dx4<1>(sSxz, r + H, z + HZ, a.a, a.one);  // Dx1 strxz
+    // YPRI:310-326: vx parts with sponges spgxn/spgxp and spgzn/spgzp, vz parts with
+    // spg1xn/spg2xp and spg1zn/spg2zp
+    if (e.plain) {
+        vxx = upd4(vxx, a.dtdx, b2, d_xx, a.one);
+        vxz = upd4(vxz, a.dtdz, b2, dz4<0, false>(sSxz, r + H, z + HZ, a, 0), a.one);
+        vzx = upd4(vzx, a.dtdx, b1, d_zx, a.one);
+        vzz = upd4(vzz, a.dtdz, b1, dz4<1, false>(sSzz, r + H, z + HZ, a, 0), a.one);
+        if (e.pad) {
+            e.xsp(vxx, a, nx, tb);
+            e.xsp(vzx, a, nx, tb + 4 * st);
+            e.zsp4(vxz, a, tb + 2 * st);
+            e.zsp4(vzz, a, tb + 6 * st);
+        }
+    } else {
+        const int d0 = FS ? e.gz - e.top : (1 << 20);
+        const float4 d_xz = dz4<0, FS>(sSxz, r + H, z + HZ, a, d0);  // Dz0 strxz
+        const float4 d_zz = dz4<1, FS>(sSzz, r + H, z + HZ, a, d0);  // Dz1 strzz
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            const int zq = min(gz + q, nz - 1);  // cells past nz are computed, not stored
-            const bool below = gz + q >= top;  // rows above the first updated row keep their values
-            // YPRI:310-316: vx parts, sponge spgxn/spgxp (x part), spgzn/spgzp (z part)
+            const int zq = min(e.gz + q, nz - 1);      // cells past nz are computed, not stored
+            const bool below = e.gz + q >= e.top;  // rows above the first updated row keep their values
             if (below) {
                 const float n_xx = fa(cmp(vxx, q), fm(fm(a.dtdx, cmp(b2, q)), cmp(d_xx, q)));
-                cmpr(vxx, q) = xs(n_xx, gx, nx, a.npx, tb + 0 * st, tb + 1 * st);
+                cmpr(vxx, q) = xs(n_xx, e.gx, nx, a.npx, tb + 0 * st, tb + 1 * st);
                 cmpr(vxz, q) = fa(cmp(vxz, q), fm(fm(a.dtdz, cmp(b2, q)), cmp(d_xz, q)));
             }
-            cmpr(vxz, q) = zsp<FS>(cmp(vxz, q), zq, top, a, tb + 2 * st, tb + 3 * st);
-            // YPRI:320-326: vz parts, sponge spg1xn/spg2xp, spg1zn/spg2zp
+            cmpr(vxz, q) = zsp<FS>(cmp(vxz, q), zq, e.top, a, tb + 2 * st, tb + 3 * st);
             if (below) {
                 const float n_zx = fa(cmp(vzx, q), fm(fm(a.dtdx, cmp(b1, q)), cmp(d_zx, q)));
-                cmpr(vzx, q) = xs(n_zx, gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
+                cmpr(vzx, q) = xs(n_zx, e.gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
                 cmpr(vzz, q) = fa(cmp(vzz, q), fm(fm(a.dtdz, cmp(b1, q)), cmp(d_zz, q)));
             }
-            cmpr(vzz, q) = zsp<FS>(cmp(vzz, q), zq, top, a, tb + 6 * st, tb + 7 * st);
+            cmpr(vzz, q) = zsp<FS>(cmp(vzz, q), zq, e.top, a, tb + 6 * st, tb + 7 * st);
         }
-        st4(a.f[I_VXX], c, nv, vxx); st4(a.f[I_VXZ], c, nv, vxz);
-        st4(a.f[I_VZX], c, nv, vzx); st4(a.f[I_VZZ], c, nv, vzz);
+        e.keep(vxx, nz); e.keep(vxz, nz); e.keep(vzx, nz); e.keep(vzz, nz);
     }
+    st4(a.f[I_VXX], e.c, vxx); st4(a.f[I_VXZ], e.c, vxz);
+    st4(a.f[I_VZX], e.c, vzx); st4(a.f[I_VZZ], e.c, vzz);
+    st4(a.f[I_VX], e.c, add4(vxx, vxz, a.one));  // YPRI:316
+    st4(a.f[I_VZ], e.c, add4(vzx, vzz, a.one));  // YPRI:326
 }
 
 template <bool FS>
-__global__ void __launch_bounds__(kThreads, 3) iso_stress_kernel(const __grid_constant__ IArgs a) {
-    __shared__ __align__(16) float sVx[SMEM];
-    __shared__ __align__(16) float sVz[SMEM];
+__global__ void __launch_bounds__(kThreads, 5) iso_stress_kernel(const __grid_constant__ IArgs a) {
+    extern __shared__ __align__(128) float smem[];
+    const float* sVx = smem;
+    const float* sVz = smem + kSmem;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + 2 * kSmem);
     TileRef t;
-    if (!tile_of(a, t)) return;
-    stage(sVx, a, t, a.f[I_VXX], a.f[I_VXZ]);  // vx = vxx + vxz (YPRI:316)
-    stage(sVz, a, t, a.f[I_VZX], a.f[I_VZZ]);  // vz = vzx + vzz (YPRI:326)
-    __syncthreads();
+    const bool on = tile_of(a, t);
+    bar_init(bar);
+    dependency();
+    if (!on) return;
+    if (threadIdx.x == 0) {
+        const int f[2] = {I_VX, I_VZ};
+        stage<2>(smem, bar, a, t, f);
+    }
     const int nx = t.sd.nx, nz = a.nz;
     const float* tb = a.spg;
     const int st = a.spg_stride;
     const ShotDev& sd = t.sd;
     const float wav = __ldg(a.wavelets + sd.wav_off + a.step);
-    const int zv = threadIdx.x & 15, z = 4 * zv, gz = t.z0 + z;
-    const int nv = min(4, nz - gz);
+    const int z = 4 * (threadIdx.x & 15);
     // YPRI:163-168: in fsbc mode strxx takes the source only below the surface at the source column
     const bool src_xx = !FS || sd.sz + 1 > __ldg(a.itopo + min(sd.x0 + sd.sx, a.nx_model - 1));
-#pragma unroll 1
-    for (int j = 0; j < kItems && nv > 0; j++) {
-        const int r = (threadIdx.x >> 4) + 16 * j, gx = t.x0 + r;
-        if (gx >= nx) break;
-        const long long c = cell(a, t.shot, gx, gz);
-        const int mc = min(sd.x0 + gx, a.nx_model - 1);
-        const long long mi = (long long)mc * a.mpitch + gz;
-        const int top = __ldg(a.itopo + mc) - (FS ? 1 : a.npz + 1);  // zs (fsbc) or t0 (abc)
-        const int d0 = FS ? gz - top : (1 << 20);
-        float4 v[6];  // strxxx strxxz strzzx strzzz strxzx strxzz
+    // YPUB:1458 wavelet*gc2d*dt/(dz**2)
+    auto source = [&](int bx, int bz) {
+        return __fdiv_rn(fm(fm(wav, __ldg(a.stamps + sd.stamp_off + bx * sd.stamp_h + bz)), a.dt), a.dz2);
+    };
+    const int r = threadIdx.x >> 4;
+    const Vec<FS> e(a, t, r, z);
+    const int bx = e.gx - sd.stamp_x0, bz0 = e.gz - sd.stamp_z0;
+    const bool stamp = bx >= 0 && bx < sd.stamp_w && bz0 + 3 >= 0 && bz0 < sd.stamp_h;
+    const bool work = t.x0 + r < nx && e.gz < nz && (!e.air || stamp);
+    float4 v[6], lm2, lam, mue;  // v: strxxx strxxz strzzx strzzz strxzx strxzz
+    if (work) {
 #pragma unroll
-        for (int k = 0; k < 6; k++) v[k] = ld4(a.f[I_SXXX + k], c, nv);
-        const float4 lm2 = __ldg(reinterpret_cast<const float4*>(a.lm2 + mi));
-        const float4 lam = __ldg(reinterpret_cast<const float4*>(a.lam + mi));
-        const float4 mue = __ldg(reinterpret_cast<const float4*>(a.mue + mi));
-        const float4 d1 = dx4<1>(sVx, r + H, z + HZ, a.a);       // Dx1 vx
-        const float4 d2 = dz4<0, FS>(sVz, r + H, z + HZ, a, d0);     // Dz0 vz
-        const float4 d3 = dx4<0>(sVz, r + H, z + HZ, a.a);       // Dx0 vz
-        const float4 d4 = dz4<1, FS>(sVx, r + H, z + HZ, a, d0);     // Dz1 vx
-        const int bx = gx - sd.stamp_x0;
-        const bool xin = bx >= 0 && bx < sd.stamp_w;
+        for (int k = 0; k < 6; k++) v[k] = ld4(a.f[I_SXXX + k], e.c);
+        lm2 = __ldg(reinterpret_cast<const float4*>(a.lm2 + e.mi));
+        lam = __ldg(reinterpret_cast<const float4*>(a.lam + e.mi));
+        mue = __ldg(reinterpret_cast<const float4*>(a.mue + e.mi));
+    }
+    if (!staged(bar, a)) return;
+    if (work) {
+        const float4 d1 = dx4<1>(sVx, r + H, z + HZ, a.a, a.one);  // Dx1 vx
+        const float4 d3 = dx4<0>(sVz, r + H, z + HZ, a.a, a.one);  // Dx0 vz
+        if (e.plain) {
+            const float4 d2 = dz4<0, false>(sVz, r + H, z + HZ, a, 0), d4 = dz4<1, false>(sVx, r + H, z + HZ, a, 0);
+            v[0] = upd4(v[0], a.dtdx, lm2, d1, a.one);
+            v[1] = upd4(v[1], a.dtdz, lam, d2, a.one);
+            v[2] = upd4(v[2], a.dtdx, lam, d1, a.one);
+            v[3] = upd4(v[3], a.dtdz, lm2, d2, a.one);
+            v[4] = upd4(v[4], a.dtdx, mue, d3, a.one);
+            v[5] = upd4(v[5], a.dtdz, mue, d4, a.one);
+            if (e.pad) {
+                e.xsp(v[0], a, nx, tb + 4 * st);
+                e.zsp4(v[1], a, tb + 2 * st);
+                e.xsp(v[2], a, nx, tb + 4 * st);
+                e.zsp4(v[3], a, tb + 2 * st);
+                e.xsp(v[4], a, nx, tb);
+                e.zsp4(v[5], a, tb + 6 * st);
+            }
+            if (stamp) {
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int zq = min(gz + q, nz - 1);  // cells past nz are computed, not stored
-            const int bz = zq - sd.stamp_z0;
-            const bool in_stamp = xin && bz >= 0 && bz < sd.stamp_h;
-            float src = 0.0f;
-            if (in_stamp)  // YPUB:1458 wavelet*gc2d*dt/(dz**2)
-                src = __fdiv_rn(fm(fm(wav, __ldg(a.stamps + sd.stamp_off + bx * sd.stamp_h + bz)), a.dt), a.dz2);
-            // rows above the first updated row keep their values (the loops start at itopo or
-            // itopo - npzn)
-            const bool below = gz + q >= top;
-            const bool zero_zz = FS && gz + q <= top;  // YPUB:978-1007, rows <= itopo
-            // YPRI:331-338: strxx parts, sponge spg1xn/spg2xp, spgzn/spgzp, then the source
-            float s0 = cmp(v[0], q), s1 = cmp(v[1], q), s2 = cmp(v[2], q), s3 = cmp(v[3], q);
-            float s4 = cmp(v[4], q), s5 = cmp(v[5], q);
-            if (below) {
-                s0 = xs(fa(s0, fm(fm(a.dtdx, cmp(lm2, q)), cmp(d1, q))), gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
-                s1 = fa(s1, fm(fm(a.dtdz, cmp(lam, q)), cmp(d2, q)));
+                for (int q = 0; q < 4; q++)
+                    if (bz0 + q >= 0 && bz0 + q < sd.stamp_h) {
+                        const float src = source(bx, bz0 + q);
+                        if (src_xx) cmpr(v[0], q) = fa(src, cmp(v[0], q));
+                        cmpr(v[2], q) = fa(src, cmp(v[2], q));
+                    }
             }
-            s1 = zsp<FS>(s1, zq, top, a, tb + 2 * st, tb + 3 * st);
-            if (in_stamp && src_xx) s0 = fa(src, s0);
-            // YPRI:342-349: strzz parts; fsbc: zero on rows <= the surface before the source
-            if (below) {
-                s2 = xs(fa(s2, fm(fm(a.dtdx, cmp(lam, q)), cmp(d1, q))), gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
-                s3 = fa(s3, fm(fm(a.dtdz, cmp(lm2, q)), cmp(d2, q)));
+        } else {
+            const int d0 = FS ? e.gz - e.top : (1 << 20);
+            const float4 d2 = dz4<0, FS>(sVz, r + H, z + HZ, a, d0);  // Dz0 vz
+            const float4 d4 = dz4<1, FS>(sVx, r + H, z + HZ, a, d0);  // Dz1 vx
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int zq = min(e.gz + q, nz - 1);  // cells past nz are computed, not stored
+                const int bz = zq - sd.stamp_z0;
+                const bool in_stamp = stamp && bz >= 0 && bz < sd.stamp_h;
+                const float src = in_stamp ? source(bx, bz) : 0.0f;
+                // rows above the first updated row keep their values (the loops start at itopo or
+                // itopo - npzn)
+                const bool below = e.gz + q >= e.top;
+                const bool zero_zz = FS && e.gz + q <= e.top;  // YPUB:978-1007, rows <= itopo
+                // YPRI:331-338: strxx parts, sponge spg1xn/spg2xp, spgzn/spgzp, then the source
+                float s0 = cmp(v[0], q), s1 = cmp(v[1], q), s2 = cmp(v[2], q), s3 = cmp(v[3], q);
+                float s4 = cmp(v[4], q), s5 = cmp(v[5], q);
+                if (below) {
+                    s0 = xs(fa(s0, fm(fm(a.dtdx, cmp(lm2, q)), cmp(d1, q))), e.gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
+                    s1 = fa(s1, fm(fm(a.dtdz, cmp(lam, q)), cmp(d2, q)));
+                }
+                s1 = zsp<FS>(s1, zq, e.top, a, tb + 2 * st, tb + 3 * st);
+                if (in_stamp && src_xx) s0 = fa(src, s0);
+                // YPRI:342-349: strzz parts; fsbc: zero on rows <= the surface before the source
+                if (below) {
+                    s2 = xs(fa(s2, fm(fm(a.dtdx, cmp(lam, q)), cmp(d1, q))), e.gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
+                    s3 = fa(s3, fm(fm(a.dtdz, cmp(lm2, q)), cmp(d2, q)));
+                }
+                s3 = zsp<FS>(s3, zq, e.top, a, tb + 2 * st, tb + 3 * st);
+                if (zero_zz) s2 = s3 = 0.0f;
+                if (in_stamp) s2 = fa(src, s2);
+                // YPRI:353-359: strxz parts, sponge spgxn/spgxp, spg1zn/spg2zp
+                if (below) {
+                    s4 = xs(fa(s4, fm(fm(a.dtdx, cmp(mue, q)), cmp(d3, q))), e.gx, nx, a.npx, tb + 0 * st, tb + 1 * st);
+                    s5 = fa(s5, fm(fm(a.dtdz, cmp(mue, q)), cmp(d4, q)));
+                }
+                s5 = zsp<FS>(s5, zq, e.top, a, tb + 6 * st, tb + 7 * st);
+                cmpr(v[0], q) = s0; cmpr(v[1], q) = s1; cmpr(v[2], q) = s2;
+                cmpr(v[3], q) = s3; cmpr(v[4], q) = s4; cmpr(v[5], q) = s5;
             }
-            s3 = zsp<FS>(s3, zq, top, a, tb + 2 * st, tb + 3 * st);
-            if (zero_zz) s2 = s3 = 0.0f;
-            if (in_stamp) s2 = fa(src, s2);
-            // YPRI:353-359: strxz parts, sponge spgxn/spgxp, spg1zn/spg2zp
-            if (below) {
-                s4 = xs(fa(s4, fm(fm(a.dtdx, cmp(mue, q)), cmp(d3, q))), gx, nx, a.npx, tb + 0 * st, tb + 1 * st);
-                s5 = fa(s5, fm(fm(a.dtdz, cmp(mue, q)), cmp(d4, q)));
-            }
-            s5 = zsp<FS>(s5, zq, top, a, tb + 6 * st, tb + 7 * st);
-            cmpr(v[0], q) = s0; cmpr(v[1], q) = s1; cmpr(v[2], q) = s2;
-            cmpr(v[3], q) = s3; cmpr(v[4], q) = s4; cmpr(v[5], q) = s5;
+#pragma unroll
+            for (int k = 0; k < 6; k++) e.keep(v[k], nz);
         }
 #pragma unroll
-        for (int k = 0; k < 6; k++) st4(a.f[I_SXXX + k], c, nv, v[k]);
+        for (int k = 0; k < 6; k++) st4(a.f[I_SXXX + k], e.c, v[k]);
+        st4(a.f[I_SXX], e.c, add4(v[0], v[1], a.one));
+        st4(a.f[I_SZZ], e.c, add4(v[2], v[3], a.one));
+        st4(a.f[I_SXZ], e.c, add4(v[4], v[5], a.one));
     }
     // receivers: record1 = vx, record2 = vz after the step (YPRI:361-367, YPUB:2-16); the
     // velocities are final after the velocity kernel and staged here
@@ -323,6 +496,7 @@ __global__ void __launch_bounds__(kThreads, 3) iso_stress_kernel(const __grid_co
     for (int j = rb + threadIdx.x; j < re; j += kThreads) {
         const int ridx = a.tile_rec_idx[j];
         const int rr = a.rec_x[sd.rec_list + ridx] - t.x0 + H, rz = a.rec_z[sd.rec_list + ridx] - t.z0 + HZ;
+        if (rr < H || rr >= H + TC) continue;  // another CTA of the 64 x 64 tile holds it
         const long long o = sd.rec_base + (long long)a.step * sd.nrec + ridx;
         a.records[o] = sVx[rr * SW + rz];
         a.records2[o] = sVz[rr * SW + rz];
@@ -332,17 +506,21 @@ __global__ void __launch_bounds__(kThreads, 3) iso_stress_kernel(const __grid_co
 // Free surface, after the stress kernel (one thread per column, zs = itopo(x) - 1): the image strxz(zs - 1) =
 // -strxz(zs) of both split parts (YPUB:1009-1024), and vz(zs - 1) = vz(zs) + lambsg/lambmusg
 // (vx(zs, x + 1) - vx(zs, x)) for both pairs of split parts (YPUB:938-976, columns but the last).
+// The velocity kernel that follows forms the sums of vx and vz again; the sum of strxz is written here.
 __global__ void iso_surface_kernel(const __grid_constant__ IArgs a) {
     const int shot = a.slot_to_shot[blockIdx.y];
     const ShotDev sd = a.shots[shot];
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    dependency();
     if (x >= sd.nx) return;
     const int mc = min(sd.x0 + x, a.nx_model - 1);
     const int zs = __ldg(a.itopo + mc) - 1;
     if (zs < 1) return;  // the row above the surface is the split fields' unused row 0
     const long long c = cell(a, shot, x, zs), cu = c - 1;
-    a.f[I_SXZX][cu] = -a.f[I_SXZX][c];
-    a.f[I_SXZZ][cu] = -a.f[I_SXZZ][c];
+    const float ux = -a.f[I_SXZX][c], uz = -a.f[I_SXZZ][c];
+    a.f[I_SXZX][cu] = ux;
+    a.f[I_SXZZ][cu] = uz;
+    a.f[I_SXZ][cu] = fa(ux, uz);
     if (x + 1 < sd.nx) {
         const long long cn = cell(a, shot, x + 1, zs);
         const long long mi = (long long)mc * a.mpitch + zs;
@@ -437,23 +615,48 @@ __global__ void __launch_bounds__(32) iso_smooth_kernel(const __grid_constant__ 
 
 }  // namespace
 
-cudaError_t elastic2d_launch_step(const IArgs& a, int active, int nx_max, cudaStream_t st, int* launches) {
-    dim3 grid(a.L.ntx * a.L.ntz, active);
-    const size_t smem = sizeof(float) * 3 * SMEM;
+namespace {
+
+cudaError_t launch_dependent(const void* fn, dim3 grid, int threads, size_t smem, cudaStream_t st, const IArgs& a) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    void* args[] = {const_cast<IArgs*>(&a)};
+    return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
+template <bool FS>
+cudaError_t launch_pair(const IArgs& a, int active, cudaStream_t st) {
+    const dim3 grid(a.L.ntx * (TX / TC) * a.L.ntz, active);
+    const int sv = (int)sizeof(float) * (3 * kSmem + 4), ss = (int)sizeof(float) * (2 * kSmem + 4);
+    const void* kv = (const void*)iso_velocity_kernel<FS>;
+    const void* ks = (const void*)iso_stress_kernel<FS>;
     static bool attr0[kMaxDevices] = {}, attr1[kMaxDevices] = {};
-    if (cudaError_t e = smem_attr_once((const void*)iso_velocity_kernel<false>, (int)smem, attr0)) return e;
-    if (cudaError_t e = smem_attr_once((const void*)iso_velocity_kernel<true>, (int)smem, attr1)) return e;
-    *launches = 2;
-    if (a.fs) {
-        iso_velocity_kernel<true><<<grid, kThreads, smem, st>>>(a);
-        iso_stress_kernel<true><<<grid, kThreads, 0, st>>>(a);
-        iso_surface_kernel<<<dim3((nx_max + 127) / 128, active), 128, 0, st>>>(a);
-        *launches = 3;
-    } else {
-        iso_velocity_kernel<false><<<grid, kThreads, smem, st>>>(a);
-        iso_stress_kernel<false><<<grid, kThreads, 0, st>>>(a);
-    }
-    return cudaGetLastError();
+    if (cudaError_t e = smem_attr_once(kv, sv, attr0)) return e;
+    if (cudaError_t e = smem_attr_once(ks, ss, attr1)) return e;
+    if (cudaError_t e = launch_dependent(kv, grid, kThreads, sv, st, a)) return e;
+    return launch_dependent(ks, grid, kThreads, ss, st, a);
+}
+
+}  // namespace
+
+void elastic2d_box(int box[2]) {
+    box[0] = SW;
+    box[1] = TC + 2 * H;
+}
+
+cudaError_t elastic2d_launch_step(const IArgs& a, int active, int nx_max, cudaStream_t st, int* launches) {
+    *launches = a.fs ? 3 : 2;
+    const cudaError_t e = a.fs ? launch_pair<true>(a, active, st) : launch_pair<false>(a, active, st);
+    if (e != cudaSuccess || !a.fs) return e;
+    return launch_dependent((const void*)iso_surface_kernel, dim3((nx_max + 127) / 128, active), 128, 0, st, a);
 }
 
 cudaError_t elastic2d_smooth(float* const arrays[5], int mpitch, int ghost, int nz, const int* itopo_dev,

@@ -154,11 +154,15 @@ void viscoel2d_prepare(int nx, int nz, const float* vp, const float* vs, const f
                        float* m3, float* rtau_out);
 
 // Isotropic elastic standard-staggered-grid split fields (elastic2d.cu), in slab order:
-// forward/yang_version_2016_2_2 vxx vxz vzx vzz strxxx strxxz strzzx strzzz strxzx strxzz.
-enum IField { I_VXX, I_VXZ, I_VZX, I_VZZ, I_SXXX, I_SXXZ, I_SZZX, I_SZZZ, I_SXZX, I_SXZZ, I_NFIELDS };
+// forward/yang_version_2016_2_2 vxx vxz vzx vzz strxxx strxxz strzzx strzzz strxzx strxzz,
+// then the sums vx vz strxx strzz strxz that the next kernel stages.
+enum IField { I_VXX, I_VXZ, I_VZX, I_VZZ, I_SXXX, I_SXXZ, I_SZZX, I_SZZZ, I_SXZX, I_SXZZ,
+              I_VX, I_VZ, I_SXX, I_SZZ, I_SXZ, I_NFIELDS };
 
-// Arguments of the isotropic elastic kernels (elastic2d.cu): ten in-place split fields.
+// Arguments of the isotropic elastic kernels (elastic2d.cu): ten in-place split fields, five sums.
 struct IArgs {
+    CUtensorMap tm[5];                    // vx vz strxx strzz strxz (elastic2d_box)
+    int* err_flag;                        // set to 1 by a CTA whose bounded wait ran out
     float* f[I_NFIELDS];
     Layout2D L;
     int nz, npx, npz;
@@ -167,6 +171,7 @@ struct IArgs {
     int mpitch, nx_model;
     float dt, dtdx, dtdz, dz2;
     float a[5];
+    float one;                            // 1.0 (elastic2d.cu add2)
     float cr[4][4];                       // M-term staggered coefficients, M = 1..4 (YMOD:7-20)
     int fs;                               // 1: free surface (fsbc mode), 0: abc mode
     const int* itopo;                     // per prepared-model column: the reference's itopo (1-based
@@ -185,6 +190,8 @@ struct IArgs {
 };
 // One step: the velocity and stress kernels, and in fsbc mode the surface kernel (YPUB:938-976
 // calfsbcv, YPUB:1009-1024 calfsbcstrxz); *launches receives the kernel count.
+constexpr int kIsoCols = 8;  // columns per CTA of the velocity and stress kernels
+void elastic2d_box(int box[2]);  // TMA box of IArgs::tm
 cudaError_t elastic2d_launch_step(const IArgs& a, int active, int nx_max, cudaStream_t st, int* launches);
 // YPUB:323-547 on one window (x-major, z fastest): substagger and the refill of the rows above
 // itopo(x) (0-based rows < itopo - 1 take row itopo - 1); out: busg2e, busg1e, lambmusg, lambsg,
