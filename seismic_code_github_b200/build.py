@@ -43,7 +43,8 @@ def _sources():
 def _compile(src: str, ptxas_v: bool) -> str:
     out = os.path.join(OBJ, os.path.splitext(src)[0] + ".o")
     path = os.path.join(CSRC, src)
-    deps = [path, os.path.join(CSRC, "sfd_internal.h"), os.path.join(ROOT, "include", "seisfd.h")]
+    deps = [path, os.path.join(CSRC, "sfd_internal.h"), os.path.join(CSRC, "tile_stage.cuh"),
+            os.path.join(ROOT, "include", "seisfd.h")]
     if os.path.exists(out) and all(os.path.getmtime(out) >= os.path.getmtime(d) for d in deps if os.path.exists(d)) \
             and not ptxas_v:
         return out

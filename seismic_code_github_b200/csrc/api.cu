@@ -79,7 +79,7 @@ struct sfd_ctx {
     int* d_err = nullptr;      // bounded-wait timeout flag written by the step kernels
     CUtensorMap tmaps[6];      // TMA descriptors: P0 P1 VX0 VX1 VZ0 VZ1
     CUtensorMap mtmaps[6];     // the same buffers with the x-marching kernel's boxes
-    CUtensorMap itmaps[5];     // isotropic elastic sums vx vz strxx strzz strxz (elastic2d.cu box)
+    CUtensorMap etmaps[5];     // elastic schemes: sums vx vz sxx szz sxz (elastic2d.cu / viscoel2d.cu box)
     CUtensorMap qtmaps[2];     // default viscoacoustic step: sigma S0 S1 (viscoac2d_fast.cu box)
 
     // 3-D scheme: dense [x][y][pitch] slabs, 8 fields (P, Vx, Vy, Vz, two buffers each)
@@ -501,12 +501,14 @@ QArgs make_qargs(const sfd_ctx* c, int step) {
     return a;
 }
 
-// Arguments of the visco-elastic step (22 in-place split fields per shot).
+// Arguments of the visco-elastic step (22 in-place split fields and five sums per shot).
 EArgs make_eargs(const sfd_ctx* c, int step) {
     EArgs a{};
     const QArgs q = make_qargs(c, step);
     const long long fs = (long long)c->nshot * c->L.shot_stride;
     for (int i = 0; i < E_NFIELDS; i++) a.f[i] = c->d_state + i * fs;
+    for (int k = 0; k < 5; k++) a.tm[k] = c->etmaps[k];
+    a.err_flag = c->d_err;
     a.L = q.L;
     a.nz = q.nz; a.npx = q.npx; a.npz = q.npz;
     a.busg = q.busg;
@@ -530,7 +532,7 @@ IArgs make_iargs(const sfd_ctx* c, int step) {
     IArgs a{};
     const long long fs = (long long)c->nshot * c->L.shot_stride;
     for (int i = 0; i < I_NFIELDS; i++) a.f[i] = c->d_state + i * fs;
-    for (int k = 0; k < 5; k++) a.tm[k] = c->itmaps[k];
+    for (int k = 0; k < 5; k++) a.tm[k] = c->etmaps[k];
     a.err_flag = c->d_err;
     a.L = c->L;
     a.nz = c->g.nz;
@@ -2391,11 +2393,12 @@ int sfd_set_shots(sfd_ctx* ctx, int nshot, const sfd_shot* shots) {
         viscoac2d_sponge_tables(ctx->g.pml, ctx->g.pml, ctx->g.dx, ctx->g.dz, ctx->spg_stride, tab.data());
         dfree(ctx->d_spg);
         if ((rc = up(&ctx->d_spg, tab))) return rc;
-        for (int f = 0; iso && f < 5; f++) {
+        for (int f = 0; (iso || elastic) && f < 5; f++) {
             int box[2];
-            elastic2d_box(box);
-            float* base = ctx->d_state + (I_VX + f) * (long long)nshot * L.shot_stride;
-            if ((rc = encode_field_map(ctx, &ctx->itmaps[f], base, L, nshot, box))) return rc;
+            if (iso) elastic2d_box(box);
+            else viscoel2d_box(box);
+            float* base = ctx->d_state + ((iso ? (int)I_VX : (int)E_VX) + f) * (long long)nshot * L.shot_stride;
+            if ((rc = encode_field_map(ctx, &ctx->etmaps[f], base, L, nshot, box))) return rc;
         }
         if (q_fast(ctx)) {
             int bs[2];

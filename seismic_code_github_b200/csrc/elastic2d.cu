@@ -54,6 +54,7 @@
 #include <vector>
 
 #include "sfd_internal.h"
+#include "tile_stage.cuh"
 
 namespace sfd {
 namespace {
@@ -110,65 +111,14 @@ __device__ __forceinline__ long long cell(const IArgs& a, int shot, int x, int z
     return (long long)shot * a.L.shot_stride + (long long)(x + a.L.gx) * a.L.pitch + a.L.gz + z;
 }
 
-__device__ __forceinline__ unsigned sptr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
 // One thread requests the tile plus halo of NF sum fields, one TMA box each (z coordinate a multiple
 // of 64, x coordinate at least 3: see Layout2D's margins), all completing on one mbarrier.
 template <int NF>
 __device__ __forceinline__ void stage(float* s, uint64_t* bar, const IArgs& a, const TileRef& t, const int* field) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sptr(bar)),
-                 "r"(4u * NF * kSmem)
-                 : "memory");
+    tile::expect(bar, 4u * NF * kSmem);
 #pragma unroll
     for (int f = 0; f < NF; f++)
-        asm volatile(
-            "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-            "[%5];" ::"r"(sptr(s + f * kSmem)),
-            "l"(reinterpret_cast<uint64_t>(&a.tm[field[f] - I_VX])), "r"(a.L.gz + t.z0 - HZ), "r"(a.L.gx + t.x0 - H),
-            "r"(t.shot), "r"(sptr(bar))
-            : "memory");
-}
-__device__ __forceinline__ void bar_init(uint64_t* bar) {
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sptr(bar)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-}
-__device__ __forceinline__ bool bar_try(uint64_t* bar) {
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(sptr(bar))
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool bar_wait_1s(uint64_t* bar) {
-    bool done = bar_try(bar);
-    if (!done) {
-        uint64_t t0, t1;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-        do {
-            done = bar_try(bar);
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-        } while (!done && t1 - t0 < 1000000000ull);
-    }
-    return done;
-}
-// every thread waits for the boxes; after a second without them it reports the timeout, gives the
-// copies another second to land before the CTA's shared memory is released, and gives up
-__device__ __forceinline__ bool staged(uint64_t* bar, const IArgs& a) {
-    if (bar_wait_1s(bar)) return true;
-    atomicExch(a.err_flag, 1);
-    bar_wait_1s(bar);
-    return false;
-}
-// programmatic dependent launch: let the next kernel's CTAs start their index work, then wait for
-// the previous kernel before the first read of its fields
-__device__ __forceinline__ void dependency() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+        tile::box(s + f * kSmem, &a.tm[field[f] - I_VX], a.L.gz + t.z0 - HZ, a.L.gx + t.x0 - H, t.shot, bar);
 }
 
 // one split-sponge factor in YPUB:851-897's order (near-side table, then far-side table)
@@ -305,8 +255,8 @@ __global__ void __launch_bounds__(kThreads, 5) iso_velocity_kernel(const __grid_
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + 3 * kSmem);
     TileRef t;
     const bool on = tile_of(a, t);
-    bar_init(bar);
-    dependency();
+    tile::bar_init(bar);
+    tile::dependency();
     if (!on) return;
     if (threadIdx.x == 0) {
         const int f[3] = {I_SXX, I_SXZ, I_SZZ};
@@ -319,14 +269,14 @@ __global__ void __launch_bounds__(kThreads, 5) iso_velocity_kernel(const __grid_
     const int r = threadIdx.x >> 4;
     const Vec<FS> e(a, t, r, z);
     if (t.x0 + r >= nx || e.gz >= nz || e.air) {
-        staged(bar, a);  // leave with the CTA's copies landed
+        tile::staged(bar, a.err_flag);  // leave with the CTA's copies landed
         return;
     }
     float4 vxx = ld4(a.f[I_VXX], e.c), vxz = ld4(a.f[I_VXZ], e.c);
     float4 vzx = ld4(a.f[I_VZX], e.c), vzz = ld4(a.f[I_VZZ], e.c);
     const float4 b2 = __ldg(reinterpret_cast<const float4*>(a.b2e + e.mi));
     const float4 b1 = __ldg(reinterpret_cast<const float4*>(a.b1e + e.mi));
-    if (!staged(bar, a)) return;
+    if (!tile::staged(bar, a.err_flag)) return;
     const float4 d_xx = dx4<0>(sSxx, r + H, z + HZ, a.a, a.one);  // Dx0 strxx
     const float4 d_zx = dx4<1>(sSxz, r + H, z + HZ, a.a, a.one);  // Dx1 strxz
     // YPRI:310-326: vx parts with sponges spgxn/spgxp and spgzn/spgzp, vz parts with
@@ -379,8 +329,8 @@ __global__ void __launch_bounds__(kThreads, 5) iso_stress_kernel(const __grid_co
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + 2 * kSmem);
     TileRef t;
     const bool on = tile_of(a, t);
-    bar_init(bar);
-    dependency();
+    tile::bar_init(bar);
+    tile::dependency();
     if (!on) return;
     if (threadIdx.x == 0) {
         const int f[2] = {I_VX, I_VZ};
@@ -411,7 +361,7 @@ __global__ void __launch_bounds__(kThreads, 5) iso_stress_kernel(const __grid_co
         lam = __ldg(reinterpret_cast<const float4*>(a.lam + e.mi));
         mue = __ldg(reinterpret_cast<const float4*>(a.mue + e.mi));
     }
-    if (!staged(bar, a)) return;
+    if (!tile::staged(bar, a.err_flag)) return;
     if (work) {
         const float4 d1 = dx4<1>(sVx, r + H, z + HZ, a.a, a.one);  // Dx1 vx
         const float4 d3 = dx4<0>(sVz, r + H, z + HZ, a.a, a.one);  // Dx0 vz
@@ -511,7 +461,7 @@ __global__ void iso_surface_kernel(const __grid_constant__ IArgs a) {
     const int shot = a.slot_to_shot[blockIdx.y];
     const ShotDev sd = a.shots[shot];
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    dependency();
+    tile::dependency();
     if (x >= sd.nx) return;
     const int mc = min(sd.x0 + x, a.nx_model - 1);
     const int zs = __ldg(a.itopo + mc) - 1;
@@ -617,21 +567,6 @@ __global__ void __launch_bounds__(32) iso_smooth_kernel(const __grid_constant__ 
 
 namespace {
 
-cudaError_t launch_dependent(const void* fn, dim3 grid, int threads, size_t smem, cudaStream_t st, const IArgs& a) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    void* args[] = {const_cast<IArgs*>(&a)};
-    return cudaLaunchKernelExC(&cfg, fn, args);
-}
-
 template <bool FS>
 cudaError_t launch_pair(const IArgs& a, int active, cudaStream_t st) {
     const dim3 grid(a.L.ntx * (TX / TC) * a.L.ntz, active);
@@ -641,8 +576,8 @@ cudaError_t launch_pair(const IArgs& a, int active, cudaStream_t st) {
     static bool attr0[kMaxDevices] = {}, attr1[kMaxDevices] = {};
     if (cudaError_t e = smem_attr_once(kv, sv, attr0)) return e;
     if (cudaError_t e = smem_attr_once(ks, ss, attr1)) return e;
-    if (cudaError_t e = launch_dependent(kv, grid, kThreads, sv, st, a)) return e;
-    return launch_dependent(ks, grid, kThreads, ss, st, a);
+    if (cudaError_t e = tile::launch(kv, grid, kThreads, sv, st, a)) return e;
+    return tile::launch(ks, grid, kThreads, ss, st, a);
 }
 
 }  // namespace
@@ -656,7 +591,7 @@ cudaError_t elastic2d_launch_step(const IArgs& a, int active, int nx_max, cudaSt
     *launches = a.fs ? 3 : 2;
     const cudaError_t e = a.fs ? launch_pair<true>(a, active, st) : launch_pair<false>(a, active, st);
     if (e != cudaSuccess || !a.fs) return e;
-    return launch_dependent((const void*)iso_surface_kernel, dim3((nx_max + 127) / 128, active), 128, 0, st, a);
+    return tile::launch((const void*)iso_surface_kernel, dim3((nx_max + 127) / 128, active), 128, 0, st, a);
 }
 
 cudaError_t elastic2d_smooth(float* const arrays[5], int mpitch, int ghost, int nz, const int* itopo_dev,

@@ -121,11 +121,14 @@ enum EField {
     E_VXX, E_VXZ, E_VZX, E_VZZ,
     E_SXXX, E_SXXZ, E_SXXR, E_SZZX, E_SZZZ, E_SZZR, E_SXZX, E_SXZZ, E_SXZR,
     E_RXXX, E_RXXZ, E_RXXR, E_RZZX, E_RZZZ, E_RZZR, E_RXZX, E_RXZZ, E_RXZR,
+    E_VX, E_VZ, E_SXX, E_SZZ, E_SXZ,  // the sums that the next kernel stages
     E_NFIELDS
 };
 
-// Arguments of the visco-elastic kernels (viscoel2d.cu): 22 in-place split fields.
+// Arguments of the visco-elastic kernels (viscoel2d.cu): 22 in-place split fields, five sums.
 struct EArgs {
+    CUtensorMap tm[5];                    // vx vz sxx szz sxz (viscoel2d_box)
+    int* err_flag;                        // set to 1 by a CTA whose bounded wait ran out
     float* f[E_NFIELDS];
     Layout2D L;
     int nz, npx, npz;
@@ -147,6 +150,7 @@ struct EArgs {
     float* records2;                      // strxx (record2)
     int step;
 };
+void viscoel2d_box(int box[2]);  // TMA box of EArgs::tm
 cudaError_t viscoel2d_launch_step(const EArgs& a, int active, cudaStream_t st);
 // QS:434-551 with vs: busg and the six stress coefficients on the padded grid, and rtaustss
 void viscoel2d_prepare(int nx, int nz, const float* vp, const float* vs, const float* rho, const float* qp,

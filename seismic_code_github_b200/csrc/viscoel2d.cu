@@ -4,11 +4,12 @@
 // (x, z and memory parts), 22 per cell:
 //   vxx vxz vzx vzz | sxxx sxxz sxxr | szzx szzz szzr | sxzx sxzz sxzr | rxxx rxxz rxxr |
 //   rzzx rzzz rzzr | rxzx rxzz rxzr
-// and one step is two kernels:
-//   velocity: sxx, sxz, szz = sums of their parts (QS:1294-1337) on the tile plus halo;
+// with the five sums vx, vz, sxx, szz, sxz (QS:1273-1337) beside them, written by the kernel that
+// completes them, and one step is two kernels:
+//   velocity: sxx, sxz, szz staged on the tile plus halo;
 //             vxx += dt b Dx0 sxx, vxz += dt b Dz0 sxz, vzx += dt b Dx0 sxz, vzz += dt b Dz0 szz,
 //             x parts times the x sponge, z parts times the z sponge        (QS:713-748, 969-990)
-//   stress:   vx = vxx + vxz, vz = vzx + vzz on the tile plus halo; d1 = Dx1 vx, d2 = Dx1 vz,
+//   stress:   vx, vz staged on the tile plus halo; d1 = Dx1 vx, d2 = Dx1 vz,
 //             d3 = Dz1 vx, d4 = Dz1 vz; with r.. the memory sums of the previous step,
 //             sxxx += dt (q1 d1), sxxz += dt (q2 d4), sxxr += dt rxx          (calpstrxx)
 //             szzx += dt (q2 d1), szzz += dt (q1 d4), szzr += dt rzz          (calpstrzz)
@@ -24,25 +25,34 @@
 //   at the receivers after the step (QM:452-459).
 // Every multiply and add is rounded separately in the reference's order, so the kernels agree
 // bit for bit with the FP32 restatement in oracle/q_oracle.cpp.
+//
+// Bound: memory.  The split fields (22 read and written) and seven model arrays are 204 B a cell; the
+// two kernels move 244 B (sums written once and read once, halos from L2).  One TMA box per sum field
+// stages a tile with its halo while every thread loads the split parts of its one cell, so that all
+// loads of a CTA are in flight together; small CTAs cover one another's waits.
 #include <cuda_runtime.h>
 
 #include <cmath>
 #include <vector>
 
 #include "sfd_internal.h"
+#include "tile_stage.cuh"
 
 namespace sfd {
 namespace {
 
-constexpr int kThreads = 256;
 constexpr int TX = kTileX, TZ = kTileZ;
+// Tiles of 64 rows by 4 columns, one thread per cell, eight (velocity) and five (stress) CTAs per SM.
+// Step of 8 shots of 780 x 580 (3.6 M cells): 64 x 64 tiles with 16 cells per thread in turn 225 us
+// (before); 8 columns 195 us; 4 columns 168 us (DRAM at 5.2 TB/s); 2 columns 165 us on this grid, with a
+// sixfold halo.
+constexpr int TC = 4, kThreads = TC * TZ;
+constexpr int kMinV = 8, kMinS = 5;
 constexpr int H = 5;                  // rotated-staggered reach
 constexpr int HZ = 8;                 // z halo rounded for float4 staging
-constexpr int SROWS = TX + 2 * H;     // 74
+constexpr int SROWS = TC + 2 * H;
 constexpr int SW = TZ + 2 * HZ;       // 80
 constexpr int SMEM = SROWS * SW;      // floats per staged field
-constexpr int kPer = TX * TZ / kThreads;
-constexpr int kNB = 2;                // cells per load batch of the stress kernel
 
 __device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float fa(float a, float b) { return __fadd_rn(a, b); }
@@ -68,6 +78,24 @@ __device__ __forceinline__ float rsg(const float* s, int r, int c, const float* 
     return fm(h, acc);
 }
 
+// both derivatives of one field: their four-point differences share the first subtraction
+template <int FLAG>
+__device__ __forceinline__ void rsg_both(const float* s, int r, int c, const float* a, float hx, float hz, float* dx,
+                                         float* dz) {
+    float ax = 0.0f, az = 0.0f;
+#pragma unroll
+    for (int m = 0; m < 5; m++) {
+        const int hi = FLAG == 0 ? m : 1 + m, lo = FLAG == 0 ? -1 - m : -m;
+        const float t = fs(s[(r + hi) * SW + c + hi], s[(r + lo) * SW + c + lo]);
+        const float p = s[(r + hi) * SW + c + lo], q = s[(r + lo) * SW + c + hi];
+        const float tx = fm(a[m], fs(fa(t, p), q)), tz = fm(a[m], fa(fs(t, p), q));
+        ax = m == 0 ? tx : fa(ax, tx);
+        az = m == 0 ? tz : fa(az, tz);
+    }
+    *dx = fm(hx, ax);
+    *dz = fm(hz, az);
+}
+
 struct TileRef {
     int shot, tile, x0, z0;
     ShotDev sd;
@@ -76,10 +104,10 @@ struct TileRef {
 __device__ __forceinline__ bool tile_of(const EArgs& a, TileRef& t) {
     t.shot = a.slot_to_shot[blockIdx.y];
     t.sd = a.shots[t.shot];
-    t.tile = blockIdx.x;
-    const int tx_i = t.tile / a.L.ntz, tz_i = t.tile - tx_i * a.L.ntz;
-    t.x0 = tx_i * TX;
+    const int tx_i = blockIdx.x / a.L.ntz, tz_i = blockIdx.x - tx_i * a.L.ntz;
+    t.x0 = tx_i * TC;
     t.z0 = tz_i * TZ;
+    t.tile = t.x0 / TX * a.L.ntz + tz_i;  // the 64 x 64 tile of the receiver lists
     return t.x0 < t.sd.nx;
 }
 
@@ -87,24 +115,13 @@ __device__ __forceinline__ long long cell(const EArgs& a, int shot, int x, int z
     return (long long)shot * a.L.shot_stride + (long long)(x + a.L.gx) * a.L.pitch + a.L.gz + z;
 }
 
-// stage (f0 + f1) + f2 (NF = 3) or f0 + f1 (NF = 2) on the tile plus halo
+// One thread requests the tile plus halo of NF sum fields (x coordinate at least 3, z a multiple of 64)
 template <int NF>
-__device__ __forceinline__ void stage(float* s, const EArgs& a, const TileRef& t, const float* f0, const float* f1,
-                                      const float* f2) {
-    constexpr int W4 = SW / 4;
-#pragma unroll 3  // several rows' loads in flight before their shared-memory stores
-    for (int i = threadIdx.x; i < SROWS * W4; i += kThreads) {
-        const int r = i / W4, c = i - r * W4;
-        const long long off = cell(a, t.shot, t.x0 - H + r, t.z0 - HZ + 4 * c);
-        const float4 u = __ldg(reinterpret_cast<const float4*>(f0 + off));
-        const float4 v = __ldg(reinterpret_cast<const float4*>(f1 + off));
-        float4 w = make_float4(fa(u.x, v.x), fa(u.y, v.y), fa(u.z, v.z), fa(u.w, v.w));
-        if (NF == 3) {
-            const float4 d = __ldg(reinterpret_cast<const float4*>(f2 + off));
-            w = make_float4(fa(w.x, d.x), fa(w.y, d.y), fa(w.z, d.z), fa(w.w, d.w));
-        }
-        *reinterpret_cast<float4*>(s + r * SW + 4 * c) = w;
-    }
+__device__ __forceinline__ void stage(float* s, uint64_t* bar, const EArgs& a, const TileRef& t, const int* field) {
+    tile::expect(bar, 4u * NF * SMEM);
+#pragma unroll
+    for (int f = 0; f < NF; f++)
+        tile::box(s + f * SMEM, &a.tm[field[f] - E_VX], a.L.gz + t.z0 - HZ, a.L.gx + t.x0 - H, t.shot, bar);
 }
 
 // one split-sponge factor applied in QS order (left table, then right table)
@@ -114,138 +131,130 @@ __device__ __forceinline__ float xs(float u, int x, int n, int np, const float* 
     return u;
 }
 
-__global__ void __launch_bounds__(kThreads) e_velocity_kernel(const __grid_constant__ EArgs a) {
-    extern __shared__ __align__(16) float smem[];
-    float* sSxx = smem;
-    float* sSxz = smem + SMEM;
-    float* sSzz = smem + 2 * SMEM;
+__global__ void __launch_bounds__(kThreads, kMinV) e_velocity_kernel(const __grid_constant__ EArgs a) {
+    extern __shared__ __align__(128) float smem[];
+    const float* sSxx = smem;
+    const float* sSxz = smem + SMEM;
+    const float* sSzz = smem + 2 * SMEM;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + 3 * SMEM);
     TileRef t;
-    if (!tile_of(a, t)) return;
-    stage<3>(sSxx, a, t, a.f[E_SXXX], a.f[E_SXXZ], a.f[E_SXXR]);
-    stage<3>(sSxz, a, t, a.f[E_SXZX], a.f[E_SXZZ], a.f[E_SXZR]);
-    stage<3>(sSzz, a, t, a.f[E_SZZX], a.f[E_SZZZ], a.f[E_SZZR]);
-    __syncthreads();
+    const bool on = tile_of(a, t);
+    tile::bar_init(bar);
+    tile::dependency();
+    if (!on) return;
+    if (threadIdx.x == 0) {
+        const int f[3] = {E_SXX, E_SXZ, E_SZZ};
+        stage<3>(smem, bar, a, t, f);
+    }
     const int nx = t.sd.nx, nz = a.nz;
+    const int r = threadIdx.x / TZ, z = threadIdx.x % TZ, gx = t.x0 + r, gz = t.z0 + z;
+    if (gx >= nx || gz >= nz) {
+        tile::staged(bar, a.err_flag);  // leave with the CTA's copies landed
+        return;
+    }
+    const long long c = cell(a, t.shot, gx, gz);
+    float n_xx = a.f[E_VXX][c], n_xz = a.f[E_VXZ][c], n_zx = a.f[E_VZX][c], n_zz = a.f[E_VZZ][c];
+    const float dtb = fm(a.dt, __ldg(a.busg + (long long)min(t.sd.x0 + gx, a.nx_model - 1) * a.mpitch + gz));
+    if (!tile::staged(bar, a.err_flag)) return;
+    n_xx = fa(n_xx, fm(dtb, rsg<true, 0>(sSxx, r + H, z + HZ, a.a, a.hx)));  // QS:713-720
+    n_zz = fa(n_zz, fm(dtb, rsg<false, 0>(sSzz, r + H, z + HZ, a.a, a.hz)));  // QS:741-748
+    float d_zx, d_xz;
+    rsg_both<0>(sSxz, r + H, z + HZ, a.a, a.hx, a.hz, &d_zx, &d_xz);
+    n_xz = fa(n_xz, fm(dtb, d_xz));  // QS:722-729
+    n_zx = fa(n_zx, fm(dtb, d_zx));  // QS:733-740
     const float* tb = a.spg;
     const int st = a.spg_stride;
-    float* vxx = a.f[E_VXX];
-    float* vxz = a.f[E_VXZ];
-    float* vzx = a.f[E_VZX];
-    float* vzz = a.f[E_VZZ];
-    // four cells per batch: the batch's global loads are issued before its arithmetic
-    for (int j0 = 0; j0 < kPer; j0 += 4) {
-        float o[4][4], bu[4];
-        long long cc[4];
-        bool ok[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int i = threadIdx.x + (j0 + u) * kThreads, r = i / TZ, z = i - r * TZ;
-            const int gx = t.x0 + r, gz = t.z0 + z;
-            ok[u] = gx < nx && gz < nz;
-            cc[u] = cell(a, t.shot, gx, gz);
-            if (ok[u]) {
-                o[u][0] = vxx[cc[u]]; o[u][1] = vxz[cc[u]]; o[u][2] = vzx[cc[u]]; o[u][3] = vzz[cc[u]];
-                bu[u] = __ldg(a.busg + (long long)min(t.sd.x0 + gx, a.nx_model - 1) * a.mpitch + gz);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            if (!ok[u]) continue;
-            const int i = threadIdx.x + (j0 + u) * kThreads, r = i / TZ, z = i - r * TZ;
-            const int gx = t.x0 + r, gz = t.z0 + z;
-            const long long c = cc[u];
-            const float dtb = fm(a.dt, bu[u]);
-            float n_xx = fa(o[u][0], fm(dtb, rsg<true, 0>(sSxx, r + H, z + HZ, a.a, a.hx)));   // QS:713-720
-            float n_xz = fa(o[u][1], fm(dtb, rsg<false, 0>(sSxz, r + H, z + HZ, a.a, a.hz)));  // QS:722-729
-            n_xx = xs(n_xx, gx, nx, a.npx, tb + 0 * st, tb + 1 * st);
-            n_xz = xs(n_xz, gz, nz, a.npz, tb + 2 * st, tb + 3 * st);
-            float n_zx = fa(o[u][2], fm(dtb, rsg<true, 0>(sSxz, r + H, z + HZ, a.a, a.hx)));   // QS:733-740
-            float n_zz = fa(o[u][3], fm(dtb, rsg<false, 0>(sSzz, r + H, z + HZ, a.a, a.hz)));  // QS:741-748
-            n_zx = xs(n_zx, gx, nx, a.npx, tb + 0 * st, tb + 1 * st);
-            n_zz = xs(n_zz, gz, nz, a.npz, tb + 2 * st, tb + 3 * st);
-            vxx[c] = n_xx; vxz[c] = n_xz; vzx[c] = n_zx; vzz[c] = n_zz;
-        }
+    if (gx <= a.npx || gx >= nx - a.npx - 1) {
+        n_xx = xs(n_xx, gx, nx, a.npx, tb + 0 * st, tb + 1 * st);
+        n_zx = xs(n_zx, gx, nx, a.npx, tb + 0 * st, tb + 1 * st);
     }
+    if (gz <= a.npz || gz >= nz - a.npz - 1) {
+        n_xz = xs(n_xz, gz, nz, a.npz, tb + 2 * st, tb + 3 * st);
+        n_zz = xs(n_zz, gz, nz, a.npz, tb + 2 * st, tb + 3 * st);
+    }
+    a.f[E_VXX][c] = n_xx; a.f[E_VXZ][c] = n_xz; a.f[E_VZX][c] = n_zx; a.f[E_VZZ][c] = n_zz;
+    a.f[E_VX][c] = fa(n_xx, n_xz);  // QS:1273-1291
+    a.f[E_VZ][c] = fa(n_zx, n_zz);
 }
 
-__global__ void __launch_bounds__(kThreads) e_stress_kernel(const __grid_constant__ EArgs a) {
-    __shared__ __align__(16) float sVx[SMEM];
-    __shared__ __align__(16) float sVz[SMEM];
+__global__ void __launch_bounds__(kThreads, kMinS) e_stress_kernel(const __grid_constant__ EArgs a) {
+    extern __shared__ __align__(128) float smem[];
+    const float* sVx = smem;
+    const float* sVz = smem + SMEM;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + 2 * SMEM);
     TileRef t;
-    if (!tile_of(a, t)) return;
-    stage<2>(sVx, a, t, a.f[E_VXX], a.f[E_VXZ], nullptr);  // vx = vxx + vxz (QS:1273-1291)
-    stage<2>(sVz, a, t, a.f[E_VZX], a.f[E_VZZ], nullptr);  // vz = vzx + vzz
-    __syncthreads();
+    const bool on = tile_of(a, t);
+    tile::bar_init(bar);
+    tile::dependency();
+    if (!on) return;
+    if (threadIdx.x == 0) {
+        const int f[2] = {E_VX, E_VZ};
+        stage<2>(smem, bar, a, t, f);
+    }
     const int nx = t.sd.nx, nz = a.nz;
-    const float* tb = a.spg;
-    const int st = a.spg_stride;
     const ShotDev& sd = t.sd;
+    const int r = threadIdx.x / TZ, z = threadIdx.x % TZ, gx = t.x0 + r, gz = t.z0 + z;
+    const bool in = gx < nx && gz < nz;
+    const long long c = cell(a, t.shot, gx, gz);
+    float w[18];  // sxxx sxxz sxxr szzx szzz szzr sxzx sxzz sxzr rxxx rxxz rxxr rzzx rzzz rzzr rxzx rxzz rxzr
+    float q1, q2, q3, m1, m2, m3;
+    if (in) {
+#pragma unroll
+        for (int k = 0; k < 18; k++) w[k] = a.f[E_SXXX + k][c];
+        const long long mi = (long long)min(sd.x0 + gx, a.nx_model - 1) * a.mpitch + gz;
+        q1 = __ldg(a.q1 + mi); q2 = __ldg(a.q2 + mi); q3 = __ldg(a.q3 + mi);
+        m1 = __ldg(a.m1 + mi); m2 = __ldg(a.m2 + mi); m3 = __ldg(a.m3 + mi);
+    }
     const float wav = __ldg(a.wavelets + sd.wav_off + a.step);
-    const float dt = a.dt, f = a.f_mem;
-    for (int j0 = 0; j0 < kPer; j0 += kNB) {
-        float v[kNB][18];
-        float q1[kNB], q2[kNB], q3[kNB], m1[kNB], m2[kNB], m3[kNB];
-        long long cc[kNB];
-        bool ok[kNB];
+    if (!tile::staged(bar, a.err_flag)) return;
+    if (in) {
+        const float dt = a.dt, f = a.f_mem;
+        float d1, d2, d3, d4;
+        rsg_both<1>(sVx, r + H, z + HZ, a.a, a.hx, a.hz, &d1, &d3);  // Dx1 vx, Dz1 vx
+        rsg_both<1>(sVz, r + H, z + HZ, a.a, a.hx, a.hz, &d2, &d4);  // Dx1 vz, Dz1 vz
+        const float rxx = fa(fa(w[9], w[10]), w[11]);   // memory sums of the previous step
+        const float rzz = fa(fa(w[12], w[13]), w[14]);
+        const float rxz = fa(fa(w[15], w[16]), w[17]);
+        // calpstrxx, calpstrzz, calpstrxz (QS:993-1132)
+        w[0] = fa(w[0], fm(dt, fm(q1, d1)));
+        w[1] = fa(w[1], fm(dt, fm(q2, d4)));
+        w[2] = fa(w[2], fm(dt, rxx));
+        w[3] = fa(w[3], fm(dt, fm(q2, d1)));
+        w[4] = fa(w[4], fm(dt, fm(q1, d4)));
+        w[5] = fa(w[5], fm(dt, rzz));
+        w[6] = fa(w[6], fm(dt, fm(q3, d2)));
+        w[7] = fa(w[7], fm(dt, fm(q3, d3)));
+        w[8] = fa(w[8], fm(dt, rxz));
+        // calprxx, calprzz, calprxz (QS:1135-1269)
+        w[9] = fa(w[9], fm(f, fm(m1, d1)));
+        w[10] = fa(w[10], fm(f, fm(m2, d4)));
+        w[11] = fa(w[11], fm(f, rxx));
+        w[12] = fa(w[12], fm(f, fm(m2, d1)));
+        w[13] = fa(w[13], fm(f, fm(m1, d4)));
+        w[14] = fa(w[14], fm(f, rzz));
+        w[15] = fa(w[15], fm(f, fm(m3, d2)));
+        w[16] = fa(w[16], fm(f, fm(m3, d3)));
+        w[17] = fa(w[17], fm(f, rxz));
+        // x parts (0, 3, ...) take the x sponge, z parts (1, 4, ...) the z sponge
+        const float* tb = a.spg;
+        const int st = a.spg_stride;
+        if (gx <= a.npx || gx >= nx - a.npx - 1)
 #pragma unroll
-        for (int u = 0; u < kNB; u++) {
-            const int i = threadIdx.x + (j0 + u) * kThreads, r = i / TZ, z = i - r * TZ;
-            const int gx = t.x0 + r, gz = t.z0 + z;
-            ok[u] = gx < nx && gz < nz;
-            cc[u] = cell(a, t.shot, gx, gz);
-            if (ok[u]) {
+            for (int k = 0; k < 18; k += 3) w[k] = xs(w[k], gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
+        if (gz <= a.npz || gz >= nz - a.npz - 1)
 #pragma unroll
-                for (int k = 0; k < 18; k++) v[u][k] = a.f[E_SXXX + k][cc[u]];
-                const long long mi = (long long)min(sd.x0 + gx, a.nx_model - 1) * a.mpitch + gz;
-                q1[u] = __ldg(a.q1 + mi); q2[u] = __ldg(a.q2 + mi); q3[u] = __ldg(a.q3 + mi);
-                m1[u] = __ldg(a.m1 + mi); m2[u] = __ldg(a.m2 + mi); m3[u] = __ldg(a.m3 + mi);
-            }
+            for (int k = 1; k < 18; k += 3) w[k] = xs(w[k], gz, nz, a.npz, tb + 6 * st, tb + 7 * st);
+        const int bx = gx - sd.stamp_x0, bz = gz - sd.stamp_z0;
+        if (bx >= 0 && bx < sd.stamp_w && bz >= 0 && bz < sd.stamp_h) {  // QS:801, 1384
+            const float src = __fdiv_rn(fm(fm(wav, __ldg(a.stamps + sd.stamp_off + bx * sd.stamp_h + bz)), dt), a.dz2);
+            w[0] = fa(src, w[0]);
+            w[3] = fa(src, w[3]);
         }
 #pragma unroll
-        for (int u = 0; u < kNB; u++) {
-            if (!ok[u]) continue;
-            const int i = threadIdx.x + (j0 + u) * kThreads, r = i / TZ, z = i - r * TZ;
-            const int gx = t.x0 + r, gz = t.z0 + z;
-            const float d1 = rsg<true, 1>(sVx, r + H, z + HZ, a.a, a.hx);   // Dx1 vx
-            const float d2 = rsg<true, 1>(sVz, r + H, z + HZ, a.a, a.hx);   // Dx1 vz
-            const float d3 = rsg<false, 1>(sVx, r + H, z + HZ, a.a, a.hz);  // Dz1 vx
-            const float d4 = rsg<false, 1>(sVz, r + H, z + HZ, a.a, a.hz);  // Dz1 vz
-            float* w = v[u];  // sxxx sxxz sxxr szzx szzz szzr sxzx sxzz sxzr rxxx rxxz rxxr rzzx rzzz rzzr rxzx rxzz rxzr
-            const float rxx = fa(fa(w[9], w[10]), w[11]);   // memory sums of the previous step
-            const float rzz = fa(fa(w[12], w[13]), w[14]);
-            const float rxz = fa(fa(w[15], w[16]), w[17]);
-            float src = 0.0f;
-            const int bx = gx - sd.stamp_x0, bz = gz - sd.stamp_z0;
-            const bool in_stamp = bx >= 0 && bx < sd.stamp_w && bz >= 0 && bz < sd.stamp_h;
-            if (in_stamp)
-                src = __fdiv_rn(fm(fm(wav, __ldg(a.stamps + sd.stamp_off + bx * sd.stamp_h + bz)), dt), a.dz2);
-            // calpstrxx (QS:993-1020)
-            w[0] = xs(fa(w[0], fm(dt, fm(q1[u], d1))), gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
-            w[1] = xs(fa(w[1], fm(dt, fm(q2[u], d4))), gz, nz, a.npz, tb + 6 * st, tb + 7 * st);
-            w[2] = fa(w[2], fm(dt, rxx));
-            if (in_stamp) w[0] = fa(src, w[0]);  // QS:801, 1384
-            // calpstrzz (QS:1023-1050)
-            w[3] = xs(fa(w[3], fm(dt, fm(q2[u], d1))), gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
-            w[4] = xs(fa(w[4], fm(dt, fm(q1[u], d4))), gz, nz, a.npz, tb + 6 * st, tb + 7 * st);
-            w[5] = fa(w[5], fm(dt, rzz));
-            if (in_stamp) w[3] = fa(src, w[3]);
-            // calpstrxz (QS:1053-1132)
-            w[6] = xs(fa(w[6], fm(dt, fm(q3[u], d2))), gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
-            w[7] = xs(fa(w[7], fm(dt, fm(q3[u], d3))), gz, nz, a.npz, tb + 6 * st, tb + 7 * st);
-            w[8] = fa(w[8], fm(dt, rxz));
-            // calprxx, calprzz, calprxz (QS:1135-1269)
-            w[9] = xs(fa(w[9], fm(f, fm(m1[u], d1))), gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
-            w[10] = xs(fa(w[10], fm(f, fm(m2[u], d4))), gz, nz, a.npz, tb + 6 * st, tb + 7 * st);
-            w[11] = fa(w[11], fm(f, rxx));
-            w[12] = xs(fa(w[12], fm(f, fm(m2[u], d1))), gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
-            w[13] = xs(fa(w[13], fm(f, fm(m1[u], d4))), gz, nz, a.npz, tb + 6 * st, tb + 7 * st);
-            w[14] = fa(w[14], fm(f, rzz));
-            w[15] = xs(fa(w[15], fm(f, fm(m3[u], d2))), gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
-            w[16] = xs(fa(w[16], fm(f, fm(m3[u], d3))), gz, nz, a.npz, tb + 6 * st, tb + 7 * st);
-            w[17] = fa(w[17], fm(f, rxz));
-#pragma unroll
-            for (int k = 0; k < 18; k++) a.f[E_SXXX + k][cc[u]] = w[k];
-        }
+        for (int k = 0; k < 18; k++) a.f[E_SXXX + k][c] = w[k];
+        a.f[E_SXX][c] = fa(fa(w[0], w[1]), w[2]);  // QS:1294-1337
+        a.f[E_SZZ][c] = fa(fa(w[3], w[4]), w[5]);
+        a.f[E_SXZ][c] = fa(fa(w[6], w[7]), w[8]);
     }
     // receivers: record1 = strzz, record2 = strxx after the step (QM:452-459)
     const int* trp = a.tile_rec_ptr + sd.tile_rec_base + t.tile;
@@ -254,26 +263,33 @@ __global__ void __launch_bounds__(kThreads) e_stress_kernel(const __grid_constan
         __syncthreads();
         for (int j = rb + threadIdx.x; j < re; j += kThreads) {
             const int ridx = a.tile_rec_idx[j];
-            const long long c = cell(a, t.shot, a.rec_x[sd.rec_list + ridx], a.rec_z[sd.rec_list + ridx]);
+            const int x = a.rec_x[sd.rec_list + ridx];
+            if (x < t.x0 || x >= t.x0 + TC) continue;  // another CTA of the 64 x 64 tile holds it
+            const long long c = cell(a, t.shot, x, a.rec_z[sd.rec_list + ridx]);
             const long long o = sd.rec_base + (long long)a.step * sd.nrec + ridx;
-            a.records[o] = fa(fa(a.f[E_SZZX][c], a.f[E_SZZZ][c]), a.f[E_SZZR][c]);
-            a.records2[o] = fa(fa(a.f[E_SXXX][c], a.f[E_SXXZ][c]), a.f[E_SXXR][c]);
+            a.records[o] = a.f[E_SZZ][c];
+            a.records2[o] = a.f[E_SXX][c];
         }
     }
 }
 
 }  // namespace
 
+void viscoel2d_box(int box[2]) {
+    box[0] = SW;
+    box[1] = SROWS;
+}
+
 cudaError_t viscoel2d_launch_step(const EArgs& a, int active, cudaStream_t st) {
-    dim3 grid(a.L.ntx * a.L.ntz, active);
-    const size_t smem = sizeof(float) * 3 * SMEM;
-    static bool attr[kMaxDevices] = {};
-    if (cudaError_t e = smem_attr_once((const void*)e_velocity_kernel, (int)smem, attr)) return e;
-    e_velocity_kernel<<<grid, kThreads, smem, st>>>(a);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    e_stress_kernel<<<grid, kThreads, 0, st>>>(a);
-    return cudaGetLastError();
+    const dim3 grid(a.L.ntx * (TX / TC) * a.L.ntz, active);
+    const int sv = (int)sizeof(float) * (3 * SMEM + 4), ss = (int)sizeof(float) * (2 * SMEM + 4);
+    const void* kv = (const void*)e_velocity_kernel;
+    const void* ks = (const void*)e_stress_kernel;
+    static bool attr0[kMaxDevices] = {}, attr1[kMaxDevices] = {};
+    if (cudaError_t e = smem_attr_once(kv, sv, attr0)) return e;
+    if (cudaError_t e = smem_attr_once(ks, ss, attr1)) return e;
+    if (cudaError_t e = tile::launch(kv, grid, kThreads, sv, st, a)) return e;
+    return tile::launch(ks, grid, kThreads, ss, st, a);
 }
 
 // QS:434-469 (density averaged in place, then buoyancy) and QS:473-551 (Blanch's tau for P and S),
