@@ -2001,6 +2001,22 @@ int run_gradient_3d(sfd_ctx* ctx, const float* obs, float* misfit, float* grad_v
 
 }  // namespace
 
+namespace sfd {
+
+bool encode_map3(CUtensorMap* m, float* base, long long d0, long long d1, long long d2, long long s1, long long s2, int b0,
+                 int b1) {
+    auto enc = tensor_map_encoder();
+    if (!enc) return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)d0, (cuuint64_t)d1, (cuuint64_t)d2};
+    const cuuint64_t strides[2] = {(cuuint64_t)s1 * 4, (cuuint64_t)s2 * 4};
+    const cuuint32_t bdim[3] = {(cuuint32_t)b0, (cuuint32_t)b1, 1}, estr[3] = {1, 1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, bdim, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+}  // namespace sfd
+
 extern "C" {
 
 int sfd_abi_version(void) { return SFD_ABI_VERSION; }

@@ -35,6 +35,10 @@ inline int num_sms() {
         return 148;
     return n;
 }
+// 3-D float32 tensor map over dense rows: extents d0 (contiguous), d1, d2, strides of d1 and d2 in
+// floats, box b0 x b1 x 1 (api.cu); false if the driver refuses.
+bool encode_map3(CUtensorMap* m, float* base, long long d0, long long d1, long long d2, long long s1, long long s2, int b0,
+                 int b1);
 // Both 2-D acoustic step kernels work on the same 64 x 64 tiles, so they share the field
 // layout and the per-tile receiver tables.
 constexpr int kTileX = 64;

@@ -69,8 +69,7 @@ __device__ __forceinline__ void dependency() {
 }
 
 // launch with the dependency() of the kernel above as a programmatic edge
-template <class Args>
-inline cudaError_t launch(const void* fn, dim3 grid, int threads, size_t smem, cudaStream_t st, const Args& a) {
+inline cudaError_t launch(const void* fn, dim3 grid, int threads, size_t smem, cudaStream_t st, void** args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
@@ -81,8 +80,12 @@ inline cudaError_t launch(const void* fn, dim3 grid, int threads, size_t smem, c
     at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    void* args[] = {const_cast<Args*>(&a)};
     return cudaLaunchKernelExC(&cfg, fn, args);
+}
+template <class Args>
+inline cudaError_t launch(const void* fn, dim3 grid, int threads, size_t smem, cudaStream_t st, const Args& a) {
+    void* args[] = {const_cast<Args*>(&a)};
+    return launch(fn, grid, threads, smem, st, args);
 }
 
 }  // namespace tile

@@ -5,17 +5,25 @@
 // Per time step the reference calls extrapolation_one_step_1 (new u from the current u and q,
 // VS:432-960) and then extrapolation_one_step_2 (new q from the current u and q, VS:965-1258).
 // Neither reads what the other writes -- step 2 takes the current u, not the new one -- so one
-// kernel does both.  A CTA stages the current u and q of a 32 x 8 tile with its 5-cell halo in
-// shared memory; each thread owns one cell of one shot, forms the stencil sums that both
-// subroutines share once, updates the split PML fields of its cell in place and writes the new
-// u and q into the slots of the old ones.  All global loads of a thread are issued before the
-// tile barrier, and the registers are bounded for five CTAs per SM (the kernel is bound by the
-// latency of those loads and of the IEEE divisions the reference order requires).  The
-// operation order is the reference's as written, every multiply, add and divide rounded
-// separately (__fmul_rn, __fadd_rn, __fdiv_rn, __fsqrt_rn), so the records equal the FP32
-// restatement in oracle/vti_oracle.cpp bit for bit.  A one-thread-per-shot kernel adds the source
-// to the current u before each step (VM:420-424, 468-472); the receiver row is written by the
-// step kernel's threads on that row.
+// kernel does both, updating the split PML fields of its cells in place and writing the new u and q
+// into the slots of the old ones.  With SFD_EXACT the operation order is the reference's as written,
+// every multiply, add and divide rounded separately (__fmul_rn, __fadd_rn, __fdiv_rn, __fsqrt_rn),
+// so the records equal the FP32 restatement in oracle/vti_oracle.cpp bit for bit.  The default mode
+// divides by grid constants through rounded reciprocals and takes the common factors h^2 and h out
+// of the PML recurrences, leaving one division per PML cell.
+//
+// Bound: memory (36 B a cell inside, 44 to 76 B more in the PML strips) and its latency.  A CTA owns
+// 64 x 2 cells, one per thread; u with a halo of 5 rows and 8 columns and q with a halo of 8 columns
+// (q is only differentiated along x) arrive by two TMA boxes while each thread loads its cell's model
+// and old u, q.  Addresses are 32-bit offsets from the shot's slab, formed on the host: with pointer
+// arithmetic in the threads integer instructions were more than half of all.  16 shots of 698 x 348,
+// 740 steps: 64 ms (default) and 83 ms (exact) with 32 x 8 tiles staged through registers; now 37 and
+// 63 ms.  Tiles of 4 and 8 rows 39 and 49 ms; one vector of four cells per thread on 64 x 8 tiles, whose
+// PML branch needs 160 registers, 44 ms.
+//
+// A one-thread-per-shot kernel adds the source to the current u before each step (VM:420-424,
+// 468-472); the receiver row is written by the step kernel's threads on that row.  The per-shot model
+// windows are built on the device from one copy of the model.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -24,252 +32,241 @@
 #include <cstring>
 #include <vector>
 
-#include "seisfd.h"
+#include "sfd_internal.h"
+#include "tile_stage.cuh"
 
 namespace {
 
-constexpr int kBX = 32, kBZ = 8;             // threads per CTA (x, z)
-constexpr int kTX = 32, kH = 5;               // cells per CTA tile in x, stencil halo
-constexpr int kSX = kTX + 2 * kH;
-// One cell per thread and registers bounded for five CTAs per SM.  Measured on the .par geometry
-// (64 shots of 348 x 698): 1, 2 and 4 cells per thread 36.9, 35.3 and 28.6 Gpts/s at four CTAs per
-// SM; one cell at five and six CTAs per SM 39.3 and 39.2 Gpts/s (the latter spills).
-constexpr int kCPT = 1, kMinBlocks = 5;
+constexpr int kTX = 64, kTZ = 2, kH = 5;      // cells of a CTA's tile (x, z), stencil halo
+constexpr int kThreads = kTX * kTZ;           // one cell per thread
+constexpr int kGX = 8;                        // ghost columns: x halo rounded to 16 bytes
+constexpr int kSX = kTX + 2 * kGX;            // staged columns
+constexpr int kMinBlocks = 10;
 
 // E = true: every operation rounded separately in the reference's order (bit-exact with the
-// restatement); E = false: multiplies and adds may contract into FMAs and divisions are the
-// approximate __fdividef (records within relative L2 1e-5 of the restatement)
+// restatement); E = false: multiplies and adds may contract into FMAs (records within relative L2
+// 1e-5 of the restatement)
 template <bool E> __device__ __forceinline__ float fm(float a, float b) { return E ? __fmul_rn(a, b) : a * b; }
 template <bool E> __device__ __forceinline__ float fa(float a, float b) { return E ? __fadd_rn(a, b) : a + b; }
 template <bool E> __device__ __forceinline__ float fs(float a, float b) { return E ? __fsub_rn(a, b) : a - b; }
-template <bool E> __device__ __forceinline__ float fd(float a, float b) { return E ? __fdiv_rn(a, b) : __fdividef(a, b); }
-template <bool E> __device__ __forceinline__ float fsq(float a) { return E ? __fsqrt_rn(a) : sqrtf(a); }
+__device__ __forceinline__ float fd(float a, float b) { return __fdiv_rn(a, b); }
+__device__ __forceinline__ float fsq(float a) { return __fsqrt_rn(a); }
 
 struct VtiDev {
-    // per shot: fields u[2], q[2] (pitch x (nz + 10), cell (i, j) 1-based at (j+4)*pitch + i+4),
-    // model vz, eps, delta in the same layout, x-strip PML fields (nxl+nxr) x nz of u (4 pairs)
-    // and q (3 pairs), z-strip PML fields nx x (nzu+nzd) of u (4 pairs)
+    CUtensorMap tm_u[2], tm_q[2];  // u and q slots (column, row, shot), boxes kSX x (kTZ + 10) and kSX x kTZ
+    int* err_flag;                 // set to 1 by a CTA whose bounded wait ran out
+    // per shot: fields u[2], q[2] and the model vz, eps, delta on rows of `pitch` floats, cell (i, j)
+    // (0-based) at (j + 5) * pitch + i + 8, all zero outside the grid; then the x-strip PML fields
+    // (nz rows of nxl + nxr floats; u: four pairs, q: three) and the z-strip ones (nzu + nzd rows of
+    // nx; u: four pairs)
     float* base;
     long long field, shot_stride;  // floats per field slab, per shot
     long long xs, zs;              // floats per x strip, per z strip
     int pitch, nx, nz, nxl, nxr, nzu, nzd, range, nt;
     float dx, dz, dt, L;
+    float rdx2, rdz2, rdx, dt2;    // default mode: 1 / dx^2, 1 / dz^2, 1 / dx, dt^2
+    float cd[4], cdd[4];           // ... damping d = speed cd idx^2 and its derivative speed cdd idx (l, r, u, d)
     float cE[5], c1[5];    // coefficient_2nd(10) (fd_coe and fd_coe_pml_2nd alike), coefficient_1st
-    const int* src;        // per shot: source cell i, j
-    const int* rrow;       // per shot: receiver row and whether it is the row-6 fallback
+    const int* src;        // per shot: source cell i, j (1-based)
+    const int* rrow;       // per shot: receiver row (1-based) and whether it is the row-6 fallback
     float* records;        // [shot][range][nt]
 };
 
-// one shot's arrays, by arithmetic on VtiDev::base (no pointer tables: the slot indices are
-// run-time values)
-struct VtiSlab {
-    float* p;
-    long long field, xs, zs;
-    __device__ float* u(int b) const { return p + b * field; }
-    __device__ float* q(int b) const { return p + (2 + b) * field; }
-    __device__ const float* vz() const { return p + 4 * field; }
-    __device__ const float* ep() const { return p + 5 * field; }
-    __device__ const float* de() const { return p + 6 * field; }
-    __device__ float* ux(int k, int b) const { return p + 7 * field + (2 * k + b) * xs; }
-    __device__ float* qx(int k, int b) const { return p + 7 * field + (8 + 2 * k + b) * xs; }
-    __device__ float* uz(int k, int b) const { return p + 7 * field + 14 * xs + (2 * k + b) * zs; }
+// Offsets (floats) of one step's arrays in a shot's slab: c = the current slots, o = the old ones that
+// take the new values.  Formed on the host, so that a thread's address is one 32-bit add.
+struct VtiOff {
+    unsigned uc, uo, qc, qo, vz, ep, de;
+    unsigned uxc[4], uxo[4], qxc[3], qxo[3], uzc[4], uzo[4];  // a1 a2 t2 a3
 };
 
-__device__ __forceinline__ VtiSlab slab(const VtiDev& a, int s) {
-    return VtiSlab{a.base + (long long)s * a.shot_stride, a.field, a.xs, a.zs};
-}
+__device__ __forceinline__ unsigned cell(const VtiDev& a, int i, int j) { return (j + kH) * a.pitch + i + kGX; }
 
 // second-derivative sum of VS:511-525: (c1 (f+1 + f-1 - 2 f0) + ... + c5 (...)) / h**2
 template <bool E>
-__device__ __forceinline__ float d2(const float* f, int c, int st, const float* cf, float h) {
-    const float two_f0 = fm<E>(2.0f, f[c]);
-    float s = fm<E>(cf[0], fs<E>(fa<E>(f[c + st], f[c - st]), two_f0));
+__device__ __forceinline__ float d2(const float* f, int st, const float* cf, float h, float rh2) {
+    const float two_f0 = fm<E>(2.0f, f[0]);
+    float s = fm<E>(cf[0], fs<E>(fa<E>(f[st], f[-st]), two_f0));
 #pragma unroll
-    for (int m = 2; m <= 5; m++) s = fa<E>(s, fm<E>(cf[m - 1], fs<E>(fa<E>(f[c + m * st], f[c - m * st]), two_f0)));
-    return fd<E>(s, fm<E>(h, h));
+    for (int m = 2; m <= 5; m++) s = fa<E>(s, fm<E>(cf[m - 1], fs<E>(fa<E>(f[m * st], f[-m * st]), two_f0)));
+    return E ? fd(s, fm<E>(h, h)) : s * rh2;
 }
 // first-derivative sum of VS:567-578: (p1 (f+1 - f-1) + ... + p5 (...)) / h
 template <bool E>
-__device__ __forceinline__ float d1(const float* f, int c, int st, const float* cf, float h) {
-    float s = fm<E>(cf[0], fs<E>(f[c + st], f[c - st]));
+__device__ __forceinline__ float d1(const float* f, int st, const float* cf, float h, float rh) {
+    float s = fm<E>(cf[0], fs<E>(f[st], f[-st]));
 #pragma unroll
-    for (int m = 2; m <= 5; m++) s = fa<E>(s, fm<E>(cf[m - 1], fs<E>(f[c + m * st], f[c - m * st])));
-    return fd<E>(s, h);
+    for (int m = 2; m <= 5; m++) s = fa<E>(s, fm<E>(cf[m - 1], fs<E>(f[m * st], f[-m * st])));
+    return E ? fd(s, h) : s * rh;
 }
 
 // the split PML recurrences of one boundary cell (VS:651-663, 840-858): a1 (second-derivative
-// part), t2 (first-derivative part with the damping derivative), a2; k2s2 = speed^2 dt^2 (s2 h^2)
-// and k2dd = speed^2 dt^2 dd (s1 h), both formed by the caller in the reference's order
+// part), t2 (first-derivative part with the damping derivative), a2; a1, t2 hold the old values and
+// a1o, t2o, a2o the current ones; k2 = speed^2 dt^2, s2 and s1 the second and first derivative
 template <bool E>
-__device__ __forceinline__ void pml_cell(float d, float dt, float h, float* a1, const float* a1o, float* t2,
-                                         const float* t2o, float* a2, const float* a2o, long long x, float k2s2,
-                                         float k2dd) {
-    const float h2 = fm<E>(h, h);
-    const float d2dt = fm<E>(fm<E>(2.0f, d), dt);
-    const float P = fs<E>(fa<E>(fm<E>(2.0f, h2), fm<E>(d2dt, h2)), fm<E>(fm<E>(fm<E>(d, d), h2), fm<E>(dt, dt)));
-    const float Den = fa<E>(h2, fm<E>(d2dt, h2));
-    const float n1 = fd<E>(fa<E>(fs<E>(fm<E>(a1o[x], P), fm<E>(h2, a1[x])), k2s2), Den);
-    const float P2 = fs<E>(fa<E>(fm<E>(2.0f, h), fm<E>(d2dt, h)), fm<E>(fm<E>(fm<E>(dt, dt), h), fm<E>(d, d)));
-    const float Den2 = fa<E>(h, fm<E>(d2dt, h));
-    const float nt = fd<E>(fs<E>(fs<E>(fm<E>(t2o[x], P2), fm<E>(h, t2[x])), k2dd), Den2);
-    a1[x] = n1;
-    t2[x] = nt;
-    a2[x] = fa<E>(fm<E>(a2o[x], fs<E>(1.0f, fm<E>(d, dt))), fm<E>(nt, dt));
+__device__ __forceinline__ void pml_cell(float d, float dd, float dt, float h, float& a1, float a1o, float& t2,
+                                         float t2o, float& a2, float a2o, float k2, float s2, float s1) {
+    if (E) {
+        const float k2s2 = fm<E>(k2, fm<E>(s2, fm<E>(h, h))), k2dd = fm<E>(fm<E>(k2, dd), fm<E>(s1, h));
+        const float h2 = fm<E>(h, h);
+        const float d2dt = fm<E>(fm<E>(2.0f, d), dt);
+        const float P = fs<E>(fa<E>(fm<E>(2.0f, h2), fm<E>(d2dt, h2)), fm<E>(fm<E>(fm<E>(d, d), h2), fm<E>(dt, dt)));
+        const float Den = fa<E>(h2, fm<E>(d2dt, h2));
+        a1 = fd(fa<E>(fs<E>(fm<E>(a1o, P), fm<E>(h2, a1)), k2s2), Den);
+        const float P2 = fs<E>(fa<E>(fm<E>(2.0f, h), fm<E>(d2dt, h)), fm<E>(fm<E>(fm<E>(dt, dt), h), fm<E>(d, d)));
+        const float Den2 = fa<E>(h, fm<E>(d2dt, h));
+        t2 = fd(fs<E>(fs<E>(fm<E>(t2o, P2), fm<E>(h, t2)), k2dd), Den2);
+        a2 = fa<E>(fm<E>(a2o, fs<E>(1.0f, fm<E>(d, dt))), fm<E>(t2, dt));
+    } else {  // the same with h^2 and h taken out of the numerators and denominators
+        const float t = d * dt, q = __frcp_rn(1.0f + 2.0f * t), P = 2.0f + 2.0f * t - t * t;
+        a1 = (P * a1o - a1 + k2 * s2) * q;
+        t2 = (P * t2o - t2 - k2 * dd * s1) * q;
+        a2 = a2o * (1.0f - t) + t2 * dt;
+    }
 }
 
-__global__ void vti_inject_kernel(VtiDev a, int cu, float w) {
+__global__ void vti_inject_kernel(const __grid_constant__ VtiDev a, unsigned uc, float w) {
+    sfd::tile::dependency();
     const int s = blockIdx.x;
     if (threadIdx.x != 0) return;
-    const VtiSlab p = slab(a, s);
-    const long long c = (long long)(a.src[2 * s + 1] + 4) * a.pitch + (a.src[2 * s] + 4);
-    p.u(cu)[c] = __fadd_rn(p.u(cu)[c], w);
+    float* u = a.base + (long long)s * a.shot_stride + uc + cell(a, a.src[2 * s] - 1, a.src[2 * s + 1] - 1);
+    *u = __fadd_rn(*u, w);
 }
 
-// one cell (i, j) of shot s: U and Q are the shared-memory tiles of the current u and q, sc the
-// cell's tile index, P the tile's row stride; c indexes the cell in the field layout
-// (v, de, ep: the cell's model; uo, qo: its old u and q, loaded by the caller ahead of time)
+// The window of every shot (get_currshot_parameters, VS:268-338, and VM:405-408) from the model
+// [nx_v][nz_v]: vz with replicated edges, epsilon and delta only inside the window and below the
+// rows nsz0 + nzu + 6.  win: per shot xmin and nsz0.
+__global__ void vti_window_kernel(const __grid_constant__ VtiDev a, const float* vz, const float* ep, const float* de,
+                                  const int* win, int nx_v, int nz_v) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, s = blockIdx.z;
+    if (i >= a.nx) return;
+    float* P = a.base + (long long)s * a.shot_stride + 4 * a.field;  // vz, eps, delta
+    const int il = min(max(i - a.nxl, 0), a.range - 1), jl = min(max(j - a.nzu, 0), nz_v - 1);
+    const long long m = (long long)min(max(il + win[2 * s], 0), nx_v - 1) * nz_v + jl;
+    const bool in = il == i - a.nxl && jl == j - a.nzu && j >= win[2 * s + 1] + a.nzu + 6;
+    const unsigned c = cell(a, i, j);
+    P[c] = vz[m];
+    P[a.field + c] = in ? ep[m] : 0.0f;
+    P[2 * a.field + c] = in ? de[m] : 0.0f;
+}
+
 template <bool E>
-__device__ __forceinline__ void vti_cell(const VtiDev& a, const VtiSlab& p, const float* U, const float* Q, int sc,
-                                         int P, int i, int j, int s, int cu, int iit, float v, float de, float ep,
-                                         float uo, float qo) {
-    const int ou = 1 - cu;
-    const int c = sc;
-    const long long g = (long long)(j + 4) * a.pitch + (i + 4);
+__global__ void __launch_bounds__(kThreads, kMinBlocks) vti_step_kernel(const __grid_constant__ VtiDev a,
+                                                                        const __grid_constant__ VtiOff o, int cu,
+                                                                        int iit) {
+    __shared__ __align__(128) float sU[(kTZ + 2 * kH) * kSX];
+    __shared__ __align__(128) float sQ[kTZ * kSX];
+    __shared__ uint64_t bar;
+    const int s = blockIdx.z, tid = threadIdx.x, tx = tid % kTX, ty = tid / kTX;
+    const int i0 = blockIdx.x * kTX, j0 = blockIdx.y * kTZ;
+    float* P = a.base + (long long)s * a.shot_stride;
+    const int gi = i0 + tx, gj = j0 + ty;  // 0-based
+    const bool in = gi < a.nx && gj < a.nz;
+    const unsigned g = cell(a, gi, gj);
+    sfd::tile::bar_init(&bar);
+    sfd::tile::dependency();
+    // u: rows j0 - 5 .. j0 + kTZ + 4, q: the tile's rows, columns i0 - 8 .. i0 + 71 (allocation columns
+    // from i0, a multiple of 64, and rows from j0; rows past the allocation read as zero)
+    if (tid == 0) {
+        sfd::tile::expect(&bar, 4u * (2 * kTZ + 2 * kH) * kSX);
+        sfd::tile::box(sU, &a.tm_u[cu], i0, j0, s, &bar);
+        sfd::tile::box(sQ, &a.tm_q[cu], i0, j0 + kH, s, &bar);
+    }
+    float v = 0.0f, de = 0.0f, ep = 0.0f, uo = 0.0f, qo = 0.0f;
+    if (in) {
+        v = P[o.vz + g];
+        de = P[o.de + g];
+        ep = P[o.ep + g];
+        uo = P[o.uo + g];
+        qo = P[o.qo + g];
+    }
+    if (!sfd::tile::staged(&bar, a.err_flag) || !in) return;
     const float dt = a.dt, dx = a.dx, dz = a.dz, L = a.L;
     const int nx = a.nx, nz = a.nz, nxl = a.nxl, nxr = a.nxr, nzu = a.nzu, nzd = a.nzd;
-    const bool xin = i > nxl && i < nx - nxr + 1;
-    float un, qn;
-
+    const float* U = sU + (ty + kH) * kSX + kGX + tx;  // the cell in the staged u and q
+    const float* Q = sQ + ty * kSX + kGX + tx;
     // The sums of the current u and q that both subroutines form: coefficient_2nd(10) is both
     // fd_coe and fd_coe_pml_2nd, the x sums of u and q appear in step 1 and step 2 (added in the
     // other order there, which IEEE addition does not distinguish), the z sum of u in every
     // region of step 1.  Each is formed once.
-    const float sxu = d2<E>(U, c, 1, a.cE, dx), sxq = d2<E>(Q, c, 1, a.cE, dx), szu = d2<E>(U, c, P, a.cE, dz);
-
-    // ---- extrapolation_one_step_1 (VS:432-960): new u; step 2's PML cells share its terms ----
-    if (xin && j > nzu && j < nz - nzd + 1) {
-        un = fa<E>(fs<E>(fm<E>(2.0f, U[c]), uo), fm<E>(fm<E>(fm<E>(dt, dt), fm<E>(v, v)), fa<E>(fm<E>(fa<E>(1.0f, fm<E>(2.0f, de)), fa<E>(sxu, sxq)), szu)));
-    } else if (!xin) {
-        const bool left = i <= nxl;
-        const float vn = fm<E>(v, fsq<E>(fa<E>(1.0f, fm<E>(2.0f, de))));
-        const float vx = fm<E>(v, fsq<E>(fa<E>(1.0f, fm<E>(2.0f, ep))));
-        const float s1 = fa<E>(d1<E>(U, c, 1, a.c1, dx), d1<E>(Q, c, 1, a.c1, dx));
-        const float s2 = fa<E>(sxu, sxq);
-        const float axis = fm<E>((float)(left ? i - (nxl + 1) : i - (nx - nxr)), dx);
-        const float thick = fm<E>((float)(left ? nxl : nxr), dx);
-        const int is = left ? i : i - (nx - nxr) + nxl;
-        const float A = fd<E>(fm<E>(3.0f, vx), fm<E>(2.0f, thick));
-        const float d = fm<E>(fm<E>(A, fm<E>(fd<E>(axis, thick), fd<E>(axis, thick))), L);
-        const float dd = fm<E>(fm<E>(A, fd<E>(fm<E>(2.0f, axis), fm<E>(thick, thick))), L);
-        const long long x = (long long)(j - 1) * (nxl + nxr) + (is - 1);
-        const float k2 = fm<E>(fm<E>(vn, vn), fm<E>(dt, dt));
-        pml_cell<E>(d, dt, dx, p.ux(0, ou), p.ux(0, cu), p.ux(2, ou), p.ux(2, cu), p.ux(1, ou), p.ux(1, cu), x,
-                 fm<E>(k2, fm<E>(s2, fm<E>(dx, dx))), fm<E>(fm<E>(k2, dd), fm<E>(s1, dx)));
-        float* a3 = p.ux(3, ou);
-        const float* a3o = p.ux(3, cu);
-        const float n3 = fa<E>(fs<E>(fm<E>(2.0f, a3o[x]), a3[x]), fd<E>(fm<E>(fm<E>(fm<E>(v, v), fm<E>(dt, dt)), fm<E>(szu, fm<E>(dz, dz))), fm<E>(dz, dz)));
-        a3[x] = n3;
-        un = fa<E>(fa<E>(p.ux(0, ou)[x], p.ux(1, ou)[x]), n3);
-        // extrapolation_one_step_2's PML cell (VS:1073-1150): the same s1, s2, d and dd
-        const float kq = fm<E>(fs<E>(fm<E>(vx, vx), fm<E>(vn, vn)), fm<E>(dt, dt));
-        pml_cell<E>(d, dt, dx, p.qx(0, ou), p.qx(0, cu), p.qx(2, ou), p.qx(2, cu), p.qx(1, ou), p.qx(1, cu), x,
-                 fm<E>(kq, fm<E>(s2, fm<E>(dx, dx))), fm<E>(fm<E>(kq, dd), fm<E>(s1, dx)));
-        qn = fa<E>(p.qx(0, ou)[x], p.qx(1, ou)[x]);
-    } else {
-        const bool top = j <= nzu;
-        const float vn = fm<E>(v, fsq<E>(fa<E>(1.0f, fm<E>(2.0f, de))));
-        const float sz1 = d1<E>(U, c, P, a.c1, dx);  // divided by dx as written (VS:796, 880)
-        const float axis = fm<E>((float)(top ? j - (nzu + 1) : j - (nz - nzd)), dz);
-        const float thick = fm<E>((float)(top ? nzu : nzd), dz);
-        const int js = top ? j : j - (nz - nzd) + nzu;
-        const float A = fd<E>(fm<E>(3.0f, v), fm<E>(2.0f, thick));
-        const float d = fm<E>(fm<E>(A, fm<E>(fd<E>(axis, thick), fd<E>(axis, thick))), L);
-        const float dd = fm<E>(fm<E>(A, fd<E>(fm<E>(2.0f, axis), fm<E>(thick, thick))), L);
-        const long long z = (long long)(js - 1) * nx + (i - 1);
-        const float k2 = fm<E>(fm<E>(v, v), fm<E>(dt, dt));
-        pml_cell<E>(d, dt, dz, p.uz(0, ou), p.uz(0, cu), p.uz(2, ou), p.uz(2, cu), p.uz(1, ou), p.uz(1, cu), z,
-                 fm<E>(k2, fm<E>(szu, fm<E>(dz, dz))), fm<E>(fm<E>(k2, dd), fm<E>(sz1, dz)));
-        float* a3 = p.uz(3, ou);
-        const float* a3o = p.uz(3, cu);
-        const float n3 = fa<E>(fs<E>(fm<E>(2.0f, a3o[z]), a3[z]), fm<E>(fm<E>(fm<E>(vn, vn), fm<E>(dt, dt)), fa<E>(sxu, sxq)));
-        a3[z] = n3;
-        un = fa<E>(fa<E>(p.uz(0, ou)[z], p.uz(1, ou)[z]), n3);
+    const float s2 = fa<E>(d2<E>(U, 1, a.cE, dx, a.rdx2), d2<E>(Q, 1, a.cE, dx, a.rdx2));
+    const float szu = d2<E>(U, kSX, a.cE, dz, a.rdz2);
+    const bool xin = gi >= nxl && gi < nx - nxr;
+    float un, qn;
+    if (xin) {  // extrapolation_one_step_1 (VS:432-960) and _2 (VS:965-1072) inside
+        const float dv = E ? fm<E>(fm<E>(dt, dt), fm<E>(v, v)) : a.dt2 * (v * v);
+        un = fa<E>(fs<E>(fm<E>(2.0f, U[0]), uo),
+                   fm<E>(dv, fa<E>(fm<E>(fa<E>(1.0f, fm<E>(2.0f, de)), s2), szu)));
+        qn = fa<E>(fs<E>(fm<E>(2.0f, Q[0]), qo), fm<E>(dv, fm<E>(fm<E>(2.0f, fs<E>(ep, de)), s2)));
+        if (gj < nzu || gj >= nz - nzd) {  // the top and bottom PML
+            const bool top = gj < nzu;
+            const int js = top ? gj : gj - (nz - nzd) + nzu, idx = top ? gj + 1 - (nzu + 1) : gj + 1 - (nz - nzd);
+            const unsigned z = js * nx + gi;
+            const float a1o = P[o.uzc[0] + z], a2o = P[o.uzc[1] + z], t2o = P[o.uzc[2] + z], a3o = P[o.uzc[3] + z];
+            float a1 = P[o.uzo[0] + z], t2 = P[o.uzo[2] + z], a3 = P[o.uzo[3] + z], a2;
+            const float sz1 = d1<E>(U, kSX, a.c1, dx, a.rdx);  // divided by dx as written (VS:796, 880)
+            float d, dd, k2, n3;
+            if (E) {
+                const float vn = fm<E>(v, fsq(fa<E>(1.0f, fm<E>(2.0f, de))));
+                const float axis = fm<E>((float)idx, dz), thick = fm<E>((float)(top ? nzu : nzd), dz);
+                const float A = fd(fm<E>(3.0f, v), fm<E>(2.0f, thick));
+                d = fm<E>(fm<E>(A, fm<E>(fd(axis, thick), fd(axis, thick))), L);
+                dd = fm<E>(fm<E>(A, fd(fm<E>(2.0f, axis), fm<E>(thick, thick))), L);
+                k2 = fm<E>(fm<E>(v, v), fm<E>(dt, dt));
+                n3 = fm<E>(fm<E>(fm<E>(vn, vn), fm<E>(dt, dt)), s2);
+            } else {
+                const float fi = (float)idx;
+                d = v * (a.cd[top ? 2 : 3] * (fi * fi));
+                dd = v * (a.cdd[top ? 2 : 3] * fi);
+                k2 = dv;
+                n3 = k2 * (1.0f + 2.0f * de) * s2;
+            }
+            pml_cell<E>(d, dd, dt, dz, a1, a1o, t2, t2o, a2, a2o, k2, szu, sz1);
+            a3 = fa<E>(fs<E>(fm<E>(2.0f, a3o), a3), n3);
+            un = fa<E>(fa<E>(a1, a2), a3);
+            P[o.uzo[0] + z] = a1; P[o.uzo[1] + z] = a2; P[o.uzo[2] + z] = t2; P[o.uzo[3] + z] = a3;
+        }
+    } else {  // the left and right PML (all rows): u, then q (VS:1073-1150) with the same s1, s2, d, dd
+        const bool left = gi < nxl;
+        const int is = left ? gi : gi - (nx - nxr) + nxl, idx = left ? gi + 1 - (nxl + 1) : gi + 1 - (nx - nxr);
+        const unsigned x = gj * (nxl + nxr) + is;
+        const float a1o = P[o.uxc[0] + x], a2o = P[o.uxc[1] + x], t2o = P[o.uxc[2] + x], a3o = P[o.uxc[3] + x];
+        const float b1o = P[o.qxc[0] + x], b2o = P[o.qxc[1] + x], r2o = P[o.qxc[2] + x];
+        float a1 = P[o.uxo[0] + x], t2 = P[o.uxo[2] + x], a3 = P[o.uxo[3] + x];
+        float b1 = P[o.qxo[0] + x], r2 = P[o.qxo[2] + x], a2, b2;
+        const float s1 = fa<E>(d1<E>(U, 1, a.c1, dx, a.rdx), d1<E>(Q, 1, a.c1, dx, a.rdx));
+        float d, dd, kn, kq, n3;
+        if (E) {
+            const float vn = fm<E>(v, fsq(fa<E>(1.0f, fm<E>(2.0f, de))));
+            const float vx = fm<E>(v, fsq(fa<E>(1.0f, fm<E>(2.0f, ep))));
+            const float axis = fm<E>((float)idx, dx), thick = fm<E>((float)(left ? nxl : nxr), dx);
+            const float A = fd(fm<E>(3.0f, vx), fm<E>(2.0f, thick));
+            d = fm<E>(fm<E>(A, fm<E>(fd(axis, thick), fd(axis, thick))), L);
+            dd = fm<E>(fm<E>(A, fd(fm<E>(2.0f, axis), fm<E>(thick, thick))), L);
+            kn = fm<E>(fm<E>(vn, vn), fm<E>(dt, dt));
+            kq = fm<E>(fs<E>(fm<E>(vx, vx), fm<E>(vn, vn)), fm<E>(dt, dt));
+            n3 = fd(fm<E>(fm<E>(fm<E>(v, v), fm<E>(dt, dt)), fm<E>(szu, fm<E>(dz, dz))), fm<E>(dz, dz));
+        } else {
+            const float k0 = a.dt2 * (v * v), sv = v * sqrtf(1.0f + 2.0f * ep), fi = (float)idx;
+            d = sv * (a.cd[left ? 0 : 1] * (fi * fi));
+            dd = sv * (a.cdd[left ? 0 : 1] * fi);
+            kn = k0 * (1.0f + 2.0f * de);
+            kq = k0 * (2.0f * (ep - de));
+            n3 = k0 * szu;
+        }
+        pml_cell<E>(d, dd, dt, dx, a1, a1o, t2, t2o, a2, a2o, kn, s2, s1);
+        a3 = fa<E>(fs<E>(fm<E>(2.0f, a3o), a3), n3);
+        un = fa<E>(fa<E>(a1, a2), a3);
+        pml_cell<E>(d, dd, dt, dx, b1, b1o, r2, r2o, b2, b2o, kq, s2, s1);
+        qn = fa<E>(b1, b2);
+        P[o.uxo[0] + x] = a1; P[o.uxo[1] + x] = a2; P[o.uxo[2] + x] = t2; P[o.uxo[3] + x] = a3;
+        P[o.qxo[0] + x] = b1; P[o.qxo[1] + x] = b2; P[o.qxo[2] + x] = r2;
     }
-
-    // ---- extrapolation_one_step_2 (VS:965-1072): new q inside, from the current u ----
-    if (xin)
-        qn = fa<E>(fs<E>(fm<E>(2.0f, Q[c]), qo), fm<E>(fm<E>(fm<E>(dt, dt), fm<E>(v, v)), fm<E>(fm<E>(2.0f, fs<E>(ep, de)), fa<E>(sxq, sxu))));
-    p.u(ou)[g] = un;
-    p.q(ou)[g] = qn;
-
+    P[o.uo + g] = un;
+    P[o.qo + g] = qn;
     // ---- recording (VM:446-453, 494-501): new u on the receiver row ----
     const int rr = a.rrow[2 * s], low = a.rrow[2 * s + 1];
-    if (j == rr && i > nxl && i <= nxl + a.range && iit <= a.nt && ((!low && iit >= 1) || (low && iit > 1)))
-        a.records[((long long)s * a.range + (i - nxl - 1)) * a.nt + (iit - 1)] = un;
-}
-
-// Tiles of 32 x (8 CPT) cells per CTA (32 x 8 threads, CPT cells per thread): the current u and
-// q of the tile and its 5-cell halo are staged in shared memory once, every stencil reads them
-// there.
-template <int CPT, int MINB, bool E>
-__global__ void __launch_bounds__(kBX * kBZ, MINB) vti_step_kernel(VtiDev a, int cu, int iit) {
-    constexpr int kTZ = kBZ * CPT, kSZ = kTZ + 2 * kH;
-    __shared__ float sU[kSX * kSZ], sQ[kSX * kSZ];
-    const int s = blockIdx.z, tx = threadIdx.x, ty = threadIdx.y, tid = ty * kBX + tx;
-    const int i0 = blockIdx.x * kTX + 1, j0 = blockIdx.y * kTZ + 1;
-    const VtiSlab p = slab(a, s);
-    const float* U = p.u(cu);
-    const float* Q = p.q(cu);
-    // tile cell (lx, lz) is field cell (i0 - 5 + lx, j0 - 5 + lz), array column i + 4 >= 0 and row
-    // j + 4 >= 0; columns past the pitch and rows past nz + 5 (only reached by the tile's own cells
-    // beyond the grid, which store nothing) read as zero.  All of the thread's global loads -- its
-    // share of the tiles and its cells' model and old u, q -- are issued before the first use.
-    constexpr int NE = kSX * kSZ, IT = (NE + kBX * kBZ - 1) / (kBX * kBZ);
-    float ru[IT], rq[IT];
-#pragma unroll
-    for (int t = 0; t < IT; t++) {
-        const int e = tid + t * kBX * kBZ;
-        const int lz = e / kSX, lx = e - lz * kSX;
-        const int gi = i0 - kH + lx + 4, gj = j0 - kH + lz + 4;
-        ru[t] = 0.0f;
-        rq[t] = 0.0f;
-        if (e < NE && gi < a.pitch && gj < a.nz + 10) {
-            const long long gg = (long long)gj * a.pitch + gi;
-            ru[t] = U[gg];
-            rq[t] = Q[gg];
-        }
-    }
-    const int i = i0 + tx, ou = 1 - cu;
-    float mv[CPT], md[CPT], me[CPT], mu[CPT], mq[CPT];
-#pragma unroll
-    for (int k = 0; k < CPT; k++) {
-        const int j = j0 + ty + kBZ * k;
-        mv[k] = md[k] = me[k] = mu[k] = mq[k] = 0.0f;
-        if (i <= a.nx && j <= a.nz) {
-            const long long g = (long long)(j + 4) * a.pitch + (i + 4);
-            mv[k] = p.vz()[g];
-            md[k] = p.de()[g];
-            me[k] = p.ep()[g];
-            mu[k] = p.u(ou)[g];
-            mq[k] = p.q(ou)[g];
-        }
-    }
-#pragma unroll
-    for (int t = 0; t < IT; t++) {
-        const int e = tid + t * kBX * kBZ;
-        if (e < NE) {
-            sU[e] = ru[t];
-            sQ[e] = rq[t];
-        }
-    }
-    __syncthreads();
-    if (i > a.nx) return;
-#pragma unroll
-    for (int k = 0; k < CPT; k++) {
-        const int lz = ty + kBZ * k, j = j0 + lz;
-        if (j > a.nz) break;
-        vti_cell<E>(a, p, sU, sQ, (lz + kH) * kSX + tx + kH, kSX, i, j, s, cu, iit, mv[k], md[k], me[k], mu[k], mq[k]);
-    }
+    if (gj + 1 == rr && gi >= nxl && gi < nxl + a.range && iit <= a.nt && ((!low && iit >= 1) || (low && iit > 1)))
+        a.records[((long long)s * a.range + (gi - nxl)) * a.nt + (iit - 1)] = un;
 }
 
 // coefficient_2nd / coefficient_1st (VS:1264-1472): a(i,j) = i^p / p! (p = 2j or 2j-1) inverted
@@ -352,49 +349,47 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
     a.L = std::log(1.0f / 1.0e-3f);  // log(1/R), R = 1.0E-3 (VS:14)
     if (coefficients(10, 0, a.cE) || coefficients(c.order_pml_1st, 1, a.c1))
         return SFD_ERR_ARG;
-    a.pitch = (nx + 10 + 31) / 32 * 32;
-    a.field = (long long)a.pitch * (nz + 10);
+    const int ntx = (nx + kTX - 1) / kTX;
+    a.pitch = (ntx * kTX + 2 * kGX + 31) / 32 * 32;
+    a.field = (long long)a.pitch * (nz + 2 * kH);
     a.xs = (long long)(nxl + nxr) * nz;
     a.zs = (long long)nx * (nzu + nzd);
+    a.rdx2 = (float)(1.0 / ((double)c.dx * c.dx));
+    a.rdz2 = (float)(1.0 / ((double)c.dz * c.dz));
+    a.rdx = (float)(1.0 / (double)c.dx);
+    a.dt2 = (float)((double)c.dt * c.dt);
+    const int pn[4] = {nxl, nxr, nzu, nzd};
+    for (int k = 0; k < 4; k++) {
+        const double h = k < 2 ? c.dx : c.dz, n3 = (double)std::max(pn[k], 1) * std::max(pn[k], 1) * std::max(pn[k], 1);
+        a.cd[k] = (float)(1.5 * (double)a.L / (n3 * h));
+        a.cdd[k] = (float)(3.0 * (double)a.L / (n3 * h * h));
+    }
+    if (7 * a.field + 14 * a.xs + 8 * a.zs > 0xffffffffLL) return SFD_ERR_NOMEM;  // 32-bit offsets in a slab
     a.shot_stride = 7 * a.field + 14 * a.xs + 8 * a.zs;
     a.shot_stride = (a.shot_stride + 31) / 32 * 32;
 
-    // per-shot windows (get_currshot_parameters, VS:268-338, and VM:405-408), source cells and
-    // receiver rows
-    std::vector<float> host((size_t)nshot * 3 * a.field, 0.0f);
-    std::vector<int> src(2 * nshot), rrow(2 * nshot);
+    // the values that enter a shot's window (vti_window_kernel) must be usable: vz in its columns, and
+    // epsilon and delta there below the zeroed rows.  Per model column: vz valid, last bad row
+    std::vector<char> vz_ok(c.nx_v, 1);
+    std::vector<int> bad(c.nx_v, 0);  // 1-based row
+    for (int i = 0; i < c.nx_v; i++)
+        for (int j = 0; j < c.nz_v; j++) {
+            const size_t m = (size_t)i * c.nz_v + j;
+            if (!(vz[m] > 0.0f) || !std::isfinite(vz[m])) vz_ok[i] = 0;
+            if (!std::isfinite(epsilon[m]) || !std::isfinite(delta[m]) || !(1.0f + 2.0f * epsilon[m] >= 0.0f) ||
+                !(1.0f + 2.0f * delta[m] >= 0.0f))
+                bad[i] = j + 1;
+        }
+    std::vector<int> src(2 * nshot), rrow(2 * nshot), win(2 * nshot);
     for (int s = 0; s < nshot; s++) {
         const sfd_vti_shot& sh = shots[s];
-        float* hv = host.data() + (size_t)s * 3 * a.field;
-        float* he = hv + a.field;
-        float* hd = he + a.field;
-        auto C = [&](int i, int j) { return (size_t)(j + 4) * a.pitch + (i + 4); };
-        for (int i = 1; i <= range; i++) {
-            int io = i + sh.xmin;
-            io = io < 1 ? 1 : (io > c.nx_v ? c.nx_v : io);
-            for (int j = 1; j <= c.nz_v; j++) {
-                const size_t m = (size_t)(io - 1) * c.nz_v + (j - 1);
-                hv[C(i + nxl, nzu + j)] = vz[m];
-                he[C(i + nxl, nzu + j)] = epsilon[m];
-                hd[C(i + nxl, nzu + j)] = delta[m];
-            }
-        }
-        for (int j = 1; j <= nzu; j++)
-            for (int i = 1; i <= nx; i++) hv[C(i, j)] = hv[C(i, nzu + 1)];
-        for (int j = nzu + c.nz_v + 1; j <= nz; j++)
-            for (int i = 1; i <= nx; i++) hv[C(i, j)] = hv[C(i, nzu + c.nz_v)];
-        for (int j = 1; j <= nz; j++)
-            for (int i = 1; i <= nxl; i++) hv[C(i, j)] = hv[C(nxl + 1, j)];
-        for (int j = 1; j <= nz; j++)
-            for (int i = nxl + range + 1; i <= nx; i++) hv[C(i, j)] = hv[C(nxl + range, j)];
-        for (int j = 1; j <= sh.nsz0 + nzu + 6 && j <= nz; j++)
-            for (int i = 1; i <= nx; i++) he[C(i, j)] = hd[C(i, j)] = 0.0f;
-        for (int j = 1; j <= nz; j++)
-            for (int i = 1; i <= nx; i++)
-                if (!(hv[C(i, j)] > 0.0f) || !std::isfinite(hv[C(i, j)]) || !std::isfinite(he[C(i, j)]) ||
-                    !std::isfinite(hd[C(i, j)]) || !(1.0f + 2.0f * he[C(i, j)] >= 0.0f) ||
-                    !(1.0f + 2.0f * hd[C(i, j)] >= 0.0f))
-                    return SFD_ERR_ARG;
+        const long long lo = (long long)sh.xmin + 1, hi = (long long)sh.xmin + range;  // 1-based columns, then clamped
+        const int c0 = (int)std::min<long long>(std::max<long long>(lo, 1), c.nx_v) - 1;
+        const int c1 = (int)std::min<long long>(std::max<long long>(hi, 1), c.nx_v) - 1;
+        for (int i = c0; i <= c1; i++)
+            if (!vz_ok[i] || bad[i] > sh.nsz0 + 6) return SFD_ERR_ARG;
+        win[2 * s] = sh.xmin;
+        win[2 * s + 1] = sh.nsz0;
         src[2 * s] = sh.nsx - sh.xmin + nxl;  // VS:294-295
         src[2 * s + 1] = sh.nsz0 + nzu;
         if (src[2 * s] < 1 || src[2 * s] > nx || src[2 * s + 1] < 1 || src[2 * s + 1] > nz) return SFD_ERR_ARG;
@@ -418,50 +413,72 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
     cudaStream_t st = nullptr;
     if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return SFD_ERR_CUDA;
     struct StreamGuard { cudaStream_t s; ~StreamGuard() { cudaStreamDestroy(s); } } sg{st};
-    DevBuf<float> state, recs;
-    DevBuf<int> dsrc, drow;
+    DevBuf<float> state, recs, model;
+    DevBuf<int> dsrc, drow, dwin, derr;
     const size_t total = (size_t)nshot * a.shot_stride;
-    const size_t rec_n = (size_t)nshot * range * c.nt;
+    const size_t rec_n = (size_t)nshot * range * c.nt, nm = (size_t)c.nx_v * c.nz_v;
     if (state.alloc(total) != cudaSuccess || recs.alloc(rec_n) != cudaSuccess || dsrc.alloc(2 * nshot) != cudaSuccess ||
-        drow.alloc(2 * nshot) != cudaSuccess) {
+        drow.alloc(2 * nshot) != cudaSuccess || dwin.alloc(2 * nshot) != cudaSuccess || derr.alloc(1) != cudaSuccess ||
+        model.alloc(3 * nm) != cudaSuccess) {
         cudaGetLastError();
         return SFD_ERR_NOMEM;
     }
     long long h2d = 0;
     if (cudaMemsetAsync(state.p, 0, total * sizeof(float), st) != cudaSuccess ||
-        cudaMemsetAsync(recs.p, 0, rec_n * sizeof(float), st) != cudaSuccess)
+        cudaMemsetAsync(recs.p, 0, rec_n * sizeof(float), st) != cudaSuccess ||
+        cudaMemsetAsync(derr.p, 0, sizeof(int), st) != cudaSuccess)
         return SFD_ERR_CUDA;
-    for (int s = 0; s < nshot; s++) {
-        if (cudaMemcpyAsync(state.p + (size_t)s * a.shot_stride + 4 * a.field, host.data() + (size_t)s * 3 * a.field,
-                            3 * a.field * sizeof(float), cudaMemcpyHostToDevice, st) != cudaSuccess)
+    const float* model_host[3] = {vz, epsilon, delta};
+    for (int k = 0; k < 3; k++)
+        if (cudaMemcpyAsync(model.p + k * nm, model_host[k], nm * sizeof(float), cudaMemcpyHostToDevice, st) != cudaSuccess)
             return SFD_ERR_CUDA;
-        h2d += 3 * a.field * (long long)sizeof(float);
-    }
+    h2d += 3 * (long long)(nm * sizeof(float));
     if (cudaMemcpyAsync(dsrc.p, src.data(), 2 * nshot * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        cudaMemcpyAsync(drow.p, rrow.data(), 2 * nshot * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess)
+        cudaMemcpyAsync(drow.p, rrow.data(), 2 * nshot * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+        cudaMemcpyAsync(dwin.p, win.data(), 2 * nshot * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess)
         return SFD_ERR_CUDA;
-    a.base = state.p; a.src = dsrc.p; a.rrow = drow.p; a.records = recs.p;
+    a.base = state.p; a.src = dsrc.p; a.rrow = drow.p; a.records = recs.p; a.err_flag = derr.p;
+    VtiOff off[2];  // by the current slot
+    for (int b = 0; b < 2; b++) {
+        VtiOff& f = off[b];
+        const unsigned F = (unsigned)a.field, X = (unsigned)a.xs, Z = (unsigned)a.zs, c0 = b, o0 = 1 - b;
+        f.uc = c0 * F; f.uo = o0 * F; f.qc = (2 + c0) * F; f.qo = (2 + o0) * F;
+        f.vz = 4 * F; f.ep = 5 * F; f.de = 6 * F;
+        for (unsigned k = 0; k < 4; k++) {
+            f.uxc[k] = 7 * F + (2 * k + c0) * X; f.uxo[k] = 7 * F + (2 * k + o0) * X;
+            if (k < 3) { f.qxc[k] = 7 * F + (8 + 2 * k + c0) * X; f.qxo[k] = 7 * F + (8 + 2 * k + o0) * X; }
+            f.uzc[k] = 7 * F + 14 * X + (2 * k + c0) * Z; f.uzo[k] = 7 * F + 14 * X + (2 * k + o0) * Z;
+        }
+        const long long rows = nz + 2 * kH;
+        if (!sfd::encode_map3(&a.tm_u[b], state.p + f.uc, a.pitch, rows, nshot, a.pitch, a.shot_stride, kSX, kTZ + 2 * kH) ||
+            !sfd::encode_map3(&a.tm_q[b], state.p + f.qc, a.pitch, rows, nshot, a.pitch, a.shot_stride, kSX, kTZ))
+            return SFD_ERR_CUDA;
+    }
+    vti_window_kernel<<<dim3((nx + 127) / 128, nz, nshot), 128, 0, st>>>(a, model.p, model.p + nm, model.p + 2 * nm, dwin.p,
+                                                                     c.nx_v, c.nz_v);
 
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     const bool exact = (c.flags & SFD_EXACT) != 0;
-    const int tz = kBZ * kCPT;
-    const dim3 grid((nx + kTX - 1) / kTX, (nz + tz - 1) / tz, nshot), block(kBX, kBZ);
+    const dim3 grid(ntx, (nz + kTZ - 1) / kTZ, nshot);
+    const void* step = exact ? (const void*)vti_step_kernel<true> : (const void*)vti_step_kernel<false>;
+    cudaError_t err = cudaSuccess;
     long long launches = 0;
     cudaEventRecord(e0, st);
-    for (int it = 1; it <= NT; it++) {
-        const int cu = (it % 2 == 1) ? 1 : 0;  // odd steps: u2 / q2 current (VM:417-505)
+    for (int it = 1; it <= NT && err == cudaSuccess; it++) {
+        int cu = (it % 2 == 1) ? 1 : 0, iit = it - half;  // odd steps: u2 / q2 current (VM:417-505)
         if (it <= nwt) {
-            vti_inject_kernel<<<nshot, 32, 0, st>>>(a, cu, w[it]);
+            void* args[] = {&a, &off[cu].uc, &w[it]};
+            err = sfd::tile::launch((const void*)vti_inject_kernel, dim3(nshot), 32, 0, st, args);
             launches++;
         }
-        if (exact) vti_step_kernel<kCPT, kMinBlocks, true><<<grid, block, 0, st>>>(a, cu, it - half);
-        else vti_step_kernel<kCPT, kMinBlocks, false><<<grid, block, 0, st>>>(a, cu, it - half);
+        void* args[] = {&a, &off[cu], &cu, &iit};
+        if (err == cudaSuccess) err = sfd::tile::launch(step, grid, kThreads, 0, st, args);
         launches++;
     }
     cudaEventRecord(e1, st);
-    cudaError_t err = cudaGetLastError();
+    if (err == cudaSuccess) err = cudaGetLastError();
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(records, recs.p, rec_n * sizeof(float), cudaMemcpyDeviceToHost, st);
     if (err == cudaSuccess) err = cudaStreamSynchronize(st);
@@ -470,6 +487,9 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (err != cudaSuccess) return SFD_ERR_CUDA;
+    int late = 0;
+    if (cudaMemcpy(&late, derr.p, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return SFD_ERR_CUDA;
+    if (late) return SFD_ERR_TIMEOUT;
     if (timing) {
         std::memset(timing, 0, sizeof(*timing));
         timing->loop_ms = ms;
