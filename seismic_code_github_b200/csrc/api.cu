@@ -794,8 +794,8 @@ int finish_nan(sfd_ctx* ctx) {
 }
 
 // Tuner for the forward step of the default (FMA) scheme.  Candidates: the tile kernel with one
-// tile per CTA (two CTAs per SM), the persistent tile kernel with double-buffered TMA, and the
-// x-marching kernel with segments of 128, 256 or 512 columns (segments longer than the shots are
+// tile per CTA (two CTAs per SM), the persistent tile kernel with double-buffered TMA, the small-tile
+// kernel (which runs untimed when the shot set has fewer tiles than the chip SMs), and the x-marching kernel with segments of 128, 256 or 512 columns (segments longer than the shots are
 // skipped).  Each runs a few steps on the real shot set, twice; the fastest is kept.  All
 // candidates give bit-identical results.  SFD_FMA_STAGES=1|2 forces a tile schedule,
 // SFD_MARCH_SEG=<columns> forces the x-marching kernel with that segment length.
@@ -807,6 +807,7 @@ int tune_schedule(sfd_ctx* ctx) {
             ctx->plan.stages = s;
             ctx->plan.seg = 0;
             ctx->plan.forced = false;
+            ctx->plan.pinned = true;
             return SFD_OK;
         }
     }
@@ -815,14 +816,25 @@ int tune_schedule(sfd_ctx* ctx) {
         if (s >= 16 && s % 16 == 0) {
             ctx->plan.stages = 1;
             ctx->plan.seg = s;
-            ctx->plan.forced = true;
+            ctx->plan.forced = ctx->plan.pinned = true;
             return SFD_OK;
         }
     }
+    ctx->plan.pinned = ctx->plan.small = false;
+    const long long tiles = (long long)active_shots(ctx, 0) * ctx->L.ntx * ctx->L.ntz;
+    if (acoustic2d_use_small(ctx->plan, ctx->L, active_shots(ctx, 0))) {  // every launch runs the small tiles
+        ctx->plan.stages = 1;
+        ctx->plan.seg = 0;
+        ctx->plan.forced = false;
+        return SFD_OK;
+    }
     struct Cand {
         int stages, seg;
+        bool small = false;
     };
     std::vector<Cand> cands = {{1, 0}, {2, 0}};
+    // beyond this the larger halo always loses (measured at 1680 tiles: equal at best)
+    if (tiles < 1500) cands.push_back({1, 0, true});
     const int width = ctx->L.ntx * ctx->L.tx;
     for (int seg : {128, 256, 512})
         if (seg < width || seg == 128) cands.push_back({1, seg});
@@ -834,6 +846,8 @@ int tune_schedule(sfd_ctx* ctx) {
             ctx->plan.stages = cands[ci].stages;
             ctx->plan.seg = cands[ci].seg;
             ctx->plan.forced = false;
+            ctx->plan.small = cands[ci].small;
+            ctx->plan.pinned = !cands[ci].small;
             int rc = prologue(ctx);
             if (rc) return rc;
             for (int k = 0; k < steps; k++) {
@@ -851,6 +865,8 @@ int tune_schedule(sfd_ctx* ctx) {
         if (best[ci] < best[pick]) pick = ci;
     ctx->plan.stages = cands[pick].stages;
     ctx->plan.seg = cands[pick].seg;
+    ctx->plan.small = cands[pick].small;
+    ctx->plan.pinned = false;
     return SFD_OK;
 }
 
@@ -860,6 +876,7 @@ int kernel_variant(const sfd_ctx* ctx) {
     if (ctx->g.scheme == SFD_VISCOEL_2D) return 45;
     if (ctx->g.scheme == SFD_ELASTIC_2D) return 50;
     if (ctx->g.flags & SFD_EXACT) return 1;
+    if (acoustic2d_use_small(ctx->plan, ctx->L, active_shots(ctx, 0))) return 11;  // tiles, one per CTA
     return acoustic2d_use_march(ctx->plan, ctx->L, active_shots(ctx, 0)) ? 13 : 10 + ctx->plan.stages;
 }
 
@@ -1121,7 +1138,9 @@ Acou2DArgs make_adj_args(const sfd_ctx* ctx, const GradRange& r, int k, const fl
 
 int grad_adj_step(sfd_ctx* ctx, const GradRange& r, int k, int act, const float* div) {
     if (ctx->g.scheme == SFD_VISCOAC_2D) return grad_adj_step_q(ctx, r, k, act, div);
-    if (acoustic2d_use_march(grad_plan(ctx), ctx->L, act))
+    if (acoustic2d_use_small(grad_plan(ctx), ctx->L, act))
+        CK(acoustic2d_small_launch(ctx->radius, make_adj_args(ctx, r, k, div), act, ctx->varden, ctx->stream, true));
+    else if (acoustic2d_use_march(grad_plan(ctx), ctx->L, act))
         CK(acoustic2d_march_launch(ctx->radius, make_adj_args(ctx, r, k, div), act, ctx->varden, ctx->plan.seg,
                                    ctx->stream, pdl_enabled(), true));
     else

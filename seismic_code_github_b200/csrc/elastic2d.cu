@@ -256,7 +256,8 @@ __global__ void __launch_bounds__(kThreads, 5) iso_velocity_kernel(const __grid_
     TileRef t;
     const bool on = tile_of(a, t);
     tile::bar_init(bar);
-    tile::dependency();
+    tile::release();
+    tile::acquire();
     if (!on) return;
     if (threadIdx.x == 0) {
         const int f[3] = {I_SXX, I_SXZ, I_SZZ};
@@ -330,7 +331,8 @@ __global__ void __launch_bounds__(kThreads, 5) iso_stress_kernel(const __grid_co
     TileRef t;
     const bool on = tile_of(a, t);
     tile::bar_init(bar);
-    tile::dependency();
+    tile::release();
+    tile::acquire();
     if (!on) return;
     if (threadIdx.x == 0) {
         const int f[2] = {I_VX, I_VZ};
@@ -461,7 +463,8 @@ __global__ void iso_surface_kernel(const __grid_constant__ IArgs a) {
     const int shot = a.slot_to_shot[blockIdx.y];
     const ShotDev sd = a.shots[shot];
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    tile::dependency();
+    tile::release();
+    tile::acquire();
     if (x >= sd.nx) return;
     const int mc = min(sd.x0 + x, a.nx_model - 1);
     const int zs = __ldg(a.itopo + mc) - 1;

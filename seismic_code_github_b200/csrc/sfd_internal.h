@@ -353,6 +353,8 @@ struct Acou2DPlan {
     int stages;  // FMA tile kernel schedule (1 or 2)
     int seg;     // > 0: forward steps run the x-marching kernel with segments of `seg` columns
     bool forced; // seg set by SFD_MARCH_SEG: x-marching even where its grid does not fill the device
+    bool pinned; // stages or seg set by the environment: no small tiles either
+    bool small;  // the small-tile kernel won the tuner's comparison on this shot set
 };
 // Model arrays on the device carry this many replicated rows above z = 0 and below z = nz - 1
 // so that vectorised halo reads stay inside the allocation and see finite values.
@@ -381,6 +383,10 @@ inline bool acoustic2d_use_march(const Acou2DPlan& plan, const Layout2D& L, int 
 }
 // Forward step of the default (FMA) scheme with the plan's kernel: x-marching when plan.seg > 0
 // and the launch fills the device, else the tile kernel with plan.stages.
+// The small-tile kernel (acoustic2d_small.cu): the tile kernel's values bit for bit, for launches with
+// few tiles; adj as in acoustic2d_fma_launch.
+cudaError_t acoustic2d_small_launch(int radius, const Acou2DArgs& a, int active, bool varden, cudaStream_t st, bool adj);
+bool acoustic2d_use_small(const Acou2DPlan& plan, const Layout2D& L, int active);
 cudaError_t acoustic2d_fwd_launch(const Acou2DPlan& plan, int radius, const Acou2DArgs& a, int active, bool varden,
                                   cudaStream_t st);
 // Programmatic dependent launch of consecutive step kernels (SFD_PDL=0 turns it off).

@@ -61,14 +61,13 @@ __device__ __forceinline__ bool staged(uint64_t* bar, int* err_flag) {
     bar_wait_1s(bar);
     return false;
 }
-// programmatic dependent launch: let the next kernel's CTAs start their index work, then wait for
-// the previous kernel before the first read of its fields
-__device__ __forceinline__ void dependency() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
+// programmatic dependent launch: release() lets the next kernel's CTAs start on what does not depend on
+// this one (indexes, model values, tables), acquire() waits for the previous kernel before the first
+// access to its fields
+__device__ __forceinline__ void release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void acquire() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// launch with the dependency() of the kernel above as a programmatic edge
+// launch whose release() and acquire() make the edge to the kernel before it a programmatic one
 inline cudaError_t launch(const void* fn, dim3 grid, int threads, size_t smem, cudaStream_t st, void** args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;

@@ -140,7 +140,8 @@ __global__ void __launch_bounds__(kThreads, kMinV) e_velocity_kernel(const __gri
     TileRef t;
     const bool on = tile_of(a, t);
     tile::bar_init(bar);
-    tile::dependency();
+    tile::release();
+    tile::acquire();
     if (!on) return;
     if (threadIdx.x == 0) {
         const int f[3] = {E_SXX, E_SXZ, E_SZZ};
@@ -185,7 +186,8 @@ __global__ void __launch_bounds__(kThreads, kMinS) e_stress_kernel(const __grid_
     TileRef t;
     const bool on = tile_of(a, t);
     tile::bar_init(bar);
-    tile::dependency();
+    tile::release();
+    tile::acquire();
     if (!on) return;
     if (threadIdx.x == 0) {
         const int f[2] = {E_VX, E_VZ};

@@ -125,7 +125,8 @@ __device__ __forceinline__ void pml_cell(float d, float dd, float dt, float h, f
 }
 
 __global__ void vti_inject_kernel(const __grid_constant__ VtiDev a, unsigned uc, float w) {
-    sfd::tile::dependency();
+    sfd::tile::release();
+    sfd::tile::acquire();
     const int s = blockIdx.x;
     if (threadIdx.x != 0) return;
     float* u = a.base + (long long)s * a.shot_stride + uc + cell(a, a.src[2 * s] - 1, a.src[2 * s + 1] - 1);
@@ -163,7 +164,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) vti_step_kernel(const __
     const bool in = gi < a.nx && gj < a.nz;
     const unsigned g = cell(a, gi, gj);
     sfd::tile::bar_init(&bar);
-    sfd::tile::dependency();
+    sfd::tile::release();
+    float v = 0.0f, de = 0.0f, ep = 0.0f, uo = 0.0f, qo = 0.0f;
+    if (in) {
+        v = P[o.vz + g];
+        de = P[o.de + g];
+        ep = P[o.ep + g];
+    }
+    sfd::tile::acquire();
     // u: rows j0 - 5 .. j0 + kTZ + 4, q: the tile's rows, columns i0 - 8 .. i0 + 71 (allocation columns
     // from i0, a multiple of 64, and rows from j0; rows past the allocation read as zero)
     if (tid == 0) {
@@ -171,11 +179,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) vti_step_kernel(const __
         sfd::tile::box(sU, &a.tm_u[cu], i0, j0, s, &bar);
         sfd::tile::box(sQ, &a.tm_q[cu], i0, j0 + kH, s, &bar);
     }
-    float v = 0.0f, de = 0.0f, ep = 0.0f, uo = 0.0f, qo = 0.0f;
     if (in) {
-        v = P[o.vz + g];
-        de = P[o.de + g];
-        ep = P[o.ep + g];
         uo = P[o.uo + g];
         qo = P[o.qo + g];
     }
