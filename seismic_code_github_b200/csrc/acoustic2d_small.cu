@@ -13,6 +13,12 @@
 // asynchronously; phase A (Vx, two columns of one vector per thread from a register window), phase B
 // (Vz), a barrier, phase C (P, one vector per thread).  Every stencil sum is the tile kernel's: first
 // product, then fused multiply-adds in the order of m.
+//
+// The same tiles run SFD_EXACT at every size (kExact): each multiply and add rounded by itself in the
+// reference's order, the scale factors and the divergence in double.  8 shots of 851 x 451 with variable
+// density, order 16: 122 us a step on 64 x 64 tiles with one stencil point per shared-memory load, 60 us
+// now (51 Gpts/s; bound by issue: two thirds of the instructions are arithmetic of the prescribed order
+// and its conversions to and from double).
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -22,12 +28,14 @@
 namespace sfd {
 namespace {
 
-constexpr int TX = 16, TZ = 32, kThreads = 128;
+constexpr int TZ = 32;
+enum Mode { kForward, kAdjoint, kExact };
 
 __host__ __device__ constexpr int r4(int v) { return (v + 3) & ~3; }
 
-template <int R>
+template <int R, int TX>
 struct SP {
+    static constexpr int kThreads = TX * TZ / 4;
     static constexpr int RQ = r4(R), HX = 2 * R, HZ = 2 * RQ;
     static constexpr int PW = TZ + 2 * HZ, PR = TX + 2 * HX;    // staged P (its corners stay unused)
     static constexpr int VXR = TX + 2 * R, VZW = TZ + 2 * RQ;   // Vx rows, Vz width
@@ -62,9 +70,38 @@ __device__ __forceinline__ void put(float* f, long long c, const float4& v, int 
         for (int q = 0; q < 4 && gz + q < nz; q++) f[c + q] = comp(v, q);
 }
 
-template <int R, bool VARDEN, bool ADJ>
-__global__ void __launch_bounds__(kThreads, 5) acoustic2d_small_kernel(const __grid_constant__ Acou2DArgs a) {
-    using T = SP<R>;
+// kExact: one stencil sum in the reference's order, every operation rounded (AFD:255-302)
+template <int R, class F>
+__device__ __forceinline__ float sum_rn(const float* C, F diff) {
+    float s = __fmul_rn(C[0], diff(0));
+#pragma unroll
+    for (int m = 1; m < R; m++) s = __fadd_rn(s, __fmul_rn(C[m], diff(m)));
+    return s;
+}
+// ... of four cells, two per instruction: the sum as fma(t, one, s) with one = 1.0 from the arguments, which
+// the compiler cannot contract with the product (see add2 in elastic2d.cu)
+template <int R, class H, class L>
+__device__ __forceinline__ float4 sum4_rn(const float* C, float one, H up, L down) {
+    float2 sl, sh;
+#pragma unroll
+    for (int m = 0; m < R; m++) {
+        const float4 p = up(m), q = down(m);
+        const float2 tl = mul2(bc(C[m]), sub2(lo(p), lo(q))), th = mul2(bc(C[m]), sub2(hi(p), hi(q)));
+        sl = m == 0 ? tl : fma2(tl, bc(one), sl);
+        sh = m == 0 ? th : fma2(th, bc(one), sh);
+    }
+    return cat(sl, sh);
+}
+// kExact: a velocity, v a - (1 / den) (dt / d) s with the scale in double (AFD:259, 276)
+__device__ __forceinline__ float vel_rn(float v, float a, double b, float s) {
+    return __double2float_rn(__dsub_rn((double)__fmul_rn(v, a), __dmul_rn(b, (double)s)));
+}
+
+template <int R, int TX, bool VARDEN, Mode MODE>
+__global__ void __launch_bounds__(TX * TZ / 4, 5) acoustic2d_small_kernel(const __grid_constant__ Acou2DArgs a) {
+    using T = SP<R, TX>;
+    constexpr bool ADJ = MODE == kAdjoint;
+    constexpr int kThreads = T::kThreads;
     __shared__ __align__(16) float smem[T::FLOATS];
     float* sP = smem;
     float* sVx = smem + T::OFF_VX;
@@ -87,10 +124,21 @@ __global__ void __launch_bounds__(kThreads, 5) acoustic2d_small_kernel(const __g
     // the x pads)
     const int row = tid >> 3, zo = 4 * (tid & 7), gx = x0 + row, gz = z0 + zo;
     const bool own = gx < nx && gz < nz;
-    const long long c = cell(gx, gz), mi = (long long)min(sd.x0 + gx, a.nx_model - 1) * a.mpitch + gz;
-    const float4 vp = __ldg(reinterpret_cast<const float4*>(a.vp + mi));
-    const float4 dn = VARDEN ? __ldg(reinterpret_cast<const float4*>(a.den + mi))
-                             : make_float4(a.den_c, a.den_c, a.den_c, a.den_c);
+    const long long c = cell(gx, gz);
+    // Model values of four cells of a column.  kExact may be given the caller's own array
+    // (sfd_forward_noalloc: any alignment, no rows around it), which is read cell by cell and only where
+    // the scheme updates; elsewhere `out` stands in, for results that are not kept
+    auto model4 = [&](const float* f, int x, int z, float out) -> float4 {
+        const long long m = (long long)min(max(sd.x0 + x, 0), a.nx_model - 1) * a.mpitch + z;
+        if (MODE != kExact || !a.model_raw) return __ldg(reinterpret_cast<const float4*>(f + m));
+        float v[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            v[q] = x >= R && x < nx - R && z + q >= R && z + q < nz - R ? __ldg(f + m + q) : out;
+        return make_float4(v[0], v[1], v[2], v[3]);
+    };
+    const float4 vp = model4(a.vp, gx, gz, 0.0f);
+    const float4 dn = VARDEN ? model4(a.den, gx, gz, 1.0f) : make_float4(a.den_c, a.den_c, a.den_c, a.den_c);
     for (int i = tid; i < T::VXR + T::VZW; i += kThreads) {
         const bool isx = i < T::VXR;
         const int p = isx ? x0 - R + i : z0 - T::RQ + i - T::VXR, n = isx ? nx : nz, pml = a.pml;
@@ -141,6 +189,23 @@ __global__ void __launch_bounds__(kThreads, 5) acoustic2d_small_kernel(const __g
         const float4 az = ld4(sAz + T::RQ + z), mz = ld4(sMz + T::RQ + z);
 #pragma unroll
         for (int o = 0; o < 2; o++) {
+            if (MODE == kExact) {
+                const float ax = sAx[r0 + o], mx = sMx[r0 + o];
+                float* v = sVx + (r0 + o) * TZ + z;
+                const float4 vo = ld4(v), sm = sum4_rn<R>(C, a.one, [&](int m) { return w[o + R + m]; },
+                                                         [&](int m) { return w[o + R - 1 - m]; });
+                float4 d = make_float4(1.f, 1.f, 1.f, 1.f);
+                if (VARDEN) d = model4(a.den, x0 - R + r0 + o, z0 + z, 1.0f);
+                float out[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const double b = VARDEN ? __dmul_rn(__drcp_rn((double)comp(d, q)), (double)a.dtdx) : a.bx_d;
+                    const float n = vel_rn(comp(vo, q), ax >= 0.0f ? ax : comp(az, q), b, comp(sm, q));
+                    out[q] = mx * comp(mz, q) != 0.0f ? n : 0.0f;
+                }
+                st4(v, make_float4(out[0], out[1], out[2], out[3]));
+                continue;
+            }
             float2 sl = mul2(bc(C[0]), sub2(lo(w[o + R]), lo(w[o + R - 1])));
             float2 sh = mul2(bc(C[0]), sub2(hi(w[o + R]), hi(w[o + R - 1])));
 #pragma unroll
@@ -189,8 +254,17 @@ __global__ void __launch_bounds__(kThreads, 5) acoustic2d_small_kernel(const __g
         const float4 vo = ld4(v), az = ld4(sAz + z), mz = ld4(sMz + z);
         const float ax = sAx[r + R], mx = sMx[r + R];
         float out[4];
+        float4 d = make_float4(1.f, 1.f, 1.f, 1.f);
+        if (MODE == kExact && VARDEN) d = model4(a.den, x0 + r, z0 - T::RQ + z, 1.0f);
 #pragma unroll
         for (int q = 0; q < 4; q++) {
+            if (MODE == kExact) {
+                const float s = sum_rn<R>(C, [&](int m) { return __fsub_rn(w[T::RQ + q + 1 + m], w[T::RQ + q - m]); });
+                const double b = VARDEN ? __dmul_rn(__drcp_rn((double)comp(d, q)), (double)a.dtdz) : a.bz_d;
+                const float n = vel_rn(comp(vo, q), ax >= 0.0f ? ax : comp(az, q), b, s);
+                out[q] = mx * comp(mz, q) != 0.0f ? n : 0.0f;
+                continue;
+            }
             float s = __fmul_rn(C[0], __fsub_rn(w[T::RQ + q + 1], w[T::RQ + q]));
 #pragma unroll
             for (int m = 1; m < R; m++) s = __fmaf_rn(C[m], __fsub_rn(w[T::RQ + q + 1 + m], w[T::RQ + q - m]), s);
@@ -212,7 +286,39 @@ __global__ void __launch_bounds__(kThreads, 5) acoustic2d_small_kernel(const __g
     // ---- phase C: P(t) on the tile, one vector per thread (AFD:289-314, 337-338) ----
     const int step = a.step;
     float4 pn = make_float4(0.f, 0.f, 0.f, 0.f);
-    {
+    if (MODE == kExact) {  // AFD:289-302: the divergence and the update in double
+        const float* vx = sVx + (row + R) * TZ + zo;
+        const float* vz = sVz + row * T::VZW + T::RQ + zo;
+        float* pc = sP + (row + T::HX) * T::PW + T::HZ + zo;
+        const float ax = sAx[row + R], mx = sMx[row + R];
+        const float4 sx = sum4_rn<R>(C, a.one, [&](int m) { return ld4(vx + m * TZ); },
+                                     [&](int m) { return ld4(vx - (m + 1) * TZ); });
+        float w[4 * T::NC], out[4], pw[4];
+#pragma unroll
+        for (int j = 0; j < T::NC; j++) {
+            const float4 v = ld4(vz - T::RQ + 4 * j);
+            w[4 * j] = v.x; w[4 * j + 1] = v.y; w[4 * j + 2] = v.z; w[4 * j + 3] = v.w;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const float sz = sum_rn<R>(C, [&](int m) { return __fsub_rn(w[T::RQ + q + m], w[T::RQ + q - 1 - m]); });
+            const float kk = __fmul_rn(__fmul_rn(__fmul_rn(comp(dn, q), comp(vp, q)), comp(vp, q)), a.dt);
+            const double div = __dadd_rn(__dmul_rn(a.rdx_d, (double)comp(sx, q)), __dmul_rn(a.rdz_d, (double)sz));
+            const float p1 = __double2float_rn(__dsub_rn((double)pc[q], __dmul_rn((double)kk, div)));
+            out[q] = mx * sMz[T::RQ + zo + q] != 0.0f ? __fmul_rn(p1, ax >= 0.0f ? ax : sAz[T::RQ + zo + q]) : 0.0f;
+            pw[q] = out[q];
+            if (gx == sd.sx && gz + q == sd.sz && step + 1 < sd.nt) {  // AFD:247-251 of the next step
+                if (a.src_pre) a.src_pre[shot] = out[q];
+                pw[q] = __fsub_rn(out[q], __fmul_rn(sd.inj_scale, __ldg(a.wavelets + sd.wav_off + step + 1)));
+            }
+        }
+        st4(pc, make_float4(out[0], out[1], out[2], out[3]));  // receivers read the recorded value here
+        if (own) {
+            put(a.p_out, c, make_float4(pw[0], pw[1], pw[2], pw[3]), gz, nz);
+            put(a.vx_out, c, ld4(vx), gz, nz);
+            put(a.vz_out, c, ld4(vz), gz, nz);
+        }
+    } else {
         const float* vx = sVx + (row + R) * TZ + zo;
         float2 sl = mul2(bc(C[0]), sub2(lo(ld4(vx)), lo(ld4(vx - TZ))));
         float2 sh = mul2(bc(C[0]), sub2(hi(ld4(vx)), hi(ld4(vx - TZ))));
@@ -321,24 +427,35 @@ __global__ void __launch_bounds__(kThreads, 5) acoustic2d_small_kernel(const __g
     }
 }
 
-template <int R, bool ADJ>
+template <int R, int TX, Mode MODE>
 cudaError_t launch_r(const Acou2DArgs& a, int active, bool varden, cudaStream_t st) {
     const dim3 grid(a.L.ntx * (kTileX / TX) * a.L.ntz * (kTileZ / TZ), active);
-    const void* k = varden ? (const void*)acoustic2d_small_kernel<R, true, ADJ>
-                           : (const void*)acoustic2d_small_kernel<R, false, ADJ>;
-    return tile::launch(k, grid, kThreads, 0, st, a);
+    const void* k = varden ? (const void*)acoustic2d_small_kernel<R, TX, true, MODE>
+                           : (const void*)acoustic2d_small_kernel<R, TX, false, MODE>;
+    return tile::launch(k, grid, SP<R, TX>::kThreads, 0, st, a);
+}
+
+template <int TX, Mode MODE>
+cudaError_t launch_mode(int radius, const Acou2DArgs& a, int active, bool varden, cudaStream_t st) {
+    switch (radius) {
+    case 1: return launch_r<1, TX, MODE>(a, active, varden, st);
+    case 2: return launch_r<2, TX, MODE>(a, active, varden, st);
+    case 4: return launch_r<4, TX, MODE>(a, active, varden, st);
+    case 5: return launch_r<5, TX, MODE>(a, active, varden, st);
+    case 8: return launch_r<8, TX, MODE>(a, active, varden, st);
+    default: return cudaErrorInvalidValue;
+    }
 }
 
 }  // namespace
 
 cudaError_t acoustic2d_small_launch(int radius, const Acou2DArgs& a, int active, bool varden, cudaStream_t st, bool adj) {
-    switch (radius) {
-#define SFD_CASE(RR) \
-    case RR: return adj ? launch_r<RR, true>(a, active, varden, st) : launch_r<RR, false>(a, active, varden, st);
-        SFD_CASE(1) SFD_CASE(2) SFD_CASE(4) SFD_CASE(5) SFD_CASE(8)
-#undef SFD_CASE
-    default: return cudaErrorInvalidValue;
-    }
+    return adj ? launch_mode<16, kAdjoint>(radius, a, active, varden, st)
+               : launch_mode<16, kForward>(radius, a, active, varden, st);
+}
+
+cudaError_t acoustic2d_exact_launch(int radius, const Acou2DArgs& a, int active, bool varden, cudaStream_t st) {
+    return launch_mode<16, kExact>(radius, a, active, varden, st);
 }
 
 // With fewer 64 x 64 tiles than SMs a step of the tile kernel costs the same 7 to 10 us however few they

@@ -357,6 +357,7 @@ Acou2DArgs make_args(const sfd_ctx* c, int step) {
     a.pml = c->g.pml;
     a.vp = c->d_vp + kModelGhostZ;  // row z = 0 of column 0
     a.den = c->varden ? c->d_den + kModelGhostZ : nullptr;
+    a.one = 1.0f;
     a.mpitch = c->mpitch;
     a.nx_model = c->g.nx;
     a.den_c = c->den_c;

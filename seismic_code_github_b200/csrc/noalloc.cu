@@ -168,6 +168,8 @@ extern "C" int sfd_forward_noalloc(const sfd_grid* g, const float* vp_dev, const
     a.pml = pml;
     a.vp = vp_dev;
     a.den = den_dev;
+    a.model_raw = 1;
+    a.one = 1.0f;
     a.mpitch = nz;  // the reference-order kernel reads the model only inside the updated region
     a.nx_model = nx;
     a.den_c = den_c;

@@ -288,6 +288,8 @@ struct Acou2DArgs {
     const float* den;       // NULL for constant density
     int mpitch;
     int nx_model;
+    int model_raw;          // SFD_EXACT only: vp and den are the caller's arrays (no ghost rows, any alignment)
+    float one;              // 1.0 (acoustic2d_small.cu sum4_rn)
     float den_c;            // constant density
     float dt;
     float dtdx, dtdz;       // float(dt/dx), float(dt/dz) (AFD:259, 276)
@@ -387,6 +389,8 @@ inline bool acoustic2d_use_march(const Acou2DPlan& plan, const Layout2D& L, int 
 // few tiles; adj as in acoustic2d_fma_launch.
 cudaError_t acoustic2d_small_launch(int radius, const Acou2DArgs& a, int active, bool varden, cudaStream_t st, bool adj);
 bool acoustic2d_use_small(const Acou2DPlan& plan, const Layout2D& L, int active);
+// SFD_EXACT: the reference's operation order
+cudaError_t acoustic2d_exact_launch(int radius, const Acou2DArgs& a, int active, bool varden, cudaStream_t st);
 cudaError_t acoustic2d_fwd_launch(const Acou2DPlan& plan, int radius, const Acou2DArgs& a, int active, bool varden,
                                   cudaStream_t st);
 // Programmatic dependent launch of consecutive step kernels (SFD_PDL=0 turns it off).

@@ -59,3 +59,32 @@ def test_small_tiles_equal_the_tile_kernel(monkeypatch, order, nx, nz, varden):
     d = den if varden else np.full_like(vp, 2400.0)
     ref, _, _ = ol.afd_forward(nx, nz, pml, nt, 10.0, 12.0, 1e-3, vp, d, w, nx // 2, nz // 2, rx, rz, radius=R)
     assert rel_l2(a[0][:len(rx) * nt].reshape(len(rx), nt), ref) <= 1e-5
+
+
+@pytest.mark.parametrize("order,nx,nz,varden", [(16, 47, 64, True), (16, 65, 33, False), (10, 49, 97, True),
+                                                (8, 80, 31, True), (4, 33, 95, False), (2, 129, 40, True)])
+def test_reference_order_tile_edges(order, nx, nz, varden):
+    """SFD_EXACT on the same tiles, and the same kernel reading a caller's unpadded model
+    (sfd_forward_noalloc), bit for bit against the oracle."""
+    import ctypes
+    import torch
+    pml, nt = 8, 60
+    rng = np.random.default_rng(order + nx)
+    vp = (2000.0 + 800.0 * rng.random((nx, nz))).astype(np.float32)
+    den = (1900.0 + 400.0 * rng.random((nx, nz))).astype(np.float32) if varden else None
+    w = S.wavelet(S.WAVELET_RIC, nt, 1e-3, 25.0, 25)
+    rx, rz = np.arange(nx, dtype=np.int32), np.full(nx, min(nz - 1, 13), np.int32)
+    ref, _, _ = ol.afd_forward(nx, nz, pml, nt, 10.0, 12.0, 1e-3, vp, den if varden else np.full_like(vp, 2400.0), w,
+                               nx // 2, nz // 2, rx, rz, radius=order // 2)
+    with S.Engine(S.ACOUSTIC_2D, nx, nz, 10.0, 12.0, 1e-3, pml, order=order, flags=S.EXACT) as e:
+        e.set_model(vp, den)
+        e.set_shots([S.ShotSpec(nx // 2, nz // 2, rx, rz, w)])
+        rec = e.forward().reshape(nx, nt)
+    assert np.abs(ref).max() > 0 and bits_equal(rec, ref)
+    g = S.Grid(S.ACOUSTIC_2D, nx, 1, nz, pml, 10.0, 0.0, 12.0, 1e-3, order, S.EXACT, 0.0)
+    dev = [None if a is None else torch.from_numpy(a).cuda() for a in (vp, den, w)]
+    out = torch.zeros(nx * nt, device="cuda")
+    torch.cuda.synchronize()
+    rc = S.load().sfd_forward_noalloc(ctypes.byref(g), dev[0].data_ptr(), None if den is None else dev[1].data_ptr(),
+                                      dev[2].data_ptr(), nt, nx // 2, nz // 2, nx, S._ip(rx), S._ip(rz), out.data_ptr(), None)
+    assert rc == 0 and bits_equal(out.cpu().numpy().reshape(nx, nt), ref)
