@@ -12,6 +12,8 @@
 // acoustic2d_small.cu) use FMA and agree with one another bit for bit.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "sfd_internal.h"
 
 namespace sfd {
@@ -27,7 +29,17 @@ __global__ void inject0_kernel(const __grid_constant__ Acou2DArgs a, int nshot, 
     a.p_out[c] = exact ? __fsub_rn(0.0f, __fmul_rn(sd.inj_scale, w)) : -(sd.inj_scale * w);
 }
 
+__global__ void buoyancy_kernel(const float* __restrict__ den, float c, float* __restrict__ out, long long n) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        out[i] = __fdiv_rn(c, den[i]);
+}
+
 }  // namespace
+
+cudaError_t launch_buoyancy(const float* den, float c, float* out, long long n, cudaStream_t st) {
+    buoyancy_kernel<<<(unsigned)std::min<long long>((n + 255) / 256, 148 * 16), 256, 0, st>>>(den, c, out, n);
+    return cudaGetLastError();
+}
 
 bool acoustic2d_plan(int radius, Acou2DPlan* plan) {
     if (radius != 1 && radius != 2 && radius != 4 && radius != 5 && radius != 8) return false;

@@ -229,9 +229,9 @@ __device__ __forceinline__ void tile_body(const Acou2DArgs& a, float* smem, floa
                 float2 bl = bc(-a.bx_f), bh = bl;
                 if (VARDEN) {
                     const int gx = min(max(sd.x0 + x0 - R + row, 0), a.nx_model - 1);
-                    const float4 d = __ldg(reinterpret_cast<const float4*>(a.den + (long long)gx * a.mpitch + z0 + zo));
-                    bl = make_float2(-a.dtdx / d.x, -a.dtdx / d.y);
-                    bh = make_float2(-a.dtdx / d.z, -a.dtdx / d.w);
+                    const float4 d = __ldg(reinterpret_cast<const float4*>(a.bxm + (long long)gx * a.mpitch + z0 + zo));
+                    bl = make_float2(-d.x, -d.y);
+                    bh = make_float2(-d.z, -d.w);
                 }
                 float2 vl = lo(vo), vh = hi(vo);
                 if (ADJ) {  // staged X'' = B M (X + rdx S+x nu), B = dt/(dx den) (1 here for constant density)
@@ -304,8 +304,8 @@ __device__ __forceinline__ void tile_body(const Acou2DArgs& a, float* smem, floa
                         const int zg = z0 - T::RQ + zi + kk;
                         const int g0 = min(sd.x0 + x0 + xr0, a.nx_model - 1);
                         const int g1 = min(sd.x0 + x0 + xr0 + 1, a.nx_model - 1);
-                        b0 = a.dtdz / __ldg(a.den + (long long)g0 * a.mpitch + zg);
-                        b1 = a.dtdz / __ldg(a.den + (long long)g1 * a.mpitch + zg);
+                        b0 = __ldg(a.bzm + (long long)g0 * a.mpitch + zg);
+                        b1 = __ldg(a.bzm + (long long)g1 * a.mpitch + zg);
                     }
                     if (ADJ) {  // staged Z'' = B M (Z + rdz S+z nu)
                         const float mz = EDGE ? sMz[zi + kk] : 1.0f;

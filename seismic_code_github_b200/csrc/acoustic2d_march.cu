@@ -160,8 +160,9 @@ __device__ __forceinline__ void chunk_body(const Acou2DArgs& a, float* smem, int
             float2 v = ld2(vrow);
             float2 b = bc(-a.bx_f), d = bc(a.den_c);
             if (VARDEN) {
-                d = __ldg(reinterpret_cast<const float2*>(a.den + midx(x, z0 + zo)));
-                b = make_float2(-a.dtdx / d.x, -a.dtdx / d.y);
+                if (ADJ) d = __ldg(reinterpret_cast<const float2*>(a.den + midx(x, z0 + zo)));
+                b = __ldg(reinterpret_cast<const float2*>(a.bxm + midx(x, z0 + zo)));
+                b = make_float2(-b.x, -b.y);
             }
             float ax = -1.0f, mx = 1.0f;
             if (EDGE) col_tables<R>(a, x, nx, ax, mx);
@@ -224,7 +225,8 @@ __device__ __forceinline__ void chunk_body(const Acou2DArgs& a, float* smem, int
             if (VARDEN) {
                 const int gz = z0 - VH + c0 + j;
                 const long long mi = midx(x, gz);
-                nb = make_float2(-(a.dtdz / __ldg(a.den + mi)), -(a.dtdz / __ldg(a.den + mi + 1)));
+                nb = __ldg(reinterpret_cast<const float2*>(a.bzm + mi));  // mi is even
+                nb = make_float2(-nb.x, -nb.y);
             }
             if (ADJ) {  // staged Z'' = B M (Z + rdz S+z nu)
                 const float2 mz = EDGE ? make_float2(sMz[c0 + j], sMz[c0 + j + 1]) : bc(1.0f);

@@ -218,9 +218,9 @@ __global__ void __launch_bounds__(TX * TZ / 4, 5) acoustic2d_small_kernel(const 
             float2 bl = bc(-a.bx_f), bh = bl;
             if (VARDEN) {
                 const int g = min(max(sd.x0 + x0 - R + r0 + o, 0), a.nx_model - 1);
-                const float4 d = __ldg(reinterpret_cast<const float4*>(a.den + (long long)g * a.mpitch + z0 + z));
-                bl = make_float2(-a.dtdx / d.x, -a.dtdx / d.y);
-                bh = make_float2(-a.dtdx / d.z, -a.dtdx / d.w);
+                const float4 d = __ldg(reinterpret_cast<const float4*>(a.bxm + (long long)g * a.mpitch + z0 + z));
+                bl = make_float2(-d.x, -d.y);
+                bh = make_float2(-d.z, -d.w);
             }
             const float ax = sAx[r0 + o], mx = sMx[r0 + o];
             float2 vl = lo(vo), vh = hi(vo);
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(TX * TZ / 4, 5) acoustic2d_small_kernel(const 
         const float ax = sAx[r + R], mx = sMx[r + R];
         float out[4];
         float4 d = make_float4(1.f, 1.f, 1.f, 1.f);
-        if (MODE == kExact && VARDEN) d = model4(a.den, x0 + r, z0 - T::RQ + z, 1.0f);
+        if (VARDEN) d = model4(MODE == kExact ? a.den : a.bzm, x0 + r, z0 - T::RQ + z, 1.0f);
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             if (MODE == kExact) {
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(TX * TZ / 4, 5) acoustic2d_small_kernel(const 
             for (int m = 1; m < R; m++) s = __fmaf_rn(C[m], __fsub_rn(w[T::RQ + q + 1 + m], w[T::RQ + q - m]), s);
             float b = a.bz_f;
             if (VARDEN)
-                b = a.dtdz / __ldg(a.den + (long long)min(sd.x0 + x0 + r, a.nx_model - 1) * a.mpitch + z0 - T::RQ + z + q);
+                b = comp(d, q);
             const float mk = mx * comp(mz, q);
             if (ADJ) {  // staged Z'' = B M (Z + rdz S+z nu)
                 out[q] = __fmul_rn(__fmaf_rn(a.rdz_f, s, comp(vo, q)), mk);

@@ -343,8 +343,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
                     const int row = r0 + h;
                     float4 b = make_float4(byc, byc, byc, byc);
                     if (VARDEN) {
-                        const float4 d = ld_model(a.den, s, y0 - R + row, z0 + zt);
-                        b = make_float4(a.dtdy / d.x, a.dtdy / d.y, a.dtdy / d.z, a.dtdy / d.w);
+                        b = ld_model(a.bym, s, y0 - R + row, z0 + zt);
                     }
                     const float4 vo = ld4s(st + K::OFF_VY + row * TZ + zt);
                     const float2 s01 = h ? b01.v : a01.v, s23 = h ? b23.v : a23.v;
@@ -386,8 +385,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
                         acc[c].add(m, a.coef[m - 1], w[K::BR + R - 1 + c + m], w[K::BR + R + c - m]);
                 float4 b = make_float4(bzc, bzc, bzc, bzc);
                 if (VARDEN) {
-                    const float4 d = ld_model(a.den, s, y0 + row, z0 - K::RQ + 4 * u);
-                    b = make_float4(a.dtdz / d.x, a.dtdz / d.y, a.dtdz / d.z, a.dtdz / d.w);
+                    b = ld_model(a.bzm, s, y0 + row, z0 - K::RQ + 4 * u);
                 }
                 const float4 vo = ld4s(st + K::OFF_VZ + row * K::VZW + 4 * u);
                 const float2 s01 = make_float2(acc[0].v, acc[1].v), s23 = make_float2(acc[2].v, acc[3].v);
@@ -432,8 +430,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
             }
             float4 b = make_float4(bxc, bxc, bxc, bxc);
             if (VARDEN) {
-                const float4 d = ld_model(a.den, xv, yo, zo);
-                b = make_float4(a.dtdx / d.x, a.dtdx / d.y, a.dtdx / d.z, a.dtdx / d.w);
+                b = ld_model(a.bxm, xv, yo, zo);
             }
             float4 vn, vout;
             if (ADJ) {

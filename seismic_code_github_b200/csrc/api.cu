@@ -39,6 +39,10 @@ struct sfd_ctx {
     float den_c = 2400.0f;
     float* d_vp = nullptr;
     float* d_den = nullptr;
+    // acoustic schemes with variable density: dt / (d_a den) per axis in d_den's layout, divided once per
+    // model instead of at every velocity update and its halo (axes of equal spacing share an array)
+    float* d_b[3] = {};         // distinct arrays
+    int b_of[3] = {0, 0, 0};    // array of the x, y, z axis
     float* d_q = nullptr;
     int mpitch = 0;
 
@@ -323,6 +327,7 @@ void free_shot_buffers(sfd_ctx* c) {
 sfd_ctx::~sfd_ctx() {
     if (device >= 0) cudaSetDevice(device);
     free_shot_buffers(this);
+    for (auto& p : d_b) dfree(p);
     dfree(d_vp); dfree(d_den); dfree(d_q); dfree(d_flag); dfree(d_err);
     dfree(q_busg); dfree(q_p1); dfree(q_p2); dfree(d_spg); dfree(d_itopo);
     for (auto& p : e_q) dfree(p);
@@ -357,6 +362,8 @@ Acou2DArgs make_args(const sfd_ctx* c, int step) {
     a.pml = c->g.pml;
     a.vp = c->d_vp + kModelGhostZ;  // row z = 0 of column 0
     a.den = c->varden ? c->d_den + kModelGhostZ : nullptr;
+    a.bxm = c->varden && c->d_b[0] ? c->d_b[c->b_of[0]] + kModelGhostZ : nullptr;
+    a.bzm = c->varden && c->d_b[0] ? c->d_b[c->b_of[2]] + kModelGhostZ : nullptr;
     a.one = 1.0f;
     a.mpitch = c->mpitch;
     a.nx_model = c->g.nx;
@@ -429,6 +436,9 @@ Acou3DArgs make_args3(const sfd_ctx* c, int step) {
     a.L = c->L3;
     a.vp = c->d_vp;
     a.den = c->varden ? c->d_den : nullptr;
+    a.bxm = c->d_b[c->b_of[0]];
+    a.bym = c->d_b[c->b_of[1]];
+    a.bzm = c->d_b[c->b_of[2]];
     a.den_c = c->den_c;
     a.dt = c->g.dt;
     a.rdx = 1.0f / c->g.dx; a.rdy = 1.0f / c->g.dy; a.rdz = 1.0f / c->g.dz;
@@ -2187,8 +2197,26 @@ int sfd_set_model(sfd_ctx* ctx, const float* vp, const float* den, const float* 
     if (urc) return urc;
     if (ctx->varden) {
         if ((urc = upload(&ctx->d_den, den))) return urc;
+        if (is3d || (ctx->g.scheme == SFD_ACOUSTIC_2D && !(ctx->g.flags & SFD_EXACT))) {
+            const float d[3] = {ctx->g.dx, is3d ? ctx->g.dy : ctx->g.dx, ctx->g.dz};
+            int n = 0;
+            for (int ax = 0; ax < 3; ax++) {
+                int k = 0;
+                while (k < ax && d[k] != d[ax]) k++;
+                if (k < ax) {
+                    ctx->b_of[ax] = ctx->b_of[k];
+                    continue;
+                }
+                ctx->b_of[ax] = n;
+                if (!ctx->d_b[n]) CK(cudaMalloc(&ctx->d_b[n], mfloats * sizeof(float)));
+                CK(launch_buoyancy(ctx->d_den, ctx->g.dt / d[ax], ctx->d_b[n], (long long)mfloats, ctx->stream));
+                n++;
+            }
+            CK(cudaStreamSynchronize(ctx->stream));
+        }
     } else {
         dfree(ctx->d_den);
+        for (auto& p : ctx->d_b) dfree(p);
     }
     if (ctx->g.scheme == SFD_ELASTIC_2D) {
         // YPUB:323-634 per shot window: staggered moduli and buoyancies, smoothed top sponge

@@ -286,6 +286,8 @@ struct Acou2DArgs {
     int pml;
     const float* vp;        // model, (nx_model x mpitch)
     const float* den;       // NULL for constant density
+    const float* bxm;       // variable density: dtdx / den and dtdz / den in den's layout (not with SFD_EXACT)
+    const float* bzm;
     int mpitch;
     int nx_model;
     int model_raw;          // SFD_EXACT only: vp and den are the caller's arrays (no ghost rows, any alignment)
@@ -390,6 +392,8 @@ inline bool acoustic2d_use_march(const Acou2DPlan& plan, const Layout2D& L, int 
 cudaError_t acoustic2d_small_launch(int radius, const Acou2DArgs& a, int active, bool varden, cudaStream_t st, bool adj);
 bool acoustic2d_use_small(const Acou2DPlan& plan, const Layout2D& L, int active);
 // SFD_EXACT: the reference's operation order
+// out[i] = c / den[i] (rounded to nearest)
+cudaError_t launch_buoyancy(const float* den, float c, float* out, long long n, cudaStream_t st);
 cudaError_t acoustic2d_exact_launch(int radius, const Acou2DArgs& a, int active, bool varden, cudaStream_t st);
 cudaError_t acoustic2d_fwd_launch(const Acou2DPlan& plan, int radius, const Acou2DArgs& a, int active, bool varden,
                                   cudaStream_t st);
@@ -448,6 +452,7 @@ struct Acou3DArgs {
     const float* p_in; const float* vx_in;
     float* p_out; float* vx_out; float* vy_out; float* vz_out;
     const float* vp; const float* den;  // model in the field layout (one shot); den NULL = constant
+    const float* bxm; const float* bym; const float* bzm;  // variable density: dt / (d_a den)
     float den_c, dt;
     float rdx, rdy, rdz;                // 1/dx, 1/dy, 1/dz
     float dtdx, dtdy, dtdz;             // dt/dx, dt/dy, dt/dz

@@ -12,3 +12,22 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("nx,order,varden", [(9, 8, False), (13, 8, True), (23, 8, False), (42, 4, True), (75, 8, True)])
 def test_segment_edges(nx, order, varden):
     check_case(nx, 37, 66, 3, 60, (nx // 2, 18, 30), seed=nx, order=order, varden=varden)
+
+
+def test_unequal_spacing_with_variable_density():
+    """Each axis has its own precomputed dt / (d den)."""
+    import numpy as np
+    import oracle_lib as ol
+    from conftest import rel_l2
+    from seismic_code_github_b200 import seisfd as S
+    from test_acoustic3d_gpu import TOL, model3d, receivers
+    nx, ny, nz, pml, nt = 30, 37, 41, 5, 60
+    vp, den = model3d(nx, ny, nz, 8, varden=True)
+    rx, ry, rz = receivers(nx, ny, nz, 8)
+    w = S.wavelet(S.WAVELET_RIC, nt, 1e-3, 25.0, 25)
+    with S.Engine(S.ACOUSTIC_3D, nx, nz, 10.0, 9.0, 1e-3, pml, order=8, ny=ny, dy=12.0) as e:
+        e.set_model(vp, den)
+        e.set_shots([S.ShotSpec(14, 20, rx, rz, w, sy=18, rec_y=ry)])
+        rec = e.forward().reshape(len(rx), nt)
+    ref, _ = ol.afd3d_forward(vp, den, w, (14, 18, 20), rx, ry, rz, pml, 10.0, 12.0, 9.0, 1e-3, radius=4)
+    assert np.abs(ref).max() > 0 and rel_l2(rec, ref) <= TOL
