@@ -32,6 +32,7 @@
 #include <type_traits>
 
 #include "sfd_internal.h"
+#include "tile_stage.cuh"
 
 namespace sfd {
 namespace {
@@ -199,6 +200,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
     using K = K3<R>;
     extern __shared__ __align__(128) float smem[];
     const int tid = threadIdx.x;
+    tile::release();
     const Layout3D& L = a.L;
     const int nx = L.nx, ny = L.ny, nz = L.nz;
     const int shot = a.slot_to_shot[blockIdx.y];
@@ -263,6 +265,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    tile::acquire();
     // The CTA's planes [xs, s_end).  iteration s: new Vx on plane s+R-1 (own points), then, for
     // s >= xs, new Vy / Vz on plane s (column + halo) and new P on plane s.  The iterations before
     // xs only fill the Vx ring (each thread its own slots: no staged box, no barrier) with planes
@@ -543,6 +546,8 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
 
 __global__ void inject3d_kernel(float* p, Layout3D L, const ShotDev* shots, const int* slot_to_shot, int active,
                                 const float* wavelets, int step, int by_slot) {
+    tile::release();
+    tile::acquire();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= active) return;
     const ShotDev sd = shots[slot_to_shot[i]];
@@ -556,6 +561,8 @@ __global__ void inject3d_kernel(float* p, Layout3D L, const ShotDev* shots, cons
 __global__ void gather3d_kernel(const float* p, Layout3D L, const ShotDev* shots, const int* slot_to_shot,
                                 const int* rec_x, const int* rec_y, const int* rec_z, float* records, int step,
                                 int by_slot) {
+    tile::release();
+    tile::acquire();
     const int shot = slot_to_shot[blockIdx.y];
     const ShotDev sd = shots[shot];
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -569,6 +576,8 @@ __global__ void gather3d_kernel(const float* p, Layout3D L, const ShotDev* shots
 // adjoint of the receiver gather: nu[receiver] += M a K res[step] (M = 1 where the step updates P)
 __global__ void adj_inject3d_kernel(float* nu, const Acou3DArgs a, const int* rec_x, const int* rec_y,
                                     const int* rec_z, const float* res) {
+    tile::release();
+    tile::acquire();
     const int shot = a.slot_to_shot[blockIdx.y];
     const ShotDev sd = a.shots[shot];
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -635,8 +644,8 @@ cudaError_t launch_t(const Acou3DArgs& a, int active, cudaStream_t st) {
     if (cudaError_t e = smem_attr_once((const void*)k, (int)smem, attr)) return e;
     const int seg = segment_planes(a.L, active, R), nseg = (a.L.nx - 2 * R + seg - 1) / seg;
     const dim3 grid(a.L.nty * a.L.ntz, active, nseg);
-    k<<<grid, kThreads, smem, st>>>(a, seg);
-    return cudaGetLastError();
+    void* args[] = {const_cast<Acou3DArgs*>(&a), const_cast<int*>(&seg)};
+    return tile::launch((const void*)k, grid, kThreads, smem, st, args);
 }
 
 template <int R>
@@ -676,9 +685,9 @@ bool acoustic3d_boxes(int radius, int bp[2], int bvy[2], int bvz[2]) {
 cudaError_t acoustic3d_launch_inject(float* p, const Layout3D& L, const ShotDev* shots, const int* slot_to_shot,
                                      int active, const float* wavelets, int step, cudaStream_t st, int slab_by_slot) {
     if (active <= 0) return cudaSuccess;
-    inject3d_kernel<<<(active + 63) / 64, 64, 0, st>>>(p, L, shots, slot_to_shot, active, wavelets, step,
-                                                       slab_by_slot);
-    return cudaGetLastError();
+    Layout3D l = L;
+    void* args[] = {&p, &l, &shots, &slot_to_shot, &active, &wavelets, &step, &slab_by_slot};
+    return tile::launch((const void*)inject3d_kernel, dim3((active + 63) / 64), 64, 0, st, args);
 }
 
 cudaError_t acoustic3d_launch_gather(const float* p, const Layout3D& L, const ShotDev* shots,
@@ -687,9 +696,9 @@ cudaError_t acoustic3d_launch_gather(const float* p, const Layout3D& L, const Sh
                                      int slab_by_slot) {
     if (active <= 0 || nrec_max <= 0) return cudaSuccess;
     const dim3 grid((nrec_max + 255) / 256, active);
-    gather3d_kernel<<<grid, 256, 0, st>>>(p, L, shots, slot_to_shot, rec_x, rec_y, rec_z, records, step,
-                                          slab_by_slot);
-    return cudaGetLastError();
+    Layout3D l = L;
+    void* args[] = {&p, &l, &shots, &slot_to_shot, &rec_x, &rec_y, &rec_z, &records, &step, &slab_by_slot};
+    return tile::launch((const void*)gather3d_kernel, grid, 256, 0, st, args);
 }
 
 cudaError_t acoustic3d_launch_adj_inject(float* nu, const Acou3DArgs& a, const int* rec_x, const int* rec_y,
@@ -697,8 +706,8 @@ cudaError_t acoustic3d_launch_adj_inject(float* nu, const Acou3DArgs& a, const i
                                          cudaStream_t st) {
     if (active <= 0 || nrec_max <= 0) return cudaSuccess;
     const dim3 grid((nrec_max + 255) / 256, active);
-    adj_inject3d_kernel<<<grid, 256, 0, st>>>(nu, a, rec_x, rec_y, rec_z, res);
-    return cudaGetLastError();
+    void* args[] = {&nu, const_cast<Acou3DArgs*>(&a), &rec_x, &rec_y, &rec_z, &res};
+    return tile::launch((const void*)adj_inject3d_kernel, grid, 256, 0, st, args);
 }
 
 cudaError_t acoustic3d_launch_gradient_reduce(const double* acc, int nslab, const Layout3D& L, const float* vp,
