@@ -84,6 +84,8 @@ struct sfd_ctx {
     CUtensorMap tmaps[6];      // TMA descriptors: P0 P1 VX0 VX1 VZ0 VZ1
     CUtensorMap mtmaps[6];     // the same buffers with the x-marching kernel's boxes
     CUtensorMap etmaps[5];     // elastic schemes: sums vx vz sxx szz sxz (elastic2d.cu / viscoel2d.cu box)
+    CUtensorMap q_maps[3];     // viscoacoustic reference-order step: vx, vz, sigma (q_box)
+    CUtensorMap q_adj_maps[4]; // ... its adjoint: T1, T4, Qx, Qz
     CUtensorMap qtmaps[2];     // default viscoacoustic step: sigma S0 S1 (viscoac2d_fast.cu box)
 
     // 3-D scheme: dense [x][y][pitch] slabs, 8 fields (P, Vx, Vy, Vz, two buffers each)
@@ -151,7 +153,7 @@ struct sfd_ctx {
     int grad_keep = 0;          // first segment whose D_k the first forward keeps (no recomputation)
     float* d_ckpt = nullptr;    // [ncp][3 fields][nshot * shot_stride]
     float* d_div = nullptr;     // D_k slots: [C] of the segment being recomputed, then the kept tail
-    float* d_adj = nullptr;     // adjoint state: nu0 nu1 x0 x1 z0 z1 (viscoacoustic: 8 adjoints + Qx Qz)
+    float* d_adj = nullptr;     // adjoint state: nu0 nu1 x0 x1 z0 z1 (viscoacoustic: 8 adjoints + Qx Qz T1 T4)
     CUtensorMap adj_tmaps[6];   // TMA descriptors of the acoustic adjoint buffers
     CUtensorMap adj_mtmaps[6];  // the same buffers with the x-marching kernel's boxes
     float* d_gseg = nullptr;    // per-segment imaging sum (float)
@@ -478,8 +480,13 @@ QFastArgs make_qfast(const sfd_ctx* c, int step) {
 QArgs make_qargs(const sfd_ctx* c, int step) {
     QArgs a{};
     const long long fs = (long long)c->nshot * c->L.shot_stride;
-    float* f[8];
-    for (int i = 0; i < 8; i++) f[i] = c->d_state + i * fs;
+    float* f[9];
+    for (int i = 0; i < 9; i++) f[i] = c->d_state + i * fs;
+    a.sg = f[8];
+    a.tm_vx = c->q_maps[0];
+    a.tm_vz = c->q_maps[1];
+    a.tm_s = c->q_maps[2];
+    a.err_flag = c->d_err;
     a.vx = f[0]; a.vz = f[1]; a.sx = f[2]; a.sz = f[3]; a.sr = f[4]; a.rx = f[5]; a.rz = f[6]; a.rr = f[7];
     a.L = c->L;
     a.nz = c->g.nz;
@@ -961,13 +968,13 @@ double q_kappa(float f0) {
 // ---------------------------------------------------------------------------------------------
 // Per scheme: fields kept in a checkpoint, forward derivatives kept per recomputed step,
 // adjoint fields, imaging sums.  Acoustic: P, Vx, Vz (one parity) / D / Q, X, Z ping-pong /
-// g.  Viscoacoustic: the eight in-place fields / Dx1 vx, Dz1 vz / eight adjoints + Qx, Qz /
+// g.  Viscoacoustic: the eight in-place fields and sigma / Dx1 vx, Dz1 vz / eight adjoints + Qx, Qz, T1, T4 /
 // g1, g2.
 struct GradShape {
     int ckpt, div, adj, img;
 };
 GradShape grad_shape(const sfd_ctx* c) {
-    return c->g.scheme == SFD_VISCOAC_2D ? GradShape{8, 2, 10, 2} : GradShape{3, 1, 6, 1};
+    return c->g.scheme == SFD_VISCOAC_2D ? GradShape{9, 2, 12, 2} : GradShape{3, 1, 6, 1};
 }
 
 int grad_alloc(sfd_ctx* ctx) {
@@ -1004,6 +1011,12 @@ int grad_alloc(sfd_ctx* ctx) {
             }
         }
         if (ctx->g.scheme == SFD_VISCOAC_2D) {
+            const int slab[4] = {10, 11, 8, 9};  // T1, T4, Qx, Qz
+            int box[2];
+            q_box(box);
+            for (int f = 0; f < 4; f++)
+                if (int rc = encode_field_map(ctx, &ctx->q_adj_maps[f], ctx->d_adj + slab[f] * fs, ctx->L, ctx->nshot, box))
+                    return rc;
             CK(cudaMalloc(&ctx->d_grad2, sizeof(double) * (size_t)ctx->g.nx * ctx->g.nz));
             CK(cudaMalloc(&ctx->d_apx0, sizeof(int) * ctx->nshot));
             CK(cudaMemcpy(ctx->d_apx0, ctx->h_ap_x0.data(), sizeof(int) * ctx->nshot, cudaMemcpyHostToDevice));
@@ -1085,6 +1098,10 @@ QAdjArgs make_qadj(const sfd_ctx* ctx, const GradRange& r, int k, const float* d
     float* A = ctx->d_adj;
     a.avx = A; a.avz = A + fs; a.asx = A + 2 * fs; a.asz = A + 3 * fs; a.asr = A + 4 * fs;
     a.arx = A + 5 * fs; a.arz = A + 6 * fs; a.arr = A + 7 * fs; a.qx = A + 8 * fs; a.qz = A + 9 * fs;
+    a.t1 = A + 10 * fs; a.t4 = A + 11 * fs;
+    a.tm_t1 = ctx->q_adj_maps[0]; a.tm_t4 = ctx->q_adj_maps[1];
+    a.tm_qx = ctx->q_adj_maps[2]; a.tm_qz = ctx->q_adj_maps[3];
+    a.err_flag = ctx->d_err;
     a.d1 = div;
     a.d4 = div ? div + fs : nullptr;
     a.g1 = ctx->d_gseg;
@@ -1165,7 +1182,7 @@ int grad_adj_step(sfd_ctx* ctx, const GradRange& r, int k, int act, const float*
 int grad_copy_state(sfd_ctx* ctx, const GradRange& r, int slot, int b, bool to_ckpt) {
     const size_t fs = (size_t)ctx->nshot * ctx->L.shot_stride;
     const size_t off = (size_t)r.first * ctx->L.shot_stride, len = (size_t)r.count * ctx->L.shot_stride;
-    const bool visco = ctx->g.scheme == SFD_VISCOAC_2D;  // eight in-place fields, no parity
+    const bool visco = ctx->g.scheme == SFD_VISCOAC_2D;  // nine in-place fields, no parity
     const int nf = grad_shape(ctx).ckpt;
     for (int f = 0; f < nf; f++) {
         float* st = ctx->d_state + (visco ? f : 2 * f + b) * fs + off;
@@ -2444,7 +2461,7 @@ int sfd_set_shots(sfd_ctx* ctx, int nshot, const sfd_shot* shots) {
         CK(cudaMalloc(&ctx->d_rec2_tn, rec_bytes));
         CK(cudaMalloc(&ctx->d_rec2_nt, rec_bytes));
     }
-    ctx->state_floats = (iso ? I_NFIELDS : elastic ? E_NFIELDS : q_fast(ctx) ? kQFastSlabs : visco ? 8 : 6) *
+    ctx->state_floats = (iso ? I_NFIELDS : elastic ? E_NFIELDS : q_fast(ctx) ? kQFastSlabs : visco ? 9 : 6) *
                         (size_t)nshot * L.shot_stride;
     CK(cudaMalloc(&ctx->d_state, ctx->state_floats * sizeof(float)));
     CK(cudaMalloc(&ctx->d_src_pre, sizeof(float) * nshot));
@@ -2463,6 +2480,12 @@ int sfd_set_shots(sfd_ctx* ctx, int nshot, const sfd_shot* shots) {
             else viscoel2d_box(box);
             float* base = ctx->d_state + ((iso ? (int)I_VX : (int)E_VX) + f) * (long long)nshot * L.shot_stride;
             if ((rc = encode_field_map(ctx, &ctx->etmaps[f], base, L, nshot, box))) return rc;
+        }
+        for (int f = 0; ctx->g.scheme == SFD_VISCOAC_2D && f < 3; f++) {
+            int box[2];
+            q_box(box);
+            float* base = ctx->d_state + (f < 2 ? f : 8) * (long long)nshot * L.shot_stride;
+            if ((rc = encode_field_map(ctx, &ctx->q_maps[f], base, L, nshot, box))) return rc;
         }
         if (q_fast(ctx)) {
             int bs[2];

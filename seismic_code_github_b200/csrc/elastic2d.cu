@@ -98,12 +98,11 @@ struct TileRef {
 
 // CTA b covers TC columns; t.tile is the 64 x 64 tile (of the receiver lists) that holds them
 __device__ __forceinline__ bool tile_of(const IArgs& a, TileRef& t) {
-    t.shot = a.slot_to_shot[blockIdx.y];
+    t.shot = a.slot_to_shot[blockIdx.z];
     t.sd = a.shots[t.shot];
-    const int tx_i = blockIdx.x / a.L.ntz, tz_i = blockIdx.x - tx_i * a.L.ntz;
-    t.x0 = tx_i * TC;
-    t.z0 = tz_i * TZ;
-    t.tile = t.x0 / TX * a.L.ntz + tz_i;
+    t.x0 = blockIdx.y * TC;
+    t.z0 = blockIdx.x * TZ;
+    t.tile = t.x0 / TX * a.L.ntz + blockIdx.x;
     return t.x0 < t.sd.nx;
 }
 
@@ -572,7 +571,7 @@ namespace {
 
 template <bool FS>
 cudaError_t launch_pair(const IArgs& a, int active, cudaStream_t st) {
-    const dim3 grid(a.L.ntx * (TX / TC) * a.L.ntz, active);
+    const dim3 grid(a.L.ntz, a.L.ntx * (TX / TC), active);
     const int sv = (int)sizeof(float) * (3 * kSmem + 4), ss = (int)sizeof(float) * (2 * kSmem + 4);
     const void* kv = (const void*)iso_velocity_kernel<FS>;
     const void* ks = (const void*)iso_stress_kernel<FS>;

@@ -13,36 +13,38 @@
 //   record = S at the receivers
 // Adjoint step k (hatted fields hold d misfit / d state after step k, with the residual of
 // step k already added at the receivers to sx^, sz^, sr^):
-//   kernel A: T1 = A'x (dt p1 sx^ + f p2 rx^), T4 = A'z (dt p1 sz^ + f p2 rz^)   (on a halo)
-//             vx^ = Ax (vx^ + Dx1^T T1),  vz^ = Az (vz^ + Dz1^T T4)
+//   T1 = A'x (dt p1 sx^ + f p2 rx^), T4 = A'z (dt p1 sz^ + f p2 rz^), kept as slabs by kernel B
+//   kernel A: vx^ = Ax (vx^ + Dx1^T T1),  vz^ = Az (vz^ + Dz1^T T4)
 //             Qx = dt b vx^, Qz = dt b vz^;   dw_k = sum stamp sx^
 //   kernel B: u1 = A'x sx^, u4 = A'z sz^, w1 = A'x rx^, w4 = A'z rz^, aR = f rr^ + dt sr^
 //             aS = Dx0^T Qx + Dz0^T Qz
 //             sx^ = u1 + aS, sz^ = u4 + aS, sr^ += aS, rx^ = w1 + aR, rz^ = w4 + aR, rr^ += aR
 //             g1 += d1 u1 + d4 u4,  g2 += d1 w1 + d4 w4;   then sx^, sz^, sr^ += res_{k-1}
 // so that d misfit / d p1 = dt sum g1 and d misfit / d p2 = f sum g2.  The transposed
-// rotated-staggered derivatives gather from the mirrored taps of QS:843-966.  Kernel A reads
-// the stress adjoints of its halo and writes only velocity adjoints and Qx, Qz; kernel B reads
-// the Qx, Qz halo and writes only its own cells, so neither launch races with itself.
+// rotated-staggered derivatives gather from the mirrored taps of QS:843-966.  Kernel A reads the halo of
+// T1, T4 and writes only velocity adjoints and Qx, Qz; kernel B reads the halo of Qx, Qz and writes only
+// its own cells (its receivers' residuals go to sx^, sz^, sr^ and, through the same factors, to T1 and
+// T4), so neither launch races with itself.
+//
+// Bound: memory (132 B a cell).  Each kernel's two differentiated fields arrive by TMA on tiles of 64 rows
+// by 8 columns with two cells per thread, as in viscoac2d.cu (measurements there); before, kernel A staged
+// six arrays with their halo to form T1 and T4 again.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 
 #include "sfd_internal.h"
+#include "tile_stage.cuh"
 
 namespace sfd {
 namespace {
 
-constexpr int kThreads = 256;
 constexpr int TX = kTileX, TZ = kTileZ;
+constexpr int TC = kQCols, kThreads = TC * TZ / 2;  // columns of a tile, two cells per thread (TC / 2 columns apart)
 constexpr int H = 5;               // rotated-staggered reach (offsets -5 .. +5)
-constexpr int HZ = 8;              // z halo rounded for float4 staging
-constexpr int SROWS = TX + 2 * H;  // staged rows x0-5 .. x0+TX+4
+constexpr int HZ = 8;              // z halo rounded to 16 bytes
 constexpr int SW = TZ + 2 * HZ;    // staged columns z0-8 .. z0+TZ+7
-constexpr int SMEM = SROWS * SW;
-constexpr int kPer = TX * TZ / kThreads;  // cells per thread
-constexpr int kNB = 4;    // cells per load batch
-constexpr int kNBS = 2;  // cells per load batch of the stress kernel (three CTAs per SM)
+constexpr int SMEM = (TC + 2 * H) * SW;
 
 struct Tile {
     int shot, tile, x0, z0;
@@ -50,12 +52,11 @@ struct Tile {
 };
 
 __device__ __forceinline__ bool tile_of(const QAdjArgs& a, Tile& t) {
-    t.shot = a.slot_to_shot[blockIdx.y];
+    t.shot = a.slot_to_shot[blockIdx.z];
     t.sd = a.shots[t.shot];
-    t.tile = blockIdx.x;
-    const int tx_i = t.tile / a.L.ntz, tz_i = t.tile - tx_i * a.L.ntz;
-    t.x0 = tx_i * TX;
-    t.z0 = tz_i * TZ;
+    t.x0 = blockIdx.y * TC;
+    t.z0 = blockIdx.x * TZ;
+    t.tile = t.x0 / TX * a.L.ntz + blockIdx.x;  // the 64 x 64 tile of the receiver lists
     return t.x0 < t.sd.nx;
 }
 
@@ -71,210 +72,188 @@ __device__ __forceinline__ float sp(int x, int n, int np, const float* tn, const
     return f;
 }
 
-__global__ void __launch_bounds__(kThreads) q_adj_velocity_kernel(const __grid_constant__ QAdjArgs a) {
-    __shared__ __align__(16) float sT1[SMEM];
-    __shared__ __align__(16) float sT4[SMEM];
+// residual v of one receiver into the stress adjoints of cell (x, z) and their share of T1, T4
+// (several receivers may share a cell, so the adds are atomic)
+__device__ __forceinline__ void add_residual(const QAdjArgs& a, int shot, const ShotDev& sd, int x, int z, float v) {
+    const long long c = cell(a, shot, x, z);
+    const float* tb = a.spg;
+    const int st = a.spg_stride;
+    const float d1 = a.dt * __ldg(a.p1 + (long long)min(sd.x0 + x, a.nx_model - 1) * a.mpitch + z);
+    atomicAdd(a.asx + c, v);
+    atomicAdd(a.asz + c, v);
+    atomicAdd(a.asr + c, v);
+    atomicAdd(a.t1 + c, sp(x, sd.nx, a.npx, tb + 4 * st, tb + 5 * st) * (d1 * v));
+    atomicAdd(a.t4 + c, sp(z, a.nz, a.npz, tb + 6 * st, tb + 7 * st) * (d1 * v));
+}
+
+__global__ void __launch_bounds__(kThreads, 8) q_adj_velocity_kernel(const __grid_constant__ QAdjArgs a) {
+    __shared__ __align__(128) float sT[2 * SMEM];
+    __shared__ uint64_t bar;
     __shared__ float s_dw;
     Tile t;
-    if (!tile_of(a, t)) return;
+    const bool on = tile_of(a, t);
+    if (threadIdx.x == 0) s_dw = 0.0f;
+    tile::bar_init(&bar);
+    tile::release();
+    tile::acquire();
+    if (!on) return;
+    if (threadIdx.x == 0) {  // zero outside the grid: the forward never updates there
+        tile::expect(&bar, 8u * SMEM);
+        tile::box(sT, &a.tm_t1, a.L.gz + t.z0 - HZ, a.L.gx + t.x0 - H, t.shot, &bar);
+        tile::box(sT + SMEM, &a.tm_t4, a.L.gz + t.z0 - HZ, a.L.gx + t.x0 - H, t.shot, &bar);
+    }
     const int nx = t.sd.nx, nz = a.nz;
     const float* tb = a.spg;
     const int st = a.spg_stride;
-    const float dt = a.dt, f = a.f_mem;
-    if (threadIdx.x == 0) s_dw = 0.0f;
-    // T1, T4 on the tile plus halo (zero outside the grid: the forward never updates there)
-    constexpr int W4 = SW / 4;
-#pragma unroll 3  // several rows' loads in flight before their shared-memory stores
-    for (int i = threadIdx.x; i < SROWS * W4; i += kThreads) {
-        const int r = i / W4, c = i - r * W4;
-        const int gx = t.x0 - H + r, gz0 = t.z0 - HZ + 4 * c;
-        float4 o1 = make_float4(0.f, 0.f, 0.f, 0.f), o4 = o1;
-        if (gx >= 0 && gx < nx && gz0 + 3 >= 0 && gz0 < nz) {
-            const long long off = cell(a, t.shot, gx, gz0);
-            const float4 SX = __ldg(reinterpret_cast<const float4*>(a.asx + off));
-            const float4 RX = __ldg(reinterpret_cast<const float4*>(a.arx + off));
-            const float4 SZ = __ldg(reinterpret_cast<const float4*>(a.asz + off));
-            const float4 RZ = __ldg(reinterpret_cast<const float4*>(a.arz + off));
-            const long long mi = (long long)min(t.sd.x0 + gx, a.nx_model - 1) * a.mpitch + gz0;
-            const float4 P1 = __ldg(reinterpret_cast<const float4*>(a.p1 + mi));
-            const float4 P2 = __ldg(reinterpret_cast<const float4*>(a.p2 + mi));
-            const float ax = sp(gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
-            const float sx_[4] = {SX.x, SX.y, SX.z, SX.w}, rx_[4] = {RX.x, RX.y, RX.z, RX.w};
-            const float sz_[4] = {SZ.x, SZ.y, SZ.z, SZ.w}, rz_[4] = {RZ.x, RZ.y, RZ.z, RZ.w};
-            const float p1_[4] = {P1.x, P1.y, P1.z, P1.w}, p2_[4] = {P2.x, P2.y, P2.z, P2.w};
-            float v1[4], v4[4];
+    const int r0 = threadIdx.x / TZ, z = threadIdx.x % TZ, gz = t.z0 + z;
+    const long long c0 = cell(a, t.shot, t.x0 + r0, gz);
+    bool in[2];
+    float vxo[2], vzo[2], bu[2];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int gz = gz0 + j;
-                const bool ok = gz >= 0 && gz < nz;
-                const float az = ok ? sp(gz, nz, a.npz, tb + 6 * st, tb + 7 * st) : 0.0f;
-                const float d1 = dt * p1_[j], d2 = f * p2_[j];
-                v1[j] = ok ? ax * fmaf(d1, sx_[j], d2 * rx_[j]) : 0.0f;
-                v4[j] = ok ? az * fmaf(d1, sz_[j], d2 * rz_[j]) : 0.0f;
-            }
-            o1 = make_float4(v1[0], v1[1], v1[2], v1[3]);
-            o4 = make_float4(v4[0], v4[1], v4[2], v4[3]);
+    for (int u = 0; u < 2; u++) {
+        const int gx = t.x0 + r0 + u * (TC / 2);
+        const long long c = c0 + (long long)u * (TC / 2) * a.L.pitch;
+        in[u] = gx < nx && gz < nz;
+        if (in[u]) {
+            vxo[u] = a.avx[c];
+            vzo[u] = a.avz[c];
+            bu[u] = __ldg(a.busg + (long long)min(t.sd.x0 + gx, a.nx_model - 1) * a.mpitch + gz);
         }
-        *reinterpret_cast<float4*>(sT1 + r * SW + 4 * c) = o1;
-        *reinterpret_cast<float4*>(sT4 + r * SW + 4 * c) = o4;
     }
-    __syncthreads();
-    float c[5];
+    if (!tile::staged(&bar, a.err_flag)) return;
 #pragma unroll
-    for (int m = 0; m < 5; m++) c[m] = a.a[m];
-    // kNB cells per batch: the global loads of a batch are issued before its arithmetic
-    for (int j0 = 0; j0 < kPer; j0 += kNB) {
-        float vxo[kNB], vzo[kNB], bu[kNB];
-        long long cc[kNB];
-        bool ok[kNB];
+    for (int u = 0; u < 2; u++) {
+        if (!in[u]) continue;
+        const int r = r0 + u * (TC / 2), gx = t.x0 + r;
+        const long long c = c0 + (long long)u * (TC / 2) * a.L.pitch;
+        const float* p1s = sT + (r + H) * SW + z + HZ;
+        const float* p4s = p1s + SMEM;
+        auto T1 = [&](int dx, int dz) { return p1s[dx * SW + dz]; };
+        auto T4 = [&](int dx, int dz) { return p4s[dx * SW + dz]; };
+        float s1 = 0.0f, s4 = 0.0f;
 #pragma unroll
-        for (int u = 0; u < kNB; u++) {
-            const int i = threadIdx.x + (j0 + u) * kThreads, r = i / TZ, z = i - r * TZ;
-            const int gx = t.x0 + r, gz = t.z0 + z;
-            ok[u] = gx < nx && gz < nz;
-            cc[u] = cell(a, t.shot, gx, gz);
-            if (ok[u]) {
-                vxo[u] = a.avx[cc[u]];
-                vzo[u] = a.avz[cc[u]];
-                bu[u] = __ldg(a.busg + (long long)min(t.sd.x0 + gx, a.nx_model - 1) * a.mpitch + gz);
-            }
+        for (int m = 0; m < 5; m++) {
+            // Dx1^T: t(x-1-m, z-1-m) - t(x+m, z+m) + t(x-1-m, z+m) - t(x+m, z-1-m); Dz1^T flips the cross terms
+            const float a1 = T1(-1 - m, -1 - m) - T1(m, m), b1 = T1(-1 - m, m) - T1(m, -1 - m);
+            const float a4 = T4(-1 - m, -1 - m) - T4(m, m), b4 = T4(-1 - m, m) - T4(m, -1 - m);
+            s1 = fmaf(a.a[m], a1 + b1, s1);
+            s4 = fmaf(a.a[m], a4 - b4, s4);
         }
-#pragma unroll
-        for (int u = 0; u < kNB; u++) {
-            if (!ok[u]) continue;
-            const int i = threadIdx.x + (j0 + u) * kThreads, r = i / TZ, z = i - r * TZ;
-            const int gx = t.x0 + r, gz = t.z0 + z;
-            const float* p1s = sT1 + (r + H) * SW + z + HZ;
-            const float* p4s = sT4 + (r + H) * SW + z + HZ;
-            auto T1 = [&](int dx, int dz) { return p1s[dx * SW + dz]; };
-            auto T4 = [&](int dx, int dz) { return p4s[dx * SW + dz]; };
-            float s1 = 0.0f, s4 = 0.0f;
-#pragma unroll
-            for (int m = 0; m < 5; m++) {
-                // Dx1^T: t(x-1-m, z-1-m) - t(x+m, z+m) + t(x-1-m, z+m) - t(x+m, z-1-m); Dz1^T flips the cross terms
-                const float a1 = T1(-1 - m, -1 - m) - T1(m, m), b1 = T1(-1 - m, m) - T1(m, -1 - m);
-                const float a4 = T4(-1 - m, -1 - m) - T4(m, m), b4 = T4(-1 - m, m) - T4(m, -1 - m);
-                s1 = fmaf(c[m], a1 + b1, s1);
-                s4 = fmaf(c[m], a4 - b4, s4);
-            }
-            const float ax = sp(gx, nx, a.npx, tb + 0 * st, tb + 1 * st);
-            const float az = sp(gz, nz, a.npz, tb + 2 * st, tb + 3 * st);
-            const float vx = ax * fmaf(a.hx, s1, vxo[u]);
-            const float vz = az * fmaf(a.hz, s4, vzo[u]);
-            const float db = dt * bu[u];
-            a.avx[cc[u]] = vx;
-            a.avz[cc[u]] = vz;
-            a.qx[cc[u]] = db * vx;
-            a.qz[cc[u]] = db * vz;
-        }
+        const float ax = sp(gx, nx, a.npx, tb + 0 * st, tb + 1 * st);
+        const float az = sp(gz, nz, a.npz, tb + 2 * st, tb + 3 * st);
+        const float vx = ax * fmaf(a.hx, s1, vxo[u]);
+        const float vz = az * fmaf(a.hz, s4, vzo[u]);
+        const float db = a.dt * bu[u];
+        a.avx[c] = vx;
+        a.avz[c] = vz;
+        a.qx[c] = db * vx;
+        a.qz[c] = db * vz;
     }
     // wavelet gradient: dw_k = dt / dz^2 sum over the source stamp of sx^ (QS:1384 transposed)
     const ShotDev& sd = t.sd;
-    const int bx0 = max(sd.stamp_x0, t.x0), bx1 = min(sd.stamp_x0 + sd.stamp_w, min(t.x0 + TX, nx));
+    const int bx0 = max(sd.stamp_x0, t.x0), bx1 = min(sd.stamp_x0 + sd.stamp_w, min(t.x0 + TC, nx));
     const int bz0 = max(sd.stamp_z0, t.z0), bz1 = min(sd.stamp_z0 + sd.stamp_h, min(t.z0 + TZ, nz));
     if (a.lam_src && bx1 > bx0 && bz1 > bz0) {
         const int w = bz1 - bz0;
         float part = 0.0f;
         for (int i = threadIdx.x; i < (bx1 - bx0) * w; i += kThreads) {
-            const int x = bx0 + i / w, z = bz0 + i % w;
-            const float g = __ldg(a.stamps + sd.stamp_off + (x - sd.stamp_x0) * sd.stamp_h + (z - sd.stamp_z0));
-            part = fmaf(g, a.asx[cell(a, t.shot, x, z)], part);
+            const int x = bx0 + i / w, zz = bz0 + i % w;
+            const float g = __ldg(a.stamps + sd.stamp_off + (x - sd.stamp_x0) * sd.stamp_h + (zz - sd.stamp_z0));
+            part = fmaf(g, a.asx[cell(a, t.shot, x, zz)], part);
         }
         for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
-        __syncthreads();
         if ((threadIdx.x & 31) == 0) atomicAdd(&s_dw, part);
         __syncthreads();
-        if (threadIdx.x == 0) atomicAdd(a.lam_src + (long long)t.shot * a.nt_max + a.step, s_dw * (dt / a.dz2));
+        if (threadIdx.x == 0) atomicAdd(a.lam_src + (long long)t.shot * a.nt_max + a.step, s_dw * (a.dt / a.dz2));
     }
 }
 
-__global__ void __launch_bounds__(kThreads, 3) q_adj_stress_kernel(const __grid_constant__ QAdjArgs a) {
-    __shared__ __align__(16) float sQx[SMEM];
-    __shared__ __align__(16) float sQz[SMEM];
+__global__ void __launch_bounds__(kThreads, 5) q_adj_stress_kernel(const __grid_constant__ QAdjArgs a) {
+    __shared__ __align__(128) float sQ[2 * SMEM];
+    __shared__ uint64_t bar;
     Tile t;
-    if (!tile_of(a, t)) return;
+    const bool on = tile_of(a, t);
+    tile::bar_init(&bar);
+    tile::release();
+    tile::acquire();
+    if (!on) return;
+    if (threadIdx.x == 0) {
+        tile::expect(&bar, 8u * SMEM);
+        tile::box(sQ, &a.tm_qx, a.L.gz + t.z0 - HZ, a.L.gx + t.x0 - H, t.shot, &bar);
+        tile::box(sQ + SMEM, &a.tm_qz, a.L.gz + t.z0 - HZ, a.L.gx + t.x0 - H, t.shot, &bar);
+    }
     const int nx = t.sd.nx, nz = a.nz;
+    const ShotDev& sd = t.sd;
+    const int r0 = threadIdx.x / TZ, z = threadIdx.x % TZ, gz = t.z0 + z;
+    const long long c0 = cell(a, t.shot, t.x0 + r0, gz);
+    bool in[2];
+    float hs[2][6], d1[2], d4[2], g1[2], g2[2], p1[2], p2[2];  // hs: sx^ sz^ sr^ rx^ rz^ rr^
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int gx = t.x0 + r0 + u * (TC / 2);
+        const long long c = c0 + (long long)u * (TC / 2) * a.L.pitch;
+        in[u] = gx < nx && gz < nz;
+        if (in[u]) {
+            hs[u][0] = a.asx[c]; hs[u][1] = a.asz[c]; hs[u][2] = a.asr[c];
+            hs[u][3] = a.arx[c]; hs[u][4] = a.arz[c]; hs[u][5] = a.arr[c];
+            d1[u] = __ldg(a.d1 + c); d4[u] = __ldg(a.d4 + c);
+            g1[u] = a.g1[c]; g2[u] = a.g2[c];
+            const long long mi = (long long)min(sd.x0 + gx, a.nx_model - 1) * a.mpitch + gz;
+            p1[u] = __ldg(a.p1 + mi); p2[u] = __ldg(a.p2 + mi);
+        }
+    }
+    if (!tile::staged(&bar, a.err_flag)) return;
     const float* tb = a.spg;
     const int st = a.spg_stride;
-    constexpr int W4 = SW / 4;
-#pragma unroll 3  // several rows' loads in flight before their shared-memory stores
-    for (int i = threadIdx.x; i < SROWS * W4; i += kThreads) {
-        const int r = i / W4, c = i - r * W4;
-        const long long off = cell(a, t.shot, t.x0 - H + r, t.z0 - HZ + 4 * c);
-        *reinterpret_cast<float4*>(sQx + r * SW + 4 * c) = __ldg(reinterpret_cast<const float4*>(a.qx + off));
-        *reinterpret_cast<float4*>(sQz + r * SW + 4 * c) = __ldg(reinterpret_cast<const float4*>(a.qz + off));
-    }
-    __syncthreads();
-    float c[5];
-#pragma unroll
-    for (int m = 0; m < 5; m++) c[m] = a.a[m];
     const float dt = a.dt, f = a.f_mem;
-    for (int j0 = 0; j0 < kPer; j0 += kNBS) {
-        float hsx[kNBS], hsz[kNBS], hsr[kNBS], hrx[kNBS], hrz[kNBS], hrr[kNBS], d1[kNBS], d4[kNBS], g1[kNBS], g2[kNBS];
-        long long cc[kNBS];
-        bool ok[kNBS];
 #pragma unroll
-        for (int u = 0; u < kNBS; u++) {
-            const int i = threadIdx.x + (j0 + u) * kThreads, r = i / TZ, z = i - r * TZ;
-            const int gx = t.x0 + r, gz = t.z0 + z;
-            ok[u] = gx < nx && gz < nz;
-            const long long c = cell(a, t.shot, gx, gz);
-            cc[u] = c;
-            if (ok[u]) {
-                hsx[u] = a.asx[c]; hsz[u] = a.asz[c]; hsr[u] = a.asr[c];
-                hrx[u] = a.arx[c]; hrz[u] = a.arz[c]; hrr[u] = a.arr[c];
-                d1[u] = __ldg(a.d1 + c); d4[u] = __ldg(a.d4 + c);
-                g1[u] = a.g1[c]; g2[u] = a.g2[c];
-            }
+    for (int u = 0; u < 2; u++) {
+        if (!in[u]) continue;
+        const int r = r0 + u * (TC / 2), gx = t.x0 + r;
+        const long long c = c0 + (long long)u * (TC / 2) * a.L.pitch;
+        const float* px = sQ + (r + H) * SW + z + HZ;
+        const float* pz = px + SMEM;
+        auto QX = [&](int dx, int dz) { return px[dx * SW + dz]; };
+        auto QZ = [&](int dx, int dz) { return pz[dx * SW + dz]; };
+        float sx = 0.0f, sz = 0.0f;
+#pragma unroll
+        for (int m = 0; m < 5; m++) {
+            // Dx0^T: t(x-m, z-m) - t(x+1+m, z+1+m) + t(x-m, z+1+m) - t(x+1+m, z-m); Dz0^T flips the cross terms
+            const float ax_ = QX(-m, -m) - QX(1 + m, 1 + m), bx_ = QX(-m, 1 + m) - QX(1 + m, -m);
+            const float az_ = QZ(-m, -m) - QZ(1 + m, 1 + m), bz_ = QZ(-m, 1 + m) - QZ(1 + m, -m);
+            sx = fmaf(a.a[m], ax_ + bx_, sx);
+            sz = fmaf(a.a[m], az_ - bz_, sz);
         }
-#pragma unroll
-        for (int u = 0; u < kNBS; u++) {
-            if (!ok[u]) continue;
-            const int i = threadIdx.x + (j0 + u) * kThreads, r = i / TZ, z = i - r * TZ;
-            const int gx = t.x0 + r, gz = t.z0 + z;
-            const float* px = sQx + (r + H) * SW + z + HZ;
-            const float* pz = sQz + (r + H) * SW + z + HZ;
-            auto QX = [&](int dx, int dz) { return px[dx * SW + dz]; };
-            auto QZ = [&](int dx, int dz) { return pz[dx * SW + dz]; };
-            float sx = 0.0f, sz = 0.0f;
-#pragma unroll
-            for (int m = 0; m < 5; m++) {
-                // Dx0^T: t(x-m, z-m) - t(x+1+m, z+1+m) + t(x-m, z+1+m) - t(x+1+m, z-m); Dz0^T flips the cross terms
-                const float ax_ = QX(-m, -m) - QX(1 + m, 1 + m), bx_ = QX(-m, 1 + m) - QX(1 + m, -m);
-                const float az_ = QZ(-m, -m) - QZ(1 + m, 1 + m), bz_ = QZ(-m, 1 + m) - QZ(1 + m, -m);
-                sx = fmaf(c[m], ax_ + bx_, sx);
-                sz = fmaf(c[m], az_ - bz_, sz);
-            }
-            const float aS = fmaf(a.hx, sx, a.hz * sz);
-            const long long cu = cc[u];
-            const float axs = sp(gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
-            const float azs = sp(gz, nz, a.npz, tb + 6 * st, tb + 7 * st);
-            const float u1 = axs * hsx[u], u4 = azs * hsz[u];
-            const float w1 = axs * hrx[u], w4 = azs * hrz[u];
-            const float aR = fmaf(f, hrr[u], dt * hsr[u]);
-            a.g1[cu] = g1[u] + fmaf(d1[u], u1, d4[u] * u4);
-            a.g2[cu] = g2[u] + fmaf(d1[u], w1, d4[u] * w4);
-            a.asx[cu] = u1 + aS;
-            a.asz[cu] = u4 + aS;
-            a.asr[cu] = hsr[u] + aS;
-            a.arx[cu] = w1 + aR;
-            a.arz[cu] = w4 + aR;
-            a.arr[cu] = hrr[u] + aR;
-        }
+        const float aS = fmaf(a.hx, sx, a.hz * sz);
+        const float axs = sp(gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
+        const float azs = sp(gz, nz, a.npz, tb + 6 * st, tb + 7 * st);
+        const float u1 = axs * hs[u][0], u4 = azs * hs[u][1];
+        const float w1 = axs * hs[u][3], w4 = azs * hs[u][4];
+        const float aR = fmaf(f, hs[u][5], dt * hs[u][2]);
+        a.g1[c] = g1[u] + fmaf(d1[u], u1, d4[u] * u4);
+        a.g2[c] = g2[u] + fmaf(d1[u], w1, d4[u] * w4);
+        const float nsx = u1 + aS, nsz = u4 + aS, nrx = w1 + aR, nrz = w4 + aR;
+        a.asx[c] = nsx;
+        a.asz[c] = nsz;
+        a.asr[c] = hs[u][2] + aS;
+        a.arx[c] = nrx;
+        a.arz[c] = nrz;
+        a.arr[c] = hs[u][5] + aR;
+        const float e1 = dt * p1[u], e2 = f * p2[u];
+        a.t1[c] = axs * fmaf(e1, nsx, e2 * nrx);
+        a.t4[c] = azs * fmaf(e1, nsz, e2 * nrz);
     }
     // residual of step k-1 at the receivers of this tile (QM:452-459 transposed): S^ -> sx^, sz^, sr^
-    const ShotDev& sd = t.sd;
     const int* trp = a.tile_rec_ptr + sd.tile_rec_base + t.tile;
     const int rb = trp[0], re = trp[1];
     if (a.step >= 1 && re > rb) {
         __syncthreads();
         for (int j = rb + threadIdx.x; j < re; j += kThreads) {
             const int ridx = a.tile_rec_idx[j];
-            const long long cc = cell(a, t.shot, a.rec_x[sd.rec_list + ridx], a.rec_z[sd.rec_list + ridx]);
-            const float v = a.res[sd.rec_base + (long long)(a.step - 1) * sd.nrec + ridx];
-            atomicAdd(a.asx + cc, v);
-            atomicAdd(a.asz + cc, v);
-            atomicAdd(a.asr + cc, v);
+            const int x = a.rec_x[sd.rec_list + ridx];
+            if (x < t.x0 || x >= t.x0 + TC) continue;  // another CTA of the 64 x 64 tile holds it
+            add_residual(a, t.shot, sd, x, a.rec_z[sd.rec_list + ridx],
+                         a.res[sd.rec_base + (long long)(a.step - 1) * sd.nrec + ridx]);
         }
     }
 }
@@ -284,11 +263,8 @@ __global__ void q_adjoint_init_kernel(QAdjArgs a, int first_shot) {
     const int s = first_shot + blockIdx.y;
     const ShotDev sd = a.shots[s];
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < sd.nrec; r += gridDim.x * blockDim.x) {
-        const long long cc = cell(a, s, a.rec_x[sd.rec_list + r], a.rec_z[sd.rec_list + r]);
-        const float v = a.res[sd.rec_base + (long long)(sd.nt - 1) * sd.nrec + r];
-        atomicAdd(a.asx + cc, v);
-        atomicAdd(a.asz + cc, v);
-        atomicAdd(a.asr + cc, v);
+        add_residual(a, s, sd, a.rec_x[sd.rec_list + r], a.rec_z[sd.rec_list + r],
+                     a.res[sd.rec_base + (long long)(sd.nt - 1) * sd.nrec + r]);
     }
 }
 
@@ -325,12 +301,9 @@ int grid_for(long long n) { return (int)std::min<long long>((n + 255) / 256, 148
 }  // namespace
 
 cudaError_t q_adjoint_launch_step(const QAdjArgs& a, int active, cudaStream_t st) {
-    dim3 grid(a.L.ntx * a.L.ntz, active);
-    q_adj_velocity_kernel<<<grid, kThreads, 0, st>>>(a);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    q_adj_stress_kernel<<<grid, kThreads, 0, st>>>(a);
-    return cudaGetLastError();
+    const dim3 grid(a.L.ntz, a.L.ntx * (TX / TC), active);
+    if (cudaError_t e = tile::launch((const void*)q_adj_velocity_kernel, grid, kThreads, 0, st, a)) return e;
+    return tile::launch((const void*)q_adj_stress_kernel, grid, kThreads, 0, st, a);
 }
 
 cudaError_t q_adjoint_launch_init(const QAdjArgs& a, int first_shot, int nshot, int nrec_max, cudaStream_t st) {

@@ -45,7 +45,7 @@ constexpr int kTileX = 64;
 constexpr int kTileZ = 64;
 
 // Per-shot descriptor in device memory (one entry per shot, indexed by shot id).
-struct ShotDev {
+struct alignas(16) ShotDev {
     int nx;            // shot-local padded width (aperture)
     int x0;            // model column of shot column 0
     int nt;            // steps
@@ -73,7 +73,11 @@ struct Layout2D {
 };
 
 // Arguments of the viscoacoustic kernels (viscoac2d.cu): in-place fields, no ping-pong.
+constexpr int kQCols = 8;  // columns per CTA of the viscoacoustic kernels and their adjoint
 struct QArgs {
+    CUtensorMap tm_s, tm_vx, tm_vz;       // sigma, vx, vz with the box of q_box (reference-order kernels)
+    int* err_flag;                        // set to 1 by a CTA whose bounded wait ran out
+    float* sg;                            // sigma = (sx + sz) + sr
     float* vx; float* vz;                 // QS vxx (= vx), vzz (= vz) for vs = 0
     float* sx; float* sz; float* sr;      // QS strxxx, strxxz, strxxr (= strzz parts for vs = 0)
     float* rx; float* rz; float* rr;      // QS rxxx, rxxz, rxxr
@@ -100,6 +104,7 @@ struct QArgs {
     float* d1_out;                        // optional: Dx1 vx of this step (field layout), for the gradient
     float* d4_out;                        // optional: Dz1 vz of this step
 };
+void q_box(int box[2]);  // TMA box (z, x) of the viscoacoustic kernels and their adjoint
 cudaError_t viscoac2d_launch_step(const QArgs& a, int active, cudaStream_t st);
 
 // Default (fast, FMA) viscoacoustic step (viscoac2d_fast.cu): merged sigma and r everywhere,
@@ -225,6 +230,9 @@ cudaError_t elastic2d_smooth(float* const arrays[5], int mpitch, int ghost, int 
 
 // Arguments of the viscoacoustic adjoint kernels (q_adjoint2d.cu): adjoint fields in place.
 struct QAdjArgs {
+    CUtensorMap tm_t1, tm_t4, tm_qx, tm_qz;  // T1, T4, Qx, Qz with the box of q_box
+    int* err_flag;                        // set to 1 by a CTA whose bounded wait ran out
+    float* t1; float* t4;                 // T1, T4 of the next adjoint step (q_adjoint2d.cu)
     float* avx; float* avz;               // adjoints of vx, vz
     float* asx; float* asz; float* asr;   // adjoints of sx, sz, sr
     float* arx; float* arz; float* arr;   // adjoints of rx, rz, rr

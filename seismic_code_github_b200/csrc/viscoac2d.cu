@@ -6,7 +6,7 @@
 //   vx, vz                (QS vxx, vzz; vx is sponged in x only, vz in z only)
 //   sx, sz, sr            (QS strxxx, strxxz, strxxr; sigma = (sx + sz) + sr)
 //   rx, rz, rr            (QS rxxx, rxxz, rxxr;       r     = (rx + rz) + rr)
-// and one step is two kernels:
+// with sigma kept as a slab of its own, written by the stress kernel, and one step is two kernels:
 //   velocity: d1 = Dx0(sigma), d2 = Dz0(sigma) (QS:843-966, xflag/zflag 0),
 //             vx = (vx + dt b d1) * x-sponge, vz = (vz + dt b d2) * z-sponge   (QS:969-990, 609-654)
 //   stress:   d1 = Dx1(vx), d4 = Dz1(vz) (flag 1),
@@ -15,27 +15,30 @@
 //             rr = rr + f r_old, f = dt (-1/tau_sigma)                       (QS:993-1337, 1340-1390)
 // Every multiply and add is rounded separately in the reference's order, so the kernels agree
 // bit for bit with the FP32 restatement in oracle/q_oracle.cpp.
+//
+// Bound: memory (eight fields read and written, three model arrays: 76 B a cell; the kernels move 100).
+// The fields that a kernel differentiates arrive by TMA, a box with halo per field, on tiles of 64 rows by
+// 8 columns with two cells per thread, while the threads load their own values.  8 shots of 700 x 420
+// (2.4 M cells), forward and adjoint step together: 160 us with 64 x 64 tiles staged through registers and
+// 16 cells per thread; 4 columns with one cell per thread 137 us (bound by issue: the fixed work of a thread
+// is half of it); two cells per thread 122 us.
 #include <cuda_runtime.h>
 
 #include <cmath>
 #include <vector>
 
 #include "sfd_internal.h"
+#include "tile_stage.cuh"
 
 namespace sfd {
 namespace {
 
-constexpr int kThreads = 256;
 constexpr int TX = kTileX, TZ = kTileZ;
+constexpr int TC = kQCols, kThreads = TC * TZ / 2;  // columns of a tile, two cells per thread (TC / 2 columns apart)
 constexpr int H = 5;                    // RSG halo (offsets -5..+5)
-constexpr int HZ = 8;                   // z halo rounded for float4 staging
-constexpr int SROWS = TX + 2 * H;       // 74
+constexpr int HZ = 8;                   // z halo rounded to 16 bytes
 constexpr int SW = TZ + 2 * HZ;         // 80
-constexpr int SMEM = SROWS * SW;        // floats per staged field
-constexpr int kPer = TX * TZ / kThreads;  // cells per thread
-constexpr int kNB = 4;    // cells per load batch
-constexpr int kNBS = 2;  // cells per load batch of the stress kernel (three CTAs per SM)
-static_assert(kPer % kNB == 0, "whole batches");
+constexpr int SMEM = (TC + 2 * H) * SW; // floats per staged field
 
 __device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float fa(float a, float b) { return __fadd_rn(a, b); }
@@ -62,42 +65,40 @@ __device__ __forceinline__ float rsg(const float* s, int r, int c, const float* 
     return fm(h, acc);
 }
 
+// both derivatives of one field: their four-point differences share the first subtraction
+template <int FLAG>
+__device__ __forceinline__ void rsg_both(const float* s, int r, int c, const float* a, float hx, float hz, float* dx,
+                                         float* dz) {
+    float ax = 0.0f, az = 0.0f;
+#pragma unroll
+    for (int m = 0; m < 5; m++) {
+        const int hi = FLAG == 0 ? m : 1 + m, lo = FLAG == 0 ? -1 - m : -m;
+        const float t = fs(s[(r + hi) * SW + c + hi], s[(r + lo) * SW + c + lo]);
+        const float p = s[(r + hi) * SW + c + lo], q = s[(r + lo) * SW + c + hi];
+        const float tx = fm(a[m], fs(fa(t, p), q)), tz = fm(a[m], fa(fs(t, p), q));
+        ax = m == 0 ? tx : fa(ax, tx);
+        az = m == 0 ? tz : fa(az, tz);
+    }
+    *dx = fm(hx, ax);
+    *dz = fm(hz, az);
+}
+
 struct TileRef {
     int shot, tile, x0, z0;
     ShotDev sd;
 };
 
 __device__ __forceinline__ bool tile_of(const QArgs& a, TileRef& t) {
-    t.shot = a.slot_to_shot[blockIdx.y];
+    t.shot = a.slot_to_shot[blockIdx.z];
     t.sd = a.shots[t.shot];
-    t.tile = blockIdx.x;
-    const int tx_i = t.tile / a.L.ntz, tz_i = t.tile - tx_i * a.L.ntz;
-    t.x0 = tx_i * TX;
-    t.z0 = tz_i * TZ;
+    t.x0 = blockIdx.y * TC;
+    t.z0 = blockIdx.x * TZ;
+    t.tile = t.x0 / TX * a.L.ntz + blockIdx.x;  // the 64 x 64 tile of the receiver lists
     return t.x0 < t.sd.nx;
 }
 
 __device__ __forceinline__ long long cell(const QArgs& a, int shot, int x, int z) {
     return (long long)shot * a.L.shot_stride + (long long)(x + a.L.gx) * a.L.pitch + a.L.gz + z;
-}
-
-// stage f0 (+ f1 + f2, summed in that order) on the tile plus halo
-template <int NF>
-__device__ __forceinline__ void stage(float* s, const QArgs& a, const TileRef& t, const float* f0, const float* f1,
-                                      const float* f2) {
-    constexpr int W4 = SW / 4;
-#pragma unroll 3  // several rows' loads in flight before their shared-memory stores
-    for (int i = threadIdx.x; i < SROWS * W4; i += kThreads) {
-        const int r = i / W4, c = i - r * W4;
-        const long long off = cell(a, t.shot, t.x0 - H + r, t.z0 - HZ + 4 * c);
-        float4 v = __ldg(reinterpret_cast<const float4*>(f0 + off));
-        if (NF == 3) {
-            const float4 b = __ldg(reinterpret_cast<const float4*>(f1 + off));
-            const float4 d = __ldg(reinterpret_cast<const float4*>(f2 + off));
-            v = make_float4(fa(fa(v.x, b.x), d.x), fa(fa(v.y, b.y), d.y), fa(fa(v.z, b.z), d.z), fa(fa(v.w, b.w), d.w));
-        }
-        *reinterpret_cast<float4*>(s + r * SW + 4 * c) = v;
-    }
 }
 
 // x / z factors of a split sponge: left/right (resp. top/bottom) tables, applied in QS order
@@ -107,116 +108,124 @@ __device__ __forceinline__ float xs(float u, int x, int nx, int np, const float*
     return u;
 }
 
-__global__ void __launch_bounds__(kThreads) q_velocity_kernel(const __grid_constant__ QArgs a) {
-    __shared__ __align__(16) float sS[SMEM];
+__global__ void __launch_bounds__(kThreads, 8) q_velocity_kernel(const __grid_constant__ QArgs a) {
+    __shared__ __align__(128) float sS[SMEM];
+    __shared__ uint64_t bar;
     TileRef t;
-    if (!tile_of(a, t)) return;
-    stage<3>(sS, a, t, a.sx, a.sz, a.sr);  // sigma = (sx + sz) + sr  (QS:1294-1314)
-    __syncthreads();
+    const bool on = tile_of(a, t);
+    tile::bar_init(&bar);
+    tile::release();
+    tile::acquire();
+    if (!on) return;
+    if (threadIdx.x == 0) {  // sigma = (sx + sz) + sr  (QS:1294-1314)
+        tile::expect(&bar, 4u * SMEM);
+        tile::box(sS, &a.tm_s, a.L.gz + t.z0 - HZ, a.L.gx + t.x0 - H, t.shot, &bar);
+    }
     const int nx = t.sd.nx, nz = a.nz;
+    const int r0 = threadIdx.x / TZ, z = threadIdx.x % TZ, gz = t.z0 + z;
+    const long long c0 = cell(a, t.shot, t.x0 + r0, gz);
+    bool in[2];
+    float vx[2], vz[2], bu[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int gx = t.x0 + r0 + u * (TC / 2);
+        const long long c = c0 + (long long)u * (TC / 2) * a.L.pitch;
+        in[u] = gx < nx && gz < nz;
+        if (in[u]) {
+            vx[u] = a.vx[c];
+            vz[u] = a.vz[c];
+            bu[u] = __ldg(a.busg + (long long)min(t.sd.x0 + gx, a.nx_model - 1) * a.mpitch + gz);
+        }
+    }
+    if (!tile::staged(&bar, a.err_flag)) return;
     const float* tb = a.spg;
     const int st = a.spg_stride;
-    // NB cells per batch: all global loads of a batch are issued before its arithmetic, so that
-    // their latencies overlap (thread t handles column z = t % TZ of rows t / TZ + 4 j)
-    for (int j0 = 0; j0 < kPer; j0 += kNB) {
-        float vxo[kNB], vzo[kNB], bu[kNB];
-        long long cc[kNB];
-        bool ok[kNB];
 #pragma unroll
-        for (int u = 0; u < kNB; u++) {
-            const int i = threadIdx.x + (j0 + u) * kThreads, r = i / TZ, z = i - r * TZ;
-            const int gx = t.x0 + r, gz = t.z0 + z;
-            ok[u] = gx < nx && gz < nz;
-            cc[u] = cell(a, t.shot, gx, gz);
-            if (ok[u]) {
-                vxo[u] = a.vx[cc[u]];
-                vzo[u] = a.vz[cc[u]];
-                bu[u] = __ldg(a.busg + (long long)min(t.sd.x0 + gx, a.nx_model - 1) * a.mpitch + gz);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < kNB; u++) {
-            if (!ok[u]) continue;
-            const int i = threadIdx.x + (j0 + u) * kThreads, r = i / TZ, z = i - r * TZ;
-            const int gx = t.x0 + r, gz = t.z0 + z;
-            const float d1 = rsg<true, 0>(sS, r + H, z + HZ, a.a, a.hx);
-            const float d2 = rsg<false, 0>(sS, r + H, z + HZ, a.a, a.hz);
-            const float dtb = fm(a.dt, bu[u]);
-            float vx = fa(vxo[u], fm(dtb, d1));
-            float vz = fa(vzo[u], fm(dtb, d2));
-            vx = xs(vx, gx, nx, a.npx, tb + 0 * st, tb + 1 * st);   // spgxn, spgxp
-            vz = xs(vz, gz, nz, a.npz, tb + 2 * st, tb + 3 * st);   // spgzn, spgzp
-            a.vx[cc[u]] = fa(vx, 0.0f);  // vx = vxx + vxz with vxz = 0
-            a.vz[cc[u]] = fa(0.0f, vz);  // vz = vzx + vzz with vzx = 0
-        }
+    for (int u = 0; u < 2; u++) {
+        if (!in[u]) continue;
+        const int r = r0 + u * (TC / 2), gx = t.x0 + r;
+        const long long c = c0 + (long long)u * (TC / 2) * a.L.pitch;
+        float d1, d2;
+        rsg_both<0>(sS, r + H, z + HZ, a.a, a.hx, a.hz, &d1, &d2);
+        const float dtb = fm(a.dt, bu[u]);
+        float x = fa(vx[u], fm(dtb, d1)), y = fa(vz[u], fm(dtb, d2));
+        x = xs(x, gx, nx, a.npx, tb + 0 * st, tb + 1 * st);   // spgxn, spgxp
+        y = xs(y, gz, nz, a.npz, tb + 2 * st, tb + 3 * st);   // spgzn, spgzp
+        a.vx[c] = fa(x, 0.0f);  // vx = vxx + vxz with vxz = 0
+        a.vz[c] = fa(0.0f, y);  // vz = vzx + vzz with vzx = 0
     }
 }
 
-__global__ void __launch_bounds__(kThreads, 3) q_stress_kernel(const __grid_constant__ QArgs a) {
-    __shared__ __align__(16) float sVx[SMEM];
-    __shared__ __align__(16) float sVz[SMEM];
+__global__ void __launch_bounds__(kThreads, 6) q_stress_kernel(const __grid_constant__ QArgs a) {
+    __shared__ __align__(128) float sV[2 * SMEM];
+    __shared__ uint64_t bar;
+    const float* sVx = sV;
+    const float* sVz = sV + SMEM;
     TileRef t;
-    if (!tile_of(a, t)) return;
-    stage<1>(sVx, a, t, a.vx, nullptr, nullptr);
-    stage<1>(sVz, a, t, a.vz, nullptr, nullptr);
-    __syncthreads();
+    const bool on = tile_of(a, t);
+    tile::bar_init(&bar);
+    tile::release();
+    tile::acquire();
+    if (!on) return;
+    if (threadIdx.x == 0) {
+        tile::expect(&bar, 8u * SMEM);
+        tile::box(sV, &a.tm_vx, a.L.gz + t.z0 - HZ, a.L.gx + t.x0 - H, t.shot, &bar);
+        tile::box(sV + SMEM, &a.tm_vz, a.L.gz + t.z0 - HZ, a.L.gx + t.x0 - H, t.shot, &bar);
+    }
     const int nx = t.sd.nx, nz = a.nz;
+    const ShotDev& sd = t.sd;
+    const int r0 = threadIdx.x / TZ, z = threadIdx.x % TZ, gz = t.z0 + z;
+    const long long c0 = cell(a, t.shot, t.x0 + r0, gz);
+    bool in[2];
+    float p1[2], p2[2], o[2][6];  // o: sx sz sr rx rz rr
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int gx = t.x0 + r0 + u * (TC / 2);
+        const long long c = c0 + (long long)u * (TC / 2) * a.L.pitch;
+        in[u] = gx < nx && gz < nz;
+        if (in[u]) {
+            const long long mi = (long long)min(sd.x0 + gx, a.nx_model - 1) * a.mpitch + gz;
+            p1[u] = __ldg(a.p1 + mi);
+            p2[u] = __ldg(a.p2 + mi);
+            o[u][0] = a.sx[c]; o[u][1] = a.sz[c]; o[u][2] = a.sr[c];
+            o[u][3] = a.rx[c]; o[u][4] = a.rz[c]; o[u][5] = a.rr[c];
+        }
+    }
+    const float wav = __ldg(a.wavelets + sd.wav_off + a.step);
+    if (!tile::staged(&bar, a.err_flag)) return;
     const float* tb = a.spg;
     const int st = a.spg_stride;
-    const int step = a.step;
-    const float wav = __ldg(a.wavelets + t.sd.wav_off + step);
-    const ShotDev& sd = t.sd;
-    for (int j0 = 0; j0 < kPer; j0 += kNBS) {
-        float p1[kNBS], p2[kNBS], sx0[kNBS], sz0[kNBS], sr0[kNBS], rx0[kNBS], rz0[kNBS], rr0[kNBS];
-        long long cc[kNBS];
-        bool ok[kNBS];
 #pragma unroll
-        for (int u = 0; u < kNBS; u++) {
-            const int i = threadIdx.x + (j0 + u) * kThreads, r = i / TZ, z = i - r * TZ;
-            const int gx = t.x0 + r, gz = t.z0 + z;
-            ok[u] = gx < nx && gz < nz;
-            cc[u] = cell(a, t.shot, gx, gz);
-            if (ok[u]) {
-                const long long mi = (long long)min(sd.x0 + gx, a.nx_model - 1) * a.mpitch + gz;
-                p1[u] = __ldg(a.p1 + mi);
-                p2[u] = __ldg(a.p2 + mi);
-                const long long c = cc[u];
-                sx0[u] = a.sx[c]; sz0[u] = a.sz[c]; sr0[u] = a.sr[c];
-                rx0[u] = a.rx[c]; rz0[u] = a.rz[c]; rr0[u] = a.rr[c];
-            }
+    for (int u = 0; u < 2; u++) {
+        if (!in[u]) continue;
+        const int r = r0 + u * (TC / 2), gx = t.x0 + r;
+        const long long c = c0 + (long long)u * (TC / 2) * a.L.pitch;
+        const float d1 = rsg<true, 1>(sVx, r + H, z + HZ, a.a, a.hx);
+        const float d4 = rsg<false, 1>(sVz, r + H, z + HZ, a.a, a.hz);
+        const float rold = fa(fa(o[u][3], o[u][4]), o[u][5]);  // QS rxx of the previous step
+        // calpstrxx (QS:993-1020) with mu = 0, split sponge (QS:800), source (QS:801)
+        float sx = fa(o[u][0], fm(a.dt, fm(p1[u], d1)));
+        float sz = fa(o[u][1], fm(a.dt, fm(p1[u], d4)));
+        const float sr = fa(o[u][2], fm(a.dt, rold));
+        sx = xs(sx, gx, nx, a.npx, tb + 4 * st, tb + 5 * st);   // spg1xn, spg2xp
+        sz = xs(sz, gz, nz, a.npz, tb + 6 * st, tb + 7 * st);   // spg1zn, spg2zp
+        const int bx = gx - sd.stamp_x0, bz = gz - sd.stamp_z0;
+        if (bx >= 0 && bx < sd.stamp_w && bz >= 0 && bz < sd.stamp_h) {
+            const float g = __ldg(a.stamps + sd.stamp_off + bx * sd.stamp_h + bz);
+            sx = fa(__fdiv_rn(fm(fm(wav, g), a.dt), a.dz2), sx);   // QS:1384
         }
-#pragma unroll
-        for (int u = 0; u < kNBS; u++) {
-            if (!ok[u]) continue;
-            const int i = threadIdx.x + (j0 + u) * kThreads, r = i / TZ, z = i - r * TZ;
-            const int gx = t.x0 + r, gz = t.z0 + z;
-            const long long c = cc[u];
-            const float d1 = rsg<true, 1>(sVx, r + H, z + HZ, a.a, a.hx);
-            const float d4 = rsg<false, 1>(sVz, r + H, z + HZ, a.a, a.hz);
-            const float rold = fa(fa(rx0[u], rz0[u]), rr0[u]);  // QS rxx of the previous step
-            // calpstrxx (QS:993-1020) with mu = 0, split sponge (QS:800), source (QS:801)
-            float sx = fa(sx0[u], fm(a.dt, fm(p1[u], d1)));
-            float sz = fa(sz0[u], fm(a.dt, fm(p1[u], d4)));
-            const float sr = fa(sr0[u], fm(a.dt, rold));
-            sx = xs(sx, gx, nx, a.npx, tb + 4 * st, tb + 5 * st);   // spg1xn, spg2xp
-            sz = xs(sz, gz, nz, a.npz, tb + 6 * st, tb + 7 * st);   // spg1zn, spg2zp
-            const int bx = gx - sd.stamp_x0, bz = gz - sd.stamp_z0;
-            if (bx >= 0 && bx < sd.stamp_w && bz >= 0 && bz < sd.stamp_h) {
-                const float g = __ldg(a.stamps + sd.stamp_off + bx * sd.stamp_h + bz);
-                sx = fa(__fdiv_rn(fm(fm(wav, g), a.dt), a.dz2), sx);   // QS:1384
-            }
-            // calprxx (QS:1135-1170)
-            float rx = fa(rx0[u], fm(a.f_mem, fm(p2[u], d1)));
-            float rz = fa(rz0[u], fm(a.f_mem, fm(p2[u], d4)));
-            const float rr = fa(rr0[u], fm(a.f_mem, rold));
-            rx = xs(rx, gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
-            rz = xs(rz, gz, nz, a.npz, tb + 6 * st, tb + 7 * st);
-            a.sx[c] = sx; a.sz[c] = sz; a.sr[c] = sr;
-            a.rx[c] = rx; a.rz[c] = rz; a.rr[c] = rr;
-            if (a.d1_out) {  // gradient recomputation keeps the derivatives for the imaging condition
-                a.d1_out[c] = d1;
-                a.d4_out[c] = d4;
-            }
+        // calprxx (QS:1135-1170)
+        float rx = fa(o[u][3], fm(a.f_mem, fm(p2[u], d1)));
+        float rz = fa(o[u][4], fm(a.f_mem, fm(p2[u], d4)));
+        const float rr = fa(o[u][5], fm(a.f_mem, rold));
+        rx = xs(rx, gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
+        rz = xs(rz, gz, nz, a.npz, tb + 6 * st, tb + 7 * st);
+        a.sx[c] = sx; a.sz[c] = sz; a.sr[c] = sr;
+        a.rx[c] = rx; a.rz[c] = rz; a.rr[c] = rr;
+        a.sg[c] = fa(fa(sx, sz), sr);
+        if (a.d1_out) {  // gradient recomputation keeps the derivatives for the imaging condition
+            a.d1_out[c] = d1;
+            a.d4_out[c] = d4;
         }
     }
     // receivers: strzz (= strxx) = (sx + sz) + sr (QM:452-459)
@@ -226,21 +235,25 @@ __global__ void __launch_bounds__(kThreads, 3) q_stress_kernel(const __grid_cons
         __syncthreads();
         for (int j = rb + threadIdx.x; j < re; j += kThreads) {
             const int ridx = a.tile_rec_idx[j];
-            const long long c = cell(a, t.shot, a.rec_x[sd.rec_list + ridx], a.rec_z[sd.rec_list + ridx]);
-            a.records[sd.rec_base + (long long)step * sd.nrec + ridx] = fa(fa(a.sx[c], a.sz[c]), a.sr[c]);
+            const int x = a.rec_x[sd.rec_list + ridx];
+            if (x < t.x0 || x >= t.x0 + TC) continue;  // another CTA of the 64 x 64 tile holds it
+            a.records[sd.rec_base + (long long)a.step * sd.nrec + ridx] =
+                a.sg[cell(a, t.shot, x, a.rec_z[sd.rec_list + ridx])];
         }
     }
 }
 
 }  // namespace
 
+void q_box(int box[2]) {
+    box[0] = SW;
+    box[1] = TC + 2 * H;
+}
+
 cudaError_t viscoac2d_launch_step(const QArgs& a, int active, cudaStream_t st) {
-    dim3 grid(a.L.ntx * a.L.ntz, active);
-    q_velocity_kernel<<<grid, kThreads, 0, st>>>(a);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    q_stress_kernel<<<grid, kThreads, 0, st>>>(a);
-    return cudaGetLastError();
+    const dim3 grid(a.L.ntz, a.L.ntx * (TX / TC), active);
+    if (cudaError_t e = tile::launch((const void*)q_velocity_kernel, grid, kThreads, 0, st, a)) return e;
+    return tile::launch((const void*)q_stress_kernel, grid, kThreads, 0, st, a);
 }
 
 // QS:434-469 (density averaged in place, then buoyancy) and QS:473-551 (Blanch's tau method),

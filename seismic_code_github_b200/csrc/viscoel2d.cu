@@ -102,12 +102,11 @@ struct TileRef {
 };
 
 __device__ __forceinline__ bool tile_of(const EArgs& a, TileRef& t) {
-    t.shot = a.slot_to_shot[blockIdx.y];
+    t.shot = a.slot_to_shot[blockIdx.z];
     t.sd = a.shots[t.shot];
-    const int tx_i = blockIdx.x / a.L.ntz, tz_i = blockIdx.x - tx_i * a.L.ntz;
-    t.x0 = tx_i * TC;
-    t.z0 = tz_i * TZ;
-    t.tile = t.x0 / TX * a.L.ntz + tz_i;  // the 64 x 64 tile of the receiver lists
+    t.x0 = blockIdx.y * TC;
+    t.z0 = blockIdx.x * TZ;
+    t.tile = t.x0 / TX * a.L.ntz + blockIdx.x;  // the 64 x 64 tile of the receiver lists
     return t.x0 < t.sd.nx;
 }
 
@@ -283,7 +282,7 @@ void viscoel2d_box(int box[2]) {
 }
 
 cudaError_t viscoel2d_launch_step(const EArgs& a, int active, cudaStream_t st) {
-    const dim3 grid(a.L.ntx * (TX / TC) * a.L.ntz, active);
+    const dim3 grid(a.L.ntz, a.L.ntx * (TX / TC), active);
     const int sv = (int)sizeof(float) * (3 * SMEM + 4), ss = (int)sizeof(float) * (2 * SMEM + 4);
     const void* kv = (const void*)e_velocity_kernel;
     const void* ks = (const void*)e_stress_kernel;
