@@ -86,7 +86,7 @@ struct sfd_ctx {
     CUtensorMap etmaps[5];     // elastic schemes: sums vx vz sxx szz sxz (elastic2d.cu / viscoel2d.cu box)
     CUtensorMap q_maps[3];     // viscoacoustic reference-order step: vx, vz, sigma (q_box)
     CUtensorMap q_adj_maps[4]; // ... its adjoint: T1, T4, Qx, Qz
-    CUtensorMap qtmaps[2];     // default viscoacoustic step: sigma S0 S1 (viscoac2d_fast.cu box)
+    CUtensorMap qtmaps[3];     // default viscoacoustic step: sigma, vx, vz (viscoac2d_fast.cu box)
 
     // 3-D scheme: dense [x][y][pitch] slabs, 8 fields (P, Vx, Vy, Vz, two buffers each)
     Layout3D L3{};
@@ -217,29 +217,10 @@ void dfree(T*& p) {
 int round_up(int v, int m) { return (v + m - 1) / m * m; }
 
 // The viscoacoustic scheme runs the fused kernel (viscoac2d_fast.cu) unless SFD_EXACT is set.
-// Its slabs: vx (2 parities), vz (2), sigma (2), r, and the six split parts of the sponge bands.
-constexpr int kQVX = 0, kQVZ = 2, kQS = 4, kQR = 6, kQSplit = 7, kQE = 13, kQFastSlabs = 15;
-constexpr int kQFastSeg = 256;  // columns per segment of the one-kernel step (SFD_QFAST_SEG overrides)
-// Segment length of a step with `act` active shots: 256 columns, halved (down to 64) while the
-// grid would not fill one wave of four CTAs per SM -- the last shots of an uneven batch get more,
-// shorter segments (each pays a warm-up chunk; the results do not depend on the length).
-int q_fast_seg(const sfd_ctx* c, int act) {
-    const char* env = std::getenv("SFD_QFAST_SEG");
-    const int v = env ? std::atoi(env) : 0;
-    if (v >= 16 && v % 16 == 0) return v;
-    static int nsm[kMaxDevices] = {};
-    if (c->device >= 0 && c->device < kMaxDevices && nsm[c->device] == 0 &&
-        cudaDeviceGetAttribute(&nsm[c->device], cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess)
-        nsm[c->device] = 0;
-    const int sms = (c->device >= 0 && c->device < kMaxDevices) ? nsm[c->device] : 0;
-    const long long width = (long long)c->L.ntx * kTileX;
-    int seg = kQFastSeg;
-    while (seg > 64 && sms > 0 && (long long)act * c->L.ntz * ((width + seg - 1) / seg) < 4LL * sms) seg /= 2;
-    return seg;
-}
-// The default viscoacoustic mode: the x-marching step kernel and the sponge-band kernel
-// (viscoac2d_fast.cu; sigma, vx, vz ping-pong, r and the split parts of the bands in place);
-// SFD_EXACT runs the reference-order pair of kernels (viscoac2d.cu, eight split fields in place).
+// Its slabs: vx, vz, sigma, r, and the six split parts of the sponge bands, all in place.
+constexpr int kQVX = 0, kQVZ = 1, kQS = 2, kQR = 3, kQSplit = 4, kQFastSlabs = 10;
+// The default viscoacoustic mode: the merged fields and the split parts of the sponge bands
+// (viscoac2d_fast.cu); SFD_EXACT runs the reference-order kernels (viscoac2d.cu) on the split fields.
 bool q_fast(const sfd_ctx* c) { return c->g.scheme == SFD_VISCOAC_2D && !(c->g.flags & SFD_EXACT); }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda).
@@ -455,24 +436,22 @@ Acou3DArgs make_args3(const sfd_ctx* c, int step) {
 // Arguments of the viscoacoustic step (fields in place, eight slabs per shot).
 QArgs make_qargs(const sfd_ctx* c, int step);
 
-// Arguments of the fused viscoacoustic step (default mode), step k: reads parity k & 1 of sigma,
-// vx, vz and writes parity (k + 1) & 1; r and the split parts of the sponge bands in place.
+// Arguments of the default viscoacoustic step k.
 QFastArgs make_qfast(const sfd_ctx* c, int step) {
     QFastArgs A{};
     A.q = make_qargs(c, step);
     const long long fs = (long long)c->nshot * c->L.shot_stride;
     float* F = c->d_state;
-    const int i = step & 1, o = (step + 1) & 1;
-    A.vx_in = F + (kQVX + i) * fs; A.vx_out = F + (kQVX + o) * fs;
-    A.vz_in = F + (kQVZ + i) * fs; A.vz_out = F + (kQVZ + o) * fs;
-    A.s_in = F + (kQS + i) * fs; A.s_out = F + (kQS + o) * fs;
+    A.vx = F + kQVX * fs;
+    A.vz = F + kQVZ * fs;
+    A.s = F + kQS * fs;
     A.r = F + kQR * fs;
     A.q.vx = A.q.vz = nullptr;
     A.q.sx = F + (kQSplit + 0) * fs; A.q.sz = F + (kQSplit + 1) * fs; A.q.sr = F + (kQSplit + 2) * fs;
     A.q.rx = F + (kQSplit + 3) * fs; A.q.rz = F + (kQSplit + 4) * fs; A.q.rr = F + (kQSplit + 5) * fs;
-    A.tm_s = c->qtmaps[i];
-    A.e1 = F + kQE * fs;
-    A.e4 = F + (kQE + 1) * fs;
+    A.tm_s = c->qtmaps[0];
+    A.tm_vx = c->qtmaps[1];
+    A.tm_vz = c->qtmaps[2];
     A.err_flag = c->d_err;
     return A;
 }
@@ -646,10 +625,9 @@ int snap_after_step(sfd_ctx* ctx, int k, const int* slots, int act, long long* l
         const long long fs = (long long)ctx->nshot * ctx->L.shot_stride;
         const float* F = ctx->d_state;
         if (q_fast(ctx)) {
-            const int o = (k + 1) & 1;  // parity written by step k
             s.nsum = 1;
-            s.f[0] = F + (sn.field == SFD_FIELD_VX ? kQVX + o : sn.field == SFD_FIELD_VZ ? kQVZ + o
-                          : sn.field == SFD_FIELD_P ? kQS + o : kQR) * fs;
+            s.f[0] = F + (sn.field == SFD_FIELD_VX ? kQVX : sn.field == SFD_FIELD_VZ ? kQVZ
+                          : sn.field == SFD_FIELD_P ? kQS : kQR) * fs;
         } else if (ctx->g.scheme == SFD_VISCOAC_2D) {
             const int f0 = sn.field == SFD_FIELD_VX ? 0 : sn.field == SFD_FIELD_VZ ? 1 : sn.field == SFD_FIELD_P ? 2 : 5;
             s.nsum = (sn.field == SFD_FIELD_P || sn.field == SFD_FIELD_R) ? 3 : 1;
@@ -717,9 +695,7 @@ int launch_one_step(sfd_ctx* ctx, int k, const int* slots, int act, long long* l
     if (q_fast(ctx)) {
         QFastArgs q = make_qfast(ctx, k);
         q.q.slot_to_shot = slots;
-        int nx_max = 0;
-        for (const auto& d : ctx->h_shots) nx_max = std::max(nx_max, d.nx);
-        CK(viscoac2d_fast_launch(q, act, q_fast_seg(ctx, act), nx_max, ctx->stream, pdl_enabled()));
+        CK(viscoac2d_fast_launch(q, act, ctx->stream));
         *launches += 2;
         return SFD_OK;
     }
@@ -2489,10 +2465,11 @@ int sfd_set_shots(sfd_ctx* ctx, int nshot, const sfd_shot* shots) {
         }
         if (q_fast(ctx)) {
             int bs[2];
-            viscoac2d_fast_boxes(bs);
+            viscoac2d_fast_box(bs);
             const long long fs = (long long)nshot * L.shot_stride;
-            for (int b = 0; b < 2; b++) {
-                const int rc2 = encode_field_map(ctx, &ctx->qtmaps[b], ctx->d_state + (kQS + b) * fs, L, nshot, bs);
+            const int slab[3] = {kQS, kQVX, kQVZ};
+            for (int b = 0; b < 3; b++) {
+                const int rc2 = encode_field_map(ctx, &ctx->qtmaps[b], ctx->d_state + slab[b] * fs, L, nshot, bs);
                 if (rc2) return rc2;
             }
         }
@@ -2625,11 +2602,10 @@ int sfd_get_wavefield(sfd_ctx* ctx, int shot, int field, float* out) {
         };
         const size_t n = (size_t)sd.nx * nz;
         int rc2;
-        if (q_fast(ctx)) {  // merged fields; the shot's last step wrote parity nt & 1
-            const int o = sd.nt & 1;
-            if (field == SFD_FIELD_VX) return fetch(kQVX + o, out);
-            if (field == SFD_FIELD_VZ) return fetch(kQVZ + o, out);
-            if (field == SFD_FIELD_P) return fetch(kQS + o, out);
+        if (q_fast(ctx)) {  // merged fields
+            if (field == SFD_FIELD_VX) return fetch(kQVX, out);
+            if (field == SFD_FIELD_VZ) return fetch(kQVZ, out);
+            if (field == SFD_FIELD_P) return fetch(kQS, out);
             if (field == SFD_FIELD_R) return fetch(kQR, out);
             return set_err(ctx, SFD_ERR_UNSUPPORTED, "field %d not available for this scheme", field);
         }

@@ -107,23 +107,18 @@ struct QArgs {
 void q_box(int box[2]);  // TMA box (z, x) of the viscoacoustic kernels and their adjoint
 cudaError_t viscoac2d_launch_step(const QArgs& a, int active, cudaStream_t st);
 
-// Default (fast, FMA) viscoacoustic step (viscoac2d_fast.cu): merged sigma and r everywhere,
-// split parts in the sponge bands only (q.sx .. q.rr); q.vx / q.vz unused.
+// Default (fast, FMA) viscoacoustic step (viscoac2d_fast.cu), all fields in place: merged sigma and r
+// everywhere, split parts in the sponge bands only (q.sx .. q.rr); q.vx / q.vz unused.
 struct QFastArgs {
-    CUtensorMap tm_s;                 // this step's input sigma (box of viscoac2d_fast_boxes)
+    CUtensorMap tm_s, tm_vx, tm_vz;   // box of viscoac2d_fast_box
     QArgs q;
-    const float* s_in; float* s_out;  // merged stress, ping-pong
-    const float* vx_in; float* vx_out;
-    const float* vz_in; float* vz_out;
-    float* r;                         // merged memory variable, in place
-    float* e1; float* e4;             // 0.5/dx Dx1 vx and 0.5/dz Dz1 vz of the cells near the bands
+    float* s; float* vx; float* vz;   // merged stress, velocities
+    float* r;                         // merged memory variable
     int* err_flag;                    // set by a CTA whose bounded wait ran out
 };
-// one step of the active shots: the step kernel (one CTA per shot, 64-wide z strip and segment of
-// `seg` columns), then the band kernel (one CTA per shot and column, nx_max >= every active nx)
-cudaError_t viscoac2d_fast_launch(const QFastArgs& a, int active, int seg, int nx_max, cudaStream_t st, bool pdl);
-// TMA box extents (z, x) of the sigma loads
-void viscoac2d_fast_boxes(int box_s[2]);
+// one step of the active shots: the velocity kernel, then the stress kernel
+cudaError_t viscoac2d_fast_launch(const QFastArgs& a, int active, cudaStream_t st);
+void viscoac2d_fast_box(int box[2]);  // TMA box (z, x) of sigma, vx and vz
 
 // Visco-elastic split fields (viscoel2d.cu), in the order of their slabs in the state buffer.
 enum EField {

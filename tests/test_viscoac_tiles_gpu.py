@@ -8,7 +8,7 @@ import pytest
 import oracle_lib as ol
 from conftest import bits_equal, rel_l2
 from test_q_gradient_gpu import DT, NPX, TOL_GRAD, engine, model, observed, oracle
-from test_viscoac_gpu import qmodel, run_gpu
+from test_viscoac_gpu import TOL_FAST, qmodel, run_gpu
 from seismic_code_github_b200 import seisfd as S
 
 pytestmark = pytest.mark.gpu
@@ -41,3 +41,24 @@ def test_gradient_tile_edges(nx, nz):
     Jo, gvo, gqo = oracle(vp, rho, q, shots, obs_list)
     assert np.abs(gqo).max() > 0 and abs(J - Jo) <= 1e-4 * Jo
     assert rel_l2(gv, gvo) <= TOL_GRAD and rel_l2(gq, gqo) <= TOL_GRAD
+
+
+@pytest.mark.parametrize("nx,nz", [(28, 44), (29, 45), (27, 41), (43, 107), (45, 110)])
+def test_default_step_tile_edges(nx, nz):
+    """The default step's tiles of 64 rows by 16 columns, four rows and four or two columns per thread:
+    the final stress everywhere on padded grids around those multiples, against the FP64 restatement."""
+    vp, rho, q = qmodel(seed=nz, nx=nx, nz=nz)
+    npx, f0, dt, dx, nt = 10, 20.0, 5e-4, 10.0, 110
+    decay = ol.q_decay(f0, dt)
+    a, b = npx + nx - 3, npx + nz // 2
+    vpp, rhop, qp = (S.pad_model(m, npx, npx, npx, npx) for m in (vp, rho, q))
+    with S.Engine(S.VISCOAC_2D, vpp.shape[0], vpp.shape[1], dx, dx, dt, npx, order=10, f0=f0) as e:
+        e.set_model(vpp, rhop, qp)
+        rx = np.arange(vpp.shape[0], dtype=np.int32)
+        e.set_shots([S.ShotSpec(a - 1, b - 1, rx, np.full_like(rx, b - 1),
+                                S.wavelet(S.WAVELET_Q, nt + decay, dt, f0))])
+        rec = e.split_records(e.forward())[0]
+        p = e.wavefield(0, S.FIELD_P)
+    _, _, fin = ol.q_forward(vp, vp * 0, rho, q, q, dx, dx, dt, f0, nt, npx, npx, a, b, fp64=True, want_final=True)
+    assert np.abs(fin).max() > 0 and rel_l2(p, fin) <= TOL_FAST
+    assert bits_equal(rec[:, -1].ravel(), p[:, b - 1].ravel())
