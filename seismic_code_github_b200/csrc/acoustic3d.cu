@@ -122,6 +122,12 @@ __device__ __forceinline__ bool bounded_wait(uint64_t* bar, unsigned parity) {
 }
 
 __device__ __forceinline__ float4 ld4s(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ const float4* at4(const float* p, unsigned bytes) {
+    return reinterpret_cast<const float4*>(reinterpret_cast<const char*>(p) + bytes);
+}
+__device__ __forceinline__ float4* at4(float* p, unsigned bytes) {
+    return reinterpret_cast<float4*>(reinterpret_cast<char*>(p) + bytes);
+}
 __device__ __forceinline__ void st4s(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 __device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
 __device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
@@ -215,7 +221,10 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
     const int yl = tid >> 3, zr = (tid & 7) * 4;
     const int yo = y0 + yl, zo = z0 + zr;
     const bool own_ok = yo < ny && zo < L.pitch;  // the float4 lies inside the allocation
-    const long long own_off = (long long)min(yo, ny - 1) * L.pitch + min(zo, L.pitch - 4);
+    // offsets inside a plane are 32-bit bytes from a base that is the same for the whole CTA, 1.5% faster
+    // than 64-bit offsets per thread (a plane of 4 GB would leave no room for the fields)
+    const unsigned pitch_b = 4u * (unsigned)L.pitch;
+    const unsigned own_off = (unsigned)min(yo, ny - 1) * pitch_b + 4u * (unsigned)min(zo, L.pitch - 4);
     const int slab = a.slab_by_slot ? (int)blockIdx.y : shot;
     const long long shot_off = (long long)slab * L.shot_stride;
     const float* p_in = a.p_in + shot_off;
@@ -240,12 +249,12 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
 
     auto ld_own = [&](const float* base, int x) -> float4 {
         if (!own_ok || x >= nx) return make_float4(0.f, 0.f, 0.f, 0.f);
-        return __ldg(reinterpret_cast<const float4*>(base + (long long)x * L.xstride + own_off));
+        return __ldg(at4(base + (long long)x * L.xstride, own_off));
     };
     auto ld_model = [&](const float* base, int x, int y, int z) -> float4 {
         y = min(max(y, 0), ny - 1);
         z = min(max(z, 0), L.pitch - 4);
-        return __ldg(reinterpret_cast<const float4*>(base + (long long)x * L.xstride + (long long)y * L.pitch + z));
+        return __ldg(at4(base + (long long)x * L.xstride, (unsigned)y * pitch_b + 4u * (unsigned)z));
     };
     const int xs = R + (int)blockIdx.z * seg, s_begin = max(1, xs - 2 * R + 1), s_end = min(xs + seg, nx - R);
     auto issue = [&](int s) {
@@ -312,9 +321,9 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
         // velocity phases so that their latency is covered
         float4 adk = make_float4(0.f, 0.f, 0.f, 0.f), agk = adk;
         if (ADJ && s >= xs && own_ok) {
-            const long long pofs = shot_off + (long long)s * L.xstride + own_off;
-            adk = __ldg(reinterpret_cast<const float4*>(a.adj_div + pofs));
-            agk = *reinterpret_cast<const float4*>(a.adj_g + pofs);
+            const long long plane = shot_off + (long long)s * L.xstride;
+            adk = __ldg(at4(a.adj_div + plane, own_off));
+            agk = *at4(a.adj_g + plane, own_off);
         }
         // the loads of the next plane's own values are issued as soon as this plane's are used
         const int xv = s + R - 1;  // plane of this iteration's new Vx
@@ -379,7 +388,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
                     st4s(nby + row * TZ + zt, vn);
                     const int y = y0 - R + row;
                     if (row >= R && row < R + TY && y < ny && z0 + zt < L.pitch)
-                        st4s(a.vy_out + plane_off + (long long)y * L.pitch + z0 + zt, vout);
+                        *at4(a.vy_out + plane_off, (unsigned)y * pitch_b + 4u * (unsigned)(z0 + zt)) = vout;
                 }
             }
             // ---- new Vz on the Vz region: rows y0 .. y0+TY-1, z0-RQ .. z0+TZ+RQ-1 ----
@@ -421,7 +430,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
                 st4s(nbz + row * K::VZW + 4 * u, vn);
                 const int y = y0 + row, z = z0 - K::RQ + 4 * u;
                 if (4 * u >= K::RQ && 4 * u < K::RQ + TZ && y < ny && z < L.pitch)
-                    st4s(a.vz_out + plane_off + (long long)y * L.pitch + z, vout);
+                    *at4(a.vz_out + plane_off, (unsigned)y * pitch_b + 4u * (unsigned)z) = vout;
             };
             if (tid >= K::NVY2) {
 #pragma unroll
@@ -457,7 +466,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
                 vout = vn;
             }
             Vxo = ld_own(vx_in, s + R);
-            if (own_ok && xv >= xs && xv < s_end) st4s(a.vx_out + shot_off + (long long)xv * L.xstride + own_off, vout);
+            if (own_ok && xv >= xs && xv < s_end) *at4(a.vx_out + shot_off + (long long)xv * L.xstride, own_off) = vout;
             cur[q * kThreads] = vn;
         }
         // every thread is done with this stage and with the new-velocity buffer of plane s-1
@@ -516,7 +525,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
             }
             const float2 k01 = __fmul2_rn(__fmul2_rn(lo2(kk), lo2(vpn)), lo2(vpn));
             const float2 k23 = __fmul2_rn(__fmul2_rn(hi2(kk), hi2(vpn)), hi2(vpn));
-            const long long pofs = shot_off + (long long)s * L.xstride + own_off;
+            const long long plane = shot_off + (long long)s * L.xstride;
             if (ADJ) {
                 // bracket = nu / K + sum (= M a Q_old + ...), nu' = M a K bracket, g += nu D_k
                 const float4 po = Pq[q];
@@ -525,12 +534,12 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
                 float4 pn = cat4(__fmul2_rn(b01, k01), __fmul2_rn(b23, k23));
                 if (edge) pn = mul4(mul4(pn, edge_f(io, xpad_s, fx_s)), edge_k(io, kx_s));
                 if (own_ok) {
-                    st4s(a.p_out + pofs, pn);
+                    *at4(a.p_out + plane, own_off) = pn;
                     const float4 dk = adk;
                     float4 g = agk;
                     g = make_float4(fmaf(po.x, dk.x, g.x), fmaf(po.y, dk.y, g.y), fmaf(po.z, dk.z, g.z),
                                     fmaf(po.w, dk.w, g.w));
-                    st4s(a.adj_g + pofs, g);
+                    *at4(a.adj_g + plane, own_off) = g;
                     const ShotDev& sd = a.shots[shot];
                     if (s == sd.sx && yo == sd.sy && sd.sz >= zo && sd.sz < zo + 4) {
                         const float bq[4] = {b01.x, b01.y, b23.x, b23.y};
@@ -543,8 +552,8 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
                                  __ffma2_rn(make_float2(-k23.x, -k23.y), d23, hi2(Pq[q])));
                 if (edge) pn = mul4(mul4(pn, edge_f(io, xpad_s, fx_s)), edge_k(io, kx_s));
                 if (own_ok) {
-                    st4s(a.p_out + pofs, pn);
-                    if (a.div_out) st4s(a.div_out + pofs, cat4(d01, d23));  // recomputation for the adjoint
+                    *at4(a.p_out + plane, own_off) = pn;
+                    if (a.div_out) *at4(a.div_out + plane, own_off) = cat4(d01, d23);  // recomputation for the adjoint
                 }
             }
         }
