@@ -318,13 +318,13 @@ def measure_gradient_sharded(args, dev, world, rank):
 
 
 # Viscoacoustic bytes per grid point and step.  Algorithmic: vx, vz, sigma, r each read and written
-# once (32 B) plus the two per-cell modulus factors (8 B).  The default one-kernel step moves 44 B
-# (the same and the buoyancy), plus 48 B at each sponge-band cell (its six split parts read and
-# written); SFD_EXACT moves 96 B (its velocity kernel reads the three split stress parts, its
-# stress kernel reads and writes all six split parts).
+# once (32 B) plus the two per-cell modulus factors (8 B).  The two kernels of the default step move
+# 52 B (vx and vz are read by both, and the buoyancy), plus 48 B at each sponge-band cell (its six
+# split parts read and written); SFD_EXACT moves 100 B (all six split parts everywhere, sigma written
+# as a sum for the velocity kernel).
 Q_ALG_BYTES = 40
-Q_KERNEL_BYTES = 44
-Q_EXACT_BYTES = 96
+Q_KERNEL_BYTES = 52
+Q_EXACT_BYTES = 100
 
 
 def measure_viscoacoustic(args, dev):
