@@ -461,6 +461,7 @@ QArgs make_qargs(const sfd_ctx* c, int step) {
     const long long fs = (long long)c->nshot * c->L.shot_stride;
     float* f[9];
     for (int i = 0; i < 9; i++) f[i] = c->d_state + i * fs;
+    a.one = 1.0f;
     a.sg = f[8];
     a.tm_vx = c->q_maps[0];
     a.tm_vz = c->q_maps[1];

@@ -72,6 +72,13 @@ __device__ __forceinline__ float sp(int x, int n, int np, const float* tn, const
     return f;
 }
 
+// values of a thread's two cells, TC / 2 staged columns apart
+__device__ __forceinline__ float2 pair(const float* s, int dx, int dz) {
+    return make_float2(s[dx * SW + dz], s[(TC / 2 + dx) * SW + dz]);
+}
+__device__ __forceinline__ float2 bc(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, bc(-1.0f), a); }
+
 // residual v of one receiver into the stress adjoints of cell (x, z) and their share of T1, T4
 // (several receivers may share a cell, so the adds are atomic)
 __device__ __forceinline__ void add_residual(const QAdjArgs& a, int shot, const ShotDev& sd, int x, int z, float v) {
@@ -121,24 +128,25 @@ __global__ void __launch_bounds__(kThreads, 8) q_adj_velocity_kernel(const __gri
         }
     }
     if (!tile::staged(&bar, a.err_flag)) return;
+    const float* p1s = sT + (r0 + H) * SW + z + HZ;
+    const float* p4s = p1s + SMEM;
+    float2 s1p = bc(0.0f), s4p = bc(0.0f);
+#pragma unroll
+    for (int m = 0; m < 5; m++) {
+        // Dx1^T: t(x-1-m, z-1-m) - t(x+m, z+m) + t(x-1-m, z+m) - t(x+m, z-1-m); Dz1^T flips the cross terms
+        const float2 a1 = sub2(pair(p1s, -1 - m, -1 - m), pair(p1s, m, m));
+        const float2 b1 = sub2(pair(p1s, -1 - m, m), pair(p1s, m, -1 - m));
+        const float2 a4 = sub2(pair(p4s, -1 - m, -1 - m), pair(p4s, m, m));
+        const float2 b4 = sub2(pair(p4s, -1 - m, m), pair(p4s, m, -1 - m));
+        s1p = __ffma2_rn(bc(a.a[m]), __fadd2_rn(a1, b1), s1p);
+        s4p = __ffma2_rn(bc(a.a[m]), sub2(a4, b4), s4p);
+    }
 #pragma unroll
     for (int u = 0; u < 2; u++) {
         if (!in[u]) continue;
-        const int r = r0 + u * (TC / 2), gx = t.x0 + r;
+        const int gx = t.x0 + r0 + u * (TC / 2);
         const long long c = c0 + (long long)u * (TC / 2) * a.L.pitch;
-        const float* p1s = sT + (r + H) * SW + z + HZ;
-        const float* p4s = p1s + SMEM;
-        auto T1 = [&](int dx, int dz) { return p1s[dx * SW + dz]; };
-        auto T4 = [&](int dx, int dz) { return p4s[dx * SW + dz]; };
-        float s1 = 0.0f, s4 = 0.0f;
-#pragma unroll
-        for (int m = 0; m < 5; m++) {
-            // Dx1^T: t(x-1-m, z-1-m) - t(x+m, z+m) + t(x-1-m, z+m) - t(x+m, z-1-m); Dz1^T flips the cross terms
-            const float a1 = T1(-1 - m, -1 - m) - T1(m, m), b1 = T1(-1 - m, m) - T1(m, -1 - m);
-            const float a4 = T4(-1 - m, -1 - m) - T4(m, m), b4 = T4(-1 - m, m) - T4(m, -1 - m);
-            s1 = fmaf(a.a[m], a1 + b1, s1);
-            s4 = fmaf(a.a[m], a4 - b4, s4);
-        }
+        const float s1 = u ? s1p.y : s1p.x, s4 = u ? s4p.y : s4p.x;
         const float ax = sp(gx, nx, a.npx, tb + 0 * st, tb + 1 * st);
         const float az = sp(gz, nz, a.npz, tb + 2 * st, tb + 3 * st);
         const float vx = ax * fmaf(a.hx, s1, vxo[u]);
@@ -206,24 +214,25 @@ __global__ void __launch_bounds__(kThreads, 5) q_adj_stress_kernel(const __grid_
     const float* tb = a.spg;
     const int st = a.spg_stride;
     const float dt = a.dt, f = a.f_mem;
+    const float* px = sQ + (r0 + H) * SW + z + HZ;
+    const float* pz = px + SMEM;
+    float2 sxp = bc(0.0f), szp = bc(0.0f);
+#pragma unroll
+    for (int m = 0; m < 5; m++) {
+        // Dx0^T: t(x-m, z-m) - t(x+1+m, z+1+m) + t(x-m, z+1+m) - t(x+1+m, z-m); Dz0^T flips the cross terms
+        const float2 ax_ = sub2(pair(px, -m, -m), pair(px, 1 + m, 1 + m));
+        const float2 bx_ = sub2(pair(px, -m, 1 + m), pair(px, 1 + m, -m));
+        const float2 az_ = sub2(pair(pz, -m, -m), pair(pz, 1 + m, 1 + m));
+        const float2 bz_ = sub2(pair(pz, -m, 1 + m), pair(pz, 1 + m, -m));
+        sxp = __ffma2_rn(bc(a.a[m]), __fadd2_rn(ax_, bx_), sxp);
+        szp = __ffma2_rn(bc(a.a[m]), sub2(az_, bz_), szp);
+    }
 #pragma unroll
     for (int u = 0; u < 2; u++) {
         if (!in[u]) continue;
-        const int r = r0 + u * (TC / 2), gx = t.x0 + r;
+        const int gx = t.x0 + r0 + u * (TC / 2);
         const long long c = c0 + (long long)u * (TC / 2) * a.L.pitch;
-        const float* px = sQ + (r + H) * SW + z + HZ;
-        const float* pz = px + SMEM;
-        auto QX = [&](int dx, int dz) { return px[dx * SW + dz]; };
-        auto QZ = [&](int dx, int dz) { return pz[dx * SW + dz]; };
-        float sx = 0.0f, sz = 0.0f;
-#pragma unroll
-        for (int m = 0; m < 5; m++) {
-            // Dx0^T: t(x-m, z-m) - t(x+1+m, z+1+m) + t(x-m, z+1+m) - t(x+1+m, z-m); Dz0^T flips the cross terms
-            const float ax_ = QX(-m, -m) - QX(1 + m, 1 + m), bx_ = QX(-m, 1 + m) - QX(1 + m, -m);
-            const float az_ = QZ(-m, -m) - QZ(1 + m, 1 + m), bz_ = QZ(-m, 1 + m) - QZ(1 + m, -m);
-            sx = fmaf(a.a[m], ax_ + bx_, sx);
-            sz = fmaf(a.a[m], az_ - bz_, sz);
-        }
+        const float sx = u ? sxp.y : sxp.x, sz = u ? szp.y : szp.x;
         const float aS = fmaf(a.hx, sx, a.hz * sz);
         const float axs = sp(gx, nx, a.npx, tb + 4 * st, tb + 5 * st);
         const float azs = sp(gz, nz, a.npz, tb + 6 * st, tb + 7 * st);

@@ -91,6 +91,7 @@ struct QArgs {
     float hx, hz;                         // 0.5/dx, 0.5/dz
     float dz2;                            // dz*dz
     float a[5];                           // a100..a104
+    float one;                            // 1 (viscoac2d.cu: a paired sum is fma(a, one, b))
     const float* spg;                     // sponge tables: xn, xp, zn, zp, 1xn, 2xp, 1zn, 2zp
     int spg_stride;
     const ShotDev* shots;

@@ -21,7 +21,7 @@
 // 8 columns with two cells per thread, while the threads load their own values.  8 shots of 700 x 420
 // (2.4 M cells), forward and adjoint step together: 160 us with 64 x 64 tiles staged through registers and
 // 16 cells per thread; 4 columns with one cell per thread 137 us (bound by issue: the fixed work of a thread
-// is half of it); two cells per thread 122 us.
+// is half of it); two cells per thread 122 us, with their stencils paired 119 us.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -42,45 +42,50 @@ constexpr int SMEM = (TC + 2 * H) * SW; // floats per staged field
 
 __device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float fa(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float fs(float a, float b) { return __fsub_rn(a, b); }
 
-// QS:843-966: 0.5/d * sum_m a_m t_m with t_m the rotated four-point difference
+// The derivatives of a thread's two cells at once, on paired FP32 instructions (half the arithmetic
+// instructions).  A difference is fma(b, -1, a) and a sum fma(a, one, b), rounded once each: the compiler
+// contracts a paired multiply and a paired add, but not through `one` (1.0 from the kernel's arguments).
+__device__ __forceinline__ float2 bc(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 fs2(float2 a, float2 b) { return __ffma2_rn(b, bc(-1.0f), a); }
+__device__ __forceinline__ float2 fa2(float2 a, float2 b, float one) { return __ffma2_rn(a, bc(one), b); }
+__device__ __forceinline__ float2 pair(const float* s, int r, int c) {
+    return make_float2(s[r * SW + c], s[(r + TC / 2) * SW + c]);
+}
+
+// QS:843-966: 0.5/d * sum_m a_m t_m with t_m the rotated four-point difference; (r, c) the staged position
+// (row = x, column = z) of the first cell
 template <bool XDIR, int FLAG>
-__device__ __forceinline__ float rsg(const float* s, int r, int c, const float* a, float h) {
-    // s(row = x, col = z) with (r, c) the staged position of the output point
-    auto u = [&](int dk, int di) { return s[(r + di) * SW + c + dk]; };
-    float acc = 0.0f;
+__device__ __forceinline__ float2 rsg(const float* s, int r, int c, const float* a, float h, float one) {
+    float2 acc;
 #pragma unroll
     for (int m = 0; m < 5; m++) {
-        float t;
-        if (FLAG == 0) {
-            t = XDIR ? fs(fa(fs(u(m, m), u(-1 - m, -1 - m)), u(-1 - m, m)), u(m, -1 - m))
-                     : fa(fs(fs(u(m, m), u(-1 - m, -1 - m)), u(-1 - m, m)), u(m, -1 - m));
-        } else {
-            t = XDIR ? fs(fa(fs(u(1 + m, 1 + m), u(-m, -m)), u(-m, 1 + m)), u(1 + m, -m))
-                     : fa(fs(fs(u(1 + m, 1 + m), u(-m, -m)), u(-m, 1 + m)), u(1 + m, -m));
-        }
-        acc = (m == 0) ? fm(a[0], t) : fa(acc, fm(a[m], t));
+        const int hi = FLAG == 0 ? m : 1 + m, lo = FLAG == 0 ? -1 - m : -m;
+        const float2 d = fs2(pair(s, r + hi, c + hi), pair(s, r + lo, c + lo));
+        const float2 p = pair(s, r + hi, c + lo), q = pair(s, r + lo, c + hi);
+        const float2 t = __fmul2_rn(bc(a[m]), XDIR ? fs2(fa2(d, p, one), q) : fa2(fs2(d, p), q, one));
+        acc = m == 0 ? t : fa2(acc, t, one);
     }
-    return fm(h, acc);
+    return __fmul2_rn(bc(h), acc);
 }
 
 // both derivatives of one field: their four-point differences share the first subtraction
 template <int FLAG>
-__device__ __forceinline__ void rsg_both(const float* s, int r, int c, const float* a, float hx, float hz, float* dx,
-                                         float* dz) {
-    float ax = 0.0f, az = 0.0f;
+__device__ __forceinline__ void rsg_both(const float* s, int r, int c, const float* a, float hx, float hz, float one,
+                                         float2* dx, float2* dz) {
+    float2 ax, az;
 #pragma unroll
     for (int m = 0; m < 5; m++) {
         const int hi = FLAG == 0 ? m : 1 + m, lo = FLAG == 0 ? -1 - m : -m;
-        const float t = fs(s[(r + hi) * SW + c + hi], s[(r + lo) * SW + c + lo]);
-        const float p = s[(r + hi) * SW + c + lo], q = s[(r + lo) * SW + c + hi];
-        const float tx = fm(a[m], fs(fa(t, p), q)), tz = fm(a[m], fa(fs(t, p), q));
-        ax = m == 0 ? tx : fa(ax, tx);
-        az = m == 0 ? tz : fa(az, tz);
+        const float2 d = fs2(pair(s, r + hi, c + hi), pair(s, r + lo, c + lo));
+        const float2 p = pair(s, r + hi, c + lo), q = pair(s, r + lo, c + hi);
+        const float2 tx = __fmul2_rn(bc(a[m]), fs2(fa2(d, p, one), q));
+        const float2 tz = __fmul2_rn(bc(a[m]), fa2(fs2(d, p), q, one));
+        ax = m == 0 ? tx : fa2(ax, tx, one);
+        az = m == 0 ? tz : fa2(az, tz, one);
     }
-    *dx = fm(hx, ax);
-    *dz = fm(hz, az);
+    *dx = __fmul2_rn(bc(hx), ax);
+    *dz = __fmul2_rn(bc(hz), az);
 }
 
 struct TileRef {
@@ -140,13 +145,14 @@ __global__ void __launch_bounds__(kThreads, 8) q_velocity_kernel(const __grid_co
     if (!tile::staged(&bar, a.err_flag)) return;
     const float* tb = a.spg;
     const int st = a.spg_stride;
+    float2 d1p, d2p;
+    rsg_both<0>(sS, r0 + H, z + HZ, a.a, a.hx, a.hz, a.one, &d1p, &d2p);
 #pragma unroll
     for (int u = 0; u < 2; u++) {
         if (!in[u]) continue;
-        const int r = r0 + u * (TC / 2), gx = t.x0 + r;
+        const int gx = t.x0 + r0 + u * (TC / 2);
         const long long c = c0 + (long long)u * (TC / 2) * a.L.pitch;
-        float d1, d2;
-        rsg_both<0>(sS, r + H, z + HZ, a.a, a.hx, a.hz, &d1, &d2);
+        const float d1 = u ? d1p.y : d1p.x, d2 = u ? d2p.y : d2p.x;
         const float dtb = fm(a.dt, bu[u]);
         float x = fa(vx[u], fm(dtb, d1)), y = fa(vz[u], fm(dtb, d2));
         x = xs(x, gx, nx, a.npx, tb + 0 * st, tb + 1 * st);   // spgxn, spgxp
@@ -195,13 +201,14 @@ __global__ void __launch_bounds__(kThreads, 6) q_stress_kernel(const __grid_cons
     if (!tile::staged(&bar, a.err_flag)) return;
     const float* tb = a.spg;
     const int st = a.spg_stride;
+    const float2 d1p = rsg<true, 1>(sVx, r0 + H, z + HZ, a.a, a.hx, a.one);
+    const float2 d4p = rsg<false, 1>(sVz, r0 + H, z + HZ, a.a, a.hz, a.one);
 #pragma unroll
     for (int u = 0; u < 2; u++) {
         if (!in[u]) continue;
-        const int r = r0 + u * (TC / 2), gx = t.x0 + r;
+        const int gx = t.x0 + r0 + u * (TC / 2);
         const long long c = c0 + (long long)u * (TC / 2) * a.L.pitch;
-        const float d1 = rsg<true, 1>(sVx, r + H, z + HZ, a.a, a.hx);
-        const float d4 = rsg<false, 1>(sVz, r + H, z + HZ, a.a, a.hz);
+        const float d1 = u ? d1p.y : d1p.x, d4 = u ? d4p.y : d4p.x;
         const float rold = fa(fa(o[u][3], o[u][4]), o[u][5]);  // QS rxx of the previous step
         // calpstrxx (QS:993-1020) with mu = 0, split sponge (QS:800), source (QS:801)
         float sx = fa(o[u][0], fm(a.dt, fm(p1[u], d1)));
