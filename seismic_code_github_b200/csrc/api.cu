@@ -214,6 +214,13 @@ void dfree(T*& p) {
     p = nullptr;
 }
 
+// Host-to-device copy in the order of the context's stream, on which every kernel that reads the copy runs.
+// A plain cudaMemcpy from pageable memory may return before its last part has reached the device, and the
+// stream, which does not wait for the default one, would read what was there before.
+cudaError_t h2d(const sfd_ctx* ctx, void* dst, const void* src, size_t bytes) {
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);
+}
+
 int round_up(int v, int m) { return (v + m - 1) / m * m; }
 
 // The viscoacoustic scheme runs the fused kernel (viscoac2d_fast.cu) unless SFD_EXACT is set.
@@ -607,7 +614,7 @@ bool snap_prepare(sfd_ctx* ctx, int* rc) {
             moved = true;
         }
         sn.total = total;
-        if (cudaMemcpy(sn.d_off, sn.off.data(), sizeof(long long) * ctx->nshot, cudaMemcpyHostToDevice) !=
+        if (h2d(ctx, sn.d_off, sn.off.data(), sizeof(long long) * ctx->nshot) !=
             cudaSuccess) {
             *rc = set_err(ctx, SFD_ERR_CUDA, "snapshot offsets upload");
             return true;
@@ -996,7 +1003,7 @@ int grad_alloc(sfd_ctx* ctx) {
                     return rc;
             CK(cudaMalloc(&ctx->d_grad2, sizeof(double) * (size_t)ctx->g.nx * ctx->g.nz));
             CK(cudaMalloc(&ctx->d_apx0, sizeof(int) * ctx->nshot));
-            CK(cudaMemcpy(ctx->d_apx0, ctx->h_ap_x0.data(), sizeof(int) * ctx->nshot, cudaMemcpyHostToDevice));
+            CK(h2d(ctx, ctx->d_apx0, ctx->h_ap_x0.data(), sizeof(int) * ctx->nshot));
         }
         CK(cudaMalloc(&ctx->d_obs_nt, sizeof(float) * nrec));
         CK(cudaMalloc(&ctx->d_obs_tn, sizeof(float) * nrec));
@@ -1441,7 +1448,7 @@ int q_prepare(sfd_ctx* ctx) {
         ctx->iso_top == ctx->prep_top && ctx->topo_gen == ctx->prep_topo_gen && width == ctx->q_width) {
         if (ctx->have_shots) {
             for (int s = 0; s < ctx->nshot; s++) ctx->h_shots[s].x0 = start[blk[s]];
-            CK(cudaMemcpy(ctx->d_shots, ctx->h_shots.data(), sizeof(ShotDev) * ctx->nshot, cudaMemcpyHostToDevice));
+            CK(h2d(ctx, ctx->d_shots, ctx->h_shots.data(), sizeof(ShotDev) * ctx->nshot));
         }
         return SFD_OK;
     }
@@ -1500,7 +1507,7 @@ int q_prepare(sfd_ctx* ctx) {
             ctx->graph_valid = false;
         }
         if (!*dst) CK(cudaMalloc(dst, mfloats * sizeof(float)));
-        CK(cudaMemcpy(*dst, staged.data(), mfloats * sizeof(float), cudaMemcpyHostToDevice));
+        CK(h2d(ctx, *dst, staged.data(), mfloats * sizeof(float)));
         return SFD_OK;
     };
     int rc;
@@ -1509,7 +1516,7 @@ int q_prepare(sfd_ctx* ctx) {
             if ((rc = upload(&ctx->e_q[i], eq[i]))) return rc;
         if (width != ctx->q_width) dfree(ctx->d_itopo);
         if (!ctx->d_itopo) CK(cudaMalloc(&ctx->d_itopo, sizeof(int) * width));
-        CK(cudaMemcpy(ctx->d_itopo, itopo.data(), sizeof(int) * width, cudaMemcpyHostToDevice));
+        CK(h2d(ctx, ctx->d_itopo, itopo.data(), sizeof(int) * width));
         // YPUB:549-634 modipapml on the device (abc mode only, YPRI:301-302): rows z < pml of the
         // five arrays, per window
         std::vector<int> win;
@@ -1540,7 +1547,7 @@ int q_prepare(sfd_ctx* ctx) {
     ctx->prep_topo_gen = ctx->topo_gen;
     if (ctx->have_shots) {
         for (int s = 0; s < ctx->nshot; s++) ctx->h_shots[s].x0 = start[blk[s]];
-        CK(cudaMemcpy(ctx->d_shots, ctx->h_shots.data(), sizeof(ShotDev) * ctx->nshot, cudaMemcpyHostToDevice));
+        CK(h2d(ctx, ctx->d_shots, ctx->h_shots.data(), sizeof(ShotDev) * ctx->nshot));
     }
     return SFD_OK;
 }
@@ -1566,8 +1573,8 @@ int build_stamps(sfd_ctx* ctx) {
     dfree(ctx->d_stamps);
     CK(cudaMalloc(&ctx->d_stamps, sizeof(float) * std::max<size_t>(1, stamps.size())));
     if (!stamps.empty())
-        CK(cudaMemcpy(ctx->d_stamps, stamps.data(), sizeof(float) * stamps.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->d_shots, ctx->h_shots.data(), sizeof(ShotDev) * ctx->nshot, cudaMemcpyHostToDevice));
+        CK(h2d(ctx, ctx->d_stamps, stamps.data(), sizeof(float) * stamps.size()));
+    CK(h2d(ctx, ctx->d_shots, ctx->h_shots.data(), sizeof(ShotDev) * ctx->nshot));
     ctx->graph_valid = false;
     return SFD_OK;
 }
@@ -1692,7 +1699,7 @@ int set_shots_3d(sfd_ctx* ctx, int nshot, const sfd_shot* shots) {
         using E = typename std::remove_reference<decltype(v)>::type::value_type;
         const size_t bytes = std::max<size_t>(1, v.size()) * sizeof(E);
         CK(cudaMalloc(dst, bytes));
-        if (!v.empty()) CK(cudaMemcpy(*dst, v.data(), v.size() * sizeof(E), cudaMemcpyHostToDevice));
+        if (!v.empty()) CK(h2d(ctx, *dst, v.data(), v.size() * sizeof(E)));
         return SFD_OK;
     };
     int rc;
@@ -2096,7 +2103,7 @@ int sfd_create(const sfd_grid* g, int device, sfd_ctx** out) {
     CK(cudaEventCreate(&c->eve));
     CK(cudaMalloc(&c->d_flag, sizeof(int)));
     CK(cudaMalloc(&c->d_err, sizeof(int)));
-    CK(cudaMemset(c->d_err, 0, sizeof(int)));
+    CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
     if (g->scheme == SFD_ACOUSTIC_2D && !acoustic2d_plan(R, &c->plan))
         return set_err(ctx, SFD_ERR_UNSUPPORTED, "no kernel for radius %d", R);
     if (g->scheme == SFD_VISCOAC_2D || g->scheme == SFD_VISCOEL_2D) {
@@ -2184,7 +2191,7 @@ int sfd_set_model(sfd_ctx* ctx, const float* vp, const float* den, const float* 
             }
         }
         if (!*dst) CK(cudaMalloc(dst, mfloats * sizeof(float)));
-        CK(cudaMemcpy(*dst, staged.data(), mfloats * sizeof(float), cudaMemcpyHostToDevice));
+        CK(h2d(ctx, *dst, staged.data(), mfloats * sizeof(float)));
         return SFD_OK;
     };
     int urc = upload(&ctx->d_vp, vp);
@@ -2250,7 +2257,7 @@ int sfd_set_model(sfd_ctx* ctx, const float* vp, const float* den, const float* 
             sc = sc * ctx->h_vp[mi];
             s.inj_scale = sc;
         }
-        CK(cudaMemcpy(ctx->d_shots, ctx->h_shots.data(), sizeof(ShotDev) * ctx->nshot, cudaMemcpyHostToDevice));
+        CK(h2d(ctx, ctx->d_shots, ctx->h_shots.data(), sizeof(ShotDev) * ctx->nshot));
     }
     return SFD_OK;
 }
@@ -2423,7 +2430,7 @@ int sfd_set_shots(sfd_ctx* ctx, int nshot, const sfd_shot* shots) {
         using E = typename std::remove_reference<decltype(v)>::type::value_type;
         const size_t bytes = std::max<size_t>(1, v.size()) * sizeof(E);
         CK(cudaMalloc(dst, bytes));
-        if (!v.empty()) CK(cudaMemcpy(*dst, v.data(), v.size() * sizeof(E), cudaMemcpyHostToDevice));
+        if (!v.empty()) CK(h2d(ctx, *dst, v.data(), v.size() * sizeof(E)));
         return SFD_OK;
     };
     int rc;
