@@ -791,6 +791,7 @@ cudaError_t acoustic2d_fwd_launch(const Acou2DPlan& plan, int radius, const Acou
 
 cudaError_t acoustic2d_fma_launch(int radius, const Acou2DArgs& a, int active, bool varden, int stages,
                                  cudaStream_t st, bool adj) {
+    if (varden && (!a.bxm || !a.bzm)) return cudaErrorInvalidValue;
     switch (radius) {
 #define SFD_CASE(RR) \
     case RR: return adj ? launch_r<RR, true>(a, active, varden, stages, st) \

@@ -620,6 +620,7 @@ cudaError_t acoustic2d_march_launch(int radius, const Acou2DArgs& a, int active,
                                    cudaStream_t st, bool pdl, bool adj) {
     if (seg_cols < CH || seg_cols % CH != 0) return cudaErrorInvalidValue;
     if (a.L.tz != TZ || a.L.tx % CH != 0) return cudaErrorInvalidValue;
+    if (varden && (!a.bxm || !a.bzm)) return cudaErrorInvalidValue;
     switch (radius) {
     case 1: return launch_r<1>(a, active, varden, seg_cols, st, pdl, adj);
     case 2: return launch_r<2>(a, active, varden, seg_cols, st, pdl, adj);

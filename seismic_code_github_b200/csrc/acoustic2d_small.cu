@@ -450,6 +450,7 @@ cudaError_t launch_mode(int radius, const Acou2DArgs& a, int active, bool varden
 }  // namespace
 
 cudaError_t acoustic2d_small_launch(int radius, const Acou2DArgs& a, int active, bool varden, cudaStream_t st, bool adj) {
+    if (varden && (!a.bxm || !a.bzm)) return cudaErrorInvalidValue;
     return adj ? launch_mode<16, kAdjoint>(radius, a, active, varden, st)
                : launch_mode<16, kForward>(radius, a, active, varden, st);
 }

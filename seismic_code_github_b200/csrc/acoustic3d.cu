@@ -692,6 +692,7 @@ cudaError_t launch_r(const Acou3DArgs& a, int active, bool varden, bool adj, cud
 cudaError_t acoustic3d_launch_step(int radius, const Acou3DArgs& a, int active, bool varden, cudaStream_t st,
                                    bool adj) {
     if (active <= 0) return cudaSuccess;
+    if (varden && (!a.bxm || !a.bym || !a.bzm)) return cudaErrorInvalidValue;
     switch (radius) {
     case 2: return launch_r<2>(a, active, varden, adj, st);
     case 4: return launch_r<4>(a, active, varden, adj, st);

@@ -440,6 +440,35 @@ Acou3DArgs make_args3(const sfd_ctx* c, int step) {
     return a;
 }
 
+// dt / (d_a den) of the uploaded density per axis.  A context with SFD_EXACT has no use for them in its
+// forwards; its first gradient, whose steps are the default kernels, forms them.  If the memory is short any
+// other context is left without a model, so that no step runs on a half-formed one.
+int form_buoyancy(sfd_ctx* ctx) {
+    const bool is3d = ctx->g.scheme == SFD_ACOUSTIC_3D;
+    const size_t mfloats = (size_t)ctx->g.nx * ctx->g.ny * ctx->mpitch;
+    const float d[3] = {ctx->g.dx, is3d ? ctx->g.dy : ctx->g.dx, ctx->g.dz};
+    int n = 0;
+    for (int ax = 0; ax < 3; ax++) {
+        int k = 0;
+        while (k < ax && d[k] != d[ax]) k++;
+        if (k < ax) {
+            ctx->b_of[ax] = ctx->b_of[k];
+            continue;
+        }
+        ctx->b_of[ax] = n;
+        if (!ctx->d_b[n] && cudaMalloc(&ctx->d_b[n], mfloats * sizeof(float)) != cudaSuccess) {
+            cudaGetLastError();
+            for (auto& p : ctx->d_b) dfree(p);
+            if (!(ctx->g.flags & SFD_EXACT)) ctx->have_model = ctx->graph_valid = ctx->grad_valid = false;
+            return set_err(ctx, SFD_ERR_CUDA, "out of device memory for the density factors of the model");
+        }
+        CK(launch_buoyancy(ctx->d_den, ctx->g.dt / d[ax], ctx->d_b[n], (long long)mfloats, ctx->stream));
+        n++;
+    }
+    CK(cudaStreamSynchronize(ctx->stream));
+    return SFD_OK;
+}
+
 // Arguments of the viscoacoustic step (fields in place, eight slabs per shot).
 QArgs make_qargs(const sfd_ctx* c, int step);
 
@@ -1324,6 +1353,7 @@ int run_gradient(sfd_ctx* ctx, const float* obs, float* misfit, float* grad_vp, 
         return set_err(ctx, SFD_ERR_UNSUPPORTED, "scheme %d has no gradient", ctx->g.scheme);
     if (grad_invq && !visco) return set_err(ctx, SFD_ERR_ARG, "grad_invq applies to the viscoacoustic scheme only");
     auto t0 = std::chrono::steady_clock::now();
+    if (!visco && ctx->varden && !ctx->d_b[0] && (rc = form_buoyancy(ctx))) return rc;
     if ((rc = grad_alloc(ctx))) return rc;
     if (!ctx->graph_valid && (rc = tune_schedule(ctx))) return rc;
     CK(cudaMemcpyAsync(ctx->d_obs_nt, obs, sizeof(float) * ctx->rec_total,
@@ -2198,23 +2228,8 @@ int sfd_set_model(sfd_ctx* ctx, const float* vp, const float* den, const float* 
     if (urc) return urc;
     if (ctx->varden) {
         if ((urc = upload(&ctx->d_den, den))) return urc;
-        if (is3d || (ctx->g.scheme == SFD_ACOUSTIC_2D && !(ctx->g.flags & SFD_EXACT))) {
-            const float d[3] = {ctx->g.dx, is3d ? ctx->g.dy : ctx->g.dx, ctx->g.dz};
-            int n = 0;
-            for (int ax = 0; ax < 3; ax++) {
-                int k = 0;
-                while (k < ax && d[k] != d[ax]) k++;
-                if (k < ax) {
-                    ctx->b_of[ax] = ctx->b_of[k];
-                    continue;
-                }
-                ctx->b_of[ax] = n;
-                if (!ctx->d_b[n]) CK(cudaMalloc(&ctx->d_b[n], mfloats * sizeof(float)));
-                CK(launch_buoyancy(ctx->d_den, ctx->g.dt / d[ax], ctx->d_b[n], (long long)mfloats, ctx->stream));
-                n++;
-            }
-            CK(cudaStreamSynchronize(ctx->stream));
-        }
+        const bool acoustic = is3d || ctx->g.scheme == SFD_ACOUSTIC_2D;
+        if (acoustic && (!(ctx->g.flags & SFD_EXACT) || ctx->d_b[0]) && (urc = form_buoyancy(ctx))) return urc;
     } else {
         dfree(ctx->d_den);
         for (auto& p : ctx->d_b) dfree(p);

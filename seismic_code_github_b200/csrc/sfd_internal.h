@@ -290,7 +290,8 @@ struct Acou2DArgs {
     int pml;
     const float* vp;        // model, (nx_model x mpitch)
     const float* den;       // NULL for constant density
-    const float* bxm;       // variable density: dtdx / den and dtdz / den in den's layout (not with SFD_EXACT)
+    const float* bxm;       // variable density: dtdx / den and dtdz / den in den's layout (NULL only in the
+                            // forwards of SFD_EXACT; the launchers of the other kernels refuse NULL)
     const float* bzm;
     int mpitch;
     int nx_model;
