@@ -61,14 +61,17 @@ __device__ __forceinline__ bool staged(uint64_t* bar, int* err_flag) {
     bar_wait_1s(bar);
     return false;
 }
-// programmatic dependent launch: release() lets the next kernel's CTAs start on what does not depend on
+// Programmatic dependent launch: release() lets the next kernel's CTAs start on what does not depend on
 // this one (indexes, model values, tables), acquire() waits for the previous kernel before the first
-// access to its fields
+// access to its fields.  What a kernel reads before acquire() must have been written before the chain of
+// programmatic dependents began: by a kernel that a plain launch followed, or a copy that was waited for.
 __device__ __forceinline__ void release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void acquire() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// launch whose release() and acquire() make the edge to the kernel before it a programmatic one
-inline cudaError_t launch(const void* fn, dim3 grid, int threads, size_t smem, cudaStream_t st, void** args) {
+// launch whose release() and acquire() make the edge to the kernel before it a programmatic one; chained =
+// false: a plain launch, which starts when everything before it is done and visible
+inline cudaError_t launch(const void* fn, dim3 grid, int threads, size_t smem, cudaStream_t st, void** args,
+                          bool chained = true) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
@@ -76,7 +79,7 @@ inline cudaError_t launch(const void* fn, dim3 grid, int threads, size_t smem, c
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    at[0].val.programmaticStreamSerializationAllowed = chained && pdl_enabled() ? 1 : 0;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelExC(&cfg, fn, args);

@@ -460,6 +460,7 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
     }
     vti_window_kernel<<<dim3((nx + 127) / 128, nz, nshot), 128, 0, st>>>(a, model.p, model.p + nm, model.p + 2 * nm, dwin.p,
                                                                      c.nx_v, c.nz_v);
+    if (cudaGetLastError() != cudaSuccess) return SFD_ERR_CUDA;
 
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
@@ -472,9 +473,12 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
     cudaEventRecord(e0, st);
     for (int it = 1; it <= NT && err == cudaSuccess; it++) {
         int cu = (it % 2 == 1) ? 1 : 0, iit = it - half;  // odd steps: u2 / q2 current (VM:417-505)
+        // The chain of programmatic dependents begins after its first kernel, an inject kernel (nwt >= 1): the
+        // steps read the model before their acquire(), which would not wait for vti_window_kernel but only for
+        // the kernel before them.
         if (it <= nwt) {
             void* args[] = {&a, &off[cu].uc, &w[it]};
-            err = sfd::tile::launch((const void*)vti_inject_kernel, dim3(nshot), 32, 0, st, args);
+            err = sfd::tile::launch((const void*)vti_inject_kernel, dim3(nshot), 32, 0, st, args, it > 1);
             launches++;
         }
         void* args[] = {&a, &off[cu], &cu, &iit};
