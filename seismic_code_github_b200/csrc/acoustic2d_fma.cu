@@ -394,7 +394,7 @@ __device__ __forceinline__ void tile_body(const Acou2DArgs& a, float* smem, floa
                 dpf[h] = gpf[h] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (gx < nx && gz + 3 < nz) {
                     const long long c = cell(gx, gz);
-                    dpf[h] = __ldg(reinterpret_cast<const float4*>(a.adj_div + c));
+                    dpf[h] = *reinterpret_cast<const float4*>(a.adj_div + c);
                     gpf[h] = *reinterpret_cast<const float4*>(a.adj_g + c);
                 }
             }
@@ -472,7 +472,7 @@ __device__ __forceinline__ void tile_body(const Acou2DArgs& a, float* smem, floa
                         *reinterpret_cast<float4*>(a.vz_out + c) = zo4;
                     } else {
                         for (int qq = 0; qq < 4 && gz + qq < nz; qq++) {
-                            a.adj_g[c + qq] = fmaf(comp(po, qq), __ldg(a.adj_div + c + qq), a.adj_g[c + qq]);
+                            a.adj_g[c + qq] = fmaf(comp(po, qq), a.adj_div[c + qq], a.adj_g[c + qq]);
                             a.p_out[c + qq] = comp(nn, qq);
                             a.vx_out[c + qq] = comp(xo, qq);
                             a.vz_out[c + qq] = comp(zo4, qq);

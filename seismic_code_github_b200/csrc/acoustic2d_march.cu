@@ -316,7 +316,7 @@ __device__ __forceinline__ void chunk_body(const Acou2DArgs& a, float* smem, int
             for (int h = 0; h < 2; h++) {
                 dk[h] = gk[h] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (own && gz + 7 < nz) {
-                    dk[h] = __ldg(reinterpret_cast<const float4*>(a.adj_div + c + 4 * h));
+                    dk[h] = *reinterpret_cast<const float4*>(a.adj_div + c + 4 * h);
                     gk[h] = ld4(a.adj_g + c + 4 * h);
                 }
             }
@@ -378,7 +378,7 @@ __device__ __forceinline__ void chunk_body(const Acou2DArgs& a, float* smem, int
                     }
                 } else {
                     for (int q = 0; q < 8 && gz + q < nz; q++) {
-                        a.adj_g[c + q] = fmaf(po8[q], __ldg(a.adj_div + c + q), a.adj_g[c + q]);
+                        a.adj_g[c + q] = fmaf(po8[q], a.adj_div[c + q], a.adj_g[c + q]);
                         a.p_out[c + q] = nn[q];
                         a.vz_out[c + q] = zo8[q];
                     }

@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(TX * TZ / 4, 5) acoustic2d_small_kernel(const 
     }
     float4 dk = make_float4(0.f, 0.f, 0.f, 0.f), gk = dk;
     if (ADJ && own) {  // cells past nz lie in the slab and are not stored
-        dk = __ldg(reinterpret_cast<const float4*>(a.adj_div + c));
+        dk = ld4(a.adj_div + c);
         gk = ld4(a.adj_g + c);
     }
     float C[R];

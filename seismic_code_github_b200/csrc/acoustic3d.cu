@@ -247,9 +247,14 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
 #pragma unroll
     for (int m = 0; m < R; m++) cc[m] = bc2(a.coef[m]);
 
+    // own points of a field (ordinary loads: the kernel before this one wrote it) and of the model
     auto ld_own = [&](const float* base, int x) -> float4 {
         if (!own_ok || x >= nx) return make_float4(0.f, 0.f, 0.f, 0.f);
-        return __ldg(at4(base + (long long)x * L.xstride, own_off));
+        return *at4(base + (long long)x * L.xstride, own_off);
+    };
+    auto ld_vp = [&](int x) -> float4 {
+        if (!own_ok || x >= nx) return make_float4(0.f, 0.f, 0.f, 0.f);
+        return __ldg(at4(a.vp + (long long)x * L.xstride, own_off));
     };
     auto ld_model = [&](const float* base, int x, int y, int z) -> float4 {
         y = min(max(y, 0), ny - 1);
@@ -293,7 +298,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
     }
     float4 Pn = ld_own(p_in, s_begin + K::NQ);
     float4 Vxo = ld_own(vx_in, s_begin + R - 1);
-    float4 vpn = ld_own(a.vp, s_begin);
+    float4 vpn = ld_vp(s_begin);
     unsigned phase = 0;
 
     // R planes per trip, so that queue, ring and stage indices are constants.  Pq[q + j] is plane s + j; the
@@ -322,7 +327,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
         float4 adk = make_float4(0.f, 0.f, 0.f, 0.f), agk = adk;
         if (ADJ && s >= xs && own_ok) {
             const long long plane = shot_off + (long long)s * L.xstride;
-            adk = __ldg(at4(a.adj_div + plane, own_off));
+            adk = *at4(a.adj_div + plane, own_off);
             agk = *at4(a.adj_g + plane, own_off);
         }
         // the loads of the next plane's own values are issued as soon as this plane's are used
@@ -557,7 +562,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
                 }
             }
         }
-        vpn = ld_own(a.vp, s + 1);
+        vpn = ld_vp(s + 1);
         Pq[K::NQ + q] = Pn;
         Pn = ld_own(p_in, s + K::NQ + 1);
     }

@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(kThreads, 5) q_adj_stress_kernel(const __grid_
         if (in[u]) {
             hs[u][0] = a.asx[c]; hs[u][1] = a.asz[c]; hs[u][2] = a.asr[c];
             hs[u][3] = a.arx[c]; hs[u][4] = a.arz[c]; hs[u][5] = a.arr[c];
-            d1[u] = __ldg(a.d1 + c); d4[u] = __ldg(a.d4 + c);
+            d1[u] = a.d1[c]; d4[u] = a.d4[c];
             g1[u] = a.g1[c]; g2[u] = a.g2[c];
             const long long mi = (long long)min(sd.x0 + gx, a.nx_model - 1) * a.mpitch + gz;
             p1[u] = __ldg(a.p1 + mi); p2[u] = __ldg(a.p2 + mi);

@@ -65,6 +65,8 @@ __device__ __forceinline__ bool staged(uint64_t* bar, int* err_flag) {
 // this one (indexes, model values, tables), acquire() waits for the previous kernel before the first
 // access to its fields.  What a kernel reads before acquire() must have been written before the chain of
 // programmatic dependents began: by a kernel that a plain launch followed, or a copy that was waited for.
+// The same goes for __ldg, whose data must not change while the kernel runs, and which the compiler may move
+// above acquire(): model, tables and receiver lists only, never what a kernel of the chain writes.
 __device__ __forceinline__ void release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void acquire() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
