@@ -42,6 +42,7 @@ constexpr int kThreads = kTX * kTZ;           // one cell per thread
 constexpr int kGX = 8;                        // ghost columns: x halo rounded to 16 bytes
 constexpr int kSX = kTX + 2 * kGX;            // staged columns
 constexpr int kMinBlocks = 10;
+constexpr int kGridY = 65535;                 // blocks that grid.y holds
 
 // E = true: every operation rounded separately in the reference's order (bit-exact with the
 // restatement); E = false: multiplies and adds may contract into FMAs (records within relative L2
@@ -75,6 +76,7 @@ struct VtiDev {
 // Offsets (floats) of one step's arrays in a shot's slab: c = the current slots, o = the old ones that
 // take the new values.  Formed on the host, so that a thread's address is one 32-bit add.
 struct VtiOff {
+    int row0;  // first tile row of the launch (grid.y holds 65535)
     unsigned uc, uo, qc, qo, vz, ep, de;
     unsigned uxc[4], uxo[4], qxc[3], qxo[3], uzc[4], uzo[4];  // a1 a2 t2 a3
 };
@@ -138,16 +140,19 @@ __global__ void vti_inject_kernel(const __grid_constant__ VtiDev a, unsigned uc,
 // rows nsz0 + nzu + 6.  win: per shot xmin and nsz0.
 __global__ void vti_window_kernel(const __grid_constant__ VtiDev a, const float* vz, const float* ep, const float* de,
                                   const int* win, int nx_v, int nz_v) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, s = blockIdx.z;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, s = blockIdx.z;
     if (i >= a.nx) return;
     float* P = a.base + (long long)s * a.shot_stride + 4 * a.field;  // vz, eps, delta
-    const int il = min(max(i - a.nxl, 0), a.range - 1), jl = min(max(j - a.nzu, 0), nz_v - 1);
-    const long long m = (long long)min(max(il + win[2 * s], 0), nx_v - 1) * nz_v + jl;
-    const bool in = il == i - a.nxl && jl == j - a.nzu && j >= win[2 * s + 1] + a.nzu + 6;
-    const unsigned c = cell(a, i, j);
-    P[c] = vz[m];
-    P[a.field + c] = in ? ep[m] : 0.0f;
-    P[2 * a.field + c] = in ? de[m] : 0.0f;
+    const int il = min(max(i - a.nxl, 0), a.range - 1);
+    for (int j = blockIdx.y; j < a.nz; j += gridDim.y) {
+        const int jl = min(max(j - a.nzu, 0), nz_v - 1);
+        const long long m = (long long)min(max(il + win[2 * s], 0), nx_v - 1) * nz_v + jl;
+        const bool in = il == i - a.nxl && jl == j - a.nzu && j >= win[2 * s + 1] + a.nzu + 6;
+        const unsigned c = cell(a, i, j);
+        P[c] = vz[m];
+        P[a.field + c] = in ? ep[m] : 0.0f;
+        P[2 * a.field + c] = in ? de[m] : 0.0f;
+    }
 }
 
 template <bool E>
@@ -158,7 +163,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) vti_step_kernel(const __
     __shared__ __align__(128) float sQ[kTZ * kSX];
     __shared__ uint64_t bar;
     const int s = blockIdx.z, tid = threadIdx.x, tx = tid % kTX, ty = tid / kTX;
-    const int i0 = blockIdx.x * kTX, j0 = blockIdx.y * kTZ;
+    const int i0 = blockIdx.x * kTX, j0 = (o.row0 + (int)blockIdx.y) * kTZ;
     float* P = a.base + (long long)s * a.shot_stride;
     const int gi = i0 + tx, gj = j0 + ty;  // 0-based
     const bool in = gi < a.nx && gj < a.nz;
@@ -442,7 +447,7 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
         cudaMemcpyAsync(dwin.p, win.data(), 2 * nshot * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess)
         return SFD_ERR_CUDA;
     a.base = state.p; a.src = dsrc.p; a.rrow = drow.p; a.records = recs.p; a.err_flag = derr.p;
-    VtiOff off[2];  // by the current slot
+    VtiOff off[2] = {};  // by the current slot
     for (int b = 0; b < 2; b++) {
         VtiOff& f = off[b];
         const unsigned F = (unsigned)a.field, X = (unsigned)a.xs, Z = (unsigned)a.zs, c0 = b, o0 = 1 - b;
@@ -458,15 +463,15 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
             !sfd::encode_map3(&a.tm_q[b], state.p + f.qc, a.pitch, rows, nshot, a.pitch, a.shot_stride, kSX, kTZ))
             return SFD_ERR_CUDA;
     }
-    vti_window_kernel<<<dim3((nx + 127) / 128, nz, nshot), 128, 0, st>>>(a, model.p, model.p + nm, model.p + 2 * nm, dwin.p,
-                                                                     c.nx_v, c.nz_v);
+    vti_window_kernel<<<dim3((nx + 127) / 128, std::min(nz, kGridY), nshot), 128, 0, st>>>(
+        a, model.p, model.p + nm, model.p + 2 * nm, dwin.p, c.nx_v, c.nz_v);
     if (cudaGetLastError() != cudaSuccess) return SFD_ERR_CUDA;
 
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     const bool exact = (c.flags & SFD_EXACT) != 0;
-    const dim3 grid(ntx, (nz + kTZ - 1) / kTZ, nshot);
+    const int rows = (nz + kTZ - 1) / kTZ;
     const void* step = exact ? (const void*)vti_step_kernel<true> : (const void*)vti_step_kernel<false>;
     cudaError_t err = cudaSuccess;
     long long launches = 0;
@@ -481,9 +486,13 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
             err = sfd::tile::launch((const void*)vti_inject_kernel, dim3(nshot), 32, 0, st, args, it > 1);
             launches++;
         }
-        void* args[] = {&a, &off[cu], &cu, &iit};
-        if (err == cudaSuccess) err = sfd::tile::launch(step, grid, kThreads, 0, st, args);
-        launches++;
+        // a cell reads the current slots and writes the old ones, so a step may be several launches
+        for (int row0 = 0; row0 < rows && err == cudaSuccess; row0 += kGridY) {
+            off[cu].row0 = row0;
+            void* args[] = {&a, &off[cu], &cu, &iit};
+            err = sfd::tile::launch(step, dim3(ntx, std::min(rows - row0, kGridY), nshot), kThreads, 0, st, args);
+            launches++;
+        }
     }
     cudaEventRecord(e1, st);
     if (err == cudaSuccess) err = cudaGetLastError();

@@ -48,3 +48,16 @@ def test_bad_model_values_outside_the_windows_are_accepted():
         with pytest.raises(S.SfdError) as err:
             S.vti_forward(m, e, de, *args, [shot])
         assert err.value.status == 1
+
+
+@pytest.mark.parametrize("nzv,row", [(65600, 65560), (131200, 131130), (262300, 262190)])
+def test_grids_of_many_rows(nzv, row):
+    """More rows than one launch's grid.y holds (65535 rows of the window kernel, 131070 of the step), the
+    source and the receivers among the last of them."""
+    vz, eps, de = model(24, nzv, seed=4)
+    args = (100.0, 100.0, 1e-2, 12.0, 14, (8, 9, 0, 10))
+    shot = (12, row, row + 8, 0, 23)
+    ref = ol.vti_forward(vz, eps, de, *args, *shot)
+    assert np.abs(ref).max() > 0
+    rec, t = S.vti_forward(vz, eps, de, *args, [shot], exact=True)
+    assert np.array_equal(rec[0].view(np.uint32), ref.view(np.uint32))
