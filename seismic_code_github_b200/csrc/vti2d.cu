@@ -74,14 +74,17 @@ struct VtiDev {
 };
 
 // Offsets (floats) of one step's arrays in a shot's slab: c = the current slots, o = the old ones that
-// take the new values.  Formed on the host, so that a thread's address is one 32-bit add.
+// take the new values.  Formed on the host, so that a thread's address is one add: of 32 bits (I =
+// unsigned) while a shot's slab has fewer than 2^32 floats, of 64 bits beyond.
+template <class I>
 struct VtiOff {
     int row0;  // first tile row of the launch (grid.y holds 65535)
-    unsigned uc, uo, qc, qo, vz, ep, de;
-    unsigned uxc[4], uxo[4], qxc[3], qxo[3], uzc[4], uzo[4];  // a1 a2 t2 a3
+    I uc, uo, qc, qo, vz, ep, de;
+    I uxc[4], uxo[4], qxc[3], qxo[3], uzc[4], uzo[4];  // a1 a2 t2 a3
 };
 
-__device__ __forceinline__ unsigned cell(const VtiDev& a, int i, int j) { return (j + kH) * a.pitch + i + kGX; }
+template <class I>
+__device__ __forceinline__ I cell(const VtiDev& a, int i, int j) { return (I)(j + kH) * a.pitch + i + kGX; }
 
 // second-derivative sum of VS:511-525: (c1 (f+1 + f-1 - 2 f0) + ... + c5 (...)) / h**2
 template <bool E>
@@ -126,12 +129,12 @@ __device__ __forceinline__ void pml_cell(float d, float dd, float dt, float h, f
     }
 }
 
-__global__ void vti_inject_kernel(const __grid_constant__ VtiDev a, unsigned uc, float w) {
+__global__ void vti_inject_kernel(const __grid_constant__ VtiDev a, long long uc, float w) {
     sfd::tile::release();
     sfd::tile::acquire();
     const int s = blockIdx.x;
     if (threadIdx.x != 0) return;
-    float* u = a.base + (long long)s * a.shot_stride + uc + cell(a, a.src[2 * s] - 1, a.src[2 * s + 1] - 1);
+    float* u = a.base + (long long)s * a.shot_stride + uc + cell<long long>(a, a.src[2 * s] - 1, a.src[2 * s + 1] - 1);
     *u = __fadd_rn(*u, w);
 }
 
@@ -148,16 +151,16 @@ __global__ void vti_window_kernel(const __grid_constant__ VtiDev a, const float*
         const int jl = min(max(j - a.nzu, 0), nz_v - 1);
         const long long m = (long long)min(max(il + win[2 * s], 0), nx_v - 1) * nz_v + jl;
         const bool in = il == i - a.nxl && jl == j - a.nzu && j >= win[2 * s + 1] + a.nzu + 6;
-        const unsigned c = cell(a, i, j);
+        const long long c = cell<long long>(a, i, j);
         P[c] = vz[m];
         P[a.field + c] = in ? ep[m] : 0.0f;
         P[2 * a.field + c] = in ? de[m] : 0.0f;
     }
 }
 
-template <bool E>
+template <bool E, class I>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) vti_step_kernel(const __grid_constant__ VtiDev a,
-                                                                        const __grid_constant__ VtiOff o, int cu,
+                                                                        const __grid_constant__ VtiOff<I> o, int cu,
                                                                         int iit) {
     __shared__ __align__(128) float sU[(kTZ + 2 * kH) * kSX];
     __shared__ __align__(128) float sQ[kTZ * kSX];
@@ -167,7 +170,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) vti_step_kernel(const __
     float* P = a.base + (long long)s * a.shot_stride;
     const int gi = i0 + tx, gj = j0 + ty;  // 0-based
     const bool in = gi < a.nx && gj < a.nz;
-    const unsigned g = cell(a, gi, gj);
+    const I g = cell<I>(a, gi, gj);
     sfd::tile::bar_init(&bar);
     sfd::tile::release();
     float v = 0.0f, de = 0.0f, ep = 0.0f, uo = 0.0f, qo = 0.0f;
@@ -209,7 +212,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) vti_step_kernel(const __
         if (gj < nzu || gj >= nz - nzd) {  // the top and bottom PML
             const bool top = gj < nzu;
             const int js = top ? gj : gj - (nz - nzd) + nzu, idx = top ? gj + 1 - (nzu + 1) : gj + 1 - (nz - nzd);
-            const unsigned z = js * nx + gi;
+            const I z = (I)js * nx + gi;
             const float a1o = P[o.uzc[0] + z], a2o = P[o.uzc[1] + z], t2o = P[o.uzc[2] + z], a3o = P[o.uzc[3] + z];
             float a1 = P[o.uzo[0] + z], t2 = P[o.uzo[2] + z], a3 = P[o.uzo[3] + z], a2;
             const float sz1 = d1<E>(U, kSX, a.c1, dx, a.rdx);  // divided by dx as written (VS:796, 880)
@@ -237,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) vti_step_kernel(const __
     } else {  // the left and right PML (all rows): u, then q (VS:1073-1150) with the same s1, s2, d, dd
         const bool left = gi < nxl;
         const int is = left ? gi : gi - (nx - nxr) + nxl, idx = left ? gi + 1 - (nxl + 1) : gi + 1 - (nx - nxr);
-        const unsigned x = gj * (nxl + nxr) + is;
+        const I x = (I)gj * (nxl + nxr) + is;
         const float a1o = P[o.uxc[0] + x], a2o = P[o.uxc[1] + x], t2o = P[o.uxc[2] + x], a3o = P[o.uxc[3] + x];
         const float b1o = P[o.qxc[0] + x], b2o = P[o.qxc[1] + x], r2o = P[o.qxc[2] + x];
         float a1 = P[o.uxo[0] + x], t2 = P[o.uxo[2] + x], a3 = P[o.uxo[3] + x];
@@ -319,6 +322,18 @@ int coefficients(int order, int first, float* out) {
     return SFD_OK;
 }
 
+VtiOff<unsigned> narrow_offsets(const VtiOff<long long>& w) {
+    VtiOff<unsigned> n{};
+    n.uc = (unsigned)w.uc; n.uo = (unsigned)w.uo; n.qc = (unsigned)w.qc; n.qo = (unsigned)w.qo;
+    n.vz = (unsigned)w.vz; n.ep = (unsigned)w.ep; n.de = (unsigned)w.de;
+    for (int k = 0; k < 4; k++) {
+        n.uxc[k] = (unsigned)w.uxc[k]; n.uxo[k] = (unsigned)w.uxo[k];
+        n.uzc[k] = (unsigned)w.uzc[k]; n.uzo[k] = (unsigned)w.uzo[k];
+        if (k < 3) { n.qxc[k] = (unsigned)w.qxc[k]; n.qxo[k] = (unsigned)w.qxo[k]; }
+    }
+    return n;
+}
+
 template <class T>
 struct DevBuf {
     T* p = nullptr;
@@ -373,7 +388,6 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
         a.cd[k] = (float)(1.5 * (double)a.L / (n3 * h));
         a.cdd[k] = (float)(3.0 * (double)a.L / (n3 * h * h));
     }
-    if (7 * a.field + 14 * a.xs + 8 * a.zs > 0xffffffffLL) return SFD_ERR_NOMEM;  // 32-bit offsets in a slab
     a.shot_stride = 7 * a.field + 14 * a.xs + 8 * a.zs;
     a.shot_stride = (a.shot_stride + 31) / 32 * 32;
 
@@ -447,13 +461,13 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
         cudaMemcpyAsync(dwin.p, win.data(), 2 * nshot * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess)
         return SFD_ERR_CUDA;
     a.base = state.p; a.src = dsrc.p; a.rrow = drow.p; a.records = recs.p; a.err_flag = derr.p;
-    VtiOff off[2] = {};  // by the current slot
+    VtiOff<long long> off[2] = {};  // by the current slot
     for (int b = 0; b < 2; b++) {
-        VtiOff& f = off[b];
-        const unsigned F = (unsigned)a.field, X = (unsigned)a.xs, Z = (unsigned)a.zs, c0 = b, o0 = 1 - b;
+        VtiOff<long long>& f = off[b];
+        const long long F = a.field, X = a.xs, Z = a.zs, c0 = b, o0 = 1 - b;
         f.uc = c0 * F; f.uo = o0 * F; f.qc = (2 + c0) * F; f.qo = (2 + o0) * F;
         f.vz = 4 * F; f.ep = 5 * F; f.de = 6 * F;
-        for (unsigned k = 0; k < 4; k++) {
+        for (int k = 0; k < 4; k++) {
             f.uxc[k] = 7 * F + (2 * k + c0) * X; f.uxo[k] = 7 * F + (2 * k + o0) * X;
             if (k < 3) { f.qxc[k] = 7 * F + (8 + 2 * k + c0) * X; f.qxo[k] = 7 * F + (8 + 2 * k + o0) * X; }
             f.uzc[k] = 7 * F + 14 * X + (2 * k + c0) * Z; f.uzo[k] = 7 * F + 14 * X + (2 * k + o0) * Z;
@@ -463,6 +477,8 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
             !sfd::encode_map3(&a.tm_q[b], state.p + f.qc, a.pitch, rows, nshot, a.pitch, a.shot_stride, kSX, kTZ))
             return SFD_ERR_CUDA;
     }
+    const bool wide = a.shot_stride > 0xffffffffLL;
+    VtiOff<unsigned> narrow[2] = {narrow_offsets(off[0]), narrow_offsets(off[1])};  // unused if wide
     vti_window_kernel<<<dim3((nx + 127) / 128, std::min(nz, kGridY), nshot), 128, 0, st>>>(
         a, model.p, model.p + nm, model.p + 2 * nm, dwin.p, c.nx_v, c.nz_v);
     if (cudaGetLastError() != cudaSuccess) return SFD_ERR_CUDA;
@@ -472,7 +488,10 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
     cudaEventCreate(&e1);
     const bool exact = (c.flags & SFD_EXACT) != 0;
     const int rows = (nz + kTZ - 1) / kTZ;
-    const void* step = exact ? (const void*)vti_step_kernel<true> : (const void*)vti_step_kernel<false>;
+    const void* step = wide ? (exact ? (const void*)vti_step_kernel<true, long long>
+                                     : (const void*)vti_step_kernel<false, long long>)
+                            : (exact ? (const void*)vti_step_kernel<true, unsigned>
+                                     : (const void*)vti_step_kernel<false, unsigned>);
     cudaError_t err = cudaSuccess;
     long long launches = 0;
     cudaEventRecord(e0, st);
@@ -488,8 +507,8 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
         }
         // a cell reads the current slots and writes the old ones, so a step may be several launches
         for (int row0 = 0; row0 < rows && err == cudaSuccess; row0 += kGridY) {
-            off[cu].row0 = row0;
-            void* args[] = {&a, &off[cu], &cu, &iit};
+            off[cu].row0 = narrow[cu].row0 = row0;
+            void* args[] = {&a, wide ? (void*)&off[cu] : (void*)&narrow[cu], &cu, &iit};
             err = sfd::tile::launch(step, dim3(ntx, std::min(rows - row0, kGridY), nshot), kThreads, 0, st, args);
             launches++;
         }

@@ -61,3 +61,19 @@ def test_grids_of_many_rows(nzv, row):
     assert np.abs(ref).max() > 0
     rec, t = S.vti_forward(vz, eps, de, *args, [shot], exact=True)
     assert np.array_equal(rec[0].view(np.uint32), ref.view(np.uint32))
+
+
+@pytest.mark.parametrize("exact", [True, False], ids=["exact", "default"])
+def test_slab_of_more_than_2_to_the_32_floats(exact):
+    """A shot whose fields take more than 2^32 floats: near the left and bottom PML, whose split fields lie
+    past that offset, it records what a grid of the same left part does (nothing returns from the right
+    edge of either within the record), bit for bit."""
+    vz, eps, de = model(1, 200000, seed=6)  # one model column, replicated over the aperture
+    args = (100.0, 100.0, 1e-2, 12.0, 8, (10, 10, 0, 10))
+    recs = []
+    for width in (200, 2990):
+        shot = (6, 199985, 199990, 0, width - 1)
+        rec, _ = S.vti_forward(vz, eps, de, *args, [shot], exact=exact)
+        recs.append(rec[0][:60].copy())
+    assert np.abs(recs[0]).max() > 0
+    assert np.array_equal(recs[0].view(np.uint32), recs[1].view(np.uint32))
