@@ -323,7 +323,9 @@ void viscoac2d_stamp(int nx, int nz, int sx, int sz, int* box, std::vector<float
     const int hw1 = (int)std::lround((n1 + 1) / 2.0), hw2 = (int)std::lround((n2 + 1) / 2.0);
     const int ixcen = (n1 + 1) / 2, izcen = (n2 + 1) / 2;
     const float pi = 3.1415926f, sigma2 = 1.5f * 1.5f;
-    auto raw = [&](int i, int j) {  // g2c(i, j) before normalisation, 1-based
+    // g2c(i, j) before normalisation, 1-based; the squares in 64 bits (a grid of more than 92680 columns
+    // would overflow 32)
+    auto raw = [&](long long i, long long j) {
         const float dis = (float)((j - izcen) * (j - izcen) + (i - ixcen) * (i - ixcen));
         return 1.0f / (2.0f * pi * sigma2) * std::exp(-dis / (2.0f * sigma2));
     };
