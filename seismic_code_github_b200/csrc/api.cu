@@ -732,15 +732,17 @@ int launch_one_step(sfd_ctx* ctx, int k, const int* slots, int act, long long* l
     if (q_fast(ctx)) {
         QFastArgs q = make_qfast(ctx, k);
         q.q.slot_to_shot = slots;
-        CK(viscoac2d_fast_launch(q, act, ctx->stream));
-        *launches += 2;
+        int n = 0;
+        CK(viscoac2d_fast_launch(q, act, ctx->stream, &n));
+        *launches += n;
         return SFD_OK;
     }
     if (ctx->g.scheme == SFD_VISCOAC_2D) {
         QArgs q = make_qargs(ctx, k);
         q.slot_to_shot = slots;
-        CK(viscoac2d_launch_step(q, act, ctx->stream));
-        *launches += 2;
+        int n = 0;
+        CK(viscoac2d_launch_step(q, act, ctx->stream, &n));
+        *launches += n;
         return SFD_OK;
     }
     if (ctx->g.scheme == SFD_ELASTIC_2D) {
@@ -754,8 +756,9 @@ int launch_one_step(sfd_ctx* ctx, int k, const int* slots, int act, long long* l
     if (ctx->g.scheme == SFD_VISCOEL_2D) {
         EArgs e = make_eargs(ctx, k);
         e.slot_to_shot = slots;
-        CK(viscoel2d_launch_step(e, act, ctx->stream));
-        *launches += 2;
+        int n = 0;
+        CK(viscoel2d_launch_step(e, act, ctx->stream, &n));
+        *launches += n;
         return SFD_OK;
     }
     Acou2DArgs a = make_args(ctx, k);
@@ -1085,7 +1088,7 @@ int range_active(const sfd_ctx* ctx, const GradRange& r, int k) {
     return ctx->h_shots[r.first].nt > k ? 1 : 0;
 }
 
-int grad_fwd_step(sfd_ctx* ctx, const GradRange& r, int k, int act, float* div_out) {
+int grad_fwd_step(sfd_ctx* ctx, const GradRange& r, int k, int act, float* div_out, long long* launches) {
     if (ctx->g.scheme == SFD_VISCOAC_2D) {
         QArgs q = make_qargs(ctx, k);
         q.slot_to_shot = r.slots;
@@ -1093,13 +1096,16 @@ int grad_fwd_step(sfd_ctx* ctx, const GradRange& r, int k, int act, float* div_o
             q.d1_out = div_out;
             q.d4_out = div_out + (size_t)ctx->nshot * ctx->L.shot_stride;
         }
-        CK(viscoac2d_launch_step(q, act, ctx->stream));
+        int n = 0;
+        CK(viscoac2d_launch_step(q, act, ctx->stream, &n));
+        *launches += n;
         return SFD_OK;
     }
     Acou2DArgs a = make_args(ctx, k);
     a.slot_to_shot = r.slots;
     a.div_out = div_out;
     CK(acoustic2d_fwd_launch(grad_plan(ctx), ctx->radius, a, act, ctx->varden, ctx->stream));
+    *launches += 1;
     return SFD_OK;
 }
 
@@ -1138,8 +1144,10 @@ QAdjArgs make_qadj(const sfd_ctx* ctx, const GradRange& r, int k, const float* d
     return a;
 }
 
-int grad_adj_step_q(sfd_ctx* ctx, const GradRange& r, int k, int act, const float* div) {
-    CK(q_adjoint_launch_step(make_qadj(ctx, r, k, div), act, ctx->stream));
+int grad_adj_step_q(sfd_ctx* ctx, const GradRange& r, int k, int act, const float* div, long long* launches) {
+    int n = 0;
+    CK(q_adjoint_launch_step(make_qadj(ctx, r, k, div), act, ctx->stream, &n));
+    *launches += n;
     return SFD_OK;
 }
 
@@ -1177,8 +1185,9 @@ Acou2DArgs make_adj_args(const sfd_ctx* ctx, const GradRange& r, int k, const fl
     return a;
 }
 
-int grad_adj_step(sfd_ctx* ctx, const GradRange& r, int k, int act, const float* div) {
-    if (ctx->g.scheme == SFD_VISCOAC_2D) return grad_adj_step_q(ctx, r, k, act, div);
+int grad_adj_step(sfd_ctx* ctx, const GradRange& r, int k, int act, const float* div, long long* launches) {
+    if (ctx->g.scheme == SFD_VISCOAC_2D) return grad_adj_step_q(ctx, r, k, act, div, launches);
+    *launches += 1;
     if (acoustic2d_use_small(grad_plan(ctx), ctx->L, act))
         CK(acoustic2d_small_launch(ctx->radius, make_adj_args(ctx, r, k, div), act, ctx->varden, ctx->stream, true));
     else if (acoustic2d_use_march(grad_plan(ctx), ctx->L, act))
@@ -1213,7 +1222,6 @@ int enqueue_gradient_range(sfd_ctx* ctx, const GradRange& r, long long* launches
     const size_t off = (size_t)r.first * ctx->L.shot_stride, len = (size_t)r.count * ctx->L.shot_stride;
     const GradShape gs = grad_shape(ctx);
     const bool visco = ctx->g.scheme == SFD_VISCOAC_2D;
-    const int per_step = visco ? 2 : 1;  // launches per forward or adjoint step
     int nrec_max = 0;
     for (int s = r.first; s < r.first + r.count; s++) nrec_max = std::max(nrec_max, ctx->h_shots[s].nrec);
     // D_k slot of step k: kept tail steps after the C recomputation slots
@@ -1227,8 +1235,7 @@ int enqueue_gradient_range(sfd_ctx* ctx, const GradRange& r, long long* launches
         const int act = range_active(ctx, r, k);
         if (act == 0) break;
         if (k % C == 0 && (rc = grad_copy_state(ctx, r, k / C, k & 1, true))) return rc;
-        if ((rc = grad_fwd_step(ctx, r, k, act, k >= kkeep ? dslot(k, 0) : nullptr))) return rc;
-        *launches += per_step;
+        if ((rc = grad_fwd_step(ctx, r, k, act, k >= kkeep ? dslot(k, 0) : nullptr, launches))) return rc;
     }
     // residuals of this range and the misfit
     const ShotDev& s0 = ctx->h_shots[r.first];
@@ -1253,15 +1260,13 @@ int enqueue_gradient_range(sfd_ctx* ctx, const GradRange& r, long long* launches
             for (int k = k0; k < k1; k++) {
                 const int act = range_active(ctx, r, k);
                 if (act == 0) break;
-                if ((rc = grad_fwd_step(ctx, r, k, act, dslot(k, k0)))) return rc;
-                *launches += per_step;
+                if ((rc = grad_fwd_step(ctx, r, k, act, dslot(k, k0), launches))) return rc;
             }
         }
         for (int k = k1 - 1; k >= k0; k--) {
             const int act = range_active(ctx, r, k);
             if (act == 0) continue;
-            if ((rc = grad_adj_step(ctx, r, k, act, dslot(k, k0)))) return rc;
-            *launches += per_step;
+            if ((rc = grad_adj_step(ctx, r, k, act, dslot(k, k0), launches))) return rc;
         }
         for (int i = 0; i < gs.img; i++) {
             CK(launch_accumulate(ctx->d_gacc + i * fs + off, ctx->d_gseg + i * fs + off, (long long)len, ctx->stream));

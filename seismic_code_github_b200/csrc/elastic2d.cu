@@ -100,7 +100,7 @@ struct TileRef {
 __device__ __forceinline__ bool tile_of(const IArgs& a, TileRef& t) {
     t.shot = a.slot_to_shot[blockIdx.z];
     t.sd = a.shots[t.shot];
-    t.x0 = blockIdx.y * TC;
+    t.x0 = (a.col0 + (int)blockIdx.y) * TC;
     t.z0 = blockIdx.x * TZ;
     t.tile = t.x0 / TX * a.L.ntz + blockIdx.x;
     return t.x0 < t.sd.nx;
@@ -570,16 +570,16 @@ __global__ void __launch_bounds__(32) iso_smooth_kernel(const __grid_constant__ 
 namespace {
 
 template <bool FS>
-cudaError_t launch_pair(const IArgs& a, int active, cudaStream_t st) {
-    const dim3 grid(a.L.ntz, a.L.ntx * (TX / TC), active);
+cudaError_t launch_pair(const IArgs& a, int active, cudaStream_t st, int* launches) {
+    const int ntz = a.L.ntz, ncol = a.L.ntx * (TX / TC);
     const int sv = (int)sizeof(float) * (3 * kSmem + 4), ss = (int)sizeof(float) * (2 * kSmem + 4);
     const void* kv = (const void*)iso_velocity_kernel<FS>;
     const void* ks = (const void*)iso_stress_kernel<FS>;
     static bool attr0[kMaxDevices] = {}, attr1[kMaxDevices] = {};
     if (cudaError_t e = smem_attr_once(kv, sv, attr0)) return e;
     if (cudaError_t e = smem_attr_once(ks, ss, attr1)) return e;
-    if (cudaError_t e = tile::launch(kv, grid, kThreads, sv, st, a)) return e;
-    return tile::launch(ks, grid, kThreads, ss, st, a);
+    if (cudaError_t e = tile::launch_columns(kv, ntz, ncol, active, kThreads, sv, st, a, launches)) return e;
+    return tile::launch_columns(ks, ntz, ncol, active, kThreads, ss, st, a, launches);
 }
 
 }  // namespace
@@ -590,9 +590,9 @@ void elastic2d_box(int box[2]) {
 }
 
 cudaError_t elastic2d_launch_step(const IArgs& a, int active, int nx_max, cudaStream_t st, int* launches) {
-    *launches = a.fs ? 3 : 2;
-    const cudaError_t e = a.fs ? launch_pair<true>(a, active, st) : launch_pair<false>(a, active, st);
+    const cudaError_t e = a.fs ? launch_pair<true>(a, active, st, launches) : launch_pair<false>(a, active, st, launches);
     if (e != cudaSuccess || !a.fs) return e;
+    ++*launches;
     return tile::launch((const void*)iso_surface_kernel, dim3((nx_max + 127) / 128, active), 128, 0, st, a);
 }
 

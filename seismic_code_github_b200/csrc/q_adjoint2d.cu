@@ -54,7 +54,7 @@ struct Tile {
 __device__ __forceinline__ bool tile_of(const QAdjArgs& a, Tile& t) {
     t.shot = a.slot_to_shot[blockIdx.z];
     t.sd = a.shots[t.shot];
-    t.x0 = blockIdx.y * TC;
+    t.x0 = (a.col0 + (int)blockIdx.y) * TC;
     t.z0 = blockIdx.x * TZ;
     t.tile = t.x0 / TX * a.L.ntz + blockIdx.x;  // the 64 x 64 tile of the receiver lists
     return t.x0 < t.sd.nx;
@@ -309,10 +309,11 @@ int grid_for(long long n) { return (int)std::min<long long>((n + 255) / 256, 148
 
 }  // namespace
 
-cudaError_t q_adjoint_launch_step(const QAdjArgs& a, int active, cudaStream_t st) {
-    const dim3 grid(a.L.ntz, a.L.ntx * (TX / TC), active);
-    if (cudaError_t e = tile::launch((const void*)q_adj_velocity_kernel, grid, kThreads, 0, st, a)) return e;
-    return tile::launch((const void*)q_adj_stress_kernel, grid, kThreads, 0, st, a);
+cudaError_t q_adjoint_launch_step(const QAdjArgs& a, int active, cudaStream_t st, int* launches) {
+    const int ntz = a.L.ntz, ncol = a.L.ntx * (TX / TC);
+    if (cudaError_t e = tile::launch_columns((const void*)q_adj_velocity_kernel, ntz, ncol, active, kThreads, 0, st, a, launches))
+        return e;
+    return tile::launch_columns((const void*)q_adj_stress_kernel, ntz, ncol, active, kThreads, 0, st, a, launches);
 }
 
 cudaError_t q_adjoint_launch_init(const QAdjArgs& a, int first_shot, int nshot, int nrec_max, cudaStream_t st) {

@@ -77,6 +77,7 @@ constexpr int kQCols = 8;  // columns per CTA of the viscoacoustic kernels and t
 struct QArgs {
     CUtensorMap tm_s, tm_vx, tm_vz;       // sigma, vx, vz with the box of q_box (reference-order kernels)
     int* err_flag;                        // set to 1 by a CTA whose bounded wait ran out
+    int col0;                             // first tile column of the launch (tile::launch_columns)
     float* sg;                            // sigma = (sx + sz) + sr
     float* vx; float* vz;                 // QS vxx (= vx), vzz (= vz) for vs = 0
     float* sx; float* sz; float* sr;      // QS strxxx, strxxz, strxxr (= strzz parts for vs = 0)
@@ -106,7 +107,8 @@ struct QArgs {
     float* d4_out;                        // optional: Dz1 vz of this step
 };
 void q_box(int box[2]);  // TMA box (z, x) of the viscoacoustic kernels and their adjoint
-cudaError_t viscoac2d_launch_step(const QArgs& a, int active, cudaStream_t st);
+// (every launcher of a step adds the kernels it launched to *launches)
+cudaError_t viscoac2d_launch_step(const QArgs& a, int active, cudaStream_t st, int* launches);
 
 // Default (fast, FMA) viscoacoustic step (viscoac2d_fast.cu), all fields in place: merged sigma and r
 // everywhere, split parts in the sponge bands only (q.sx .. q.rr); q.vx / q.vz unused.
@@ -116,9 +118,10 @@ struct QFastArgs {
     float* s; float* vx; float* vz;   // merged stress, velocities
     float* r;                         // merged memory variable
     int* err_flag;                    // set by a CTA whose bounded wait ran out
+    int col0;                         // first tile column of the launch
 };
 // one step of the active shots: the velocity kernel, then the stress kernel
-cudaError_t viscoac2d_fast_launch(const QFastArgs& a, int active, cudaStream_t st);
+cudaError_t viscoac2d_fast_launch(const QFastArgs& a, int active, cudaStream_t st, int* launches);
 void viscoac2d_fast_box(int box[2]);  // TMA box (z, x) of sigma, vx and vz
 
 // Visco-elastic split fields (viscoel2d.cu), in the order of their slabs in the state buffer.
@@ -134,6 +137,7 @@ enum EField {
 struct EArgs {
     CUtensorMap tm[5];                    // vx vz sxx szz sxz (viscoel2d_box)
     int* err_flag;                        // set to 1 by a CTA whose bounded wait ran out
+    int col0;                             // first tile column of the launch
     float* f[E_NFIELDS];
     Layout2D L;
     int nz, npx, npz;
@@ -156,7 +160,7 @@ struct EArgs {
     int step;
 };
 void viscoel2d_box(int box[2]);  // TMA box of EArgs::tm
-cudaError_t viscoel2d_launch_step(const EArgs& a, int active, cudaStream_t st);
+cudaError_t viscoel2d_launch_step(const EArgs& a, int active, cudaStream_t st, int* launches);
 // QS:434-551 with vs: busg and the six stress coefficients on the padded grid, and rtaustss
 void viscoel2d_prepare(int nx, int nz, const float* vp, const float* vs, const float* rho, const float* qp,
                        const float* qs, float f0, float* busg, float* q1, float* q2, float* q3, float* m1, float* m2,
@@ -172,6 +176,7 @@ enum IField { I_VXX, I_VXZ, I_VZX, I_VZZ, I_SXXX, I_SXXZ, I_SZZX, I_SZZZ, I_SXZX
 struct IArgs {
     CUtensorMap tm[5];                    // vx vz strxx strzz strxz (elastic2d_box)
     int* err_flag;                        // set to 1 by a CTA whose bounded wait ran out
+    int col0;                             // first tile column of the launch
     float* f[I_NFIELDS];
     Layout2D L;
     int nz, npx, npz;
@@ -228,6 +233,7 @@ cudaError_t elastic2d_smooth(float* const arrays[5], int mpitch, int ghost, int 
 struct QAdjArgs {
     CUtensorMap tm_t1, tm_t4, tm_qx, tm_qz;  // T1, T4, Qx, Qz with the box of q_box
     int* err_flag;                        // set to 1 by a CTA whose bounded wait ran out
+    int col0;                             // first tile column of the launch
     float* t1; float* t4;                 // T1, T4 of the next adjoint step (q_adjoint2d.cu)
     float* avx; float* avz;               // adjoints of vx, vz
     float* asx; float* asz; float* asr;   // adjoints of sx, sz, sr
@@ -254,7 +260,7 @@ struct QAdjArgs {
     int step;
 };
 // adjoint of forward step a.step for the active shots (two launches)
-cudaError_t q_adjoint_launch_step(const QAdjArgs& a, int active, cudaStream_t st);
+cudaError_t q_adjoint_launch_step(const QAdjArgs& a, int active, cudaStream_t st, int* launches);
 // adjoint initial state: sx^, sz^, sr^ += residual of each shot's last step at its receivers
 cudaError_t q_adjoint_launch_init(const QAdjArgs& a, int first_shot, int nshot, int nrec_max, cudaStream_t st);
 // model-grid d misfit / d vp and d misfit / d (1/Q) from the per-shot double imaging sums

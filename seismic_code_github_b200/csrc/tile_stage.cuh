@@ -91,6 +91,20 @@ inline cudaError_t launch(const void* fn, dim3 grid, int threads, size_t smem, c
     void* args[] = {const_cast<Args*>(&a)};
     return launch(fn, grid, threads, smem, st, args);
 }
+// Launch over columns of tiles (grid: 64-row tiles, tile columns, shots), in as many launches as grid.y,
+// which holds 65535, asks for: the kernels write only their own cells of fields that no other of their CTAs
+// reads.  a.col0 is the first tile column of the launch; *launches counts them.
+template <class Args>
+inline cudaError_t launch_columns(const void* fn, int ntz, int ncol, int active, int threads, size_t smem, cudaStream_t st,
+                                  const Args& args, int* launches) {
+    Args a = args;
+    for (a.col0 = 0; a.col0 < ncol; a.col0 += 65535) {
+        const int n = ncol - a.col0 < 65535 ? ncol - a.col0 : 65535;
+        if (cudaError_t e = launch(fn, dim3(ntz, n, active), threads, smem, st, a)) return e;
+        ++*launches;
+    }
+    return cudaSuccess;
+}
 
 }  // namespace tile
 }  // namespace sfd

@@ -96,7 +96,7 @@ struct TileRef {
 __device__ __forceinline__ bool tile_of(const QArgs& a, TileRef& t) {
     t.shot = a.slot_to_shot[blockIdx.z];
     t.sd = a.shots[t.shot];
-    t.x0 = blockIdx.y * TC;
+    t.x0 = (a.col0 + (int)blockIdx.y) * TC;
     t.z0 = blockIdx.x * TZ;
     t.tile = t.x0 / TX * a.L.ntz + blockIdx.x;  // the 64 x 64 tile of the receiver lists
     return t.x0 < t.sd.nx;
@@ -257,10 +257,11 @@ void q_box(int box[2]) {
     box[1] = TC + 2 * H;
 }
 
-cudaError_t viscoac2d_launch_step(const QArgs& a, int active, cudaStream_t st) {
-    const dim3 grid(a.L.ntz, a.L.ntx * (TX / TC), active);
-    if (cudaError_t e = tile::launch((const void*)q_velocity_kernel, grid, kThreads, 0, st, a)) return e;
-    return tile::launch((const void*)q_stress_kernel, grid, kThreads, 0, st, a);
+cudaError_t viscoac2d_launch_step(const QArgs& a, int active, cudaStream_t st, int* launches) {
+    const int ntz = a.L.ntz, ncol = a.L.ntx * (TX / TC);
+    if (cudaError_t e = tile::launch_columns((const void*)q_velocity_kernel, ntz, ncol, active, kThreads, 0, st, a, launches))
+        return e;
+    return tile::launch_columns((const void*)q_stress_kernel, ntz, ncol, active, kThreads, 0, st, a, launches);
 }
 
 // QS:434-469 (density averaged in place, then buoyancy) and QS:473-551 (Blanch's tau method),

@@ -72,10 +72,11 @@ struct Place {
 };
 
 template <int U>
-__device__ __forceinline__ Place place(const QArgs& a, const ShotDev& sd, int shot) {
+__device__ __forceinline__ Place place(const QFastArgs& A, const ShotDev& sd, int shot) {
+    const QArgs& a = A.q;
     Place t;
     t.shot = shot;
-    t.x0 = blockIdx.y * TC;
+    t.x0 = (A.col0 + (int)blockIdx.y) * TC;
     t.z0 = blockIdx.x * TZ;
     t.row = U * (int)(threadIdx.x / (TZ / 4));
     t.zq = threadIdx.x % (TZ / 4);
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(threads_of(UV), 8) viscoac2d_fast_velocity_ker
     const QArgs& a = A.q;
     const int shot = a.slot_to_shot[blockIdx.z];
     const ShotDev sd = a.shots[shot];
-    const Place t = place<U>(a, sd, shot);
+    const Place t = place<U>(A, sd, shot);
     tile::bar_init(&bar);
     tile::release();
     tile::acquire();
@@ -193,7 +194,7 @@ __global__ void __launch_bounds__(threads_of(US), 5) viscoac2d_fast_stress_kerne
     const QArgs& a = A.q;
     const int shot = a.slot_to_shot[blockIdx.z];
     const ShotDev sd = a.shots[shot];
-    const Place t = place<U>(a, sd, shot);
+    const Place t = place<U>(A, sd, shot);
     tile::bar_init(&bar);
     tile::release();
     tile::acquire();
@@ -344,10 +345,13 @@ __global__ void __launch_bounds__(threads_of(US), 5) viscoac2d_fast_stress_kerne
 
 }  // namespace
 
-cudaError_t viscoac2d_fast_launch(const QFastArgs& A, int active, cudaStream_t st) {
-    const dim3 grid(A.q.L.ntz, A.q.L.ntx * (TX / TC), active);
-    if (cudaError_t e = tile::launch((const void*)viscoac2d_fast_velocity_kernel, grid, threads_of(UV), 0, st, A)) return e;
-    return tile::launch((const void*)viscoac2d_fast_stress_kernel, grid, threads_of(US), 0, st, A);
+cudaError_t viscoac2d_fast_launch(const QFastArgs& A, int active, cudaStream_t st, int* launches) {
+    const int ntz = A.q.L.ntz, ncol = A.q.L.ntx * (TX / TC);
+    if (cudaError_t e = tile::launch_columns((const void*)viscoac2d_fast_velocity_kernel, ntz, ncol, active, threads_of(UV), 0,
+                                             st, A, launches))
+        return e;
+    return tile::launch_columns((const void*)viscoac2d_fast_stress_kernel, ntz, ncol, active, threads_of(US), 0, st, A,
+                                launches);
 }
 
 void viscoac2d_fast_box(int box[2]) {

@@ -104,7 +104,7 @@ struct TileRef {
 __device__ __forceinline__ bool tile_of(const EArgs& a, TileRef& t) {
     t.shot = a.slot_to_shot[blockIdx.z];
     t.sd = a.shots[t.shot];
-    t.x0 = blockIdx.y * TC;
+    t.x0 = (a.col0 + (int)blockIdx.y) * TC;
     t.z0 = blockIdx.x * TZ;
     t.tile = t.x0 / TX * a.L.ntz + blockIdx.x;  // the 64 x 64 tile of the receiver lists
     return t.x0 < t.sd.nx;
@@ -281,16 +281,16 @@ void viscoel2d_box(int box[2]) {
     box[1] = SROWS;
 }
 
-cudaError_t viscoel2d_launch_step(const EArgs& a, int active, cudaStream_t st) {
-    const dim3 grid(a.L.ntz, a.L.ntx * (TX / TC), active);
+cudaError_t viscoel2d_launch_step(const EArgs& a, int active, cudaStream_t st, int* launches) {
+    const int ntz = a.L.ntz, ncol = a.L.ntx * (TX / TC);
     const int sv = (int)sizeof(float) * (3 * SMEM + 4), ss = (int)sizeof(float) * (2 * SMEM + 4);
     const void* kv = (const void*)e_velocity_kernel;
     const void* ks = (const void*)e_stress_kernel;
     static bool attr0[kMaxDevices] = {}, attr1[kMaxDevices] = {};
     if (cudaError_t e = smem_attr_once(kv, sv, attr0)) return e;
     if (cudaError_t e = smem_attr_once(ks, ss, attr1)) return e;
-    if (cudaError_t e = tile::launch(kv, grid, kThreads, sv, st, a)) return e;
-    return tile::launch(ks, grid, kThreads, ss, st, a);
+    if (cudaError_t e = tile::launch_columns(kv, ntz, ncol, active, kThreads, sv, st, a, launches)) return e;
+    return tile::launch_columns(ks, ntz, ncol, active, kThreads, ss, st, a, launches);
 }
 
 // QS:434-469 (density averaged in place, then buoyancy) and QS:473-551 (Blanch's tau for P and S),

@@ -10,6 +10,7 @@ from seismic_code_github_b200 import seisfd as S
 pytestmark = pytest.mark.gpu
 
 NZ, PML, NT = 32, 6, 8
+COLUMNS = {"viscoel": 4, "visco_exact": 8, "visco_gradient": 8, "elastic": 8, "visco": 16}  # per tile
 
 
 def run(kind, nx):
@@ -59,3 +60,10 @@ def compare(kind, nx):
 def test_source_stamp_of_a_long_line(kind):
     """The squared distances of the Gaussian stamp's normalising sum exceed 31 bits."""
     compare(kind, 100000)
+
+
+@pytest.mark.parametrize("kind", list(COLUMNS))
+def test_more_tile_columns_than_a_grid_holds(kind):
+    """More tile columns than one launch's grid.y holds (65535): a step takes several launches."""
+    n, n_wide = compare(kind, 65535 * COLUMNS[kind] + 100)
+    assert n_wide > n
