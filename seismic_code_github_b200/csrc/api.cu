@@ -97,6 +97,7 @@ struct sfd_ctx {
 
     cudaGraphExec_t graph = nullptr;
     bool graph_valid = false;
+    bool tuned = false;         // plan holds tune_schedule's pick for these shots and this kind of density
 
     // wavefield snapshot streams (sfd_set_snapshots)
     struct Snap {
@@ -298,7 +299,7 @@ void free_shot_buffers(sfd_ctx* c) {
     }
     if (c->graph) cudaGraphExecDestroy(c->graph);
     c->graph = nullptr;
-    c->graph_valid = false;
+    c->graph_valid = c->tuned = false;
     dfree(c->d_ckpt); dfree(c->d_div); dfree(c->d_adj); dfree(c->d_gseg); dfree(c->d_gacc);
     dfree(c->d_obs_nt); dfree(c->d_obs_tn); dfree(c->d_res); dfree(c->d_lam); dfree(c->d_misfit);
     dfree(c->d_grad); dfree(c->d_grad2); dfree(c->d_apx0); dfree(c->d_gsrc);
@@ -830,7 +831,9 @@ int finish_nan(sfd_ctx* ctx) {
 // Tuner for the forward step of the default (FMA) scheme.  Candidates: the tile kernel with one
 // tile per CTA (two CTAs per SM), the persistent tile kernel with double-buffered TMA, the small-tile
 // kernel (which runs untimed when the shot set has fewer tiles than the chip SMs), and the x-marching kernel with segments of 128, 256 or 512 columns (segments longer than the shots are
-// skipped).  Each runs a few steps on the real shot set, twice; the fastest is kept.  All
+// skipped).  Each runs a few steps on the real shot set, twice; the fastest is kept until the shots or the
+// kind of density change (a gradient, which never makes the forward's captured loop valid, would otherwise
+// time them again on every call).  All
 // candidates give bit-identical results.  SFD_FMA_STAGES=1|2 forces a tile schedule,
 // SFD_MARCH_SEG=<columns> forces the x-marching kernel with that segment length.
 int tune_schedule(sfd_ctx* ctx) {
@@ -842,6 +845,7 @@ int tune_schedule(sfd_ctx* ctx) {
             ctx->plan.seg = 0;
             ctx->plan.forced = false;
             ctx->plan.pinned = true;
+            ctx->tuned = false;
             return SFD_OK;
         }
     }
@@ -851,15 +855,18 @@ int tune_schedule(sfd_ctx* ctx) {
             ctx->plan.stages = 1;
             ctx->plan.seg = s;
             ctx->plan.forced = ctx->plan.pinned = true;
+            ctx->tuned = false;
             return SFD_OK;
         }
     }
+    if (ctx->tuned) return SFD_OK;
     ctx->plan.pinned = ctx->plan.small = false;
     const long long tiles = (long long)active_shots(ctx, 0) * ctx->L.ntx * ctx->L.ntz;
     if (acoustic2d_use_small(ctx->plan, ctx->L, active_shots(ctx, 0))) {  // every launch runs the small tiles
         ctx->plan.stages = 1;
         ctx->plan.seg = 0;
         ctx->plan.forced = false;
+        ctx->tuned = true;
         return SFD_OK;
     }
     struct Cand {
@@ -901,6 +908,7 @@ int tune_schedule(sfd_ctx* ctx) {
     ctx->plan.seg = cands[pick].seg;
     ctx->plan.small = cands[pick].small;
     ctx->plan.pinned = false;
+    ctx->tuned = true;
     return SFD_OK;
 }
 
@@ -1360,7 +1368,7 @@ int run_gradient(sfd_ctx* ctx, const float* obs, float* misfit, float* grad_vp, 
     auto t0 = std::chrono::steady_clock::now();
     if (!visco && ctx->varden && !ctx->d_b[0] && (rc = form_buoyancy(ctx))) return rc;
     if ((rc = grad_alloc(ctx))) return rc;
-    if (!ctx->graph_valid && (rc = tune_schedule(ctx))) return rc;
+    if ((rc = tune_schedule(ctx))) return rc;
     CK(cudaMemcpyAsync(ctx->d_obs_nt, obs, sizeof(float) * ctx->rec_total,
                        dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->stream));
     long long launches = 0;
@@ -2262,6 +2270,7 @@ int sfd_set_model(sfd_ctx* ctx, const float* vp, const float* den, const float* 
         ctx->have_model = true;
         if ((urc = q_prepare(ctx))) return urc;
     }
+    if (ctx->varden != varden_old) ctx->tuned = false;
     if (ctx->varden != varden_old || (!ctx->varden && ctx->den_c != den_c_old)) {
         ctx->graph_valid = false;
         ctx->grad_valid = false;
@@ -2767,6 +2776,7 @@ int sfd_test_wait_timeout(sfd_ctx* ctx, int cta, int step, double limit_s) {
     ctx->test_wait_ns = cta < 0 ? 0ull : (unsigned long long)(limit_s * 1e9);
     ctx->graph_valid = false;  // the captured loop holds the step arguments
     ctx->grad_valid = false;
+    ctx->tuned = false;        // a wait that runs out would be timed with its candidate
     return SFD_OK;
 }
 
