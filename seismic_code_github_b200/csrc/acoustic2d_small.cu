@@ -459,14 +459,20 @@ cudaError_t acoustic2d_exact_launch(int radius, const Acou2DArgs& a, int active,
     return launch_mode<16, kExact>(radius, a, active, varden, st);
 }
 
-// With fewer 64 x 64 tiles than SMs a step of the tile kernel costs the same 7 to 10 us however few they
-// are.  Measured (us a step, tile kernel / small tiles): order 16, 36 to 108 tiles 7.7 / 5.4 to 6.0, 144 tiles
-// 7.7 / 8.5, 576 tiles 20.5 / 24.5; order 8 with variable density (whose divisions the tile kernel repeats
-// in longer chains) 36 tiles 9.9 / 5.2, 315 tiles 21.9 / 15.2, 1680 tiles 82 / 80.  Above one tile per SM the
-// plan's `small` decides, which the tuner sets by timing both.
+// One wave of small tiles (five CTAs per SM, 92 tiles of 64 x 64) takes the same time however few they are, and so
+// do up to one of the tile kernel's persistent CTAs per SM.  Measured (us a step; small tiles / persistent CTAs
+// / one tile per CTA): order 16, 64 to 90 tiles 5.4 / 7.2 / 9.5, 99 tiles 7.5 / 7.0 / 9.9, 147 tiles 9.2 / 7.4 / 8.9;
+// order 16 with variable density 5.7 / 8.0 / 11, 8.0 / 7.8 / 11.8, 9.8 / 8.2 / 10.6; order 8 4.4 / 6.6 / 8.5, 6.2 / 6.4 /
+// 9.0, 7.6 / 6.7 / 8.0; order 4 4.4 / 6.2 / 8, 4.4 / 6.1 / 8.2, 6.8 / 6.3 / 7.3; gradients alike.  So one wave runs the
+// small tiles, and beyond it the tuner times both.  Steps with fewer tiles than SMs, but more than a wave, under
+// a plan that does not run persistent CTAs (the last shots of an uneven batch) take the small tiles too.
+bool acoustic2d_one_small_wave(const Layout2D& L, int active) {
+    return (long long)active * L.ntx * L.ntz * (kTileX / 16) * (kTileZ / TZ) <= 5LL * num_sms();
+}
 bool acoustic2d_use_small(const Acou2DPlan& plan, const Layout2D& L, int active) {
     if (plan.pinned) return false;
-    return plan.small || (long long)active * L.ntx * L.ntz < num_sms();
+    return plan.small || acoustic2d_one_small_wave(L, active) ||
+           (plan.stages == 1 && (long long)active * L.ntx * L.ntz < num_sms());
 }
 
 }  // namespace sfd

@@ -830,11 +830,11 @@ int finish_nan(sfd_ctx* ctx) {
 
 // Tuner for the forward step of the default (FMA) scheme.  Candidates: the tile kernel with one
 // tile per CTA (two CTAs per SM), the persistent tile kernel with double-buffered TMA, the small-tile
-// kernel (which runs untimed when the shot set has fewer tiles than the chip SMs), and the x-marching kernel with segments of 128, 256 or 512 columns (segments longer than the shots are
-// skipped).  Each runs a few steps on the real shot set, twice; the fastest is kept until the shots or the
-// kind of density change (a gradient, which never makes the forward's captured loop valid, would otherwise
-// time them again on every call).  All
-// candidates give bit-identical results.  SFD_FMA_STAGES=1|2 forces a tile schedule,
+// kernel (which runs untimed when the shot set is one wave of its CTAs), and the x-marching kernel with
+// segments of 128, 256 or 512 columns (segments longer than the shots are skipped).  Each runs a few steps
+// on the real shot set, twice; the fastest is kept until the shots or the kind of density change (a
+// gradient, which never makes the forward's captured loop valid, would otherwise time them again on every
+// call).  All candidates give bit-identical results.  SFD_FMA_STAGES=1|2 forces a tile schedule,
 // SFD_MARCH_SEG=<columns> forces the x-marching kernel with that segment length.
 int tune_schedule(sfd_ctx* ctx) {
     if ((ctx->g.flags & SFD_EXACT) || ctx->g.scheme != SFD_ACOUSTIC_2D) return SFD_OK;
@@ -862,7 +862,7 @@ int tune_schedule(sfd_ctx* ctx) {
     if (ctx->tuned) return SFD_OK;
     ctx->plan.pinned = ctx->plan.small = false;
     const long long tiles = (long long)active_shots(ctx, 0) * ctx->L.ntx * ctx->L.ntz;
-    if (acoustic2d_use_small(ctx->plan, ctx->L, active_shots(ctx, 0))) {  // every launch runs the small tiles
+    if (acoustic2d_one_small_wave(ctx->L, active_shots(ctx, 0))) {  // every launch runs the small tiles
         ctx->plan.stages = 1;
         ctx->plan.seg = 0;
         ctx->plan.forced = false;

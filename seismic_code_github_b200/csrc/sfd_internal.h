@@ -401,6 +401,7 @@ inline bool acoustic2d_use_march(const Acou2DPlan& plan, const Layout2D& L, int 
 // The small-tile kernel (acoustic2d_small.cu): the tile kernel's values bit for bit, for launches with
 // few tiles; adj as in acoustic2d_fma_launch.
 cudaError_t acoustic2d_small_launch(int radius, const Acou2DArgs& a, int active, bool varden, cudaStream_t st, bool adj);
+bool acoustic2d_one_small_wave(const Layout2D& L, int active);  // the small tiles run untimed
 bool acoustic2d_use_small(const Acou2DPlan& plan, const Layout2D& L, int active);
 // SFD_EXACT: the reference's operation order
 // out[i] = c / den[i] (rounded to nearest)

@@ -59,3 +59,28 @@ def test_schedules_are_timed_once_per_shot_set():
         assert bits_equal(grads[0], grads[1]) and not bits_equal(grads[1], grads[2])
     assert n[0] > n[1] == n[2]
     assert 2 * nt <= n[1] <= 3 * nt  # forward, adjoint, and the recomputation of what is not kept
+
+
+@pytest.mark.parametrize("order,varden", [(16, False), (8, True)])
+def test_small_tiles_run_untimed_in_one_wave_only(monkeypatch, order, varden):
+    """Up to one wave of its CTAs (92 tiles of 64 x 64 on 148 SMs) the small-tile kernel runs alone, forward
+    and gradient; beyond it (110 and 143 tiles) it is one candidate among those that are timed.  The
+    records equal those of a pinned schedule, which never runs it, bit for bit."""
+    nt = 20
+    for tx, tz in ((10, 9), (11, 10), (13, 11)):
+        recs = []
+        for pin in (None, "2"):
+            monkeypatch.delenv("SFD_FMA_STAGES", raising=False)
+            if pin:
+                monkeypatch.setenv("SFD_FMA_STAGES", pin)
+            e, _ = engine(64 * tx - 3, 64 * tz, order, 1, nt, varden)
+            with e:
+                first = launched(lambda: recs.append(e.forward().copy()))
+                grad = launched(lambda: e.gradient(np.zeros(e.record_size(), np.float32)))
+            if pin:
+                assert first == {"tile": nt} and set(grad) == {"tile"}
+            elif tx * tz <= 92:
+                assert first == {"small": nt} and set(grad) == {"small"}
+            else:
+                assert first["small"] >= 20 and first["tile"] >= 40
+        assert np.abs(recs[0]).max() > 0 and bits_equal(recs[0], recs[1])
