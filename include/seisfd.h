@@ -222,7 +222,8 @@ int sfd_get_wavelet_gradient(sfd_ctx* ctx, int shot, float* out);
  * device waits): in the forwards and gradients that follow, CTA `cta` of the 2-D acoustic FMA
  * step `step` issues none of its TMA box loads and gives up waiting for them after limit_s
  * seconds (0 < limit_s <= 10; every other wait keeps its limit of about one second).  That call
- * returns SFD_ERR_TIMEOUT and leaves the context usable.  cta < 0 removes the hook. */
+ * returns SFD_ERR_TIMEOUT and leaves the context usable.  Small launches, which otherwise run a kernel
+ * without such loads, run the tile kernel while the hook is set.  cta < 0 removes the hook. */
 int sfd_test_wait_timeout(sfd_ctx* ctx, int cta, int step, double limit_s);
 
 /* Checkpoint interval of sfd_gradient in steps (0 = ceil(sqrt(nt))).  The forward state of

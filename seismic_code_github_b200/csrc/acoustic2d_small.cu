@@ -470,7 +470,7 @@ bool acoustic2d_one_small_wave(const Layout2D& L, int active) {
     return (long long)active * L.ntx * L.ntz * (kTileX / 16) * (kTileZ / TZ) <= 5LL * num_sms();
 }
 bool acoustic2d_use_small(const Acou2DPlan& plan, const Layout2D& L, int active) {
-    if (plan.pinned) return false;
+    if (plan.pinned || plan.hooked) return false;
     return plan.small || acoustic2d_one_small_wave(L, active) ||
            (plan.stages == 1 && (long long)active * L.ntx * L.ntz < num_sms());
 }

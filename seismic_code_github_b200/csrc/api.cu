@@ -862,7 +862,7 @@ int tune_schedule(sfd_ctx* ctx) {
     if (ctx->tuned) return SFD_OK;
     ctx->plan.pinned = ctx->plan.small = false;
     const long long tiles = (long long)active_shots(ctx, 0) * ctx->L.ntx * ctx->L.ntz;
-    if (acoustic2d_one_small_wave(ctx->L, active_shots(ctx, 0))) {  // every launch runs the small tiles
+    if (!ctx->plan.hooked && acoustic2d_one_small_wave(ctx->L, active_shots(ctx, 0))) {  // every launch runs the small tiles
         ctx->plan.stages = 1;
         ctx->plan.seg = 0;
         ctx->plan.forced = false;
@@ -875,7 +875,7 @@ int tune_schedule(sfd_ctx* ctx) {
     };
     std::vector<Cand> cands = {{1, 0}, {2, 0}};
     // beyond this the larger halo always loses (measured at 1680 tiles: equal at best)
-    if (tiles < 1500) cands.push_back({1, 0, true});
+    if (tiles < 1500 && !ctx->plan.hooked) cands.push_back({1, 0, true});
     const int width = ctx->L.ntx * ctx->L.tx;
     for (int seg : {128, 256, 512})
         if (seg < width || seg == 128) cands.push_back({1, seg});
@@ -2773,6 +2773,7 @@ int sfd_test_wait_timeout(sfd_ctx* ctx, int cta, int step, double limit_s) {
     if (!ctx || (cta >= 0 && (step < 0 || !(limit_s > 0.0) || limit_s > 10.0))) return SFD_ERR_ARG;
     ctx->test_cta = cta < 0 ? -1 : cta;
     ctx->test_step = step;
+    ctx->plan.hooked = cta >= 0;
     ctx->test_wait_ns = cta < 0 ? 0ull : (unsigned long long)(limit_s * 1e9);
     ctx->graph_valid = false;  // the captured loop holds the step arguments
     ctx->grad_valid = false;

@@ -370,6 +370,7 @@ struct Acou2DPlan {
     bool forced; // seg set by SFD_MARCH_SEG: x-marching even where its grid does not fill the device
     bool pinned; // stages or seg set by the environment: no small tiles either
     bool small;  // the small-tile kernel won the tuner's comparison on this shot set
+    bool hooked; // sfd_test_wait_timeout is set: no small tiles, which have no wait to run out
 };
 // Model arrays on the device carry this many replicated rows above z = 0 and below z = nz - 1
 // so that vectorised halo reads stay inside the allocation and see finite values.
