@@ -1256,7 +1256,7 @@ int enqueue_gradient_range(sfd_ctx* ctx, const GradRange& r, long long* launches
         CK(launch_adjoint_init(ctx->d_adj, ctx->d_adj + fs, make_adj_args(ctx, r, 0, nullptr), ctx->radius, r.first,
                                r.count, nrec_max, ctx->stream));
     }
-    *launches += 2;
+    *launches += visco && nrec_max > 0 ? 3 : 2;
     // segments, last to first
     for (int j = ncp - 1; j >= 0; j--) {
         const int k0 = j * C, k1 = std::min(k0 + C, ctx->nt_max);

@@ -23,8 +23,8 @@
 // so that d misfit / d p1 = dt sum g1 and d misfit / d p2 = f sum g2.  The transposed
 // rotated-staggered derivatives gather from the mirrored taps of QS:843-966.  Kernel A reads the halo of
 // T1, T4 and writes only velocity adjoints and Qx, Qz; kernel B reads the halo of Qx, Qz and writes only
-// its own cells (its receivers' residuals go to sx^, sz^, sr^ and, through the same factors, to T1 and
-// T4), so neither launch races with itself.
+// its own cells (with its receivers' residuals in sx^, sz^, sr^ before T1 and T4 are formed), so neither
+// launch races with itself.
 //
 // Bound: memory (132 B a cell).  Each kernel's two differentiated fields arrive by TMA on tiles of 64 rows
 // by 8 columns with two cells per thread, as in viscoac2d.cu (measurements there); before, kernel A staged
@@ -78,20 +78,6 @@ __device__ __forceinline__ float2 pair(const float* s, int dx, int dz) {
 }
 __device__ __forceinline__ float2 bc(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, bc(-1.0f), a); }
-
-// residual v of one receiver into the stress adjoints of cell (x, z) and their share of T1, T4
-// (several receivers may share a cell, so the adds are atomic)
-__device__ __forceinline__ void add_residual(const QAdjArgs& a, int shot, const ShotDev& sd, int x, int z, float v) {
-    const long long c = cell(a, shot, x, z);
-    const float* tb = a.spg;
-    const int st = a.spg_stride;
-    const float d1 = a.dt * __ldg(a.p1 + (long long)min(sd.x0 + x, a.nx_model - 1) * a.mpitch + z);
-    atomicAdd(a.asx + c, v);
-    atomicAdd(a.asz + c, v);
-    atomicAdd(a.asr + c, v);
-    atomicAdd(a.t1 + c, sp(x, sd.nx, a.npx, tb + 4 * st, tb + 5 * st) * (d1 * v));
-    atomicAdd(a.t4 + c, sp(z, a.nz, a.npz, tb + 6 * st, tb + 7 * st) * (d1 * v));
-}
 
 __global__ void __launch_bounds__(kThreads, 8) q_adj_velocity_kernel(const __grid_constant__ QAdjArgs a) {
     __shared__ __align__(128) float sT[2 * SMEM];
@@ -178,9 +164,24 @@ __global__ void __launch_bounds__(kThreads, 8) q_adj_velocity_kernel(const __gri
 
 __global__ void __launch_bounds__(kThreads, 5) q_adj_stress_kernel(const __grid_constant__ QAdjArgs a) {
     __shared__ __align__(128) float sQ[2 * SMEM];
+    __shared__ float sR[TC * TZ];
     __shared__ uint64_t bar;
     Tile t;
     const bool on = tile_of(a, t);
+    // receivers of the 64 x 64 tile (their lists, before the wait for the kernel before) ...
+    const int* trp = a.tile_rec_ptr + t.sd.tile_rec_base + t.tile;
+    const int rb = on ? __ldg(trp) : 0, re = on ? __ldg(trp + 1) : 0, j0 = rb + threadIdx.x;
+    const bool res = a.step >= 1 && re > rb;
+    int ridx = 0, rx = 0, rz = 0;
+    auto receiver = [&](int j) {
+        ridx = a.tile_rec_idx[j];
+        rx = a.rec_x[t.sd.rec_list + ridx] - t.x0;
+        rz = a.rec_z[t.sd.rec_list + ridx] - t.z0;
+    };
+    if (res) {
+        if (j0 < re) receiver(j0);
+        for (int i = threadIdx.x; i < TC * TZ; i += kThreads) sR[i] = 0.0f;
+    }
     tile::bar_init(&bar);
     tile::release();
     tile::acquire();
@@ -209,6 +210,16 @@ __global__ void __launch_bounds__(kThreads, 5) q_adj_stress_kernel(const __grid_
             const long long mi = (long long)min(sd.x0 + gx, a.nx_model - 1) * a.mpitch + gz;
             p1[u] = __ldg(a.p1 + mi); p2[u] = __ldg(a.p2 + mi);
         }
+    }
+    // ... and the residual of step k-1 there (QM:452-459 transposed), S^ -> sx^, sz^, sr^, summed per cell while
+    // the boxes are on their way
+    if (res) {
+        for (int j = j0; j < re; j += kThreads) {
+            if (j > j0) receiver(j);
+            if (rx >= 0 && rx < TC)  // else another CTA of the 64 x 64 tile holds it
+                atomicAdd(&sR[rx * TZ + rz], a.res[sd.rec_base + (long long)(a.step - 1) * sd.nrec + ridx]);
+        }
+        __syncthreads();
     }
     if (!tile::staged(&bar, a.err_flag)) return;
     const float* tb = a.spg;
@@ -241,10 +252,17 @@ __global__ void __launch_bounds__(kThreads, 5) q_adj_stress_kernel(const __grid_
         const float aR = fmaf(f, hs[u][5], dt * hs[u][2]);
         a.g1[c] = g1[u] + fmaf(d1[u], u1, d4[u] * u4);
         a.g2[c] = g2[u] + fmaf(d1[u], w1, d4[u] * w4);
-        const float nsx = u1 + aS, nsz = u4 + aS, nrx = w1 + aR, nrz = w4 + aR;
+        float nsx = u1 + aS, nsz = u4 + aS, nsr = hs[u][2] + aS;
+        const float nrx = w1 + aR, nrz = w4 + aR;
+        const float v = res ? sR[(r0 + u * (TC / 2)) * TZ + z] : 0.0f;
+        if (v != 0.0f) {
+            nsx += v;
+            nsz += v;
+            nsr += v;
+        }
         a.asx[c] = nsx;
         a.asz[c] = nsz;
-        a.asr[c] = hs[u][2] + aS;
+        a.asr[c] = nsr;
         a.arx[c] = nrx;
         a.arz[c] = nrz;
         a.arr[c] = hs[u][5] + aR;
@@ -252,28 +270,32 @@ __global__ void __launch_bounds__(kThreads, 5) q_adj_stress_kernel(const __grid_
         a.t1[c] = axs * fmaf(e1, nsx, e2 * nrx);
         a.t4[c] = azs * fmaf(e1, nsz, e2 * nrz);
     }
-    // residual of step k-1 at the receivers of this tile (QM:452-459 transposed): S^ -> sx^, sz^, sr^
-    const int* trp = a.tile_rec_ptr + sd.tile_rec_base + t.tile;
-    const int rb = trp[0], re = trp[1];
-    if (a.step >= 1 && re > rb) {
-        __syncthreads();
-        for (int j = rb + threadIdx.x; j < re; j += kThreads) {
-            const int ridx = a.tile_rec_idx[j];
-            const int x = a.rec_x[sd.rec_list + ridx];
-            if (x < t.x0 || x >= t.x0 + TC) continue;  // another CTA of the 64 x 64 tile holds it
-            add_residual(a, t.shot, sd, x, a.rec_z[sd.rec_list + ridx],
-                         a.res[sd.rec_base + (long long)(a.step - 1) * sd.nrec + ridx]);
-        }
-    }
 }
 
-// sx^, sz^, sr^ of every shot in [first, first + n) += res of the shot's last step
+// sx^, sz^, sr^ of every shot in [first, first + n) += res of the shot's last step (several receivers may share
+// a cell, so the adds are atomic); then T1, T4 there, from the sums
 __global__ void q_adjoint_init_kernel(QAdjArgs a, int first_shot) {
     const int s = first_shot + blockIdx.y;
     const ShotDev sd = a.shots[s];
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < sd.nrec; r += gridDim.x * blockDim.x) {
-        add_residual(a, s, sd, a.rec_x[sd.rec_list + r], a.rec_z[sd.rec_list + r],
-                     a.res[sd.rec_base + (long long)(sd.nt - 1) * sd.nrec + r]);
+        const long long c = cell(a, s, a.rec_x[sd.rec_list + r], a.rec_z[sd.rec_list + r]);
+        const float v = a.res[sd.rec_base + (long long)(sd.nt - 1) * sd.nrec + r];
+        atomicAdd(a.asx + c, v);
+        atomicAdd(a.asz + c, v);
+        atomicAdd(a.asr + c, v);
+    }
+}
+__global__ void q_adjoint_init_t_kernel(QAdjArgs a, int first_shot) {
+    const int s = first_shot + blockIdx.y;
+    const ShotDev sd = a.shots[s];
+    const float* tb = a.spg;
+    const int st = a.spg_stride;
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < sd.nrec; r += gridDim.x * blockDim.x) {
+        const int x = a.rec_x[sd.rec_list + r], z = a.rec_z[sd.rec_list + r];
+        const long long c = cell(a, s, x, z), mi = (long long)min(sd.x0 + x, a.nx_model - 1) * a.mpitch + z;
+        const float e1 = a.dt * __ldg(a.p1 + mi), e2 = a.f_mem * __ldg(a.p2 + mi);
+        a.t1[c] = sp(x, sd.nx, a.npx, tb + 4 * st, tb + 5 * st) * fmaf(e1, a.asx[c], e2 * a.arx[c]);
+        a.t4[c] = sp(z, a.nz, a.npz, tb + 6 * st, tb + 7 * st) * fmaf(e1, a.asz[c], e2 * a.arz[c]);
     }
 }
 
@@ -320,6 +342,8 @@ cudaError_t q_adjoint_launch_init(const QAdjArgs& a, int first_shot, int nshot, 
     if (nrec_max <= 0 || nshot <= 0) return cudaSuccess;
     dim3 grid((nrec_max + 255) / 256, nshot);
     q_adjoint_init_kernel<<<grid, 256, 0, st>>>(a, first_shot);
+    if (cudaError_t e = cudaGetLastError()) return e;
+    q_adjoint_init_t_kernel<<<grid, 256, 0, st>>>(a, first_shot);
     return cudaGetLastError();
 }
 
