@@ -1063,7 +1063,8 @@ int grad_alloc(sfd_ctx* ctx) {
     const long long extra = budget > 0 ? (long long)(budget / (double)slot) : 0;
     int keep = ncp;  // segments keep .. ncp-1 are kept
     while (keep > 0 && (long long)ctx->nt_max - (long long)(keep - 1) * C <= extra) keep--;
-    const long long nslots = C + ((long long)ctx->nt_max - (long long)keep * C);
+    // (the last segment may be shorter than C: with nothing kept, keep * C lies beyond nt_max)
+    const long long nslots = C + std::max(0LL, (long long)ctx->nt_max - (long long)keep * C);
     if (cudaMalloc(&ctx->d_div, slot * nslots) != cudaSuccess) {
         cudaGetLastError();
         keep = ncp;
