@@ -204,9 +204,11 @@ int set_err(sfd_ctx* c, int code, const char* fmt, ...) {
 #define CK(call)                                                                               \
     do {                                                                                       \
         cudaError_t e_ = (call);                                                               \
-        if (e_ != cudaSuccess)                                                                 \
+        if (e_ != cudaSuccess) {                                                               \
+            (void)cudaGetLastError(); /* not the next call's launch checks' error */           \
             return set_err(ctx, e_ == cudaErrorMemoryAllocation ? SFD_ERR_NOMEM : SFD_ERR_CUDA, \
                            "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
+        }                                                                                      \
     } while (0)
 
 template <typename T>
@@ -285,7 +287,23 @@ float sponge3(const sfd_grid& g, int x, int y, int z) {
     return k < 0 ? 1.0f : (float)(-0.38 * k * k / (1.0 * g.pml * g.pml) + 1);
 }
 
+// The gradient's buffers.  Also called when one of them could not be allocated: the next gradient starts
+// from none, not from some.
+void free_gradient_buffers(sfd_ctx* c) {
+    dfree(c->d_ckpt); dfree(c->d_div); dfree(c->d_adj); dfree(c->d_gseg); dfree(c->d_gacc);
+    dfree(c->d_obs_nt); dfree(c->d_obs_tn); dfree(c->d_res); dfree(c->d_lam); dfree(c->d_misfit);
+    dfree(c->d_grad); dfree(c->d_grad2); dfree(c->d_apx0); dfree(c->d_gsrc);
+    dfree(c->g3_adj); dfree(c->g3_div); dfree(c->g3_ck1); dfree(c->g3_ck2); dfree(c->g3_gseg); dfree(c->g3_gacc);
+    c->g3_G = c->g3_C1 = c->g3_C2 = c->g3_n1 = c->g3_n2 = 0;
+    if (c->grad_graph) cudaGraphExecDestroy(c->grad_graph);
+    c->grad_graph = nullptr;
+    c->grad_valid = false;
+    c->have_grad = false;
+    c->grad_C = c->grad_ncp = 0;
+}
+
 void free_shot_buffers(sfd_ctx* c) {
+    c->have_shots = false;  // until the new ones are complete
     dfree(c->d_shots); dfree(c->d_slot); dfree(c->d_ident); dfree(c->d_wav);
     dfree(c->d_rec_x); dfree(c->d_rec_z); dfree(c->d_trp); dfree(c->d_tri); dfree(c->d_torder); dfree(c->d_rec_y);
     dfree(c->d_rec_tn); dfree(c->d_rec_nt); dfree(c->d_state); dfree(c->d_stamps); dfree(c->d_src_pre);
@@ -300,17 +318,8 @@ void free_shot_buffers(sfd_ctx* c) {
     if (c->graph) cudaGraphExecDestroy(c->graph);
     c->graph = nullptr;
     c->graph_valid = c->tuned = false;
-    dfree(c->d_ckpt); dfree(c->d_div); dfree(c->d_adj); dfree(c->d_gseg); dfree(c->d_gacc);
-    dfree(c->d_obs_nt); dfree(c->d_obs_tn); dfree(c->d_res); dfree(c->d_lam); dfree(c->d_misfit);
-    dfree(c->d_grad); dfree(c->d_grad2); dfree(c->d_apx0); dfree(c->d_gsrc);
-    dfree(c->g3_adj); dfree(c->g3_div); dfree(c->g3_ck1); dfree(c->g3_ck2); dfree(c->g3_gseg); dfree(c->g3_gacc);
-    c->g3_G = c->g3_C1 = c->g3_C2 = c->g3_n1 = c->g3_n2 = 0;
+    free_gradient_buffers(c);
     c->state_slabs = 0;
-    if (c->grad_graph) cudaGraphExecDestroy(c->grad_graph);
-    c->grad_graph = nullptr;
-    c->grad_valid = false;
-    c->have_grad = false;
-    c->grad_C = c->grad_ncp = 0;
 }
 
 }  // namespace
@@ -461,7 +470,7 @@ int form_buoyancy(sfd_ctx* ctx) {
             cudaGetLastError();
             for (auto& p : ctx->d_b) dfree(p);
             if (!(ctx->g.flags & SFD_EXACT)) ctx->have_model = ctx->graph_valid = ctx->grad_valid = false;
-            return set_err(ctx, SFD_ERR_CUDA, "out of device memory for the density factors of the model");
+            return set_err(ctx, SFD_ERR_NOMEM, "out of device memory for the density factors of the model");
         }
         CK(launch_buoyancy(ctx->d_den, ctx->g.dt / d[ax], ctx->d_b[n], (long long)mfloats, ctx->stream));
         n++;
@@ -1001,7 +1010,7 @@ GradShape grad_shape(const sfd_ctx* c) {
     return c->g.scheme == SFD_VISCOAC_2D ? GradShape{9, 2, 12, 2} : GradShape{3, 1, 6, 1};
 }
 
-int grad_alloc(sfd_ctx* ctx) {
+int grad_alloc_buffers(sfd_ctx* ctx) {
     const int C = ctx->ckpt_interval > 0 ? std::min(ctx->ckpt_interval, ctx->nt_max)
                                          : (int)std::ceil(std::sqrt((double)ctx->nt_max));
     const int ncp = (ctx->nt_max + C - 1) / C;
@@ -1074,6 +1083,12 @@ int grad_alloc(sfd_ctx* ctx) {
     ctx->grad_C = C;
     ctx->grad_ncp = ncp;
     return SFD_OK;
+}
+
+int grad_alloc(sfd_ctx* ctx) {
+    const int rc = grad_alloc_buffers(ctx);
+    if (rc) free_gradient_buffers(ctx);
+    return rc;
 }
 
 // shots [first, first + count) as one schedule; `slots` maps launch slots to shots
@@ -1837,7 +1852,7 @@ int plan3_choose(sfd_ctx* ctx, int Gmax, Plan3* out) {
                    budget / 1e9);
 }
 
-int g3_alloc(sfd_ctx* ctx, const Plan3& p) {
+int g3_alloc_buffers(sfd_ctx* ctx, const Plan3& p) {
     int rc;
     const bool same = ctx->g3_adj && p.G == ctx->g3_G && p.C1 == ctx->g3_C1 && p.C2 == ctx->g3_C2 &&
                       ctx->state_slabs == p.G;
@@ -1874,6 +1889,12 @@ int g3_alloc(sfd_ctx* ctx, const Plan3& p) {
         CK(cudaMalloc(&ctx->d_grad, sizeof(double) * (size_t)ctx->g.nx * ctx->g.ny * ctx->g.nz));
     }
     return SFD_OK;
+}
+
+int g3_alloc(sfd_ctx* ctx, const Plan3& p) {
+    const int rc = g3_alloc_buffers(ctx, p);
+    if (rc) free_gradient_buffers(ctx);
+    return rc;
 }
 
 // one forward step of the group's active slots (source before, receivers after when `gather`)

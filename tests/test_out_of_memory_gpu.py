@@ -1,0 +1,94 @@
+"""Calls that run out of device memory return SFD_ERR_NOMEM and leave a context that can be used: shots that
+could not be set are not there (SFD_ERR_STATE, no launch on missing buffers), and once there is memory the
+same context gives the records and gradients of one that never ran short, bit for bit."""
+import numpy as np
+import pytest
+
+from conftest import bits_equal, rel_l2
+from seismic_code_github_b200 import seisfd as S
+
+pytestmark = pytest.mark.gpu
+
+
+class Hog:
+    """Holds the device's free memory but for `leave` bytes."""
+
+    def __init__(self, leave):
+        import torch
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        self.t = torch.empty(max(0, torch.cuda.mem_get_info()[0] - leave), dtype=torch.uint8, device="cuda")
+
+    def release(self):
+        import torch
+        self.t = None
+        torch.cuda.empty_cache()
+
+
+def setup(kind):
+    rng = np.random.default_rng(7)
+    nt = 60
+    if kind == "cube":
+        n = 64
+        vp = (2000.0 + 300.0 * rng.random((n, n, n))).astype(np.float32)
+        e = S.Engine(S.ACOUSTIC_3D, n, n, 10.0, 10.0, 1e-3, 8, order=8, ny=n, dy=10.0)
+        e.set_model(vp, (1900.0 + 300.0 * rng.random(vp.shape)).astype(np.float32))
+        r = np.arange(10, 54, dtype=np.int32)
+        w = S.wavelet(S.WAVELET_RIC, nt, 1e-3, 25.0, 20)
+        return e, lambda k: [S.ShotSpec(30 + i % 4, 12, r, np.full(r.size, 12, np.int32), w, sy=30,
+                                        rec_y=np.full(r.size, 30, np.int32)) for i in range(k)]
+    nx = nz = 300
+    vp = (2000.0 + 300.0 * rng.random((nx, nz))).astype(np.float32)
+    den = (1900.0 + 300.0 * rng.random((nx, nz))).astype(np.float32)
+    rx, rz = np.arange(10, nx - 10, dtype=np.int32), np.full(nx - 20, 13, np.int32)
+    if kind == "visco":
+        e = S.Engine(S.VISCOAC_2D, nx, nz, 10.0, 10.0, 5e-4, 10, order=10, f0=20.0)
+        e.set_model(vp, den, (30.0 + 60.0 * rng.random((nx, nz))).astype(np.float32))
+        w = S.wavelet(S.WAVELET_Q, nt, 5e-4, 20.0)
+    else:
+        e = S.Engine(S.ACOUSTIC_2D, nx, nz, 10.0, 10.0, 1e-3, 10, order=16)
+        e.set_model(vp, den)
+        w = S.wavelet(S.WAVELET_RIC, nt, 1e-3, 25.0, 20)
+    return e, lambda k: [S.ShotSpec(nx // 2 + i % 16, 15, rx, rz, w) for i in range(k)]
+
+
+@pytest.mark.parametrize("kind", ["acoustic", "visco", "cube"])
+def test_a_context_survives_running_short(kind):
+    mb = 1 << 20
+    e, shots = setup(kind)
+    with e:
+        e.set_shots(shots(6))
+        obs = np.zeros(e.record_size(), np.float32)
+        rec, grad = e.forward().copy(), e.gradient(obs)[1].copy()
+    assert np.abs(rec).max() > 0 and np.abs(grad).max() > 0
+    e, shots = setup(kind)
+    with e:
+        e.set_shots(shots(6))
+        hog = Hog(64 * mb)
+        try:
+            with pytest.raises(S.SfdError) as err:
+                e.set_shots(shots(600))
+            assert err.value.status == S.ERR_NOMEM
+            with pytest.raises(S.SfdError) as err:
+                e.forward()
+            assert err.value.status == S.ERR_STATE
+        finally:
+            hog.release()
+        e.set_shots(shots(6))
+        assert bits_equal(e.forward(), rec)
+        failed = 0
+        for leave in (8, 40, 64, 72, 80, 90, 110, 140, 180):
+            hog = Hog(leave * mb)
+            try:
+                g = e.gradient(obs)[1]
+                # the 3-D schedule follows the memory, and with it the order of the imaging sums
+                assert rel_l2(g, grad) <= 1e-6 if kind == "cube" else bits_equal(g, grad)
+                break
+            except S.SfdError as err:
+                assert err.status == S.ERR_NOMEM, err
+                failed += 1
+            finally:
+                hog.release()
+        assert failed > 0
+        assert bits_equal(e.gradient(obs)[1], grad)
+        assert bits_equal(e.forward(), rec)
