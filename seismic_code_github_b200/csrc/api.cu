@@ -1001,13 +1001,13 @@ double q_kappa(float f0) {
 // ---------------------------------------------------------------------------------------------
 // Per scheme: fields kept in a checkpoint, forward derivatives kept per recomputed step,
 // adjoint fields, imaging sums.  Acoustic: P, Vx, Vz (one parity) / D / Q, X, Z ping-pong /
-// g.  Viscoacoustic: the eight in-place fields and sigma / Dx1 vx, Dz1 vz / eight adjoints + Qx, Qz, T1, T4 /
-// g1, g2.
+// g.  Viscoacoustic: the eight in-place fields (sigma is formed again) / Dx1 vx, Dz1 vz / eight adjoints + Qx,
+// Qz, T1, T4 / g1, g2.
 struct GradShape {
     int ckpt, div, adj, img;
 };
 GradShape grad_shape(const sfd_ctx* c) {
-    return c->g.scheme == SFD_VISCOAC_2D ? GradShape{9, 2, 12, 2} : GradShape{3, 1, 6, 1};
+    return c->g.scheme == SFD_VISCOAC_2D ? GradShape{8, 2, 12, 2} : GradShape{3, 1, 6, 1};
 }
 
 int grad_alloc_buffers(sfd_ctx* ctx) {
@@ -1228,7 +1228,7 @@ int grad_adj_step(sfd_ctx* ctx, const GradRange& r, int k, int act, const float*
 int grad_copy_state(sfd_ctx* ctx, const GradRange& r, int slot, int b, bool to_ckpt) {
     const size_t fs = (size_t)ctx->nshot * ctx->L.shot_stride;
     const size_t off = (size_t)r.first * ctx->L.shot_stride, len = (size_t)r.count * ctx->L.shot_stride;
-    const bool visco = ctx->g.scheme == SFD_VISCOAC_2D;  // nine in-place fields, no parity
+    const bool visco = ctx->g.scheme == SFD_VISCOAC_2D;  // in-place fields, no parity
     const int nf = grad_shape(ctx).ckpt;
     for (int f = 0; f < nf; f++) {
         float* st = ctx->d_state + (visco ? f : 2 * f + b) * fs + off;
@@ -1236,6 +1236,7 @@ int grad_copy_state(sfd_ctx* ctx, const GradRange& r, int slot, int b, bool to_c
         CK(cudaMemcpyAsync(to_ckpt ? ck : st, to_ckpt ? st : ck, len * sizeof(float), cudaMemcpyDeviceToDevice,
                            ctx->stream));
     }
+    if (visco && !to_ckpt) CK(viscoac2d_launch_sigma(make_qargs(ctx, 0), (long long)off, (long long)len, ctx->stream));
     return SFD_OK;
 }
 
@@ -1281,6 +1282,7 @@ int enqueue_gradient_range(sfd_ctx* ctx, const GradRange& r, long long* launches
             CK(cudaMemsetAsync(ctx->d_gseg + i * fs + off, 0, len * sizeof(float), ctx->stream));
         if (j < ctx->grad_keep) {  // recompute the segment from its checkpoint, keeping D_k
             if ((rc = grad_copy_state(ctx, r, j, k0 & 1, false))) return rc;
+            if (visco) (*launches)++;
             for (int k = k0; k < k1; k++) {
                 const int act = range_active(ctx, r, k);
                 if (act == 0) break;

@@ -109,6 +109,8 @@ struct QArgs {
 void q_box(int box[2]);  // TMA box (z, x) of the viscoacoustic kernels and their adjoint
 // (every launcher of a step adds the kernels it launched to *launches)
 cudaError_t viscoac2d_launch_step(const QArgs& a, int active, cudaStream_t st, int* launches);
+// sigma of the cells [first, first + n) of the slabs from the restored split parts
+cudaError_t viscoac2d_launch_sigma(const QArgs& a, long long first, long long n, cudaStream_t st);
 
 // Default (fast, FMA) viscoacoustic step (viscoac2d_fast.cu), all fields in place: merged sigma and r
 // everywhere, split parts in the sponge bands only (q.sx .. q.rr); q.vx / q.vz unused.

@@ -24,6 +24,7 @@
 // is half of it); two cells per thread 122 us, with their stencils paired 119 us.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -262,6 +263,20 @@ cudaError_t viscoac2d_launch_step(const QArgs& a, int active, cudaStream_t st, i
     if (cudaError_t e = tile::launch_columns((const void*)q_velocity_kernel, ntz, ncol, active, kThreads, 0, st, a, launches))
         return e;
     return tile::launch_columns((const void*)q_stress_kernel, ntz, ncol, active, kThreads, 0, st, a, launches);
+}
+
+// sigma = (sx + sz) + sr of n cells from each pointer on (n a multiple of four), as the stress kernel forms it
+__global__ void q_sigma_kernel(const float4* sx, const float4* sz, const float4* sr, float4* sg, long long n4) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
+        const float4 a = sx[i], b = sz[i], c = sr[i];
+        sg[i] = make_float4(fa(fa(a.x, b.x), c.x), fa(fa(a.y, b.y), c.y), fa(fa(a.z, b.z), c.z), fa(fa(a.w, b.w), c.w));
+    }
+}
+cudaError_t viscoac2d_launch_sigma(const QArgs& a, long long first, long long n, cudaStream_t st) {
+    auto at = [&](float* f) { return reinterpret_cast<float4*>(f + first); };
+    q_sigma_kernel<<<(unsigned)std::min<long long>((n / 4 + 255) / 256, 148 * 16), 256, 0, st>>>(at(a.sx), at(a.sz), at(a.sr),
+                                                                                            at(a.sg), n / 4);
+    return cudaGetLastError();
 }
 
 // QS:434-469 (density averaged in place, then buoyancy) and QS:473-551 (Blanch's tau method),

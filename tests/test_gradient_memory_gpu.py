@@ -1,6 +1,7 @@
 """The 2-D gradients when memory is short: with no room for kept derivatives every segment is recomputed from
 its checkpoint, and misfit and gradients equal those with everything kept bit for bit -- with a last
-segment shorter than the others too."""
+segment shorter than the others too; the viscoacoustic checkpoints hold the eight fields of the reference's
+state (sigma is formed from them)."""
 import numpy as np
 import pytest
 
@@ -42,3 +43,21 @@ def test_recomputed_segments_equal_kept_ones(kind, flags, interval):
     for j, g, gq, _ in out[1:]:
         assert np.abs(g).max() > 0 and rel_l2(j, out[0][0]) <= 1e-6 and bits_equal(g, out[0][1])
         assert not visco or bits_equal(gq, out[0][2])
+
+
+def test_viscoacoustic_checkpoints_hold_eight_fields():
+    import torch
+    nx = nz = 300
+    nt, nshot = 64, 8
+    with engine("visco", nx, nz, 8, (nt,) * nshot, S.EXACT) as e:
+        e.set_memory_limit(1)
+        e.forward()
+        obs = np.zeros(e.record_size(), np.float32)
+        torch.cuda.synchronize()
+        free0 = torch.cuda.mem_get_info()[0]
+        e.gradient(obs)
+        used = free0 - torch.cuda.mem_get_info()[0]
+    # slabs of the 64 x 64 tiles with margins of 8 columns and 8 rows, rows rounded to 32 floats: eight
+    # checkpoints, 12 adjoint fields, two imaging sums in float and double, two derivatives per step of a segment
+    slab = 4 * nshot * (8 + 320 + 8) * 352
+    assert used <= (8 * 8 + 12 + 2 + 4 + 2 * 8) * slab + (16 << 20)
