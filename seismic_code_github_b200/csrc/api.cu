@@ -97,6 +97,7 @@ struct sfd_ctx {
 
     cudaGraphExec_t graph = nullptr;
     bool graph_valid = false;
+    bool sums = true;           // the state has the slabs of the sums that the split schemes stage
     bool tuned = false;         // plan holds tune_schedule's pick for these shots and this kind of density
 
     // wavefield snapshot streams (sfd_set_snapshots)
@@ -508,7 +509,7 @@ QArgs make_qargs(const sfd_ctx* c, int step) {
     float* f[9];
     for (int i = 0; i < 9; i++) f[i] = c->d_state + i * fs;
     a.one = 1.0f;
-    a.sg = f[8];
+    a.sg = c->sums ? f[8] : nullptr;
     a.tm_vx = c->q_maps[0];
     a.tm_vz = c->q_maps[1];
     a.tm_s = c->q_maps[2];
@@ -550,7 +551,7 @@ EArgs make_eargs(const sfd_ctx* c, int step) {
     EArgs a{};
     const QArgs q = make_qargs(c, step);
     const long long fs = (long long)c->nshot * c->L.shot_stride;
-    for (int i = 0; i < E_NFIELDS; i++) a.f[i] = c->d_state + i * fs;
+    for (int i = 0; i < E_NFIELDS; i++) a.f[i] = i < E_VX || c->sums ? c->d_state + i * fs : nullptr;
     for (int k = 0; k < 5; k++) a.tm[k] = c->etmaps[k];
     a.err_flag = c->d_err;
     a.L = q.L;
@@ -575,7 +576,7 @@ EArgs make_eargs(const sfd_ctx* c, int step) {
 IArgs make_iargs(const sfd_ctx* c, int step) {
     IArgs a{};
     const long long fs = (long long)c->nshot * c->L.shot_stride;
-    for (int i = 0; i < I_NFIELDS; i++) a.f[i] = c->d_state + i * fs;
+    for (int i = 0; i < I_NFIELDS; i++) a.f[i] = i < I_VX || c->sums ? c->d_state + i * fs : nullptr;
     for (int k = 0; k < 5; k++) a.tm[k] = c->etmaps[k];
     a.err_flag = c->d_err;
     a.L = c->L;
@@ -1236,7 +1237,7 @@ int grad_copy_state(sfd_ctx* ctx, const GradRange& r, int slot, int b, bool to_c
         CK(cudaMemcpyAsync(to_ckpt ? ck : st, to_ckpt ? st : ck, len * sizeof(float), cudaMemcpyDeviceToDevice,
                            ctx->stream));
     }
-    if (visco && !to_ckpt) CK(viscoac2d_launch_sigma(make_qargs(ctx, 0), (long long)off, (long long)len, ctx->stream));
+    if (visco && !to_ckpt && ctx->sums) CK(viscoac2d_launch_sigma(make_qargs(ctx, 0), (long long)off, (long long)len, ctx->stream));
     return SFD_OK;
 }
 
@@ -1282,7 +1283,7 @@ int enqueue_gradient_range(sfd_ctx* ctx, const GradRange& r, long long* launches
             CK(cudaMemsetAsync(ctx->d_gseg + i * fs + off, 0, len * sizeof(float), ctx->stream));
         if (j < ctx->grad_keep) {  // recompute the segment from its checkpoint, keeping D_k
             if ((rc = grad_copy_state(ctx, r, j, k0 & 1, false))) return rc;
-            if (visco) (*launches)++;
+            if (visco && ctx->sums) (*launches)++;
             for (int k = k0; k < k1; k++) {
                 const int act = range_active(ctx, r, k);
                 if (act == 0) break;
@@ -2498,9 +2499,20 @@ int sfd_set_shots(sfd_ctx* ctx, int nshot, const sfd_shot* shots) {
         CK(cudaMalloc(&ctx->d_rec2_tn, rec_bytes));
         CK(cudaMalloc(&ctx->d_rec2_nt, rec_bytes));
     }
-    ctx->state_floats = (iso ? I_NFIELDS : elastic ? E_NFIELDS : q_fast(ctx) ? kQFastSlabs : visco ? 9 : 6) *
-                        (size_t)nshot * L.shot_stride;
-    CK(cudaMalloc(&ctx->d_state, ctx->state_floats * sizeof(float)));
+    // The slabs of the state; without those of the sums where they do not fit, so that a batch may be as large as
+    // its split parts allow.
+    const size_t fields = (size_t)nshot * L.shot_stride;
+    const int slabs = iso ? I_NFIELDS : elastic ? E_NFIELDS : q_fast(ctx) ? kQFastSlabs : visco ? 9 : 6;
+    const int fewer = iso ? (int)I_VX : elastic ? (int)E_VX : visco && !q_fast(ctx) ? 8 : slabs;
+    ctx->sums = true;
+    ctx->state_floats = slabs * fields;
+    if (fewer < slabs && cudaMalloc(&ctx->d_state, ctx->state_floats * sizeof(float)) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->d_state = nullptr;
+        ctx->sums = false;
+        ctx->state_floats = fewer * fields;
+    }
+    if (!ctx->d_state) CK(cudaMalloc(&ctx->d_state, ctx->state_floats * sizeof(float)));
     CK(cudaMalloc(&ctx->d_src_pre, sizeof(float) * nshot));
     if (visco) {
         // Gaussian source stamps (QS:1340-1444, YPUB:1429-1466) and the split cosine sponge tables
@@ -2511,14 +2523,14 @@ int sfd_set_shots(sfd_ctx* ctx, int nshot, const sfd_shot* shots) {
         viscoac2d_sponge_tables(ctx->g.pml, ctx->g.pml, ctx->g.dx, ctx->g.dz, ctx->spg_stride, tab.data());
         dfree(ctx->d_spg);
         if ((rc = up(&ctx->d_spg, tab))) return rc;
-        for (int f = 0; (iso || elastic) && f < 5; f++) {
+        for (int f = 0; (iso || elastic) && ctx->sums && f < 5; f++) {
             int box[2];
             if (iso) elastic2d_box(box);
             else viscoel2d_box(box);
             float* base = ctx->d_state + ((iso ? (int)I_VX : (int)E_VX) + f) * (long long)nshot * L.shot_stride;
             if ((rc = encode_field_map(ctx, &ctx->etmaps[f], base, L, nshot, box))) return rc;
         }
-        for (int f = 0; ctx->g.scheme == SFD_VISCOAC_2D && f < 3; f++) {
+        for (int f = 0; ctx->g.scheme == SFD_VISCOAC_2D && f < (ctx->sums ? 3 : 2); f++) {
             int box[2];
             q_box(box);
             float* base = ctx->d_state + (f < 2 ? f : 8) * (long long)nshot * L.shot_stride;

@@ -120,6 +120,16 @@ __device__ __forceinline__ void stage(float* s, uint64_t* bar, const IArgs& a, c
         tile::box(s + f * kSmem, &a.tm[field[f] - I_VX], a.L.gz + t.z0 - HZ, a.L.gx + t.x0 - H, t.shot, bar);
 }
 
+// The same without the slabs of the sums, from the split parts f0, f0 + 1 (the caller's __syncthreads follows)
+__device__ __forceinline__ void stage_parts(float* s, const IArgs& a, const TileRef& t, int f0) {
+    for (int i = threadIdx.x; i < kSmem / 4; i += kThreads) {
+        const int r = i / (SW / 4), c = 4 * (i % (SW / 4));
+        const long long off = cell(a, t.shot, t.x0 - H + r, t.z0 - HZ + c);
+        const float4 p = *reinterpret_cast<const float4*>(a.f[f0] + off), q = *reinterpret_cast<const float4*>(a.f[f0 + 1] + off);
+        *reinterpret_cast<float4*>(s + r * SW + c) = add4(p, q, a.one);
+    }
+}
+
 // one split-sponge factor in YPUB:851-897's order (near-side table, then far-side table)
 __device__ __forceinline__ float xs(float u, int x, int n, int np, const float* tn, const float* tp) {
     if (x <= np) u = fm(u, tn[x]);
@@ -245,7 +255,9 @@ struct Vec {
     }
 };
 
-template <bool FS>
+// SUMS = false: no memory for the slabs of the sums, two thirds of the state.  The tile and its halo are summed
+// by the threads: 58 ms against 35 for 275 steps of 8 shots of 1280 x 483.
+template <bool FS, bool SUMS>
 __global__ void __launch_bounds__(kThreads, 5) iso_velocity_kernel(const __grid_constant__ IArgs a) {
     extern __shared__ __align__(128) float smem[];
     const float* sSxx = smem;
@@ -258,7 +270,12 @@ __global__ void __launch_bounds__(kThreads, 5) iso_velocity_kernel(const __grid_
     tile::release();
     tile::acquire();
     if (!on) return;
-    if (threadIdx.x == 0) {
+    if (!SUMS) {
+        stage_parts(smem, a, t, I_SXXX);
+        stage_parts(smem + kSmem, a, t, I_SXZX);
+        stage_parts(smem + 2 * kSmem, a, t, I_SZZX);
+        __syncthreads();
+    } else if (threadIdx.x == 0) {
         const int f[3] = {I_SXX, I_SXZ, I_SZZ};
         stage<3>(smem, bar, a, t, f);
     }
@@ -269,14 +286,14 @@ __global__ void __launch_bounds__(kThreads, 5) iso_velocity_kernel(const __grid_
     const int r = threadIdx.x >> 4;
     const Vec<FS> e(a, t, r, z);
     if (t.x0 + r >= nx || e.gz >= nz || e.air) {
-        tile::staged(bar, a.err_flag);  // leave with the CTA's copies landed
+        if (SUMS) tile::staged(bar, a.err_flag);  // leave with the CTA's copies landed
         return;
     }
     float4 vxx = ld4(a.f[I_VXX], e.c), vxz = ld4(a.f[I_VXZ], e.c);
     float4 vzx = ld4(a.f[I_VZX], e.c), vzz = ld4(a.f[I_VZZ], e.c);
     const float4 b2 = __ldg(reinterpret_cast<const float4*>(a.b2e + e.mi));
     const float4 b1 = __ldg(reinterpret_cast<const float4*>(a.b1e + e.mi));
-    if (!tile::staged(bar, a.err_flag)) return;
+    if (SUMS && !tile::staged(bar, a.err_flag)) return;
     const float4 d_xx = dx4<0>(sSxx, r + H, z + HZ, a.a, a.one);  // Dx0 strxx
     const float4 d_zx = dx4<1>(sSxz, r + H, z + HZ, a.a, a.one);  // Dx1 strxz
     // YPRI:310-326: vx parts with sponges spgxn/spgxp and spgzn/spgzp, vz parts with
@@ -317,11 +334,13 @@ __global__ void __launch_bounds__(kThreads, 5) iso_velocity_kernel(const __grid_
     }
     st4(a.f[I_VXX], e.c, vxx); st4(a.f[I_VXZ], e.c, vxz);
     st4(a.f[I_VZX], e.c, vzx); st4(a.f[I_VZZ], e.c, vzz);
-    st4(a.f[I_VX], e.c, add4(vxx, vxz, a.one));  // YPRI:316
-    st4(a.f[I_VZ], e.c, add4(vzx, vzz, a.one));  // YPRI:326
+    if (SUMS) {
+        st4(a.f[I_VX], e.c, add4(vxx, vxz, a.one));  // YPRI:316
+        st4(a.f[I_VZ], e.c, add4(vzx, vzz, a.one));  // YPRI:326
+    }
 }
 
-template <bool FS>
+template <bool FS, bool SUMS>
 __global__ void __launch_bounds__(kThreads, 5) iso_stress_kernel(const __grid_constant__ IArgs a) {
     extern __shared__ __align__(128) float smem[];
     const float* sVx = smem;
@@ -333,7 +352,11 @@ __global__ void __launch_bounds__(kThreads, 5) iso_stress_kernel(const __grid_co
     tile::release();
     tile::acquire();
     if (!on) return;
-    if (threadIdx.x == 0) {
+    if (!SUMS) {
+        stage_parts(smem, a, t, I_VXX);
+        stage_parts(smem + kSmem, a, t, I_VZX);
+        __syncthreads();
+    } else if (threadIdx.x == 0) {
         const int f[2] = {I_VX, I_VZ};
         stage<2>(smem, bar, a, t, f);
     }
@@ -362,7 +385,7 @@ __global__ void __launch_bounds__(kThreads, 5) iso_stress_kernel(const __grid_co
         lam = __ldg(reinterpret_cast<const float4*>(a.lam + e.mi));
         mue = __ldg(reinterpret_cast<const float4*>(a.mue + e.mi));
     }
-    if (!tile::staged(bar, a.err_flag)) return;
+    if (SUMS && !tile::staged(bar, a.err_flag)) return;
     if (work) {
         const float4 d1 = dx4<1>(sVx, r + H, z + HZ, a.a, a.one);  // Dx1 vx
         const float4 d3 = dx4<0>(sVz, r + H, z + HZ, a.a, a.one);  // Dx0 vz
@@ -436,9 +459,11 @@ __global__ void __launch_bounds__(kThreads, 5) iso_stress_kernel(const __grid_co
         }
 #pragma unroll
         for (int k = 0; k < 6; k++) st4(a.f[I_SXXX + k], e.c, v[k]);
-        st4(a.f[I_SXX], e.c, add4(v[0], v[1], a.one));
-        st4(a.f[I_SZZ], e.c, add4(v[2], v[3], a.one));
-        st4(a.f[I_SXZ], e.c, add4(v[4], v[5], a.one));
+        if (SUMS) {
+            st4(a.f[I_SXX], e.c, add4(v[0], v[1], a.one));
+            st4(a.f[I_SZZ], e.c, add4(v[2], v[3], a.one));
+            st4(a.f[I_SXZ], e.c, add4(v[4], v[5], a.one));
+        }
     }
     // receivers: record1 = vx, record2 = vz after the step (YPRI:361-367, YPUB:2-16); the
     // velocities are final after the velocity kernel and staged here
@@ -472,7 +497,7 @@ __global__ void iso_surface_kernel(const __grid_constant__ IArgs a) {
     const float ux = -a.f[I_SXZX][c], uz = -a.f[I_SXZZ][c];
     a.f[I_SXZX][cu] = ux;
     a.f[I_SXZZ][cu] = uz;
-    a.f[I_SXZ][cu] = fa(ux, uz);
+    if (a.f[I_SXZ]) a.f[I_SXZ][cu] = fa(ux, uz);
     if (x + 1 < sd.nx) {
         const long long cn = cell(a, shot, x + 1, zs);
         const long long mi = (long long)mc * a.mpitch + zs;
@@ -569,12 +594,12 @@ __global__ void __launch_bounds__(32) iso_smooth_kernel(const __grid_constant__ 
 
 namespace {
 
-template <bool FS>
+template <bool FS, bool SUMS>
 cudaError_t launch_pair(const IArgs& a, int active, cudaStream_t st, int* launches) {
     const int ntz = a.L.ntz, ncol = a.L.ntx * (TX / TC);
     const int sv = (int)sizeof(float) * (3 * kSmem + 4), ss = (int)sizeof(float) * (2 * kSmem + 4);
-    const void* kv = (const void*)iso_velocity_kernel<FS>;
-    const void* ks = (const void*)iso_stress_kernel<FS>;
+    const void* kv = (const void*)iso_velocity_kernel<FS, SUMS>;
+    const void* ks = (const void*)iso_stress_kernel<FS, SUMS>;
     static bool attr0[kMaxDevices] = {}, attr1[kMaxDevices] = {};
     if (cudaError_t e = smem_attr_once(kv, sv, attr0)) return e;
     if (cudaError_t e = smem_attr_once(ks, ss, attr1)) return e;
@@ -590,7 +615,11 @@ void elastic2d_box(int box[2]) {
 }
 
 cudaError_t elastic2d_launch_step(const IArgs& a, int active, int nx_max, cudaStream_t st, int* launches) {
-    const cudaError_t e = a.fs ? launch_pair<true>(a, active, st, launches) : launch_pair<false>(a, active, st, launches);
+    const bool sums = a.f[I_VX] != nullptr;
+    const cudaError_t e = a.fs ? (sums ? launch_pair<true, true>(a, active, st, launches)
+                                       : launch_pair<true, false>(a, active, st, launches))
+                               : (sums ? launch_pair<false, true>(a, active, st, launches)
+                                       : launch_pair<false, false>(a, active, st, launches));
     if (e != cudaSuccess || !a.fs) return e;
     ++*launches;
     return tile::launch((const void*)iso_surface_kernel, dim3((nx_max + 127) / 128, active), 128, 0, st, a);

@@ -78,7 +78,7 @@ struct QArgs {
     CUtensorMap tm_s, tm_vx, tm_vz;       // sigma, vx, vz with the box of q_box (reference-order kernels)
     int* err_flag;                        // set to 1 by a CTA whose bounded wait ran out
     int col0;                             // first tile column of the launch (tile::launch_columns)
-    float* sg;                            // sigma = (sx + sz) + sr
+    float* sg;                            // sigma = (sx + sz) + sr; NULL: not kept (the kernels sum the parts)
     float* vx; float* vz;                 // QS vxx (= vx), vzz (= vz) for vs = 0
     float* sx; float* sz; float* sr;      // QS strxxx, strxxz, strxxr (= strzz parts for vs = 0)
     float* rx; float* rz; float* rr;      // QS rxxx, rxxz, rxxr
@@ -131,7 +131,7 @@ enum EField {
     E_VXX, E_VXZ, E_VZX, E_VZZ,
     E_SXXX, E_SXXZ, E_SXXR, E_SZZX, E_SZZZ, E_SZZR, E_SXZX, E_SXZZ, E_SXZR,
     E_RXXX, E_RXXZ, E_RXXR, E_RZZX, E_RZZZ, E_RZZR, E_RXZX, E_RXZZ, E_RXZR,
-    E_VX, E_VZ, E_SXX, E_SZZ, E_SXZ,  // the sums that the next kernel stages
+    E_VX, E_VZ, E_SXX, E_SZZ, E_SXZ,  // the sums that the next kernel stages (f[] NULL: not kept)
     E_NFIELDS
 };
 
@@ -170,7 +170,7 @@ void viscoel2d_prepare(int nx, int nz, const float* vp, const float* vs, const f
 
 // Isotropic elastic standard-staggered-grid split fields (elastic2d.cu), in slab order:
 // forward/yang_version_2016_2_2 vxx vxz vzx vzz strxxx strxxz strzzx strzzz strxzx strxzz,
-// then the sums vx vz strxx strzz strxz that the next kernel stages.
+// then the sums vx vz strxx strzz strxz that the next kernel stages (f[] NULL: not kept).
 enum IField { I_VXX, I_VXZ, I_VZX, I_VZZ, I_SXXX, I_SXXZ, I_SZZX, I_SZZZ, I_SXZX, I_SXZZ,
               I_VX, I_VZ, I_SXX, I_SZZ, I_SXZ, I_NFIELDS };
 
