@@ -201,9 +201,15 @@ __device__ __forceinline__ float4 adj_vel(float4 xo, float rd, float2 s01, float
     return cat4(v01, v23);
 }
 
-template <int R, bool VARDEN, bool ADJ>
+// Density: constant, or variable with the factors dt / (d_a den) per cell in memory, or -- where there is no
+// memory for them (one to three slabs beside the ten of a shot and its model) -- divided in the step, with the
+// same rounding
+enum Density { kConstant, kFactors, kDivide };
+
+template <int R, Density DEN, bool ADJ>
 __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __grid_constant__ Acou3DArgs a, int seg) {
     using K = K3<R>;
+    constexpr bool VARDEN = DEN != kConstant;
     extern __shared__ __align__(128) float smem[];
     const int tid = threadIdx.x;
     tile::release();
@@ -260,6 +266,11 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
         y = min(max(y, 0), ny - 1);
         z = min(max(z, 0), L.pitch - 4);
         return __ldg(at4(base + (long long)x * L.xstride, (unsigned)y * pitch_b + 4u * (unsigned)z));
+    };
+    auto ld_factor = [&](const float* b, float dtd, int x, int y, int z) -> float4 {
+        if (DEN == kFactors) return ld_model(b, x, y, z);
+        const float4 d = ld_model(a.den, x, y, z);
+        return make_float4(dtd / d.x, dtd / d.y, dtd / d.z, dtd / d.w);
     };
     const int xs = R + (int)blockIdx.z * seg, s_begin = max(1, xs - 2 * R + 1), s_end = min(xs + seg, nx - R);
     auto issue = [&](int s) {
@@ -371,7 +382,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
                     const int row = r0 + h;
                     float4 b = make_float4(byc, byc, byc, byc);
                     if (VARDEN) {
-                        b = ld_model(a.bym, s, y0 - R + row, z0 + zt);
+                        b = ld_factor(a.bym, a.dtdy, s, y0 - R + row, z0 + zt);
                     }
                     const float4 vo = ld4s(st + K::OFF_VY + row * TZ + zt);
                     const float2 s01 = h ? b01.v : a01.v, s23 = h ? b23.v : a23.v;
@@ -413,7 +424,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
                         acc[c].add(m, a.coef[m - 1], w[K::BR + R - 1 + c + m], w[K::BR + R + c - m]);
                 float4 b = make_float4(bzc, bzc, bzc, bzc);
                 if (VARDEN) {
-                    b = ld_model(a.bzm, s, y0 + row, z0 - K::RQ + 4 * u);
+                    b = ld_factor(a.bzm, a.dtdz, s, y0 + row, z0 - K::RQ + 4 * u);
                 }
                 const float4 vo = ld4s(st + K::OFF_VZ + row * K::VZW + 4 * u);
                 const float2 s01 = make_float2(acc[0].v, acc[1].v), s23 = make_float2(acc[2].v, acc[3].v);
@@ -458,7 +469,7 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
             }
             float4 b = make_float4(bxc, bxc, bxc, bxc);
             if (VARDEN) {
-                b = ld_model(a.bxm, xv, yo, zo);
+                b = ld_factor(a.bxm, a.dtdx, xv, yo, zo);
             }
             float4 vn, vout;
             if (ADJ) {
@@ -666,10 +677,10 @@ int segment_planes(const Layout3D& L, int active, int R) {
     return best;
 }
 
-template <int R, bool VARDEN, bool ADJ>
+template <int R, Density DEN, bool ADJ>
 cudaError_t launch_t(const Acou3DArgs& a, int active, cudaStream_t st) {
     const size_t smem = sizeof(float) * K3<R>::SMEM_FLOATS;
-    auto k = acoustic3d_step_kernel<R, VARDEN, ADJ>;
+    auto k = acoustic3d_step_kernel<R, DEN, ADJ>;
     static bool attr[kMaxDevices] = {};
     if (cudaError_t e = smem_attr_once((const void*)k, (int)smem, attr)) return e;
     const int seg = segment_planes(a.L, active, R), nseg = (a.L.nx - 2 * R + seg - 1) / seg;
@@ -688,16 +699,20 @@ void boxes_t(int bp[2], int bvy[2], int bvz[2]) {
 
 }  // namespace
 
+template <int R, bool ADJ>
+cudaError_t launch_d(const Acou3DArgs& a, int active, bool varden, cudaStream_t st) {
+    if (!varden) return launch_t<R, kConstant, ADJ>(a, active, st);
+    return a.bxm ? launch_t<R, kFactors, ADJ>(a, active, st) : launch_t<R, kDivide, ADJ>(a, active, st);
+}
 template <int R>
 cudaError_t launch_r(const Acou3DArgs& a, int active, bool varden, bool adj, cudaStream_t st) {
-    if (adj) return varden ? launch_t<R, true, true>(a, active, st) : launch_t<R, false, true>(a, active, st);
-    return varden ? launch_t<R, true, false>(a, active, st) : launch_t<R, false, false>(a, active, st);
+    return adj ? launch_d<R, true>(a, active, varden, st) : launch_d<R, false>(a, active, varden, st);
 }
 
 cudaError_t acoustic3d_launch_step(int radius, const Acou3DArgs& a, int active, bool varden, cudaStream_t st,
                                    bool adj) {
     if (active <= 0) return cudaSuccess;
-    if (varden && (!a.bxm || !a.bym || !a.bzm)) return cudaErrorInvalidValue;
+    if (varden && (!a.bxm != !a.bym || !a.bxm != !a.bzm || !a.den)) return cudaErrorInvalidValue;
     switch (radius) {
     case 2: return launch_r<2>(a, active, varden, adj, st);
     case 4: return launch_r<4>(a, active, varden, adj, st);

@@ -437,9 +437,11 @@ Acou3DArgs make_args3(const sfd_ctx* c, int step) {
     a.L = c->L3;
     a.vp = c->d_vp;
     a.den = c->varden ? c->d_den : nullptr;
-    a.bxm = c->d_b[c->b_of[0]];
-    a.bym = c->d_b[c->b_of[1]];
-    a.bzm = c->d_b[c->b_of[2]];
+    if (c->d_b[0]) {
+        a.bxm = c->d_b[c->b_of[0]];
+        a.bym = c->d_b[c->b_of[1]];
+        a.bzm = c->d_b[c->b_of[2]];
+    }
     a.den_c = c->den_c;
     a.dt = c->g.dt;
     a.rdx = 1.0f / c->g.dx; a.rdy = 1.0f / c->g.dy; a.rdz = 1.0f / c->g.dz;
@@ -452,10 +454,16 @@ Acou3DArgs make_args3(const sfd_ctx* c, int step) {
 }
 
 // dt / (d_a den) of the uploaded density per axis.  A context with SFD_EXACT has no use for them in its
-// forwards; its first gradient, whose steps are the default kernels, forms them.  If the memory is short any
-// other context is left without a model, so that no step runs on a half-formed one.
+// forwards; its first gradient, whose steps are the default kernels, forms them.  If the memory is short the
+// 3-D step divides by the density itself; another 2-D context is left without a model, so that no step runs
+// on a half-formed one.
+void drop_buoyancy(sfd_ctx* ctx) {
+    for (auto& p : ctx->d_b) dfree(p);
+    if (ctx->g.scheme == SFD_ACOUSTIC_3D) ctx->graph_valid = false;  // the captured steps read them
+}
 int form_buoyancy(sfd_ctx* ctx) {
     const bool is3d = ctx->g.scheme == SFD_ACOUSTIC_3D;
+    if (is3d && !ctx->d_b[0]) ctx->graph_valid = false;
     const size_t mfloats = (size_t)ctx->g.nx * ctx->g.ny * ctx->mpitch;
     const float d[3] = {ctx->g.dx, is3d ? ctx->g.dy : ctx->g.dx, ctx->g.dz};
     int n = 0;
@@ -469,7 +477,8 @@ int form_buoyancy(sfd_ctx* ctx) {
         ctx->b_of[ax] = n;
         if (!ctx->d_b[n] && cudaMalloc(&ctx->d_b[n], mfloats * sizeof(float)) != cudaSuccess) {
             cudaGetLastError();
-            for (auto& p : ctx->d_b) dfree(p);
+            drop_buoyancy(ctx);
+            if (is3d) return SFD_OK;
             if (!(ctx->g.flags & SFD_EXACT)) ctx->have_model = ctx->graph_valid = ctx->grad_valid = false;
             return set_err(ctx, SFD_ERR_NOMEM, "out of device memory for the density factors of the model");
         }
@@ -1652,7 +1661,13 @@ int alloc_state_3d(sfd_ctx* ctx, int nslab) {
     ctx->graph_valid = false;
     const Layout3D& L = ctx->L3;
     ctx->state_floats = 8 * (size_t)nslab * L.shot_stride;
-    if (cudaMalloc(&ctx->d_state, ctx->state_floats * sizeof(float)) != cudaSuccess) {
+    cudaError_t e = cudaMalloc(&ctx->d_state, ctx->state_floats * sizeof(float));
+    if (e != cudaSuccess && ctx->d_b[0]) {  // the density factors make room
+        cudaGetLastError();
+        drop_buoyancy(ctx);
+        e = cudaMalloc(&ctx->d_state, ctx->state_floats * sizeof(float));
+    }
+    if (e != cudaSuccess) {
         cudaGetLastError();
         ctx->d_state = nullptr;
         return set_err(ctx, SFD_ERR_NOMEM, "3-D wavefields of %d shots need %.1f GB of device memory", nslab,
@@ -2030,8 +2045,16 @@ int run_gradient_3d(sfd_ctx* ctx, const float* obs, float* misfit, float* grad_v
     int rc;
     auto t0 = std::chrono::steady_clock::now();
     Plan3 p;
-    if ((rc = plan3_choose(ctx, batched ? ctx->nshot : 1, &p))) return rc;
-    if ((rc = g3_alloc(ctx, p))) return rc;
+    auto plan = [&]() -> int {
+        const int r = plan3_choose(ctx, batched ? ctx->nshot : 1, &p);
+        return r ? r : g3_alloc(ctx, p);
+    };
+    rc = plan();
+    if (rc == SFD_ERR_NOMEM && ctx->d_b[0]) {  // the density factors make room
+        drop_buoyancy(ctx);
+        rc = plan();
+    }
+    if (rc) return rc;
     CK(cudaMemcpyAsync(ctx->d_obs_nt, obs, sizeof(float) * ctx->rec_total,
                        dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->stream));
     long long launches = 0;

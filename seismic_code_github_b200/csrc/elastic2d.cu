@@ -255,8 +255,8 @@ struct Vec {
     }
 };
 
-// SUMS = false: no memory for the slabs of the sums, two thirds of the state.  The tile and its halo are summed
-// by the threads: 58 ms against 35 for 275 steps of 8 shots of 1280 x 483.
+// SUMS = false: no memory for the slabs of the sums, a third of the state.  The tile and its halo are summed by
+// the threads: 58 ms against 35 for 275 steps of 8 shots of 1280 x 483.
 template <bool FS, bool SUMS>
 __global__ void __launch_bounds__(kThreads, 5) iso_velocity_kernel(const __grid_constant__ IArgs a) {
     extern __shared__ __align__(128) float smem[];

@@ -467,7 +467,7 @@ struct Acou3DArgs {
     const float* p_in; const float* vx_in;
     float* p_out; float* vx_out; float* vy_out; float* vz_out;
     const float* vp; const float* den;  // model in the field layout (one shot); den NULL = constant
-    const float* bxm; const float* bym; const float* bzm;  // variable density: dt / (d_a den)
+    const float* bxm; const float* bym; const float* bzm;  // variable density: dt / (d_a den), or NULL: not kept
     float den_c, dt;
     float rdx, rdy, rdz;                // 1/dx, 1/dy, 1/dz
     float dtdx, dtdy, dtdz;             // dt/dx, dt/dy, dt/dz
