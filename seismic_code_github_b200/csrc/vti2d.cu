@@ -154,19 +154,23 @@ __global__ void vti_inject_kernel(const __grid_constant__ VtiDev a, long long uc
     *u = __fadd_rn(*u, w);
 }
 
-// The window of every shot (get_currshot_parameters, VS:268-338, and VM:405-408) from the model
-// [nx_v][nz_v]: vz with replicated edges, epsilon and delta only inside the window and below the
-// rows nsz0 + nzu + 6.  win: per shot xmin and nsz0.
-__global__ void vti_window_kernel(const __grid_constant__ VtiDev a, const float* vz, const float* ep, const float* de,
+// The window of every shot (get_currshot_parameters, VS:268-338, and VM:405-408) from the model: vz with
+// replicated edges, epsilon and delta only inside the window and below the rows nsz0 + nzu + 6.  mdl: the three
+// arrays, marr floats apart, of shot s from mdl + s * mshot on (0: one copy for all), columns of nz_v values.
+// win: per shot xmin, nsz0 and the model column that its copy starts with.
+__global__ void vti_window_kernel(const __grid_constant__ VtiDev a, const float* mdl, long long mshot, long long marr,
                                   const int* win, int nx_v, int nz_v) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, s = blockIdx.z;
     if (i >= a.nx) return;
     float* P = a.base + (long long)s * a.shot_stride + 4 * a.field;  // vz, eps, delta
+    const float* vz = mdl + s * mshot;
+    const float *ep = vz + marr, *de = ep + marr;
+    win += 3 * s;
     const int il = min(max(i - a.nxl, 0), a.range - 1);
     for (int j = blockIdx.y; j < a.nz; j += gridDim.y) {
         const int jl = min(max(j - a.nzu, 0), nz_v - 1);
-        const long long m = (long long)min(max(il + win[2 * s], 0), nx_v - 1) * nz_v + jl;
-        const bool in = il == i - a.nxl && jl == j - a.nzu && j >= win[2 * s + 1] + a.nzu + 6;
+        const long long m = (long long)(min(max(il + win[0], 0), nx_v - 1) - win[2]) * nz_v + jl;
+        const bool in = il == i - a.nxl && jl == j - a.nzu && j >= win[1] + a.nzu + 6;
         const long long c = cell<long long>(a, i, j);
         P[c] = vz[m];
         P[a.field + c] = in ? ep[m] : 0.0f;
@@ -423,7 +427,7 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
                 !(1.0f + 2.0f * delta[m] >= 0.0f))
                 bad[i] = j + 1;
         }
-    std::vector<int> src(2 * nshot), rrow(2 * nshot), win(2 * nshot);
+    std::vector<int> src(2 * nshot), rrow(2 * nshot), win(3 * nshot), cols(nshot);
     for (int s = 0; s < nshot; s++) {
         const sfd_vti_shot& sh = shots[s];
         const long long lo = (long long)sh.xmin + 1, hi = (long long)sh.xmin + range;  // 1-based columns, then clamped
@@ -431,8 +435,10 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
         const int c1 = (int)std::min<long long>(std::max<long long>(hi, 1), c.nx_v) - 1;
         for (int i = c0; i <= c1; i++)
             if (!vz_ok[i] || bad[i] > sh.nsz0 + 6) return SFD_ERR_ARG;
-        win[2 * s] = sh.xmin;
-        win[2 * s + 1] = sh.nsz0;
+        win[3 * s] = sh.xmin;
+        win[3 * s + 1] = sh.nsz0;
+        win[3 * s + 2] = c0;
+        cols[s] = c1 - c0 + 1;
         src[2 * s] = sh.nsx - sh.xmin + nxl;  // VS:294-295
         src[2 * s + 1] = sh.nsz0 + nzu;
         if (src[2 * s] < 1 || src[2 * s] > nx || src[2 * s + 1] < 1 || src[2 * s + 1] > nz) return SFD_ERR_ARG;
@@ -461,24 +467,34 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
     const size_t total = (size_t)nshot * a.shot_stride;
     const size_t rec_n = (size_t)nshot * range * c.nt, nm = (size_t)c.nx_v * c.nz_v;
     if (state.alloc(total) != cudaSuccess || recs.alloc(rec_n) != cudaSuccess || dsrc.alloc(2 * nshot) != cudaSuccess ||
-        drow.alloc(2 * nshot) != cudaSuccess || dwin.alloc(2 * nshot) != cudaSuccess || derr.alloc(1) != cudaSuccess ||
-        model.alloc(3 * nm) != cudaSuccess) {
+        drow.alloc(2 * nshot) != cudaSuccess || dwin.alloc(3 * nshot) != cudaSuccess || derr.alloc(1) != cudaSuccess) {
         cudaGetLastError();
         return SFD_ERR_NOMEM;
     }
+    // One copy of the model for all windows; where it does not fit beside the fields, every shot's columns go to
+    // its own u and q slots, which are cleared again after the windows are built.
+    const bool shared = model.alloc(3 * nm) == cudaSuccess;
+    if (!shared) cudaGetLastError();
     long long h2d = 0;
     if (cudaMemsetAsync(state.p, 0, total * sizeof(float), st) != cudaSuccess ||
         cudaMemsetAsync(recs.p, 0, rec_n * sizeof(float), st) != cudaSuccess ||
         cudaMemsetAsync(derr.p, 0, sizeof(int), st) != cudaSuccess)
         return SFD_ERR_CUDA;
     const float* model_host[3] = {vz, epsilon, delta};
-    for (int k = 0; k < 3; k++)
-        if (cudaMemcpyAsync(model.p + k * nm, model_host[k], nm * sizeof(float), cudaMemcpyHostToDevice, st) != cudaSuccess)
-            return SFD_ERR_CUDA;
-    h2d += 3 * (long long)(nm * sizeof(float));
+    if (shared) std::fill(cols.begin(), cols.end(), c.nx_v);
+    for (int s = 0; s < (shared ? 1 : nshot); s++) {
+        const size_t n = (size_t)cols[s] * c.nz_v, first = shared ? 0 : (size_t)win[3 * s + 2] * c.nz_v;
+        for (int k = 0; k < 3; k++) {
+            float* dst = shared ? model.p + k * nm : state.p + (size_t)s * a.shot_stride + k * a.field;
+            if (cudaMemcpyAsync(dst, model_host[k] + first, n * sizeof(float), cudaMemcpyHostToDevice, st) != cudaSuccess)
+                return SFD_ERR_CUDA;
+            h2d += (long long)(n * sizeof(float));
+        }
+    }
+    for (int s = 0; shared && s < nshot; s++) win[3 * s + 2] = 0;
     if (cudaMemcpyAsync(dsrc.p, src.data(), 2 * nshot * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaMemcpyAsync(drow.p, rrow.data(), 2 * nshot * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        cudaMemcpyAsync(dwin.p, win.data(), 2 * nshot * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess)
+        cudaMemcpyAsync(dwin.p, win.data(), 3 * nshot * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess)
         return SFD_ERR_CUDA;
     a.base = state.p; a.src = dsrc.p; a.rrow = drow.p; a.records = recs.p; a.err_flag = derr.p;
     VtiOff<long long> off[2] = {};  // by the current slot
@@ -500,8 +516,11 @@ int sfd_vti_forward(const sfd_vti_par* par, const float* vz, const float* epsilo
     const bool wide = a.shot_stride > 0xffffffffLL;
     VtiOff<unsigned> narrow[2] = {narrow_offsets(off[0]), narrow_offsets(off[1])};  // unused if wide
     vti_window_kernel<<<dim3((nx + 127) / 128, std::min(nz, kGridY), nshot), 128, 0, st>>>(
-        a, model.p, model.p + nm, model.p + 2 * nm, dwin.p, c.nx_v, c.nz_v);
+        a, shared ? model.p : state.p, shared ? 0 : a.shot_stride, shared ? (long long)nm : a.field, dwin.p, c.nx_v, c.nz_v);
     if (cudaGetLastError() != cudaSuccess) return SFD_ERR_CUDA;
+    for (int s = 0; !shared && s < nshot; s++)
+        if (cudaMemsetAsync(state.p + (size_t)s * a.shot_stride, 0, 4 * a.field * sizeof(float), st) != cudaSuccess)
+            return SFD_ERR_CUDA;
 
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
