@@ -11,13 +11,24 @@ pytestmark = pytest.mark.gpu
 
 
 class Hog:
-    """Holds the device's free memory but for `leave` bytes."""
+    """Holds the device's memory but for one block of `leave` bytes.  What the driver reports as free is not
+    all that it can give (it keeps blocks of memory freed before), so the rest is taken until nothing is
+    left, and the block that was set aside first is given back."""
 
     def __init__(self, leave):
         import torch
         torch.cuda.synchronize()
         torch.cuda.empty_cache()
-        self.t = torch.empty(max(0, torch.cuda.mem_get_info()[0] - leave), dtype=torch.uint8, device="cuda")
+        aside = torch.empty(leave, dtype=torch.uint8, device="cuda")
+        self.t = []
+        size = torch.cuda.mem_get_info()[0]
+        while size >= 2 << 20:
+            try:
+                self.t.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+            except torch.cuda.OutOfMemoryError:
+                size //= 2
+        del aside
+        torch.cuda.empty_cache()
 
     def release(self):
         import torch
