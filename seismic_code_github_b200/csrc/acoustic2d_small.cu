@@ -5,8 +5,8 @@
 // Bound: latency.  One shot of 351 x 351 is 36 tiles of 64 x 64 on 148 SMs, each a serial chain of
 // loads and three phases over 16 points per thread; here it is 242 tiles of one vector of four points
 // per thread.  The price is the halo (P is read 2.5 times, Vx twice, Vz 1.5 times, from L2) and the
-// velocities recomputed on it, which costs less than the idle SMs until the launch has several waves
-// (acoustic2d_use_small).
+// velocities recomputed on it, which costs less than the idle SMs up to one wave of these CTAs and at
+// low orders somewhat beyond (acoustic2d_use_small).
 //
 // A CTA of 128 threads: P on a cross (the tile with 2R columns on each side, and with 2 round4(R) rows
 // above and below), Vx with R columns and Vz with round4(R) rows on each side, copied to shared memory
@@ -17,8 +17,7 @@
 // The same tiles run SFD_EXACT at every size (kExact): each multiply and add rounded by itself in the
 // reference's order, the scale factors and the divergence in double.  8 shots of 851 x 451 with variable
 // density, order 16: 122 us a step on 64 x 64 tiles with one stencil point per shared-memory load, 60 us
-// now (51 Gpts/s; bound by issue: two thirds of the instructions are arithmetic of the prescribed order
-// and its conversions to and from double).
+// now (51 Gpts/s; latency: 18 warps an SM at 96 registers, issue 55%, L1 data pipe 58%, FP64 pipe 9%).
 #include <cuda.h>
 #include <cuda_runtime.h>
 

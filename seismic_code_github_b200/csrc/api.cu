@@ -227,11 +227,9 @@ cudaError_t h2d(const sfd_ctx* ctx, void* dst, const void* src, size_t bytes) {
 
 int round_up(int v, int m) { return (v + m - 1) / m * m; }
 
-// The viscoacoustic scheme runs the fused kernel (viscoac2d_fast.cu) unless SFD_EXACT is set.
-// Its slabs: vx, vz, sigma, r, and the six split parts of the sponge bands, all in place.
+// The default viscoacoustic mode (viscoac2d_fast.cu) keeps vx, vz, sigma, r and the six split parts of the
+// sponge bands, all in place; SFD_EXACT runs the reference-order kernels (viscoac2d.cu) on the split fields.
 constexpr int kQVX = 0, kQVZ = 1, kQS = 2, kQR = 3, kQSplit = 4, kQFastSlabs = 10;
-// The default viscoacoustic mode: the merged fields and the split parts of the sponge bands
-// (viscoac2d_fast.cu); SFD_EXACT runs the reference-order kernels (viscoac2d.cu) on the split fields.
 bool q_fast(const sfd_ctx* c) { return c->g.scheme == SFD_VISCOAC_2D && !(c->g.flags & SFD_EXACT); }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda).

@@ -26,7 +26,8 @@
 // its own cells (with its receivers' residuals in sx^, sz^, sr^ before T1 and T4 are formed), so neither
 // launch races with itself.
 //
-// Bound: memory (132 B a cell).  Each kernel's two differentiated fields arrive by TMA on tiles of 64 rows
+// Bound: issue and shared-memory loads in the velocity kernel (72% and 67%, DRAM 1.8 TB/s), memory and issue in
+// the stress kernel (4.1 TB/s, 61%); 132 B a cell.  Each kernel's two differentiated fields arrive by TMA on tiles of 64 rows
 // by 8 columns with two cells per thread, as in viscoac2d.cu (measurements there); before, kernel A staged
 // six arrays with their halo to form T1 and T4 again.
 #include <cuda_runtime.h>

@@ -399,17 +399,17 @@ bool acoustic2d_march_fills(const Layout2D& L, int active, int seg_cols);
 inline bool acoustic2d_use_march(const Acou2DPlan& plan, const Layout2D& L, int active) {
     return plan.seg > 0 && (plan.forced || acoustic2d_march_fills(L, active, plan.seg));
 }
-// Forward step of the default (FMA) scheme with the plan's kernel: x-marching when plan.seg > 0
-// and the launch fills the device, else the tile kernel with plan.stages.
 // The small-tile kernel (acoustic2d_small.cu): the tile kernel's values bit for bit, for launches with
 // few tiles; adj as in acoustic2d_fma_launch.
 cudaError_t acoustic2d_small_launch(int radius, const Acou2DArgs& a, int active, bool varden, cudaStream_t st, bool adj);
 bool acoustic2d_one_small_wave(const Layout2D& L, int active);  // the small tiles run untimed
 bool acoustic2d_use_small(const Acou2DPlan& plan, const Layout2D& L, int active);
-// SFD_EXACT: the reference's operation order
 // out[i] = c / den[i] (rounded to nearest)
 cudaError_t launch_buoyancy(const float* den, float c, float* out, long long n, cudaStream_t st);
+// SFD_EXACT: the reference's operation order
 cudaError_t acoustic2d_exact_launch(int radius, const Acou2DArgs& a, int active, bool varden, cudaStream_t st);
+// Forward step of the default (FMA) scheme with the plan's kernel: the small tiles (acoustic2d_use_small),
+// x-marching when plan.seg > 0 and the launch fills the device, else the tile kernel with plan.stages.
 cudaError_t acoustic2d_fwd_launch(const Acou2DPlan& plan, int radius, const Acou2DArgs& a, int active, bool varden,
                                   cudaStream_t st);
 // Programmatic dependent launch of consecutive step kernels (SFD_PDL=0 turns it off).

@@ -19,7 +19,7 @@
 // values in registers and adds each tap with one FMA into the outputs that use it.
 //
 // Bound: memory (40 B a cell and step of state, 88 B in the bands; the model stays in L2).  16 shots of
-// 1124 x 1124 (20.2 M cells): 76 us velocity at 4.9 TB/s, about 150 us stress.  A kernel that marched down x
+// 1124 x 1124 (20.2 M cells): 76 us velocity at 4.9 TB/s, 165 us stress at 4.2.  A kernel that marched down x
 // with both phases in one CTA (32 B a cell, but 280 B of shared loads a cell, the velocities of the z halo
 // computed twice, and a second kernel for the bands) took 258 + 63 us: few warps in flight behind its
 // barriers, and the shared-memory pipe at 86%.  Stress with four columns per thread: 2% slower (10 warps an

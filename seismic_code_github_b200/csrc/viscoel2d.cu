@@ -26,7 +26,8 @@
 // Every multiply and add is rounded separately in the reference's order, so the kernels agree
 // bit for bit with the FP32 restatement in oracle/q_oracle.cpp.
 //
-// Bound: memory.  The split fields (22 read and written) and seven model arrays are 204 B a cell; the
+// Bound: memory in the stress kernel (DRAM at 4.9 TB/s), issue and shared-memory loads in the velocity kernel
+// (72% and 66%, DRAM at 3.0 TB/s).  The split fields (22 read and written) and seven model arrays are 204 B a cell; the
 // two kernels move 244 B (sums written once and read once, halos from L2).  One TMA box per sum field
 // stages a tile with its halo while every thread loads the split parts of its one cell, so that all
 // loads of a CTA are in flight together; small CTAs cover one another's waits.
@@ -44,7 +45,7 @@ namespace {
 constexpr int TX = kTileX, TZ = kTileZ;
 // Tiles of 64 rows by 4 columns, one thread per cell, eight (velocity) and five (stress) CTAs per SM.
 // Step of 8 shots of 780 x 580 (3.6 M cells): 64 x 64 tiles with 16 cells per thread in turn 225 us
-// (before); 8 columns 195 us; 4 columns 168 us (DRAM at 5.2 TB/s); 2 columns 165 us on this grid, with a
+// (before); 8 columns 195 us; 4 columns 168 us; 2 columns 165 us on this grid, with a
 // sixfold halo.
 constexpr int TC = 4, kThreads = TC * TZ;
 constexpr int kMinV = 8, kMinS = 5;

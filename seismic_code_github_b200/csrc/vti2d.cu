@@ -14,7 +14,8 @@
 // relative L2 distance from a 64-bit run is 2.2 to 4.1e-6 for grids of 220 to 490 columns and 350 to 630 steps,
 // with or without a top PML; the reference order's is 2.3 to 3.2e-6 without and 4.9 to 9.6e-6 with one.
 //
-// Bound: memory (36 B a cell inside, 44 to 76 B more in the PML strips) and its latency.  A CTA owns
+// Bound: issue (77%; DRAM at 3.5 TB/s): the stencil's arithmetic on 36 B a cell inside and 44 to 76 B more in
+// the PML strips.  A CTA owns
 // 64 x 2 cells, one per thread; u with a halo of 5 rows and 8 columns and q with a halo of 8 columns
 // (q is only differentiated along x) arrive by two TMA boxes while each thread loads its cell's model
 // and old u, q.  Addresses are 32-bit offsets from the shot's slab, formed on the host: with pointer

@@ -243,7 +243,7 @@ def vti_forward(vz: np.ndarray, epsilon: np.ndarray, delta: np.ndarray, dx: floa
     x-major; bounds = (nx_bound_l, nx_bound_r, nz_bound_u, nz_bound_d) PML cells; shots a list of
     (nsx, nsz0, nrz0, xmin, xmax) in the reference's 1-based grid numbers, all with the same
     xmax - xmin.  exact: the reference's operation order, bit-exact with the restatement
-    (SFD_EXACT); otherwise FMA contraction and approximate divisions (relative L2 <= 1e-5).
+    (SFD_EXACT); otherwise FMA contraction and PML factors as reciprocals (relative L2 <= 1e-5).
     Returns (records [nshot][xmax - xmin + 1][nt], timing dict)."""
     arrs = [np.ascontiguousarray(a, np.float32) for a in (vz, epsilon, delta)]
     nx_v, nz_v = arrs[0].shape
