@@ -320,80 +320,122 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
     float4 *cur = sVq, *prv = sVq + R * kThreads;
     for (int s0 = s_begin; s0 < s_end; s0 += R) {
 #pragma unroll
-    for (int q = 0; q < R; q++) {
-        const int s = s0 + q;
-        if (s >= s_end) return;
-        static_assert(R % 2 == 0, "a plane's stage is the parity of q");
-        const int stg = q & 1;
-        bool got = true;
-        if (s >= xs) {
-            got = bounded_wait(bars + stg, (phase >> stg) & 1u);
-            phase ^= 1u << stg;
-        }
-        const float* st = smem + stg * K::STAGE;
-        float* nby = smem + K::OFF_NB + stg * K::NBUF;  // new Vy region of this plane
-        float* nbz = nby + K::NB_NZ;                     // new Vz region of this plane
-        // adjoint: D_k and the imaging sum of the own points of plane s, requested before the
-        // velocity phases so that their latency is covered
-        float4 adk = make_float4(0.f, 0.f, 0.f, 0.f), agk = adk;
-        if (ADJ && s >= xs && own_ok) {
-            const long long plane = shot_off + (long long)s * L.xstride;
-            adk = *at4(a.adj_div + plane, own_off);
-            agk = *at4(a.adj_g + plane, own_off);
-        }
-        // the loads of the next plane's own values are issued as soon as this plane's are used
-        const int xv = s + R - 1;  // plane of this iteration's new Vx
-        const bool edge = !yz_int || !(s >= E && xv < nx - E);
-        bool xpad_s, xpad_v;
-        const float fx_s = axis_taper(a, s, nx, &xpad_s);
-        const float fx_v = axis_taper(a, xv, nx, &xpad_v);
-        const float kx_s = (s >= R && s < nx - R) ? 1.0f : 0.0f, kx_v = (xv >= R && xv < nx - R) ? 1.0f : 0.0f;
-        // damping factors and masks of four points of the region at table index i, plane s
-        auto edge_f = [&](int i, bool xpad, float fx) {
-            return xpad ? make_float4(fx, fx, fx, fx) : ld4s(sFA + i);
-        };
-        auto edge_k = [&](int i, float kx) {
-            const float4 k = ld4s(sFK + i);
-            return make_float4(k.x * kx, k.y * kx, k.z * kx, k.w * kx);
-        };
+        for (int q = 0; q < R; q++) {
+            const int s = s0 + q;
+            if (s >= s_end) return;
+            static_assert(R % 2 == 0, "a plane's stage is the parity of q");
+            const int stg = q & 1;
+            bool got = true;
+            if (s >= xs) {
+                got = bounded_wait(bars + stg, (phase >> stg) & 1u);
+                phase ^= 1u << stg;
+            }
+            const float* st = smem + stg * K::STAGE;
+            float* nby = smem + K::OFF_NB + stg * K::NBUF;  // new Vy region of this plane
+            float* nbz = nby + K::NB_NZ;                     // new Vz region of this plane
+            // adjoint: D_k and the imaging sum of the own points of plane s, requested before the
+            // velocity phases so that their latency is covered
+            float4 adk = make_float4(0.f, 0.f, 0.f, 0.f), agk = adk;
+            if (ADJ && s >= xs && own_ok) {
+                const long long plane = shot_off + (long long)s * L.xstride;
+                adk = *at4(a.adj_div + plane, own_off);
+                agk = *at4(a.adj_g + plane, own_off);
+            }
+            // the loads of the next plane's own values are issued as soon as this plane's are used
+            const int xv = s + R - 1;  // plane of this iteration's new Vx
+            const bool edge = !yz_int || !(s >= E && xv < nx - E);
+            bool xpad_s, xpad_v;
+            const float fx_s = axis_taper(a, s, nx, &xpad_s);
+            const float fx_v = axis_taper(a, xv, nx, &xpad_v);
+            const float kx_s = (s >= R && s < nx - R) ? 1.0f : 0.0f, kx_v = (xv >= R && xv < nx - R) ? 1.0f : 0.0f;
+            // damping factors and masks of four points of the region at table index i, plane s
+            auto edge_f = [&](int i, bool xpad, float fx) {
+                return xpad ? make_float4(fx, fx, fx, fx) : ld4s(sFA + i);
+            };
+            auto edge_k = [&](int i, float kx) {
+                const float4 k = ld4s(sFK + i);
+                return make_float4(k.x * kx, k.y * kx, k.z * kx, k.w * kx);
+            };
 
-        if (s >= xs) {
-            const long long plane_off = shot_off + (long long)s * L.xstride;
-            // ---- new Vy on the Vy region: rows y0-R .. y0+TY+R-1, two rows x float4 per task ----
-            if (tid < K::NVY2) {
-                const int r0 = (tid >> 3) * 2, zt = (tid & 7) * 4;
-                // P rows r0+R+1-m (lo, row r0) ... r0+R+1+m (hi, row r0+1), center row shared
-                const float* pc = st + K::HZ + zt;
-                Acc2 a01, a23, b01, b23;  // rows r0 and r0+1
-                float4 hi_a = ld4s(pc + (r0 + R + 1) * K::PZ), lo_b = hi_a;
+            if (s >= xs) {
+                const long long plane_off = shot_off + (long long)s * L.xstride;
+                // ---- new Vy on the Vy region: rows y0-R .. y0+TY+R-1, two rows x float4 per task ----
+                if (tid < K::NVY2) {
+                    const int r0 = (tid >> 3) * 2, zt = (tid & 7) * 4;
+                    // P rows r0+R+1-m (lo, row r0) ... r0+R+1+m (hi, row r0+1), center row shared
+                    const float* pc = st + K::HZ + zt;
+                    Acc2 a01, a23, b01, b23;  // rows r0 and r0+1
+                    float4 hi_a = ld4s(pc + (r0 + R + 1) * K::PZ), lo_b = hi_a;
 #pragma unroll
-                for (int m = 1; m <= R; m++) {
-                    const float4 lo_a = ld4s(pc + (r0 + R + 1 - m) * K::PZ);
-                    const float4 hi_b = ld4s(pc + (r0 + R + 1 + m) * K::PZ);
-                    a01.add(m, cc[m - 1], lo2(hi_a), lo2(lo_a));
-                    a23.add(m, cc[m - 1], hi2(hi_a), hi2(lo_a));
-                    b01.add(m, cc[m - 1], lo2(hi_b), lo2(lo_b));
-                    b23.add(m, cc[m - 1], hi2(hi_b), hi2(lo_b));
-                    hi_a = hi_b;
-                    lo_b = lo_a;
-                }
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int row = r0 + h;
-                    float4 b = make_float4(byc, byc, byc, byc);
-                    if (VARDEN) {
-                        b = ld_factor(a.bym, a.dtdy, s, y0 - R + row, z0 + zt);
+                    for (int m = 1; m <= R; m++) {
+                        const float4 lo_a = ld4s(pc + (r0 + R + 1 - m) * K::PZ);
+                        const float4 hi_b = ld4s(pc + (r0 + R + 1 + m) * K::PZ);
+                        a01.add(m, cc[m - 1], lo2(hi_a), lo2(lo_a));
+                        a23.add(m, cc[m - 1], hi2(hi_a), hi2(lo_a));
+                        b01.add(m, cc[m - 1], lo2(hi_b), lo2(lo_b));
+                        b23.add(m, cc[m - 1], hi2(hi_b), hi2(lo_b));
+                        hi_a = hi_b;
+                        lo_b = lo_a;
                     }
-                    const float4 vo = ld4s(st + K::OFF_VY + row * TZ + zt);
-                    const float2 s01 = h ? b01.v : a01.v, s23 = h ? b23.v : a23.v;
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const int row = r0 + h;
+                        float4 b = make_float4(byc, byc, byc, byc);
+                        if (VARDEN) {
+                            b = ld_factor(a.bym, a.dtdy, s, y0 - R + row, z0 + zt);
+                        }
+                        const float4 vo = ld4s(st + K::OFF_VY + row * TZ + zt);
+                        const float2 s01 = h ? b01.v : a01.v, s23 = h ? b23.v : a23.v;
+                        float4 vn, vout;
+                        const int i = row * K::VZW + K::RQ + zt;
+                        if (ADJ) {
+                            if (edge)
+                                vn = adj_vel<true, VARDEN>(vo, a.rdy, s01, s23, edge_f(i, xpad_s, fx_s), edge_k(i, kx_s), b,
+                                                           &vout);
+                            else
+                                vn = adj_vel<false, VARDEN>(vo, a.rdy, s01, s23, vo, vo, b, &vout);
+                        } else {
+                            if (edge)
+                                vn = vel_update<true>(vo, b, s01, s23, edge_f(i, xpad_s, fx_s), edge_k(i, kx_s));
+                            else
+                                vn = vel_update<false>(vo, b, s01, s23, vo, vo);
+                            vout = vn;
+                        }
+                        st4s(nby + row * TZ + zt, vn);
+                        const int y = y0 - R + row;
+                        if (row >= R && row < R + TY && y < ny && z0 + zt < L.pitch)
+                            *at4(a.vy_out + plane_off, (unsigned)y * pitch_b + 4u * (unsigned)(z0 + zt)) = vout;
+                    }
+                }
+                // ---- new Vz on the Vz region: rows y0 .. y0+TY-1, z0-RQ .. z0+TZ+RQ-1 ----
+                auto vz_task = [&](int t) {
+                    const int row = t / (K::VZW / 4), u = t % (K::VZW / 4);
+                    float w[4 * K::NFZ];
+#pragma unroll
+                    for (int f = 0; f < K::NFZ; f++) {
+                        const float4 v = ld4s(st + (row + K::HY) * K::PZ + 4 * u + K::B4 + 4 * f);
+                        w[4 * f] = v.x; w[4 * f + 1] = v.y; w[4 * f + 2] = v.z; w[4 * f + 3] = v.w;
+                    }
+                    Acc acc[4];
+#pragma unroll
+                    for (int c = 0; c < 4; c++)
+#pragma unroll
+                        for (int m = 1; m <= R; m++)
+                            acc[c].add(m, a.coef[m - 1], w[K::BR + R - 1 + c + m], w[K::BR + R + c - m]);
+                    float4 b = make_float4(bzc, bzc, bzc, bzc);
+                    if (VARDEN) {
+                        b = ld_factor(a.bzm, a.dtdz, s, y0 + row, z0 - K::RQ + 4 * u);
+                    }
+                    const float4 vo = ld4s(st + K::OFF_VZ + row * K::VZW + 4 * u);
+                    const float2 s01 = make_float2(acc[0].v, acc[1].v), s23 = make_float2(acc[2].v, acc[3].v);
                     float4 vn, vout;
-                    const int i = row * K::VZW + K::RQ + zt;
+                    const int i = (row + R) * K::VZW + 4 * u;
                     if (ADJ) {
                         if (edge)
-                            vn = adj_vel<true, VARDEN>(vo, a.rdy, s01, s23, edge_f(i, xpad_s, fx_s), edge_k(i, kx_s), b,
+                            vn = adj_vel<true, VARDEN>(vo, a.rdz, s01, s23, edge_f(i, xpad_s, fx_s), edge_k(i, kx_s), b,
                                                        &vout);
                         else
-                            vn = adj_vel<false, VARDEN>(vo, a.rdy, s01, s23, vo, vo, b, &vout);
+                            vn = adj_vel<false, VARDEN>(vo, a.rdz, s01, s23, vo, vo, b, &vout);
                     } else {
                         if (edge)
                             vn = vel_update<true>(vo, b, s01, s23, edge_f(i, xpad_s, fx_s), edge_k(i, kx_s));
@@ -401,187 +443,145 @@ __global__ void __launch_bounds__(kThreads, 2) acoustic3d_step_kernel(const __gr
                             vn = vel_update<false>(vo, b, s01, s23, vo, vo);
                         vout = vn;
                     }
-                    st4s(nby + row * TZ + zt, vn);
-                    const int y = y0 - R + row;
-                    if (row >= R && row < R + TY && y < ny && z0 + zt < L.pitch)
-                        *at4(a.vy_out + plane_off, (unsigned)y * pitch_b + 4u * (unsigned)(z0 + zt)) = vout;
+                    st4s(nbz + row * K::VZW + 4 * u, vn);
+                    const int y = y0 + row, z = z0 - K::RQ + 4 * u;
+                    if (4 * u >= K::RQ && 4 * u < K::RQ + TZ && y < ny && z < L.pitch)
+                        *at4(a.vz_out + plane_off, (unsigned)y * pitch_b + 4u * (unsigned)z) = vout;
+                };
+                if (tid >= K::NVY2) {
+#pragma unroll
+                    for (int k = 0; k < 3; k++) {
+                        const int j = (tid - K::NVY2) + k * K::HVZ;
+                        if (j < K::NVZ) vz_task(j);
+                    }
+                } else if (K::RVZ > 0 && tid >= K::NVY2 - K::RVZ) {
+                    vz_task(3 * K::HVZ + tid - (K::NVY2 - K::RVZ));
                 }
             }
-            // ---- new Vz on the Vz region: rows y0 .. y0+TY-1, z0-RQ .. z0+TZ+RQ-1 ----
-            auto vz_task = [&](int t) {
-                const int row = t / (K::VZW / 4), u = t % (K::VZW / 4);
-                float w[4 * K::NFZ];
+            const int io = (yl + R) * K::VZW + K::RQ + zr;  // table index of the own points
+            // ---- new Vx on plane xv (own points, P from the register queue) ----
+            {
+                Acc2 s01, s23;
 #pragma unroll
-                for (int f = 0; f < K::NFZ; f++) {
-                    const float4 v = ld4s(st + (row + K::HY) * K::PZ + 4 * u + K::B4 + 4 * f);
-                    w[4 * f] = v.x; w[4 * f + 1] = v.y; w[4 * f + 2] = v.z; w[4 * f + 3] = v.w;
+                for (int m = 1; m <= R; m++) {
+                    s01.add(m, cc[m - 1], lo2(Pq[q + R - 1 + m]), lo2(Pq[q + R - m]));
+                    s23.add(m, cc[m - 1], hi2(Pq[q + R - 1 + m]), hi2(Pq[q + R - m]));
                 }
-                Acc acc[4];
+                float4 b = make_float4(bxc, bxc, bxc, bxc);
+                if (VARDEN) {
+                    b = ld_factor(a.bxm, a.dtdx, xv, yo, zo);
+                }
+                float4 vn, vout;
+                if (ADJ) {
+                    vn = edge ? adj_vel<true, VARDEN>(Vxo, a.rdx, s01.v, s23.v, edge_f(io, xpad_v, fx_v), edge_k(io, kx_v),
+                                                      b, &vout)
+                              : adj_vel<false, VARDEN>(Vxo, a.rdx, s01.v, s23.v, Vxo, Vxo, b, &vout);
+                } else {
+                    vn = edge ? vel_update<true>(Vxo, b, s01.v, s23.v, edge_f(io, xpad_v, fx_v), edge_k(io, kx_v))
+                              : vel_update<false>(Vxo, b, s01.v, s23.v, Vxo, Vxo);
+                    vout = vn;
+                }
+                Vxo = ld_own(vx_in, s + R);
+                if (own_ok && xv >= xs && xv < s_end) *at4(a.vx_out + shot_off + (long long)xv * L.xstride, own_off) = vout;
+                cur[q * kThreads] = vn;
+            }
+            // every thread is done with this stage and with the new-velocity buffer of plane s-1
+            if (s >= xs && __syncthreads_or(!got)) {
+                if (tid == 0) {
+                    atomicExch(a.err_flag, 1);
+                    // let the copies still in flight land before the CTA's shared memory is released
+                    bounded_wait(bars + stg, ((phase >> stg) & 1u) ^ 1u);
+                    if (s + 1 < s_end) bounded_wait(bars + (stg ^ 1), (phase >> (stg ^ 1)) & 1u);
+                }
+                return;
+            }
+            if (tid == 0 && s >= xs && s + 2 < s_end) issue(s + 2);
+            if (s >= xs) {
+                // ---- new P on plane s (own points) ----
+                float wz[4 * K::NFD];
+#pragma unroll
+                for (int f = 0; f < K::NFD; f++) {
+                    const float4 v = ld4s(nbz + yl * K::VZW + zr + K::D4 + 4 * f);
+                    wz[4 * f] = v.x; wz[4 * f + 1] = v.y; wz[4 * f + 2] = v.z; wz[4 * f + 3] = v.w;
+                }
+                Acc2 ax01, ax23, ay01, ay23;
+#pragma unroll
+                for (int m = 1; m <= R; m++) {
+                    const int hi = q + m - R, lo = q - m - R + 1;  // positions from cur[0]
+                    const float4 xhi = hi >= 0 ? cur[hi * kThreads] : prv[(hi + R) * kThreads];
+                    const float4 xlo = lo >= -R ? prv[(lo + R) * kThreads] : cur[(lo + 2 * R) * kThreads];
+                    ax01.add(m, cc[m - 1], lo2(xhi), lo2(xlo));
+                    ax23.add(m, cc[m - 1], hi2(xhi), hi2(xlo));
+                    const float4 yhi = ld4s(nby + (yl + R + m - 1) * TZ + zr);
+                    const float4 ylo = ld4s(nby + (yl + R - m) * TZ + zr);
+                    ay01.add(m, cc[m - 1], lo2(yhi), lo2(ylo));
+                    ay23.add(m, cc[m - 1], hi2(yhi), hi2(ylo));
+                }
+                Acc az[4];
 #pragma unroll
                 for (int c = 0; c < 4; c++)
 #pragma unroll
                     for (int m = 1; m <= R; m++)
-                        acc[c].add(m, a.coef[m - 1], w[K::BR + R - 1 + c + m], w[K::BR + R + c - m]);
-                float4 b = make_float4(bzc, bzc, bzc, bzc);
+                        az[c].add(m, a.coef[m - 1], wz[K::DR + R + c + m - 1], wz[K::DR + R + c - m]);
+                // div = ((Sx / dx) + Sy / dy) + Sz / dz, then P = P - (den dt vp vp) div; the adjoint
+                // weighs the sums by B (constant density) instead
+                const float2 rdx = bc2(ADJ ? a.adj_c[0] : a.rdx), rdy = bc2(ADJ ? a.adj_c[1] : a.rdy),
+                             rdz = bc2(ADJ ? a.adj_c[2] : a.rdz);
+                float2 d01 = __fmul2_rn(ax01.v, rdx), d23 = __fmul2_rn(ax23.v, rdx);
+                d01 = __ffma2_rn(ay01.v, rdy, d01);
+                d23 = __ffma2_rn(ay23.v, rdy, d23);
+                d01 = __ffma2_rn(make_float2(az[0].v, az[1].v), rdz, d01);
+                d23 = __ffma2_rn(make_float2(az[2].v, az[3].v), rdz, d23);
+                float4 kk;
                 if (VARDEN) {
-                    b = ld_factor(a.bzm, a.dtdz, s, y0 + row, z0 - K::RQ + 4 * u);
-                }
-                const float4 vo = ld4s(st + K::OFF_VZ + row * K::VZW + 4 * u);
-                const float2 s01 = make_float2(acc[0].v, acc[1].v), s23 = make_float2(acc[2].v, acc[3].v);
-                float4 vn, vout;
-                const int i = (row + R) * K::VZW + 4 * u;
-                if (ADJ) {
-                    if (edge)
-                        vn = adj_vel<true, VARDEN>(vo, a.rdz, s01, s23, edge_f(i, xpad_s, fx_s), edge_k(i, kx_s), b,
-                                                   &vout);
-                    else
-                        vn = adj_vel<false, VARDEN>(vo, a.rdz, s01, s23, vo, vo, b, &vout);
+                    const float4 d = ld_model(a.den, s, yo, zo);
+                    kk = make_float4(d.x * a.dt, d.y * a.dt, d.z * a.dt, d.w * a.dt);
                 } else {
-                    if (edge)
-                        vn = vel_update<true>(vo, b, s01, s23, edge_f(i, xpad_s, fx_s), edge_k(i, kx_s));
-                    else
-                        vn = vel_update<false>(vo, b, s01, s23, vo, vo);
-                    vout = vn;
+                    kk = make_float4(kc, kc, kc, kc);
                 }
-                st4s(nbz + row * K::VZW + 4 * u, vn);
-                const int y = y0 + row, z = z0 - K::RQ + 4 * u;
-                if (4 * u >= K::RQ && 4 * u < K::RQ + TZ && y < ny && z < L.pitch)
-                    *at4(a.vz_out + plane_off, (unsigned)y * pitch_b + 4u * (unsigned)z) = vout;
-            };
-            if (tid >= K::NVY2) {
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    const int j = (tid - K::NVY2) + k * K::HVZ;
-                    if (j < K::NVZ) vz_task(j);
-                }
-            } else if (K::RVZ > 0 && tid >= K::NVY2 - K::RVZ) {
-                vz_task(3 * K::HVZ + tid - (K::NVY2 - K::RVZ));
-            }
-        }
-        const int io = (yl + R) * K::VZW + K::RQ + zr;  // table index of the own points
-        // ---- new Vx on plane xv (own points, P from the register queue) ----
-        {
-            Acc2 s01, s23;
-#pragma unroll
-            for (int m = 1; m <= R; m++) {
-                s01.add(m, cc[m - 1], lo2(Pq[q + R - 1 + m]), lo2(Pq[q + R - m]));
-                s23.add(m, cc[m - 1], hi2(Pq[q + R - 1 + m]), hi2(Pq[q + R - m]));
-            }
-            float4 b = make_float4(bxc, bxc, bxc, bxc);
-            if (VARDEN) {
-                b = ld_factor(a.bxm, a.dtdx, xv, yo, zo);
-            }
-            float4 vn, vout;
-            if (ADJ) {
-                vn = edge ? adj_vel<true, VARDEN>(Vxo, a.rdx, s01.v, s23.v, edge_f(io, xpad_v, fx_v), edge_k(io, kx_v),
-                                                  b, &vout)
-                          : adj_vel<false, VARDEN>(Vxo, a.rdx, s01.v, s23.v, Vxo, Vxo, b, &vout);
-            } else {
-                vn = edge ? vel_update<true>(Vxo, b, s01.v, s23.v, edge_f(io, xpad_v, fx_v), edge_k(io, kx_v))
-                          : vel_update<false>(Vxo, b, s01.v, s23.v, Vxo, Vxo);
-                vout = vn;
-            }
-            Vxo = ld_own(vx_in, s + R);
-            if (own_ok && xv >= xs && xv < s_end) *at4(a.vx_out + shot_off + (long long)xv * L.xstride, own_off) = vout;
-            cur[q * kThreads] = vn;
-        }
-        // every thread is done with this stage and with the new-velocity buffer of plane s-1
-        if (s >= xs && __syncthreads_or(!got)) {
-            if (tid == 0) {
-                atomicExch(a.err_flag, 1);
-                // let the copies still in flight land before the CTA's shared memory is released
-                bounded_wait(bars + stg, ((phase >> stg) & 1u) ^ 1u);
-                if (s + 1 < s_end) bounded_wait(bars + (stg ^ 1), (phase >> (stg ^ 1)) & 1u);
-            }
-            return;
-        }
-        if (tid == 0 && s >= xs && s + 2 < s_end) issue(s + 2);
-        if (s >= xs) {
-            // ---- new P on plane s (own points) ----
-            float wz[4 * K::NFD];
-#pragma unroll
-            for (int f = 0; f < K::NFD; f++) {
-                const float4 v = ld4s(nbz + yl * K::VZW + zr + K::D4 + 4 * f);
-                wz[4 * f] = v.x; wz[4 * f + 1] = v.y; wz[4 * f + 2] = v.z; wz[4 * f + 3] = v.w;
-            }
-            Acc2 ax01, ax23, ay01, ay23;
-#pragma unroll
-            for (int m = 1; m <= R; m++) {
-                const int hi = q + m - R, lo = q - m - R + 1;  // positions from cur[0]
-                const float4 xhi = hi >= 0 ? cur[hi * kThreads] : prv[(hi + R) * kThreads];
-                const float4 xlo = lo >= -R ? prv[(lo + R) * kThreads] : cur[(lo + 2 * R) * kThreads];
-                ax01.add(m, cc[m - 1], lo2(xhi), lo2(xlo));
-                ax23.add(m, cc[m - 1], hi2(xhi), hi2(xlo));
-                const float4 yhi = ld4s(nby + (yl + R + m - 1) * TZ + zr);
-                const float4 ylo = ld4s(nby + (yl + R - m) * TZ + zr);
-                ay01.add(m, cc[m - 1], lo2(yhi), lo2(ylo));
-                ay23.add(m, cc[m - 1], hi2(yhi), hi2(ylo));
-            }
-            Acc az[4];
-#pragma unroll
-            for (int c = 0; c < 4; c++)
-#pragma unroll
-                for (int m = 1; m <= R; m++)
-                    az[c].add(m, a.coef[m - 1], wz[K::DR + R + c + m - 1], wz[K::DR + R + c - m]);
-            // div = ((Sx / dx) + Sy / dy) + Sz / dz, then P = P - (den dt vp vp) div; the adjoint
-            // weighs the sums by B (constant density) instead
-            const float2 rdx = bc2(ADJ ? a.adj_c[0] : a.rdx), rdy = bc2(ADJ ? a.adj_c[1] : a.rdy),
-                         rdz = bc2(ADJ ? a.adj_c[2] : a.rdz);
-            float2 d01 = __fmul2_rn(ax01.v, rdx), d23 = __fmul2_rn(ax23.v, rdx);
-            d01 = __ffma2_rn(ay01.v, rdy, d01);
-            d23 = __ffma2_rn(ay23.v, rdy, d23);
-            d01 = __ffma2_rn(make_float2(az[0].v, az[1].v), rdz, d01);
-            d23 = __ffma2_rn(make_float2(az[2].v, az[3].v), rdz, d23);
-            float4 kk;
-            if (VARDEN) {
-                const float4 d = ld_model(a.den, s, yo, zo);
-                kk = make_float4(d.x * a.dt, d.y * a.dt, d.z * a.dt, d.w * a.dt);
-            } else {
-                kk = make_float4(kc, kc, kc, kc);
-            }
-            const float2 k01 = __fmul2_rn(__fmul2_rn(lo2(kk), lo2(vpn)), lo2(vpn));
-            const float2 k23 = __fmul2_rn(__fmul2_rn(hi2(kk), hi2(vpn)), hi2(vpn));
-            const long long plane = shot_off + (long long)s * L.xstride;
-            if (ADJ) {
-                // bracket = nu / K + sum (= M a Q_old + ...), nu' = M a K bracket, g += nu D_k
-                const float4 po = Pq[q];
-                const float2 b01 = __fadd2_rn(d01, make_float2(__fdividef(po.x, k01.x), __fdividef(po.y, k01.y)));
-                const float2 b23 = __fadd2_rn(d23, make_float2(__fdividef(po.z, k23.x), __fdividef(po.w, k23.y)));
-                float4 pn = cat4(__fmul2_rn(b01, k01), __fmul2_rn(b23, k23));
-                if (edge) pn = mul4(mul4(pn, edge_f(io, xpad_s, fx_s)), edge_k(io, kx_s));
-                if (own_ok) {
-                    *at4(a.p_out + plane, own_off) = pn;
-                    const float4 dk = adk;
-                    float4 g = agk;
-                    g = make_float4(fmaf(po.x, dk.x, g.x), fmaf(po.y, dk.y, g.y), fmaf(po.z, dk.z, g.z),
-                                    fmaf(po.w, dk.w, g.w));
-                    *at4(a.adj_g + plane, own_off) = g;
-                    const ShotDev& sd = a.shots[shot];
-                    if (s == sd.sx && yo == sd.sy && sd.sz >= zo && sd.sz < zo + 4) {
-                        const float bq[4] = {b01.x, b01.y, b23.x, b23.y};
-                        for (int c = 0; c < 4; c++)
-                            if (sd.sz == zo + c) a.adj_lam[(long long)shot * a.nt_max + a.step] = bq[c];
+                const float2 k01 = __fmul2_rn(__fmul2_rn(lo2(kk), lo2(vpn)), lo2(vpn));
+                const float2 k23 = __fmul2_rn(__fmul2_rn(hi2(kk), hi2(vpn)), hi2(vpn));
+                const long long plane = shot_off + (long long)s * L.xstride;
+                if (ADJ) {
+                    // bracket = nu / K + sum (= M a Q_old + ...), nu' = M a K bracket, g += nu D_k
+                    const float4 po = Pq[q];
+                    const float2 b01 = __fadd2_rn(d01, make_float2(__fdividef(po.x, k01.x), __fdividef(po.y, k01.y)));
+                    const float2 b23 = __fadd2_rn(d23, make_float2(__fdividef(po.z, k23.x), __fdividef(po.w, k23.y)));
+                    float4 pn = cat4(__fmul2_rn(b01, k01), __fmul2_rn(b23, k23));
+                    if (edge) pn = mul4(mul4(pn, edge_f(io, xpad_s, fx_s)), edge_k(io, kx_s));
+                    if (own_ok) {
+                        *at4(a.p_out + plane, own_off) = pn;
+                        const float4 dk = adk;
+                        float4 g = agk;
+                        g = make_float4(fmaf(po.x, dk.x, g.x), fmaf(po.y, dk.y, g.y), fmaf(po.z, dk.z, g.z),
+                                        fmaf(po.w, dk.w, g.w));
+                        *at4(a.adj_g + plane, own_off) = g;
+                        const ShotDev& sd = a.shots[shot];
+                        if (s == sd.sx && yo == sd.sy && sd.sz >= zo && sd.sz < zo + 4) {
+                            const float bq[4] = {b01.x, b01.y, b23.x, b23.y};
+                            for (int c = 0; c < 4; c++)
+                                if (sd.sz == zo + c) a.adj_lam[(long long)shot * a.nt_max + a.step] = bq[c];
+                        }
+                    }
+                } else {
+                    float4 pn = cat4(__ffma2_rn(make_float2(-k01.x, -k01.y), d01, lo2(Pq[q])),
+                                     __ffma2_rn(make_float2(-k23.x, -k23.y), d23, hi2(Pq[q])));
+                    if (edge) pn = mul4(mul4(pn, edge_f(io, xpad_s, fx_s)), edge_k(io, kx_s));
+                    if (own_ok) {
+                        *at4(a.p_out + plane, own_off) = pn;
+                        if (a.div_out) *at4(a.div_out + plane, own_off) = cat4(d01, d23);  // recomputation for the adjoint
                     }
                 }
-            } else {
-                float4 pn = cat4(__ffma2_rn(make_float2(-k01.x, -k01.y), d01, lo2(Pq[q])),
-                                 __ffma2_rn(make_float2(-k23.x, -k23.y), d23, hi2(Pq[q])));
-                if (edge) pn = mul4(mul4(pn, edge_f(io, xpad_s, fx_s)), edge_k(io, kx_s));
-                if (own_ok) {
-                    *at4(a.p_out + plane, own_off) = pn;
-                    if (a.div_out) *at4(a.div_out + plane, own_off) = cat4(d01, d23);  // recomputation for the adjoint
-                }
             }
+            vpn = ld_vp(s + 1);
+            Pq[K::NQ + q] = Pn;
+            Pn = ld_own(p_in, s + K::NQ + 1);
         }
-        vpn = ld_vp(s + 1);
-        Pq[K::NQ + q] = Pn;
-        Pn = ld_own(p_in, s + K::NQ + 1);
-    }
 #pragma unroll
-    for (int j = 0; j < K::NQ; j++) Pq[j] = Pq[j + R];
-    float4* const other = cur;
-    cur = prv;
-    prv = other;
+        for (int j = 0; j < K::NQ; j++) Pq[j] = Pq[j + R];
+        float4* const other = cur;
+        cur = prv;
+        prv = other;
     }
 }
 
