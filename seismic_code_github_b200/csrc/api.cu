@@ -957,6 +957,7 @@ int run_forward(sfd_ctx* ctx, float* out_dev) {
         }
         CK(e);
         if (ctx->graph) cudaGraphExecDestroy(ctx->graph);
+        ctx->graph = nullptr;
         e = cudaGraphInstantiate(&ctx->graph, g, 0);
         cudaGraphDestroy(g);
         CK(e);
@@ -1411,6 +1412,7 @@ int run_gradient(sfd_ctx* ctx, const float* obs, float* misfit, float* grad_vp, 
             }
             CK(e);
             if (ctx->grad_graph) cudaGraphExecDestroy(ctx->grad_graph);
+            ctx->grad_graph = nullptr;
             e = cudaGraphInstantiate(&ctx->grad_graph, g, 0);
             cudaGraphDestroy(g);
             CK(e);
@@ -1490,7 +1492,7 @@ int run_gradient(sfd_ctx* ctx, const float* obs, float* misfit, float* grad_vp, 
 // and its edge rule stop at the window's last row and column.  Every distinct window (aperture
 // start and width) gets its own block of the prepared arrays; shot x0 becomes that block's start.
 // Without shots the whole grid is one window.
-int q_prepare(sfd_ctx* ctx) {
+int q_prepare_arrays(sfd_ctx* ctx) {
     const bool elastic = ctx->g.scheme == SFD_VISCOEL_2D;
     const bool iso = ctx->g.scheme == SFD_ELASTIC_2D;
     if ((ctx->g.scheme != SFD_VISCOAC_2D && !elastic && !iso) || !ctx->have_model) return SFD_OK;
@@ -1619,6 +1621,17 @@ int q_prepare(sfd_ctx* ctx) {
         CK(h2d(ctx, ctx->d_shots, ctx->h_shots.data(), sizeof(ShotDev) * ctx->nshot));
     }
     return SFD_OK;
+}
+
+// Arrays that could not be formed for want of memory leave the context without a model, not with some of them.
+int q_prepare(sfd_ctx* ctx) {
+    const int rc = q_prepare_arrays(ctx);
+    if (rc == SFD_ERR_NOMEM || rc == SFD_ERR_CUDA) {
+        ctx->have_model = ctx->graph_valid = ctx->grad_valid = false;
+        ctx->q_width = 0;
+        ctx->prep_wins.clear();
+    }
+    return rc;
 }
 
 // Gaussian source stamps of the current shots (QS:1340-1444; YPUB:1429-1466 with the context's
@@ -2283,6 +2296,8 @@ int sfd_set_model(sfd_ctx* ctx, const float* vp, const float* den, const float* 
         CK(h2d(ctx, *dst, staged.data(), mfloats * sizeof(float)));
         return SFD_OK;
     };
+    const bool had_model = ctx->have_model;
+    ctx->have_model = false;  // until the uploads are complete
     int urc = upload(&ctx->d_vp, vp);
     if (urc) return urc;
     if (ctx->varden) {
@@ -2293,6 +2308,7 @@ int sfd_set_model(sfd_ctx* ctx, const float* vp, const float* den, const float* 
         dfree(ctx->d_den);
         for (auto& p : ctx->d_b) dfree(p);
     }
+    ctx->have_model = had_model;
     if (ctx->g.scheme == SFD_ELASTIC_2D) {
         // YPUB:323-634 per shot window: staggered moduli and buoyancies, smoothed top sponge
         if (q) return set_err(ctx, SFD_ERR_ARG, "the yang_version scheme has no quality factor");

@@ -103,3 +103,99 @@ def test_a_context_survives_running_short(kind):
         assert failed > 0
         assert bits_equal(e.gradient(obs)[1], grad)
         assert bits_equal(e.forward(), rec)
+
+
+def test_a_model_that_could_not_be_uploaded_is_not_there():
+    """SFD_EXACT acoustic: a constant-density model, then one of variable density without memory for it."""
+    mb = 1 << 20
+    rng = np.random.default_rng(9)
+    nx, nz, nt = 2000, 1500, 20
+    vp = (2000.0 + 300.0 * rng.random((nx, nz))).astype(np.float32)
+    den = (1900.0 + 300.0 * rng.random((nx, nz))).astype(np.float32)
+    rx, rz = np.arange(10, nx - 10, dtype=np.int32), np.full(nx - 20, 13, np.int32)
+    shots = [S.ShotSpec(nx // 2, 15, rx, rz, S.wavelet(S.WAVELET_RIC, nt, 1e-3, 25.0, 10))]
+
+    def engine():
+        return S.Engine(S.ACOUSTIC_2D, nx, nz, 10.0, 10.0, 1e-3, 10, order=8, flags=S.EXACT)
+
+    with engine() as e:
+        e.set_model(vp, den)
+        e.set_shots(shots)
+        want = e.forward().copy()
+    with engine() as e:
+        e.set_model(vp)
+        e.set_shots(shots)
+        assert not bits_equal(e.forward(), want)
+        hog = Hog(2 * mb)  # den is 12 MB
+        try:
+            with pytest.raises(S.SfdError) as err:
+                e.set_model(vp, den)
+            assert err.value.status == S.ERR_NOMEM
+            with pytest.raises(S.SfdError) as err:
+                e.forward()
+            assert err.value.status == S.ERR_STATE
+        finally:
+            hog.release()
+        e.set_model(vp, den)
+        assert np.abs(want).max() > 0 and bits_equal(e.forward(), want)
+
+
+@pytest.mark.parametrize("kind", ["visco", "viscoel", "elastic"])
+def test_prepared_model_arrays_that_do_not_fit(kind):
+    """The per-window model arrays of the Fortran schemes are formed after the state: shots that leave no room
+    for them are refused, and the context goes on."""
+    rng = np.random.default_rng(10)
+    nx, nz, pml, nt, n = 1400, 500, 10, 12, 24
+    vp = (2000.0 + 300.0 * rng.random((nx, nz))).astype(np.float32)
+    den = (1900.0 + 300.0 * rng.random((nx, nz))).astype(np.float32)
+    scheme = {"visco": S.VISCOAC_2D, "viscoel": S.VISCOEL_2D, "elastic": S.ELASTIC_2D}[kind]
+    w = S.wavelet(S.WAVELET_Q, nt, 5e-4, 20.0)
+    rx, rz = np.arange(20, 300, dtype=np.int32), np.full(280, 14, np.int32)
+    one = [S.ShotSpec(100, 16, rx, rz, w, ap_x0=0, ap_nx=320)]
+    many = [S.ShotSpec(100, 16, rx, rz, w, ap_x0=40 * i, ap_nx=320) for i in range(n)]  # 24 windows
+
+    def model(e):
+        if kind == "visco":
+            e.set_model(vp, den)
+        else:
+            e.set_model_elastic(vp, vp / np.float32(1.8), den)
+
+    def engine():
+        e = S.Engine(scheme, nx, nz, 5.0, 5.0, 5e-4, pml, order=10, f0=20.0)
+        if kind == "elastic":
+            e.set_gauss_radius(6)
+            e.set_free_surface(pml)
+        model(e)
+        e.set_shots(one)
+        return e
+
+    with engine() as e:
+        first = e.forward().copy()
+        e.set_shots(many)
+        want = e.forward().copy()
+    slabs = {"visco": 10, "viscoel": 22, "elastic": 10}[kind]
+    slab = 4 * n * (8 + 320 + 8) * 544
+    state = slabs * slab
+    failed = 0
+    with engine() as e:
+        for extra in (4, 16, 24, 32, 44, 60, 90, 140, 200, 400):
+            hog = Hog(state + (extra << 20))
+            try:
+                e.set_shots(many)
+            except S.SfdError as err:
+                assert err.status == S.ERR_NOMEM, err
+                with pytest.raises(S.SfdError) as again:
+                    e.forward()
+                assert again.value.status == S.ERR_STATE
+                failed += 1
+            else:
+                hog.release()  # the captured loop needs a little memory of its own
+                assert bits_equal(e.forward(), want)
+                break
+            finally:
+                hog.release()
+            model(e)
+            e.set_shots(one)
+            assert bits_equal(e.forward(), first)
+        assert 0 < failed < 10
+        assert np.abs(want).max() > 0
