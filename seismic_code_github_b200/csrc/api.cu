@@ -2551,15 +2551,9 @@ int sfd_set_shots(sfd_ctx* ctx, int nshot, const sfd_shot* shots) {
     }
     if (!ctx->d_state) CK(cudaMalloc(&ctx->d_state, ctx->state_floats * sizeof(float)));
     CK(cudaMalloc(&ctx->d_src_pre, sizeof(float) * nshot));
-    if (visco) {
-        // Gaussian source stamps (QS:1340-1444, YPUB:1429-1466) and the split cosine sponge tables
-        // (QS:555-605, YPUB:796-849)
-        if ((rc = build_stamps(ctx))) return rc;
-        ctx->spg_stride = ctx->g.pml + 1;
-        std::vector<float> tab(8 * (size_t)ctx->spg_stride);
-        viscoac2d_sponge_tables(ctx->g.pml, ctx->g.pml, ctx->g.dx, ctx->g.dz, ctx->spg_stride, tab.data());
-        dfree(ctx->d_spg);
-        if ((rc = up(&ctx->d_spg, tab))) return rc;
+    // TMA descriptors of what the split schemes' kernels stage: the sums, and vx, vz, sigma
+    auto split_maps = [&]() -> int {
+        int rc;
         for (int f = 0; (iso || elastic) && ctx->sums && f < 5; f++) {
             int box[2];
             if (iso) elastic2d_box(box);
@@ -2573,6 +2567,18 @@ int sfd_set_shots(sfd_ctx* ctx, int nshot, const sfd_shot* shots) {
             float* base = ctx->d_state + (f < 2 ? f : 8) * (long long)nshot * L.shot_stride;
             if ((rc = encode_field_map(ctx, &ctx->q_maps[f], base, L, nshot, box))) return rc;
         }
+        return SFD_OK;
+    };
+    if (visco) {
+        // Gaussian source stamps (QS:1340-1444, YPUB:1429-1466) and the split cosine sponge tables
+        // (QS:555-605, YPUB:796-849)
+        if ((rc = build_stamps(ctx))) return rc;
+        ctx->spg_stride = ctx->g.pml + 1;
+        std::vector<float> tab(8 * (size_t)ctx->spg_stride);
+        viscoac2d_sponge_tables(ctx->g.pml, ctx->g.pml, ctx->g.dx, ctx->g.dz, ctx->spg_stride, tab.data());
+        dfree(ctx->d_spg);
+        if ((rc = up(&ctx->d_spg, tab))) return rc;
+        if ((rc = split_maps())) return rc;
         if (q_fast(ctx)) {
             int bs[2];
             viscoac2d_fast_box(bs);
@@ -2602,8 +2608,21 @@ int sfd_set_shots(sfd_ctx* ctx, int nshot, const sfd_shot* shots) {
     for (int s = 0; s < nshot; s++) ctx->h_ap_x0[s] = shots[s].ap_x0;
     ctx->have_shots = true;
     ctx->graph_valid = false;
-    if (visco) return q_prepare(ctx);
-    return SFD_OK;
+    if (!visco) return SFD_OK;
+    const bool had_model = ctx->have_model;
+    rc = q_prepare(ctx);
+    if (rc == SFD_ERR_NOMEM && ctx->sums && fewer < slabs) {  // the slabs of the sums make room for the model's arrays
+        dfree(ctx->d_state);
+        ctx->sums = false;
+        ctx->state_floats = fewer * fields;
+        ctx->have_shots = false;
+        CK(cudaMalloc(&ctx->d_state, ctx->state_floats * sizeof(float)));
+        if ((rc = split_maps())) return rc;
+        ctx->have_shots = true;
+        ctx->have_model = had_model;
+        rc = q_prepare(ctx);
+    }
+    return rc;
 }
 
 int sfd_forward_device(sfd_ctx* ctx, float* records_dev) {
