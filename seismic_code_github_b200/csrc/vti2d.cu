@@ -68,9 +68,10 @@ struct VtiDev {
     long long xs, zs;              // floats per x strip, per z strip
     int pitch, nx, nz, nxl, nxr, nzu, nzd, range, nt;
     float dx, dz, dt, L;
-    float cx[2], cz[2], cx1;       // default mode: dt^2 / dx^2 and dt^2 / dz^2 as sums of two, dt^2 / dx
+    float cx[2], cz[2];            // default mode: dt^2 / dx^2 and dt^2 / dz^2 as sums of two
     float cd[4], cdd[4];           // ... damping d = speed cd idx^2 and its derivative speed cdd idx (l, r, u, d)
     float cE[5], c1[5];    // coefficient_2nd(10) (fd_coe and fd_coe_pml_2nd alike), coefficient_1st
+    float cx1;             // default mode: dt^2 / dx (after the coefficients, which it would shift off 8 bytes: 1%)
     const int* src;        // per shot: source cell i, j (1-based)
     const int* rrow;       // per shot: receiver row (1-based) and whether it is the row-6 fallback
     float* records;        // [shot][range][nt]
@@ -101,7 +102,7 @@ __device__ __forceinline__ float d2(const float* f, int st, const float* cf, flo
 }
 // default mode: s dt^2 / h^2 with the factor as the sum of two.  A grid constant that is rounded once has the
 // same error at every cell and step, which shifts the wave's speed; this one is exact to 48 bits.
-__device__ __forceinline__ float scaled(float s, const float* c) { return fmaf(s, c[0], s * c[1]); }
+template <bool E> __device__ __forceinline__ float scaled(float s, const float* c) { return E ? s : fmaf(s, c[0], s * c[1]); }
 // first-derivative sum of VS:567-578: (p1 (f+1 - f-1) + ... + p5 (...)) / h (default mode: times rh)
 template <bool E>
 __device__ __forceinline__ float d1(const float* f, int st, const float* cf, float h, float rh) {
@@ -220,12 +221,9 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) vti_step_kernel(const __
     // The sums of the current u and q that both subroutines form: coefficient_2nd(10) is both
     // fd_coe and fd_coe_pml_2nd, the x sums of u and q appear in step 1 and step 2 (added in the
     // other order there, which IEEE addition does not distinguish), the z sum of u in every
-    // region of step 1.  Each is formed once.
-    float s2 = fa<E>(d2<E>(U, 1, a.cE, dx), d2<E>(Q, 1, a.cE, dx)), szu = d2<E>(U, kSX, a.cE, dz);
-    if (!E) {  // times dt^2
-        s2 = scaled(s2, a.cx);
-        szu = scaled(szu, a.cz);
-    }
+    // region of step 1.  Each is formed once (in the default mode times dt^2).
+    const float s2 = scaled<E>(fa<E>(d2<E>(U, 1, a.cE, dx), d2<E>(Q, 1, a.cE, dx)), a.cx);
+    const float szu = scaled<E>(d2<E>(U, kSX, a.cE, dz), a.cz);
     const bool xin = gi >= nxl && gi < nx - nxr;
     float un, qn;
     if (xin) {  // extrapolation_one_step_1 (VS:432-960) and _2 (VS:965-1072) inside
